@@ -64,7 +64,7 @@ constexpr int kMaskAxisZ = (1 << 2) | (1 << 3) | (1 << 4);  // J = (0, 0, s, s r
 
 // solve6, avbd/src/lib.rs:107-180 (unpivoted LDL^T); solves H x = -g.  Each
 // quotient by a pivot is the IEEE quotient (div_rn.cuh: one reciprocal per
-// pivot, a correction step per quotient).
+// pivot, a correction step per quotient, one range test per pivot's column).
 template <class R>
 __device__ __forceinline__ void solve6(const Block6<R>& B, R x[6]) {
     const R* H = B.h;
@@ -75,27 +75,31 @@ __device__ __forceinline__ void solve6(const Block6<R>& B, R x[6]) {
     R a43 = H[tri(3, 2)], a53 = H[tri(4, 2)], a63 = H[tri(5, 2)];
     R a44 = H[tri(3, 3)], a54 = H[tri(4, 3)], a64 = H[tri(5, 3)], a55 = H[tri(4, 4)], a65 = H[tri(5, 4)],
       a66 = H[tri(5, 5)];
-    const Divisor<R> p1(a11);
-    R l21 = p1.div(a21), l31 = p1.div(a31), l41 = p1.div(a41), l51 = p1.div(a51), l61 = p1.div(a61);
+    const Pivot<R> p1(a11);
+    R q1[5] = {a21, a31, a41, a51, a61};
+    divide_all(p1, q1);
+    const R l21 = q1[0], l31 = q1[1], l41 = q1[2], l51 = q1[3], l61 = q1[4];
     R d1 = a11;
     R d2 = a22 - l21 * l21 * d1;
-    const Divisor<R> p2(d2);
-    R l32 = p2.div(a32 - l21 * l31 * d1);
-    R l42 = p2.div(a42 - l21 * l41 * d1);
-    R l52 = p2.div(a52 - l21 * l51 * d1);
-    R l62 = p2.div(a62 - l21 * l61 * d1);
+    const Pivot<R> p2(d2);
+    R q2[4] = {a32 - l21 * l31 * d1, a42 - l21 * l41 * d1, a52 - l21 * l51 * d1, a62 - l21 * l61 * d1};
+    divide_all(p2, q2);
+    const R l32 = q2[0], l42 = q2[1], l52 = q2[2], l62 = q2[3];
     R d3 = a33 - (l31 * l31 * d1 + l32 * l32 * d2);
-    const Divisor<R> p3(d3);
-    R l43 = p3.div(a43 - l31 * l41 * d1 - l32 * l42 * d2);
-    R l53 = p3.div(a53 - l31 * l51 * d1 - l32 * l52 * d2);
-    R l63 = p3.div(a63 - l31 * l61 * d1 - l32 * l62 * d2);
+    const Pivot<R> p3(d3);
+    R q3[3] = {a43 - l31 * l41 * d1 - l32 * l42 * d2, a53 - l31 * l51 * d1 - l32 * l52 * d2,
+               a63 - l31 * l61 * d1 - l32 * l62 * d2};
+    divide_all(p3, q3);
+    const R l43 = q3[0], l53 = q3[1], l63 = q3[2];
     R d4 = a44 - (l41 * l41 * d1 + l42 * l42 * d2 + l43 * l43 * d3);
-    const Divisor<R> p4(d4);
-    R l54 = p4.div(a54 - l41 * l51 * d1 - l42 * l52 * d2 - l43 * l53 * d3);
-    R l64 = p4.div(a64 - l41 * l61 * d1 - l42 * l62 * d2 - l43 * l63 * d3);
+    const Pivot<R> p4(d4);
+    R q4[2] = {a54 - l41 * l51 * d1 - l42 * l52 * d2 - l43 * l53 * d3,
+               a64 - l41 * l61 * d1 - l42 * l62 * d2 - l43 * l63 * d3};
+    divide_all(p4, q4);
+    const R l54 = q4[0], l64 = q4[1];
     R d5 = a55 - (l51 * l51 * d1 + l52 * l52 * d2 + l53 * l53 * d3 + l54 * l54 * d4);
     const Divisor<R> p5(d5);
-    R l65 = p5.div(a65 - l51 * l61 * d1 - l52 * l62 * d2 - l53 * l63 * d3 - l54 * l64 * d4);
+    const R l65 = p5.div(a65 - l51 * l61 * d1 - l52 * l62 * d2 - l53 * l63 * d3 - l54 * l64 * d4);
     R d6 = a66 - (l61 * l61 * d1 + l62 * l62 * d2 + l63 * l63 * d3 + l64 * l64 * d4 + l65 * l65 * d5);
     R b0 = -B.g[0], b1 = -B.g[1], b2 = -B.g[2], b3 = -B.g[3], b4 = -B.g[4], b5 = -B.g[5];
     R y1 = b0;
@@ -104,7 +108,16 @@ __device__ __forceinline__ void solve6(const Block6<R>& B, R x[6]) {
     R y4 = b3 - l41 * y1 - l42 * y2 - l43 * y3;
     R y5 = b4 - l51 * y1 - l52 * y2 - l53 * y3 - l54 * y4;
     R y6 = b5 - l61 * y1 - l62 * y2 - l63 * y3 - l64 * y4 - l65 * y5;
-    R z1 = p1.div(y1), z2 = p2.div(y2), z3 = p3.div(y3), z4 = p4.div(y4), z5 = p5.div(y5), z6 = y6 / d6;
+    Quotients<R> qz;
+    R z1 = qz.div(p1, y1), z2 = qz.div(p2, y2), z3 = qz.div(p3, y3), z4 = qz.div(p4, y4), z5 = qz.div(p5.p, y5);
+    if (!(qz.in_range() && p1.ok() && p2.ok() && p3.ok() && p4.ok() && p5.p.ok())) {
+        z1 = y1 / d1;
+        z2 = y2 / d2;
+        z3 = y3 / d3;
+        z4 = y4 / d4;
+        z5 = y5 / d5;
+    }
+    R z6 = y6 / d6;
     x[5] = z6;
     x[4] = z5 - l65 * x[5];
     x[3] = z4 - l54 * x[4] - l64 * x[5];
@@ -375,8 +388,9 @@ __device__ __forceinline__ void primal_joint(const DevWorld<P, R>& w, const DioC
         R target = R(jt.anchor_a[3]);
         bool active = len > R(1.0e-6) && (jt.kind != DIO_CONSTRAINT_ROPE || len > target);
         if (active) {
-            const Divisor<R> dl(len);  // the IEEE quotients (div_rn.cuh)
-            const V3<R> nn{dl.div(delta.x), dl.div(delta.y), dl.div(delta.z)};
+            R dn[3] = {delta.x, delta.y, delta.z};
+            divide_all(Pivot<R>(len), dn);  // the IEEE quotients (div_rn.cuh)
+            const V3<R> nn{dn[0], dn[1], dn[2]};
             V3<R> jl = scale(nn, sign);
             V3<R> ja = cross(r_self, jl);
             stamp(B, jl, ja, stiff, stiff * (len - target));
@@ -427,8 +441,9 @@ __device__ __forceinline__ void primal_jview_p(const JView& jv, A4<P> op4, A4<P>
         R target = R(jv.self_anchor.w);
         bool active = len > R(1.0e-6) && (kind != DIO_CONSTRAINT_ROPE || len > target);
         if (active) {
-            const Divisor<R> dl(len);  // the IEEE quotients (div_rn.cuh)
-            const V3<R> nn{dl.div(delta.x), dl.div(delta.y), dl.div(delta.z)};
+            R dn[3] = {delta.x, delta.y, delta.z};
+            divide_all(Pivot<R>(len), dn);  // the IEEE quotients (div_rn.cuh)
+            const V3<R> nn{dn[0], dn[1], dn[2]};
             V3<R> jl = scale(nn, sign);
             V3<R> ja = cross(r_self, jl);
             stamp(B, jl, ja, stiff, stiff * (len - target));
