@@ -35,7 +35,7 @@ DioConfig default_config() {
     c.precision = DIO_PREC_F32;
     c.contacts_per_pair = DIO_CONTACTS_PER_PAIR;
     c.use_graph = 1;
-    c.primal_variant = 5;  // {64 threads, 10 CTAs/SM}: 96 registers, no spills
+    c.primal_variant = 5;  // bodies grouped per warp by the size of the world
     c.block_size = 0;
     c.batched_solver = 0;
     return c;

@@ -586,10 +586,10 @@ class Engine final : public EngineBase {
         DIO_CK(cudaFuncSetAttribute(k_scene_tree<R, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, tree_bytes));
         DIO_CK(cudaFuncSetAttribute(k_chunk_build<R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)chunk_build_bytes<R>()));
-        DIO_CK(cudaFuncSetAttribute(k_primal_warp<P, R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)primal_warp_smem<R>()));
-        DIO_CK(cudaFuncSetAttribute(k_primal_color_warp<P, R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)primal_warp_smem<R>()));
+        DIO_CK(cudaFuncSetAttribute(k_primal_group<P, R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)primal_group_smem<R>()));
+        DIO_CK(cudaFuncSetAttribute(k_primal_color<P, R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)primal_group_smem<R>()));
         DIO_CK(cudaFuncSetAttribute(k_solve_chunks<P, R, kChunkThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)chunk_smem_bytes<P>(solve_chunk_cap<P>())));
         DIO_CK(cudaFuncSetAttribute(k_solve_chunks<P, R, kChunkThreadsWide>,
@@ -1664,7 +1664,7 @@ class Engine final : public EngineBase {
         for (uint32_t k = 0; k < o.iterations; ++k) {
             int par = (int)(k % 2);
             cudaEvent_t e0 = span_begin();
-            launch_primal<P, R>((int)cfg_.primal_variant, pdl, w_, par, 1 - par, o, stream_);
+            launch_primal<P, R>((int)cfg_.primal_variant, pdl, w_, par, 1 - par, o, sms_, stream_);
             span_end(e0, 0);
             ++launches_;
             if (m) {
@@ -2071,11 +2071,9 @@ class Engine final : public EngineBase {
                     uint32_t c0 = color_off_h_[c], c1 = color_off_h_[c + 1];
                     if (c1 <= c0) continue;
                     cudaEvent_t e0 = span_begin();
-                    if (cfg_.primal_variant == 10)  // warp per body
-                        k_primal_color_warp<P, R><<<grid_for(c1 - c0, kPrimalWarpWarps), kPrimalWarpWarps * 32,
-                                                    primal_warp_smem<R>(), stream_>>>(w_, c0, c1, so);
-                    else
-                        k_primal_color<P, R><<<grid_for(c1 - c0, 128), 128, 0, stream_>>>(w_, c0, c1, so);
+                    const uint32_t g = cfg_.primal_variant == 10 ? 1u : primal_group_size(c1 - c0, sms_);
+                    k_primal_color<P, R><<<grid_for(c1 - c0, kPrimalGroupWarps * (int)g), kPrimalGroupWarps * 32,
+                                           primal_group_smem<R>(), stream_>>>(w_, c0, c1, g, so);
                     span_end(e0, 0);
                     ++launches_;
                 }

@@ -574,111 +574,201 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_primal(DevWorld<P, R> w, int rd
         primal_body(w, w.dyn_list[t], rd, o);
 }
 
-// Warp per dynamic body, for worlds whose bodies carry many contact rows
-// (a thread per body walks its rows one dependent gather after another):
-// lane l forms the three stamps of the body's incidence j0 + 32 q + l and
-// writes their 27 products each (21 Hessian terms, 6 gradient terms, the
-// products exactly as stamp() forms them) to shared memory; lane e < 27 then
-// adds entry e of the 6x6 system over the incidences and stamps in the
-// serial order -- the same sums, term for term, as primal_body_f.  Lane 0
-// adds the joint rows and solves.
-constexpr int kPrimalWarpWarps = 4;
+// A group of up to 32 bodies by one warp, for bodies with contact rows.  A
+// thread per body walks its rows one dependent gather and one chain of sums
+// after another (about 900 cycles a row), so the warp lasts as long as its
+// body with the most rows, and a world of a few thousand bodies leaves most
+// of the GPU idle.  Here lane b holds body b, and the group's incidences --
+// the bodies' row lists one after another -- are taken 32 at a time, a lane
+// each whatever its body: the lane forms the incidence's three stamps
+// (Jacobian row, stiffness, force) and stages them in shared memory; then
+// lane e < 27 adds entry e of each body's 6x6 system (21 Hessian terms, 6
+// gradient terms, each product formed as stamp() forms it) over the body's
+// incidences and stamps in the serial order.  The sums see the same terms in
+// the same order as primal_body_f, so the bits are the same; joints, the
+// 6x6 solve and the pose update follow with a lane per body again.
+// The staged sums cost about three times the instructions of a row in a warp
+// whose bodies have equally many rows, so they are taken when the longest
+// list exceeds kGroupSerial times the rounds of 32 (else: a thread per body).
+// Measured (us per primal launch, cold caches): 31.8 -> 15.1 on the
+// 8,192-cube field (8 incidences a body, groups of 4), 22.8 -> 18.1 on the
+// 50,000-body pile (under one incidence a body, clustered), 18.6 -> 15.3 on
+// 715 stacks of 7 cubes.  Serial threshold 1, 2 or 3: equal within 1 %, but 1
+// takes the split-precision brick wall (7 incidences a body, evenly spread)
+// 3.90 -> 4.47 ms a step.  Four CTAs an SM (128 registers) against five (96,
+// spills): the field's two steps 922 against 976 us, the pile's 1672 against
+// 1657.  Half the bodies a warp (24 warps an SM): every case slower.
+constexpr uint32_t kGroupSerial = 2;
+constexpr int kGroupStage = 25;  // 3 stamps of (J[6], k, f) padded to an odd stride
+constexpr int kGroupSums = 27;
 template <class R>
-__host__ __device__ constexpr size_t primal_warp_smem() {
-    return (size_t)kPrimalWarpWarps * 32 * 3 * 28 * sizeof(R);
+__host__ __device__ constexpr size_t primal_group_words() {
+    return (size_t)32 * (kGroupStage + kGroupSums);
 }
-// One body's primal by the calling warp (all 32 lanes, the same i);
-// prod: the warp's [32][3][28] product staging in shared memory.
+constexpr int kPrimalGroupWarps = 4;
+template <class R>
+__host__ __device__ constexpr size_t primal_group_smem() {
+    return (size_t)kPrimalGroupWarps * primal_group_words<R>() * sizeof(R);
+}
+
+// Bodies list[0 .. nb) (dynamic ones, nb <= 32), all lanes of the warp;
+// stage: the warp's primal_group_words<R>() words of shared memory.
 template <class P, class R, class F>
-__device__ __forceinline__ void primal_warp_body(const DevWorld<P, R>& w, uint32_t i, const SolveParams<R>& o,
-                                                 const F& fetch, R* prod, uint32_t lane) {
-    const A4<R> inv = w.inv[i];
-    if (inv.w == R(0)) return;  // warp-uniform
-    const V3<P> sp = xyz(fetch.pos(i));
-    const Q4<P> sq = quat(fetch.rot(i));
-    const Q4<R> sqr = castq<R>(sq);
+__device__ __forceinline__ void primal_group(const DevWorld<P, R>& w, const uint32_t* list, uint32_t nb,
+                                             const SolveParams<R>& o, const F& fetch, R* stage, uint32_t lane) {
+    constexpr uint32_t kAll = 0xFFFFFFFFu;
+    R* const sums = stage + 32 * kGroupStage;  // [body][27]
+    const bool live = lane < nb;
+    uint32_t i = 0, j0 = 0, n = 0;
+    V3<P> sp{P(0), P(0), P(0)};
+    Q4<P> sq{P(0), P(0), P(0), P(1)};
     Block6<R> B;
-    primal_inertia(w, i, inv, sp, sqr, o, B);
-    // lane e holds entry e: h[0..20], then g[0..5]
-    R acc = R(0);
+    if (live) {
+        i = list[lane];
+        j0 = w.row_off[i];
+        n = w.row_off[i + 1] - j0;
+        sp = xyz(fetch.pos(i));
+        sq = quat(fetch.rot(i));
+    }
+    const Q4<R> sqr = castq<R>(sq);
+    if (live) primal_inertia(w, i, A4<R>{}, sp, sqr, o, B);
+    uint32_t incl = n;  // inclusive sums of the row counts
 #pragma unroll
-    for (int e = 0; e < 21; ++e)
-        if (lane == (uint32_t)e) acc = B.h[e];
-#pragma unroll
-    for (int e = 0; e < 6; ++e)
-        if (lane == (uint32_t)(21 + e)) acc = B.g[e];
-    const uint32_t j0 = w.row_off[i], j1 = w.row_off[i + 1];
-    if (j0 < j1) {
-        const V3<R> dqsl = cast3<R>(sub(sp, xyz(fetch.ipos(i))));
-        const V3<R> dqsa = ang_diff(sqr, castq<R>(quat(fetch.irot(i))));
+    for (int off = 1; off < 32; off <<= 1) {
+        const uint32_t t = __shfl_up_sync(kAll, incl, off);
+        if (lane >= (uint32_t)off) incl += t;
+    }
+    const uint32_t total = __shfl_sync(kAll, incl, 31);
+    if (total) {
         const R k_alpha = R(1) - o.alpha;
-        for (uint32_t base = j0; base < j1; base += 32u) {
-            const uint32_t cnt = min(32u, j1 - base);
-            if (lane < cnt) {
-                const uint32_t j = base + lane;
-                const uint32_t r = w.row_idx[j];
-                V3<R> jl[3], ja[3];
-                R k[3], f[3];
-                primal_row_terms<P, R>(w.rs[r], w.rd[r], w.row_oth[j], fetch, sqr, dqsl, dqsa, k_alpha, jl, ja, k,
-                                       f);
-                R* mine = prod + lane * (3 * 28);
+        V3<R> dqsl{R(0), R(0), R(0)}, dqsa{R(0), R(0), R(0)};
+        if (n) {
+            dqsl = cast3<R>(sub(sp, xyz(fetch.ipos(i))));
+            dqsa = ang_diff(sqr, castq<R>(quat(fetch.irot(i))));
+        }
+        if (__reduce_max_sync(kAll, n) <= kGroupSerial * ((total + 31u) / 32u)) {
+            for (uint32_t j = j0; j < j0 + n; ++j)
+                primal_row_f(w, w.row_idx[j], w.row_oth[j], fetch, sqr, dqsl, dqsa, k_alpha, B);
+        } else {
+            if (n) {
 #pragma unroll
-                for (int s = 0; s < 3; ++s) {
-                    const R J[6] = {jl[s].x, jl[s].y, jl[s].z, ja[s].x, ja[s].y, ja[s].z};
+                for (int e = 0; e < 21; ++e) sums[lane * kGroupSums + e] = B.h[e];
 #pragma unroll
-                    for (int a = 0; a < 6; ++a)
-#pragma unroll
-                        for (int b = 0; b <= a; ++b) mine[s * 28 + tri(a, b)] = J[a] * J[b] * k[s];
-#pragma unroll
-                    for (int a = 0; a < 6; ++a) mine[s * 28 + 21 + a] = J[a] * f[s];
-                }
+                for (int e = 0; e < 6; ++e) sums[lane * kGroupSums + 21 + e] = B.g[e];
             }
-            __syncwarp();
-            if (lane < 27u)
-                for (uint32_t q = 0; q < cnt; ++q) {
-                    const R* pq = prod + q * (3 * 28) + lane;
-                    acc = acc + pq[0];
-                    acc = acc + pq[28];
-                    acc = acc + pq[56];
+            // lane e's entry: H[ra][rb] (product J[ra] J[rb] k) or g[ra] (J[ra] f)
+            const bool is_h = lane < 21u;
+            uint32_t ra = 0, rb = 7;
+            if (is_h) {
+                while ((ra + 1) * (ra + 2) / 2 <= lane) ++ra;
+                rb = lane - ra * (ra + 1) / 2;
+            } else if (lane < (uint32_t)kGroupSums) {
+                ra = lane - 21u;
+            }
+            for (uint32_t base = 0; base < total; base += 32u) {
+                const uint32_t cnt = min(32u, total - base), f = base + lane;
+                uint32_t s = 0;  // the incidence's body: the first with incl > f
+#pragma unroll
+                for (uint32_t step = 16; step; step >>= 1)
+                    if (__shfl_sync(kAll, incl, s + step - 1) <= f) s += step;
+                const uint32_t j = __shfl_sync(kAll, j0, s) + f - __shfl_sync(kAll, incl - n, s);
+                auto from = [&](R v) { return __shfl_sync(kAll, v, s); };
+                const Q4<R> q{from(sqr.x), from(sqr.y), from(sqr.z), from(sqr.w)};
+                const V3<R> dl{from(dqsl.x), from(dqsl.y), from(dqsl.z)};
+                const V3<R> da{from(dqsa.x), from(dqsa.y), from(dqsa.z)};
+                if (lane < cnt) {
+                    const uint32_t r = w.row_idx[j];
+                    V3<R> jl[3], ja[3];
+                    R k[3], ff[3];
+                    primal_row_terms<P, R>(w.rs[r], w.rd[r], w.row_oth[j], fetch, q, dl, da, k_alpha, jl, ja, k, ff);
+                    R* mine = stage + lane * kGroupStage;
+#pragma unroll
+                    for (int t = 0; t < 3; ++t) {
+                        mine[t * 8 + 0] = jl[t].x;
+                        mine[t * 8 + 1] = jl[t].y;
+                        mine[t * 8 + 2] = jl[t].z;
+                        mine[t * 8 + 3] = ja[t].x;
+                        mine[t * 8 + 4] = ja[t].y;
+                        mine[t * 8 + 5] = ja[t].z;
+                        mine[t * 8 + 6] = k[t];
+                        mine[t * 8 + 7] = ff[t];
+                    }
                 }
-            __syncwarp();
+                __syncwarp();
+                const uint32_t b1 = __shfl_sync(kAll, s, cnt - 1u);
+                for (uint32_t b = __shfl_sync(kAll, s, 0); b <= b1; ++b) {
+                    const uint32_t end = __shfl_sync(kAll, incl, b), cb = __shfl_sync(kAll, n, b);
+                    const uint32_t q0 = max(end - cb, base) - base, q1 = min(end - base, cnt);
+                    if (cb && lane < (uint32_t)kGroupSums) {
+                        R acc = sums[b * kGroupSums + lane];
+                        for (uint32_t t = q0; t < q1; ++t) {
+                            const R* p = stage + t * kGroupStage;
+#pragma unroll
+                            for (int u = 0; u < 3; ++u) {
+                                const R v = p[u * 8 + ra] * p[u * 8 + rb];
+                                const R vk = v * p[u * 8 + 6];
+                                acc = acc + (is_h ? vk : v);
+                            }
+                        }
+                        sums[b * kGroupSums + lane] = acc;
+                    }
+                }
+                __syncwarp();
+            }
+            if (n) {
+#pragma unroll
+                for (int e = 0; e < 21; ++e) B.h[e] = sums[lane * kGroupSums + e];
+#pragma unroll
+                for (int e = 0; e < 6; ++e) B.g[e] = sums[lane * kGroupSums + 21 + e];
+            }
+            __syncwarp();  // the next group's sums
         }
     }
-#pragma unroll
-    for (int e = 0; e < 21; ++e) B.h[e] = __shfl_sync(0xFFFFFFFFu, acc, e);
-#pragma unroll
-    for (int e = 0; e < 6; ++e) B.g[e] = __shfl_sync(0xFFFFFFFFu, acc, 21 + e);
-    if (lane == 0u) {
+    if (live) {
         const uint32_t k0 = w.n_joints ? w.joint_off[i] : 0u, k1 = w.n_joints ? w.joint_off[i + 1] : 0u;
         primal_finish(w, i, k0, k1, fetch, sp, sq, sqr, B);
     }
 }
 
-template <class P, class R>
-__global__ void __launch_bounds__(kPrimalWarpWarps * 32) k_primal_warp(DevWorld<P, R> w, int rd, int wr,
-                                                                        SolveParams<R> o) {
-    pdl_enter();
-    extern __shared__ __align__(16) unsigned char primal_warp_smem_raw[];
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    R* prod = reinterpret_cast<R*>(primal_warp_smem_raw) + (size_t)warp * 32 * 3 * 28;  // [32][3][28]
-    const GlobalFetch<P, R> fetch{w, rd};
-    const uint32_t nwarps = gridDim.x * kPrimalWarpWarps;
-    for (uint32_t t = blockIdx.x * kPrimalWarpWarps + warp; t < w.n_dyn; t += nwarps)
-        primal_warp_body(w, w.dyn_list[t], o, fetch, prod, lane);
+// Bodies per warp: all 32 lanes once that gives every SM 12 warps, fewer
+// (down to one) in smaller worlds, which would leave SMs idle.
+inline uint32_t primal_group_size(uint32_t n_dyn, int sms) {
+    uint32_t g = 32;
+    while (g > 1 && n_dyn / g < (uint32_t)sms * 12u) g /= 2;
+    return g;
 }
 
-// variants: 0-5 k_primal over the dynamic-body list with {threads per CTA,
-// min CTAs per SM}; 6-9 k_primal_tile over body tiles; 10 k_primal_warp
+template <class P, class R, class F>
+__device__ __forceinline__ void primal_groups(const DevWorld<P, R>& w, const uint32_t* list, uint32_t n, uint32_t g,
+                                              const SolveParams<R>& o, const F& fetch) {
+    extern __shared__ __align__(16) unsigned char primal_group_smem_raw[];
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    R* stage = reinterpret_cast<R*>(primal_group_smem_raw) + warp * primal_group_words<R>();
+    for (uint32_t t = (blockIdx.x * kPrimalGroupWarps + warp) * g; t < n; t += gridDim.x * kPrimalGroupWarps * g)
+        primal_group(w, list + t, min(g, n - t), o, fetch, stage, lane);
+}
+template <class P, class R>
+__global__ void __launch_bounds__(kPrimalGroupWarps * 32, sizeof(R) == 4 ? 4 : 2)
+    k_primal_group(DevWorld<P, R> w, int rd, uint32_t g, SolveParams<R> o) {
+    pdl_enter();
+    primal_groups(w, w.dyn_list, w.n_dyn, g, o, GlobalFetch<P, R>{w, rd});
+}
+
+// variants: 0-4 k_primal over the dynamic-body list with {threads per CTA,
+// min CTAs per SM}; 5 (the default) k_primal_group, or k_primal in worlds of
+// jointed bodies; 6-9 k_primal_tile over body tiles; 10 k_primal_group with a
+// warp per body
 constexpr int kPrimalVariants = DIO_PRIMAL_VARIANTS;
-constexpr int kPrimalShape[kPrimalVariants][2] = {{128, 4}, {128, 5}, {128, 6}, {256, 2}, {256, 3},
-                                                  {64, 10}, {128, 5}, {128, 6}, {256, 3}, {64, 10},
-                                                  {kPrimalWarpWarps * 32, 1}};
 
 template <class P, class R>
 inline void launch_primal(int variant, bool pdl, const DevWorld<P, R>& w, int rd, int wr, const SolveParams<R>& o,
-                          cudaStream_t s) {
+                          int sms, cudaStream_t s) {
     const uint32_t nd = w.n_dyn > 0 ? w.n_dyn : 1;
     auto grid = [&](int block) { return grid_for(nd, block); };
+    auto group = [&](uint32_t g) {
+        launch_k(pdl, k_primal_group<P, R>, grid_for(nd, kPrimalGroupWarps * (int)g), kPrimalGroupWarps * 32,
+                 primal_group_smem<R>(), s, w, rd, g, o);
+    };
     switch (variant) {
         case 0:
             launch_k(pdl, k_primal<P, R, 128, 4>, grid(128), 128, 0, s, w, rd, wr, o);
@@ -693,7 +783,13 @@ inline void launch_primal(int variant, bool pdl, const DevWorld<P, R>& w, int rd
             launch_k(pdl, k_primal<P, R, 256, 3>, grid(256), 256, 0, s, w, rd, wr, o);
             break;
         case 5:
-            launch_k(pdl, k_primal<P, R, 64, 10>, grid(64), 64, 0, s, w, rd, wr, o);
+            // jointed bodies carry few rows and their joints are spread
+            // evenly by the list's order: a thread per body with 20 warps an
+            // SM (the 257-scene split batch: 2.21 ms against 2.27 in groups)
+            if ((uint64_t)w.n_joints * 2 > nd)
+                launch_k(pdl, k_primal<P, R, 64, 10>, grid(64), 64, 0, s, w, rd, wr, o);
+            else
+                group(primal_group_size(nd, sms));
             break;
         case 6:
             launch_k(pdl, k_primal_tile<P, R, 128, 5>, grid_for(w.n, 128), 128, 0, s, w, rd, wr, o);
@@ -708,8 +804,7 @@ inline void launch_primal(int variant, bool pdl, const DevWorld<P, R>& w, int rd
             launch_k(pdl, k_primal_tile<P, R, 64, 10>, grid_for(w.n, 64), 64, 0, s, w, rd, wr, o);
             break;
         case 10:
-            launch_k(pdl, k_primal_warp<P, R>, grid_for(nd, kPrimalWarpWarps), kPrimalWarpWarps * 32,
-                     primal_warp_smem<R>(), s, w, rd, wr, o);
+            group(1);
             break;
         default:
             launch_k(pdl, k_primal<P, R, 128, 5>, grid(128), 128, 0, s, w, rd, wr, o);
@@ -733,24 +828,9 @@ struct InPlaceFetch {
 
 // Coloured Gauss-Seidel sweep: bodies color_order[c0 .. c1) in place.
 template <class P, class R>
-__global__ void __launch_bounds__(128) k_primal_color(DevWorld<P, R> w, uint32_t c0, uint32_t c1, SolveParams<R> o) {
-    for (uint32_t t = c0 + blockIdx.x * blockDim.x + threadIdx.x; t < c1; t += gridDim.x * blockDim.x) {
-        const uint32_t i = w.color_order[t];
-        const uint32_t k0 = w.n_joints ? w.joint_off[i] : 0u, k1 = w.n_joints ? w.joint_off[i + 1] : 0u;
-        primal_body_f(w, i, k0, k1, o, InPlaceFetch<P, R>{w});
-    }
-}
-
-// The same sweep with a warp per body (primal variant 10)
-template <class P, class R>
-__global__ void __launch_bounds__(kPrimalWarpWarps * 32)
-    k_primal_color_warp(DevWorld<P, R> w, uint32_t c0, uint32_t c1, SolveParams<R> o) {
-    extern __shared__ __align__(16) unsigned char primal_warp_smem_raw[];
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    R* prod = reinterpret_cast<R*>(primal_warp_smem_raw) + (size_t)warp * 32 * 3 * 28;
-    const InPlaceFetch<P, R> fetch{w};
-    for (uint32_t t = c0 + blockIdx.x * kPrimalWarpWarps + warp; t < c1; t += gridDim.x * kPrimalWarpWarps)
-        primal_warp_body(w, w.color_order[t], o, fetch, prod, lane);
+__global__ void __launch_bounds__(kPrimalGroupWarps * 32, sizeof(R) == 4 ? 4 : 2)
+    k_primal_color(DevWorld<P, R> w, uint32_t c0, uint32_t c1, uint32_t g, SolveParams<R> o) {
+    primal_groups(w, w.color_order + c0, c1 - c0, g, o, InPlaceFetch<P, R>{w});
 }
 
 // avbd_dual, avbd/src/lib.rs:565-663: the row's dual update from its bodies' new poses (a, and b unless the

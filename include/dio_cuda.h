@@ -230,8 +230,9 @@ typedef struct DioConfig {
     uint32_t contacts_per_pair; /* 4 (reference) or 8 (extended manifold) */
     uint32_t use_graph;         /* replay each step as a CUDA graph       */
     uint32_t primal_variant;    /* primal kernel variant, 0 .. DIO_PRIMAL_VARIANTS-1
-                                   (launch shape, body tiles; every variant
-                                   computes the same bits; autotuned)     */
+                                   (launch shape, body tiles, bodies per warp;
+                                   every variant computes the same bits;
+                                   autotuned)                             */
     uint32_t block_size;        /* threads per CTA of the scene-chunk
                                    solve: 0 (512) or 640 (autotuned)      */
     uint32_t batched_solver;    /* DioSolveLaunch: DIO_SOLVE_AUTO (0) runs
