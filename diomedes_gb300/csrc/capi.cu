@@ -171,7 +171,7 @@ int dio_ctx_configure(DioCtx* ctx, const DioConfig* config) {
     if (config->contacts_per_pair != 4 && config->contacts_per_pair != 8)
         return fail(ctx, DIO_ERR_INVALID, "contacts_per_pair must be 4 or 8");
     if (config->block_size != 0 && config->block_size != 640)
-        return fail(ctx, DIO_ERR_INVALID, "block_size must be 0 (512 threads) or 640");
+        return fail(ctx, DIO_ERR_INVALID, "block_size must be 0 or 640");
     if (config->batched_solver > DIO_SOLVE_PER_PHASE) return fail(ctx, DIO_ERR_INVALID, "unknown solve launch");
     bool realloc = config->contacts_per_pair > ctx->cfg.contacts_per_pair;
     ctx->cfg = *config;
@@ -475,7 +475,7 @@ int dio_autotune(DioCtx* ctx, const DioAvbdOptions* options, uint32_t trial_step
             best_cfg = c;
         }
     }
-    // 2) the scene-chunk solve's CTA size when it won, else the primal
+    // 2) the scene-chunk solve's CTA shape when it won, else the primal
     // launch shape
     if (best_cfg.batched_solver == DIO_SOLVE_AUTO) {
         DioConfig c = best_cfg;

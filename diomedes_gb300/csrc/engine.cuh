@@ -11,7 +11,8 @@
 //            scene                scene index of the body
 //   pairs    DioPair list sorted by (a, b), count in counters
 //   slots    narrow-phase output, `per_pair` slots per pair
-//   rows     RowStatic (80 B at FP32) + RowDual (penalty, lambda) + (a, b)
+//   rows     RowStatic (5 arrays of 4-vectors) + RowDual (penalty, lambda)
+//            + (a, b)
 //   CSR      row_off[n+1], row_idx[2m] (row), row_oth[2m] (other body | B flag)
 //   joints   DioConstraint records + per-body joint CSR
 // Pose arrays use P (float or double), everything else R.
@@ -74,6 +75,36 @@ struct RowDual {
     A4<R> penalty;  // xyz
     A4<P> lambda;   // xyz
 };
+// A buffer of rows, one array per 4-vector: a warp's loads of one field of
+// consecutive rows are one 512-byte run (records of 80 bytes made each such
+// load touch 20 to 32 cache lines, and the dual was bound by them).
+template <class R>
+struct RowStatics {
+    A4<R>* v;  // field f of row r at v[f * stride + r]
+    size_t stride;
+    __device__ __forceinline__ RowStatic<R> operator[](uint32_t r) const {
+        return RowStatic<R>{v[r], v[stride + r], v[2 * stride + r], v[3 * stride + r], v[4 * stride + r]};
+    }
+    __device__ __forceinline__ void put(uint32_t r, const RowStatic<R>& s) const {
+        v[r] = s.n;
+        v[stride + r] = s.t1;
+        v[2 * stride + r] = s.t2;
+        v[3 * stride + r] = s.ra;
+        v[4 * stride + r] = s.rb;
+    }
+};
+template <class P, class R>
+struct RowDuals {
+    A4<R>* penalty;
+    A4<P>* lambda;
+    __device__ __forceinline__ RowDual<P, R> operator[](uint32_t r) const {
+        return RowDual<P, R>{penalty[r], lambda[r]};
+    }
+    __device__ __forceinline__ void put(uint32_t r, const RowDual<P, R>& d) const {
+        penalty[r] = d.penalty;
+        lambda[r] = d.lambda;
+    }
+};
 
 // Narrow-phase slot; at R = float its bytes are exactly DioContactOut.
 template <class R>
@@ -102,12 +133,27 @@ struct JView {
     uint32_t pad[2];
 };
 
+// The scene-chunk solve's per-body data by position in the dynamic-body list
+// (the inertial targets and m / dt^2, I / dt^2 are kept by position too in a
+// step solved that way).  joints and the joint arrays are built with the
+// list; rows every step.
+constexpr uint32_t kListJoints = 2;  // joints of a body kept by position
+struct SolveList {
+    uint2* rows;                // row list: first CSR entry, count
+    const uint32_t* joints;     // number of joints
+    const float4* joint_self;   // JView fields of joint q at [q * stride + t]
+    const float4* joint_other;
+    const uint2* joint_meta;    // other body, kind
+    uint32_t stride;
+};
+
 template <class P, class R>
 struct DevWorld {
     uint32_t n;  // bodies
     const uint32_t* dyn_list;  // dynamic bodies, ordered by work signature
     uint32_t n_dyn;
     const JView* jview;        // per-body joint views (joint CSR order)
+    SolveList solve;
     // poses
     A4<P>* pos[2];
     A4<P>* rot[2];
@@ -139,8 +185,8 @@ struct DevWorld {
     uint32_t* epa_list;
     uint32_t epa_wait_polls;  // budget of the EPA's first wait for its hull copies
     // rows
-    RowStatic<R>* rs;
-    RowDual<P, R>* rd;
+    RowStatics<R> rs;
+    RowDuals<P, R> rd;
     uint2* ab;
     uint32_t max_rows;
     uint32_t* row_off;
@@ -218,20 +264,35 @@ __device__ __forceinline__ uint32_t warp_append(uint32_t* cursor) {
     return base + (uint32_t)__popc(m & lt);
 }
 
+// cluster: CTAs per thread-block cluster (0: none)
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_k(bool pdl, void (*kern)(KArgs...), int grid, int block, size_t smem, cudaStream_t s,
-                            Args&&... args) {
+inline cudaError_t launch_clusters(bool pdl, uint32_t cluster, void (*kern)(KArgs...), int grid, int block, size_t smem,
+                                   cudaStream_t s, Args&&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)grid);
     cfg.blockDim = dim3((unsigned)block);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
+    unsigned n = 0;
+    if (pdl) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = cluster;
+        attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+        ++n;
+    }
     cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
+    cfg.numAttrs = n;
     return cudaLaunchKernelEx(&cfg, kern, std::forward<Args>(args)...);
+}
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_k(bool pdl, void (*kern)(KArgs...), int grid, int block, size_t smem, cudaStream_t s,
+                            Args&&... args) {
+    return launch_clusters(pdl, 0u, kern, grid, block, smem, s, std::forward<Args>(args)...);
 }
 
 }  // namespace dio

@@ -131,7 +131,7 @@ __global__ void k_unpack_state(DevWorld<P, R> w, const DioBodyState* st, uint32_
 }
 
 template <class P, class R>
-__global__ void k_unpack_contacts(RowStatic<R>* rs, RowDual<P, R>* rd, uint2* ab, const DioContact* c, uint32_t m,
+__global__ void k_unpack_contacts(RowStatics<R> rs, RowDuals<P, R> rd, uint2* ab, const DioContact* c, uint32_t m,
                                   uint32_t n, uint32_t* err) {
     for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < m; r += gridDim.x * blockDim.x) {
         const DioContact x = c[r];
@@ -141,18 +141,18 @@ __global__ void k_unpack_contacts(RowStatic<R>* rs, RowDual<P, R>* rd, uint2* ab
         s.t2 = A4<R>{R(x.tangent2[0]), R(x.tangent2[1]), R(x.tangent2[2]), R(0)};
         s.ra = A4<R>{R(x.r_a[0]), R(x.r_a[1]), R(x.r_a[2]), R(x.c0[0])};
         s.rb = A4<R>{R(x.r_b[0]), R(x.r_b[1]), R(x.r_b[2]), R(x.c0[1])};
-        rs[r] = s;
+        rs.put(r, s);
         RowDual<P, R> d;
         d.penalty = A4<R>{R(x.penalty[0]), R(x.penalty[1]), R(x.penalty[2]), R(0)};
         d.lambda = A4<P>{P(x.lambda[0]), P(x.lambda[1]), P(x.lambda[2]), P(0)};
-        rd[r] = d;
+        rd.put(r, d);
         ab[r] = make_uint2(x.a, x.b);
         if (x.a >= n || (x.b != kContainer && x.b >= n)) atomicOr(err, kErrBadIndex);
     }
 }
 
 template <class P, class R>
-__global__ void k_pack_contacts(const RowStatic<R>* rs, const RowDual<P, R>* rd, const uint2* ab, DioContact* out,
+__global__ void k_pack_contacts(RowStatics<R> rs, RowDuals<P, R> rd, const uint2* ab, DioContact* out,
                                 const uint32_t* m_dev) {
     uint32_t m = *m_dev;
     for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < m; r += gridDim.x * blockDim.x) {
@@ -263,7 +263,7 @@ __global__ void k_pack_result(DevWorld<P, R> w, uint32_t n, int buf, float* pos3
 }
 
 template <class P, class R>
-__global__ void k_pack_dual(const RowDual<P, R>* rd, uint32_t m, float* lambda, float* penalty) {
+__global__ void k_pack_dual(RowDuals<P, R> rd, uint32_t m, float* lambda, float* penalty) {
     for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < m; r += gridDim.x * blockDim.x) {
         RowDual<P, R> d = rd[r];
         lambda[3 * r] = float(d.lambda.x);
@@ -346,11 +346,21 @@ static __global__ void k_dyn_fill(const uint32_t* flags, const uint32_t* pos, ui
 // incidences (three rows each) first, then distance joints, then the shape.
 // Bodies with one signature run the same code path, so sorting the list by
 // it keeps warps convergent; the Jacobi primal does not depend on the order.
-// With `scene_chunk` set the key leads with the body's solve chunk, so each
-// chunk's dynamic bodies form one signature-ordered run of the list.
+// With `units.scene_chunk` set the key leads with the solve's CTA that holds
+// the body, so each CTA's dynamic bodies form one signature-ordered run of
+// the list.
+struct SolveUnits {
+    const uint32_t* scene_chunk;  // solve chunk of every scene, or null
+    const uint2* chunks;
+    const SceneDesc* scenes;
+    SolveShape shape;
+    __device__ __forceinline__ uint32_t of(uint32_t i, uint32_t scene) const {
+        const uint32_t c = scene_chunk[scene];
+        return (c << shape.cl) | shape.owner(i - scenes[chunks[c].x].body_lo);
+    }
+};
 template <class P, class R>
-__global__ void k_dyn_keys(DevWorld<P, R> w, const uint32_t* list, uint32_t nd, const uint32_t* scene_chunk,
-                           uint32_t* keys) {
+__global__ void k_dyn_keys(DevWorld<P, R> w, const uint32_t* list, uint32_t nd, SolveUnits units, uint32_t* keys) {
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < nd; t += gridDim.x * blockDim.x) {
         const uint32_t i = list[t];
         uint32_t nb = 0, nl = 0;
@@ -364,20 +374,36 @@ __global__ void k_dyn_keys(DevWorld<P, R> w, const uint32_t* list, uint32_t nd, 
         nb = nb > 3u ? 3u : nb;
         nl = nl > 3u ? 3u : nl;
         const uint32_t tag = w.shape[i].tag > 7u ? 7u : w.shape[i].tag;
-        const uint32_t chunk = scene_chunk ? scene_chunk[w.scene[i]] : 0u;
-        keys[t] = (chunk << 7) | ((3u - nb) << 5) | ((3u - nl) << 3) | tag;
+        const uint32_t unit = units.scene_chunk ? units.of(i, w.scene[i]) : 0u;
+        keys[t] = (unit << 7) | ((3u - nb) << 5) | ((3u - nl) << 3) | tag;
     }
 }
 
-// [first, last) of each solve chunk's run in the chunk-ordered dynamic-body
-// list (runs start zeroed: a chunk without dynamic bodies keeps (0, 0))
+// [first, last) of each solve CTA's run in the dynamic-body list (runs start
+// zeroed: a CTA without dynamic bodies keeps (0, 0))
 template <class P, class R>
-__global__ void k_chunk_dyn_runs(DevWorld<P, R> w, const uint32_t* list, uint32_t nd, const uint32_t* scene_chunk,
-                                 uint2* runs) {
+__global__ void k_chunk_dyn_runs(DevWorld<P, R> w, const uint32_t* list, uint32_t nd, SolveUnits units, uint2* runs) {
+    auto unit = [&](uint32_t t) { return units.of(list[t], w.scene[list[t]]); };
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < nd; t += gridDim.x * blockDim.x) {
-        const uint32_t c = scene_chunk[w.scene[list[t]]];
-        if (t == 0 || scene_chunk[w.scene[list[t - 1]]] != c) runs[c].x = t;
-        if (t + 1 == nd || scene_chunk[w.scene[list[t + 1]]] != c) runs[c].y = t + 1;
+        const uint32_t c = unit(t);
+        if (t == 0 || unit(t - 1) != c) runs[c].x = t;
+        if (t + 1 == nd || unit(t + 1) != c) runs[c].y = t + 1;
+    }
+}
+
+// the bodies' first joints by position in the dynamic-body list (SolveList)
+template <class P, class R>
+__global__ void k_list_joints(DevWorld<P, R> w, const uint32_t* list, uint32_t nd, uint32_t* count, float4* self,
+                              float4* other, uint2* meta) {
+    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < nd; t += gridDim.x * blockDim.x) {
+        const uint32_t k0 = w.joint_off[list[t]], n = w.joint_off[list[t] + 1] - k0;
+        count[t] = n;
+        for (uint32_t q = 0; q < n && q < kListJoints; ++q) {
+            const JView v = w.jview[k0 + q];
+            self[q * w.solve.stride + t] = v.self_anchor;
+            other[q * w.solve.stride + t] = v.other_anchor;
+            meta[q * w.solve.stride + t] = make_uint2(v.other, v.kind);
+        }
     }
 }
 
@@ -503,8 +529,10 @@ class Engine final : public EngineBase {
         DIO_TRY(alloc(&lb_long_, N));
         DIO_TRY(alloc(&lb_long_count_, 1));
         for (int b = 0; b < 2; ++b) {
-            DIO_TRY(alloc(&rs_[b], M));
-            DIO_TRY(alloc(&rd_[b], M));
+            DIO_TRY(alloc(&rs_[b].v, 5ull * M));
+            rs_[b].stride = M;
+            DIO_TRY(alloc(&rd_[b].penalty, M));
+            DIO_TRY(alloc(&rd_[b].lambda, M));
             DIO_TRY(alloc(&ab_[b], M));
             DIO_TRY(alloc(&keys_s_[b], M));
             DIO_TRY(alloc(&ids_s_[b], M));
@@ -526,6 +554,12 @@ class Engine final : public EngineBase {
         DIO_TRY(alloc(&dyn_list_, N));
         DIO_TRY(alloc(&dyn_tmp_, N));
         DIO_TRY(alloc(&dyn_keep_, N));
+        DIO_TRY(alloc(&list_rows_, N));
+        DIO_TRY(alloc(&list_joints_, N));
+        DIO_TRY(alloc(&list_joint_self_, (size_t)kListJoints * N));
+        DIO_TRY(alloc(&list_joint_other_, (size_t)kListJoints * N));
+        DIO_TRY(alloc(&list_joint_meta_, (size_t)kListJoints * N));
+        w_.solve = SolveList{list_rows_, list_joints_, list_joint_self_, list_joint_other_, list_joint_meta_, N};
         DIO_TRY(alloc(&color_hist_, kMaxColors + 2));
         const size_t CNT = std::max<size_t>(std::max<size_t>(N, (size_t)PP * per_cap_), 2ull * M) + 2;
         DIO_TRY(alloc(&counts_, CNT));
@@ -535,7 +569,7 @@ class Engine final : public EngineBase {
         DIO_TRY(alloc(&scenes_, S));
         DIO_TRY(alloc(&chunks_, S));
         DIO_TRY(alloc(&solve_chunks_, S));
-        DIO_TRY(alloc(&chunk_dyn_, S));
+        DIO_TRY(alloc(&chunk_dyn_, (size_t)S << kMaxClusterShift));
         DIO_TRY(alloc(&scene_chunk_, S));
         DIO_TRY(alloc(&chunk_n_, S));
         DIO_TRY(alloc(&chunk_ovf_, S));
@@ -590,17 +624,14 @@ class Engine final : public EngineBase {
                                     (int)primal_group_smem<R>()));
         DIO_CK(cudaFuncSetAttribute(k_primal_color<P, R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     (int)primal_group_smem<R>()));
-        DIO_CK(cudaFuncSetAttribute(k_solve_chunks<P, R, kChunkThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)chunk_smem_bytes<P>(solve_chunk_cap<P>())));
-        DIO_CK(cudaFuncSetAttribute(k_solve_chunks<P, R, kChunkThreadsWide>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)chunk_smem_bytes<P>(solve_chunk_cap<P>())));
-        DIO_CK(cudaFuncSetAttribute(k_solve_chunks_colored<P, R, kChunkThreads>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)chunk_colored_smem_bytes<P>(solve_chunk_cap<P>())));
-        DIO_CK(cudaFuncSetAttribute(k_solve_chunks_colored<P, R, kChunkThreadsWide>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)chunk_colored_smem_bytes<P>(solve_chunk_cap<P>())));
+        auto allow = [&](auto* kernel, size_t bytes) {
+            return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+        };
+        constexpr uint32_t spread_cap = solve_cta_cap<P, true>(), packed_cap = solve_cta_cap<P, false>();
+        DIO_CK(allow(k_solve_chunks<P, R, true, true>, chunk_smem_bytes<P, R, true>(spread_cap)));
+        DIO_CK(allow(k_solve_chunks<P, R, false, false>, chunk_smem_bytes<P, R, false>(packed_cap)));
+        DIO_CK(allow(k_solve_chunks_colored<P, R, true, true>, chunk_colored_smem_bytes<P, R, true>(spread_cap)));
+        DIO_CK(allow(k_solve_chunks_colored<P, R, false, false>, chunk_colored_smem_bytes<P, R, false>(packed_cap)));
         return DIO_OK;
     }
     // largest scene, and the chunks of consecutive scenes (each of at most
@@ -639,61 +670,131 @@ class Engine final : public EngineBase {
                          [&](const uint2& a, const uint2& b) { return bodies_of(a) > bodies_of(b); });
         return largest;
     }
-    // Chunks of the scene-chunk solve.  It runs one CTA per chunk and one CTA
-    // per SM, so it takes about (waves) x (largest chunk): for k = 1, 2, ...
-    // waves the smallest chunk size that packs every scene into at most k x
-    // SMs chunks (greedy over consecutive scenes) is found by bisection, and
-    // the k with the smallest k x size wins.  Returns the largest chunk's
-    // bodies (0: some scene exceeds solve_chunk_cap).
+    // Chunks of the scene-chunk solve and how each is dealt to CTAs: the
+    // cheapest of the spread shapes (clusters of 1 to 8 CTAs) and the packed
+    // ones (a CTA a chunk, chunks of up to `target` bodies), by estimates
+    // fitted to measured solves (us for 10 iterations of the jointed batches
+    // of scenes.batched, 2 to 1024 scenes): a cluster costs 56 plus 47 per
+    // round of 256 bodies of a CTA and a little per body (coloured 139 more;
+    // FP64 poses 1.7 times that) whatever the number of scenes, until the clusters exceed what the
+    // GPU holds; a packed CTA 18 plus 0.092 a body (coloured 1.6 times), the
+    // SMs taking the next largest chunk as they fall free; packed only when
+    // there are more chunks than SMs (contact-dense scenes are twice as slow
+    // packed: the 901-body pile 225 against 127).  33 scenes: 104
+    // spread over 8 CTAs, 148 over 4, 203 packed; 257: 244, 193, 209; 1024:
+    // 850, 585, 413.  Returns the largest chunk's bodies (0: some scene
+    // exceeds the cap).
     uint32_t pack_solve_chunks() {
-        const uint32_t cap = solve_chunk_cap<P>();
-        uint32_t largest = 0;
-        for (const SceneDesc& sd : scenes_host_) largest = std::max(largest, sd.body_hi - sd.body_lo);
-        solve_chunks_host_.clear();
-        if (scenes_host_.empty() || largest == 0 || largest > cap) return 0;
-        auto count_at = [&](uint32_t m) {
-            uint64_t count = 0, open = 0;
-            for (const SceneDesc& sd : scenes_host_) {
-                const uint32_t sz = sd.body_hi - sd.body_lo;
-                if (!count || open + sz > m) {
-                    ++count;
-                    open = 0;
-                }
-                open += sz;
-            }
-            return count;
-        };
-        const uint64_t sm = (uint64_t)std::max(1, sms_);
-        uint64_t best_cost = ~0ull;
-        uint32_t best_m = cap;
-        for (uint64_t k = 1; k <= 64; ++k) {
-            if (count_at(cap) > k * sm) continue;
-            uint32_t lo = largest, hi = cap;  // the smallest size with at most k x SMs chunks
-            while (lo < hi) {
-                const uint32_t mid = lo + (hi - lo) / 2;
-                if (count_at(mid) <= k * sm)
-                    hi = mid;
-                else
-                    lo = mid + 1;
-            }
-            if (k * lo < best_cost) {
-                best_cost = k * lo;
-                best_m = lo;
-            }
-            if (lo == largest || k * sm >= scenes_host_.size()) break;  // more waves cannot help
+        uint32_t largest = 0, total = 0;
+        for (const SceneDesc& sd : scenes_host_) {
+            largest = std::max(largest, sd.body_hi - sd.body_lo);
+            total = std::max(total, sd.body_hi);
         }
-        return pack_chunks(best_m, solve_chunks_host_);
+        solve_chunks_host_.clear();
+        shape_mode_ = cfg_.solver_mode;
+        shape_block_ = cfg_.block_size;
+        solve_estimate_ = 0.0;
+        if (scenes_host_.empty() || largest == 0 || largest > kSolveChunkCap) return 0;
+        const bool colored = cfg_.solver_mode == DIO_SOLVER_COLORED;
+        const double wide = sizeof(P) == 4 ? 1.0 : 1.7;
+        double best = 1e300;
+        std::vector<uint2> chunks;
+        auto consider = [&](bool spread, SolveShape sh, double us) {
+            if (us >= best) return;
+            best = us;
+            spread_ = spread;
+            shape_ = sh;
+            solve_chunks_host_ = chunks;
+        };
+        if (cfg_.block_size == 0 || largest > solve_cta_cap<P, false>()) {
+            const uint32_t most = pack_solve(kSolveChunkCap, chunks);
+            for (uint32_t cl = 0; cl <= kMaxClusterShift; ++cl) {
+                SolveShape sh{cl, 5};
+                while (sh.blk && (most >> sh.blk) < (1u << cl)) --sh.blk;
+                const uint32_t slots = sh.slots(most);
+                if (slots > solve_cta_cap<P, true>() || (cl && most < (4u << cl))) continue;
+                const int held = std::max(1, clusters_held(sh, slots, colored));
+                const uint64_t waves = (chunks.size() + held - 1) / held;
+                const double over = double(chunks.size() << cl) / sms_ - 1.0;  // CTAs beyond one an SM
+                const double share = 1.0 + 0.25 * std::min(1.0, std::max(0.0, over));
+                const uint32_t rounds = (slots + 255u) / 256u;
+                consider(true, sh,
+                         (56.0 + 47.0 * rounds + 0.05 * slots + (colored ? 139.0 : 0.0)) * wide * share * waves);
+            }
+        }
+        if (largest <= solve_cta_cap<P, false>())
+            for (uint32_t target : {512u, 768u, 1024u}) {
+                pack_solve(std::min(target, solve_cta_cap<P, false>()), chunks);
+                if (chunks.size() <= (size_t)sms_ && !solve_chunks_host_.empty()) continue;
+                // longest first over the SMs
+                std::vector<double> sm(std::min<size_t>((size_t)sms_, chunks.size()), 0.0);
+                auto later = [](double x, double y) { return x > y; };
+                for (const uint2& c : chunks) {
+                    const uint32_t bodies = scenes_host_[c.y - 1].body_hi - scenes_host_[c.x].body_lo;
+                    std::pop_heap(sm.begin(), sm.end(), later);
+                    sm.back() += 18.0 + 0.092 * bodies;
+                    std::push_heap(sm.begin(), sm.end(), later);
+                }
+                const double us = *std::max_element(sm.begin(), sm.end()) * (chunks.size() > (size_t)sms_ ? 1.35 : 1.0);
+                consider(false, SolveShape{0, 5}, us * wide * (colored ? 1.6 : 1.0));
+            }
+        solve_estimate_ = best;
+        solve_total_ = total;
+        uint32_t most = 0;
+        for (const uint2& c : solve_chunks_host_)
+            most = std::max(most, scenes_host_[c.y - 1].body_hi - scenes_host_[c.x].body_lo);
+        return most;
+    }
+    // clusters of the spread solve that the GPU holds at once
+    int clusters_held(const SolveShape& sh, uint32_t slots, bool colored) const {
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3(1u << sh.cl);
+        cfg.blockDim = dim3(chunk_threads<R, true>());
+        cfg.dynamicSmemBytes = colored ? chunk_colored_smem_bytes<P, R, true>(slots) : chunk_smem_bytes<P, R, true>(slots);
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = 1u << sh.cl;
+        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int n = 0;
+        const cudaError_t e = colored ? cudaOccupancyMaxActiveClusters(&n, k_solve_chunks_colored<P, R, true, true>, &cfg)
+                                      : cudaOccupancyMaxActiveClusters(&n, k_solve_chunks<P, R, true, true>, &cfg);
+        return e == cudaSuccess ? n : 0;
+    }
+    // consecutive scenes packed into chunks of up to `target` bodies (a larger
+    // scene is a chunk by itself), largest first; returns the largest's bodies
+    uint32_t pack_solve(uint32_t target, std::vector<uint2>& out) const {
+        out.clear();
+        auto bodies_of = [&](const uint2& c) { return scenes_host_[c.y - 1].body_hi - scenes_host_[c.x].body_lo; };
+        for (uint32_t s = 0; s < (uint32_t)scenes_host_.size(); ++s) {
+            if (!out.empty() && scenes_host_[s].body_hi - scenes_host_[out.back().x].body_lo <= target)
+                out.back().y = s + 1;
+            else
+                out.push_back(make_uint2(s, s + 1));
+        }
+        std::stable_sort(out.begin(), out.end(),
+                         [&](const uint2& a, const uint2& b) { return bodies_of(a) > bodies_of(b); });
+        return bodies_of(out.front());
+    }
+    // the solve's shape follows the solver mode and the CTA shape asked for;
+    // both may change after the upload
+    int reshape_solve() {
+        if (!chunk_world_ || (shape_mode_ == cfg_.solver_mode && shape_block_ == cfg_.block_size)) return DIO_OK;
+        drop_graphs();
+        DIO_TRY(note_scene_sizes());
+        return order_dyn_list();
     }
     // largest scene; the chunks of the broad phase's shared-memory trees
     // (scene_tree_cap<R> bodies) and of the scene-chunk solve
-    // (solve_chunk_cap<P> bodies)
+    // (kSolveChunkCap bodies)
     int note_scene_sizes() {
         scene_max_ = 0;
         for (const SceneDesc& sd : scenes_host_) scene_max_ = std::max(scene_max_, sd.body_hi - sd.body_lo);
         chunk_max_ = pack_chunks(scene_tree_cap<R>(), chunks_host_);
         solve_chunk_max_ = pack_solve_chunks();
         // solve chunk of every scene (when every scene has one)
-        chunked_scenes_ = !solve_chunks_host_.empty() && scene_max_ <= solve_chunk_cap<P>();
+        chunked_scenes_ = !solve_chunks_host_.empty() && scene_max_ <= kSolveChunkCap;
         if (chunked_scenes_) {
             std::vector<uint32_t> sch(scenes_host_.size(), 0u);
             for (uint32_t c = 0; c < (uint32_t)solve_chunks_host_.size(); ++c)
@@ -1018,6 +1119,7 @@ class Engine final : public EngineBase {
     int step_async(const DioAvbdOptions* options, uint32_t steps) override {
         if (!options) return inval("null options");
         if (!world_ready_) return state_err("no world uploaded");
+        DIO_TRY(reshape_solve());
         if (cfg_.contact_lag) {
             if (!slots_[1]) DIO_TRY(alloc(&slots_[1], (size_t)cap_.max_pairs * per_cap_));
             if (!lag_primed_) {
@@ -1305,17 +1407,23 @@ class Engine final : public EngineBase {
     // index order is kept inside a signature
     int order_dyn_list() {
         const uint32_t nd = w_.n_dyn;
-        const uint32_t nc = (uint32_t)solve_chunks_host_.size();
+        const uint32_t nc = (uint32_t)solve_chunks_host_.size() << shape_.cl;
         if (nc) DIO_CK(cudaMemsetAsync(chunk_dyn_, 0, nc * sizeof(uint2), stream_));
         if (!nd) return DIO_OK;
-        // in chunk order when every scene has a solve chunk (the scene-chunk
-        // solve walks its chunk's run), else by signature alone
-        const uint32_t* sch = chunked_scenes_ ? scene_chunk_ : nullptr;
-        k_dyn_keys<P, R><<<grid_for(nd, 256), 256, 0, stream_>>>(w_, dyn_list_, nd, sch, counts2_);
-        const uint32_t end_bit = 7u + (sch ? bits_for(nc) : 0u);
+        // in the order of the solve's CTAs when every scene has a solve chunk
+        // (a CTA walks its run), else by signature alone
+        const SolveUnits units{chunked_scenes_ ? scene_chunk_ : nullptr, solve_chunks_, scenes_, shape_};
+        k_dyn_keys<P, R><<<grid_for(nd, 256), 256, 0, stream_>>>(w_, dyn_list_, nd, units, counts2_);
+        const uint32_t end_bit = 7u + (chunked_scenes_ ? bits_for(nc) : 0u);
         DIO_CK(ss_.sort_pairs(counts2_, offsets2_, dyn_list_, dyn_tmp_, nd, 0u, end_bit, false, stream_));
         DIO_CK(cudaMemcpyAsync(dyn_list_, dyn_tmp_, (size_t)nd * 4, cudaMemcpyDeviceToDevice, stream_));
-        if (sch) k_chunk_dyn_runs<P, R><<<grid_for(nd, 256), 256, 0, stream_>>>(w_, dyn_list_, nd, sch, chunk_dyn_);
+        if (chunked_scenes_) {
+            k_chunk_dyn_runs<P, R><<<grid_for(nd, 256), 256, 0, stream_>>>(w_, dyn_list_, nd, units, chunk_dyn_);
+            if (w_.n_joints)
+                k_list_joints<P, R><<<grid_for(nd, 256), 256, 0, stream_>>>(w_, dyn_list_, nd, list_joints_,
+                                                                            list_joint_self_, list_joint_other_,
+                                                                            list_joint_meta_);
+        }
         return DIO_OK;
     }
     int single_scene(uint32_t n, const DioContainer* c) {
@@ -1339,6 +1447,7 @@ class Engine final : public EngineBase {
         // the API path is single-scene FP32; keep host scene table in sync
         scenes_host_.assign(1, x);
         DIO_TRY(note_scene_sizes());
+        chunked_scenes_ = false;  // these calls solve per phase: the list needs no CTA order
         DIO_CK(cudaStreamSynchronize(stream_));
         return DIO_OK;
     }
@@ -1357,33 +1466,35 @@ class Engine final : public EngineBase {
         return true;
     }
     // the whole solve of a world step as one launch (k_solve_chunks)
-    bool use_chunk_solve() const { return chunk_world_ && cfg_.batched_solver == DIO_SOLVE_AUTO; }
+    // unless, with FP64 poses (half the bodies a CTA), the per-phase launches
+    // are the faster: 297 us plus 2 per 1,000 bodies (coloured 670 plus 3.1),
+    // measured as above
+    bool use_chunk_solve() const {
+        if (!chunk_world_ || cfg_.batched_solver != DIO_SOLVE_AUTO) return false;
+        if (sizeof(P) == 4) return true;
+        return solve_estimate_ <= (cfg_.solver_mode == DIO_SOLVER_COLORED ? 670.0 + 3.1e-3 * solve_total_
+                                                                           : 297.0 + 2.0e-3 * solve_total_);
+    }
     bool chunk_solve_possible() const override { return chunk_world_; }
     int solve_chunks(const SolveParams<R>& o) {
-        const uint32_t cap = solve_chunk_max_;  // shared memory sized to the largest chunk
+        const uint32_t cap = shape_.slots(solve_chunk_max_);  // shared memory sized to the largest chunk
         cudaEvent_t e0 = span_begin();
-        const int grid = (int)solve_chunks_host_.size();
-        const bool wide = cfg_.block_size == (uint32_t)kChunkThreadsWide;
-        if (cfg_.solver_mode == DIO_SOLVER_COLORED) {
-            // the coloured Gauss-Seidel schedule, colouring included
-            const size_t cs = chunk_colored_smem_bytes<P>(cap);
-            if (wide)
-                DIO_CK(launch_k(pdl(), k_solve_chunks_colored<P, R, kChunkThreadsWide>, grid, kChunkThreadsWide, cs,
-                                stream_, w_, (const uint2*)solve_chunks_, (const uint2*)chunk_dyn_, scenes_, cap, o));
-            else
-                DIO_CK(launch_k(pdl(), k_solve_chunks_colored<P, R, kChunkThreads>, grid, kChunkThreads, cs,
-                                stream_, w_, (const uint2*)solve_chunks_, (const uint2*)chunk_dyn_, scenes_, cap, o));
-            span_end(e0, 6);
-            ++launches_;
-            return DIO_OK;
-        }
-        const size_t smem = chunk_smem_bytes<P>(cap);
-        if (wide)
-            DIO_CK(launch_k(pdl(), k_solve_chunks<P, R, kChunkThreadsWide>, grid, kChunkThreadsWide, smem, stream_, w_,
-                            (const uint2*)solve_chunks_, (const uint2*)chunk_dyn_, scenes_, cap, o));
+        const int grid = (int)(solve_chunks_host_.size() << shape_.cl);
+        const bool colored = cfg_.solver_mode == DIO_SOLVER_COLORED;
+        auto run = [&](auto* kernel, int threads, size_t smem) {
+            return launch_clusters(pdl(), spread_ ? 1u << shape_.cl : 0u, kernel, grid, threads, smem, stream_, w_,
+                                   (const uint2*)solve_chunks_, (const uint2*)chunk_dyn_, (const SceneDesc*)scenes_,
+                                   cap, shape_, o);
+        };
+        if (spread_)
+            DIO_CK(colored ? run(k_solve_chunks_colored<P, R, true, true>, chunk_threads<R, true>(),
+                                 chunk_colored_smem_bytes<P, R, true>(cap))
+                           : run(k_solve_chunks<P, R, true, true>, chunk_threads<R, true>(), chunk_smem_bytes<P, R, true>(cap)));
         else
-            DIO_CK(launch_k(pdl(), k_solve_chunks<P, R, kChunkThreads>, grid, kChunkThreads, smem, stream_, w_,
-                            (const uint2*)solve_chunks_, (const uint2*)chunk_dyn_, scenes_, cap, o));
+            DIO_CK(colored ? run(k_solve_chunks_colored<P, R, false, false>, chunk_threads<R, false>(),
+                                 chunk_colored_smem_bytes<P, R, false>(cap))
+                           : run(k_solve_chunks<P, R, false, false>, chunk_threads<R, false>(),
+                                 chunk_smem_bytes<P, R, false>(cap)));
         span_end(e0, 6);
         ++launches_;
         return DIO_OK;
@@ -1804,6 +1915,21 @@ class Engine final : public EngineBase {
         }
         return o;
     }
+    // the image keeps rows as records (RowStatic, RowDual), the device field
+    // by field: strided copies between the two
+    int copy_rows(char* statics, char* duals, int buf, uint32_t rows, bool to_device) {
+        auto field = [&](char* host, size_t pitch, void* dev, size_t bytes) {
+            return to_device ? cudaMemcpy2DAsync(dev, bytes, host, pitch, bytes, rows, cudaMemcpyHostToDevice, stream_)
+                             : cudaMemcpy2DAsync(host, pitch, dev, bytes, bytes, rows, cudaMemcpyDeviceToHost, stream_);
+        };
+        for (size_t f = 0; f < 5; ++f)
+            DIO_CK(field(statics + f * sizeof(A4<R>), sizeof(RowStatic<R>), rs_[buf].v + f * rs_[buf].stride,
+                         sizeof(A4<R>)));
+        DIO_CK(field(duals + offsetof(DualRecord, penalty), sizeof(DualRecord), rd_[buf].penalty, sizeof(A4<R>)));
+        DIO_CK(field(duals + offsetof(DualRecord, lambda), sizeof(DualRecord), rd_[buf].lambda, sizeof(A4<P>)));
+        return DIO_OK;
+    }
+    using DualRecord = RowDual<P, R>;
     static constexpr char kCkptMagic[8] = {'D', 'I', 'O', 'C', 'K', 'P', 'T', '1'};
 
    public:
@@ -1852,10 +1978,7 @@ class Engine final : public EngineBase {
             if (a4) DIO_CK(cudaMemcpyAsync(b + off[kCkPos + k], src[k], a4, cudaMemcpyDeviceToHost, stream_));
         const int pb = 1 - cur_;  // the last step's rows
         if (h.rows) {
-            DIO_CK(cudaMemcpyAsync(b + off[kCkRowStatic], rs_[pb], (size_t)h.rows * sizeof(RowStatic<R>),
-                                   cudaMemcpyDeviceToHost, stream_));
-            DIO_CK(cudaMemcpyAsync(b + off[kCkRowDual], rd_[pb], (size_t)h.rows * sizeof(RowDual<P, R>),
-                                   cudaMemcpyDeviceToHost, stream_));
+            DIO_TRY(copy_rows(b + off[kCkRowStatic], b + off[kCkRowDual], pb, h.rows, false));
             DIO_CK(cudaMemcpyAsync(b + off[kCkRowAb], ab_[pb], (size_t)h.rows * sizeof(uint2), cudaMemcpyDeviceToHost,
                                    stream_));
         }
@@ -1921,10 +2044,8 @@ class Engine final : public EngineBase {
         // the last step's rows: the next step's warm-start source
         const int pb = 1 - cur_;
         if (h.rows) {
-            DIO_CK(cudaMemcpyAsync(rs_[pb], b + off[kCkRowStatic], (size_t)h.rows * sizeof(RowStatic<R>),
-                                   cudaMemcpyHostToDevice, stream_));
-            DIO_CK(cudaMemcpyAsync(rd_[pb], b + off[kCkRowDual], (size_t)h.rows * sizeof(RowDual<P, R>),
-                                   cudaMemcpyHostToDevice, stream_));
+            DIO_TRY(copy_rows(const_cast<char*>(b) + off[kCkRowStatic], const_cast<char*>(b) + off[kCkRowDual], pb,
+                              h.rows, true));
             DIO_CK(cudaMemcpyAsync(ab_[pb], b + off[kCkRowAb], (size_t)h.rows * sizeof(uint2), cudaMemcpyHostToDevice,
                                    stream_));
         }
@@ -1968,8 +2089,9 @@ class Engine final : public EngineBase {
         DIO_CK(cp(w_.ang, a4));
         DIO_CK(cp(w_.prev_vel, a4));
         for (int b = 0; b < 2; ++b) {
-            DIO_CK(cp(rs_[b], nr * sizeof(RowStatic<R>)));
-            DIO_CK(cp(rd_[b], nr * sizeof(RowDual<P, R>)));
+            DIO_CK(cp(rs_[b].v, nr * sizeof(RowStatic<R>)));
+            DIO_CK(cp(rd_[b].penalty, nr * sizeof(A4<R>)));
+            DIO_CK(cp(rd_[b].lambda, nr * sizeof(A4<P>)));
             DIO_CK(cp(ab_[b], nr * sizeof(uint2)));
         }
         DIO_CK(cp(ctr_, sizeof(Counters)));
@@ -2071,9 +2193,13 @@ class Engine final : public EngineBase {
                     uint32_t c0 = color_off_h_[c], c1 = color_off_h_[c + 1];
                     if (c1 <= c0) continue;
                     cudaEvent_t e0 = span_begin();
-                    const uint32_t g = cfg_.primal_variant == 10 ? 1u : primal_group_size(c1 - c0, sms_);
-                    k_primal_color<P, R><<<grid_for(c1 - c0, kPrimalGroupWarps * (int)g), kPrimalGroupWarps * 32,
-                                           primal_group_smem<R>(), stream_>>>(w_, c0, c1, g, so);
+                    if (cfg_.primal_variant != 10 && mostly_jointed(w_)) {
+                        k_primal_color_bodies<P, R><<<grid_for(c1 - c0, 128), 128, 0, stream_>>>(w_, c0, c1, so);
+                    } else {
+                        const uint32_t g = cfg_.primal_variant == 10 ? 1u : primal_group_size(c1 - c0, sms_);
+                        k_primal_color<P, R><<<grid_for(c1 - c0, kPrimalGroupWarps * (int)g), kPrimalGroupWarps * 32,
+                                               primal_group_smem<R>(), stream_>>>(w_, c0, c1, g, so);
+                    }
                     span_end(e0, 0);
                     ++launches_;
                 }
@@ -2149,7 +2275,7 @@ class Engine final : public EngineBase {
         int pb = 1 - cur_;
         const int gf = std::min(grid_for(cap_.max_contacts, 256), sms_ * 8);
         DIO_CK(launch_k(pdl(), k_warm_sections<P, R>, gf, 256, 0, stream_, w_, (const uint2*)ab_[pb],
-                        (const RowDual<P, R>*)rd_[pb], o));
+                        rd_[pb], o));
         // counts2_ was cleared by k_cont_rows (build_rows, bodies [0, n))
         if (!n) DIO_CK(cudaMemsetAsync(counts2_, 0, 4, stream_));
         DIO_CK(launch_k(pdl() && n, k_csr_count_dyn<P, R>, gf, 256, 0, stream_, w_, counts2_));
@@ -2268,8 +2394,8 @@ class Engine final : public EngineBase {
     std::vector<void*> allocs_;
     uint32_t per_cap_ = 4;
     int sms_ = 152;
-    RowStatic<R>* rs_[2] = {};
-    RowDual<P, R>* rd_[2] = {};
+    RowStatics<R> rs_[2] = {};
+    RowDuals<P, R> rd_[2] = {};
     uint2* ab_[2] = {};
     unsigned long long* keys_s_[2] = {};
     uint32_t* ids_s_[2] = {};
@@ -2299,6 +2425,15 @@ class Engine final : public EngineBase {
     uint32_t* scene_chunk_ = nullptr;   // solve chunk of every scene
     bool chunked_scenes_ = false;       // every scene has a solve chunk
     uint32_t solve_chunk_max_ = 0;      // bodies of the largest solve chunk
+    SolveShape shape_{0, 5};            // how a solve chunk is dealt to its cluster's CTAs
+    bool spread_ = false;               // clusters of small CTAs, or a CTA a chunk
+    uint32_t shape_mode_ = 0, shape_block_ = 0;  // solver_mode, block_size the shape was chosen for
+    double solve_estimate_ = 0.0;       // of the chosen shape, us
+    uint32_t solve_total_ = 0;          // bodies of all scenes
+    uint2* list_rows_ = nullptr;        // SolveList arrays
+    uint32_t* list_joints_ = nullptr;
+    float4 *list_joint_self_ = nullptr, *list_joint_other_ = nullptr;
+    uint2* list_joint_meta_ = nullptr;
     uint2* chunks_ = nullptr;
     Slot<R>* slots_[2] = {nullptr, nullptr};
     // inside step_body_dev: its scratch zeroing is done by k_roll_counters and

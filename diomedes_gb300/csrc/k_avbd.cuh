@@ -126,41 +126,41 @@ __device__ __forceinline__ void solve6(const Block6<R>& B, R x[6]) {
     x[0] = z1 - l21 * x[1] - l31 * x[2] - l41 * x[3] - l51 * x[4] - l61 * x[5];
 }
 
-// avbd_init, avbd/src/lib.rs:202-254 (+ seeding buffer 1 with the
-// un-warm-started pose, render/gpu_physics.rs:479-482)
+// avbd_init, avbd/src/lib.rs:202-254, for one body: the inertial target and
+// the diagonal m / dt^2, I / dt^2 go to index `at` of their arrays, the
+// step-start pose and the (for dynamic bodies) warm-started one come back.
+template <class P>
+struct InitPose {
+    A4<P> start_pos, start_rot, pos, rot;
+};
 template <class P, class R>
-__device__ __forceinline__ void init_body(const DevWorld<P, R>& w, uint32_t i, const SolveParams<R>& o) {
-    A4<P> p4 = w.pos[0][i];
-    A4<P> q4 = w.rot[0][i];
-    R inv_mass = w.inv[i].w;
-    // buffer 1 holds the un-warm-started pose for bodies the primal never
-    // writes (static ones); a dynamic body's copy is overwritten by the first
-    // primal before anything reads it, unless there is no iteration at all
-    if (inv_mass == R(0) || o.iterations == 0) {
-        w.pos[1][i] = p4;
-        w.rot[1][i] = q4;
-    }
-    V3<P> pos = xyz(p4);
-    Q4<P> rot = quat(q4);
+__device__ __forceinline__ InitPose<P> init_pose(const DevWorld<P, R>& w, uint32_t i, uint32_t at,
+                                                 const SolveParams<R>& o) {
+    InitPose<P> r;
+    r.pos = w.pos[0][i];
+    r.rot = w.rot[0][i];
+    const A4<R> inv = w.inv[i];
+    const R inv_mass = inv.w;
+    V3<P> pos = xyz(r.pos);
+    Q4<P> rot = quat(r.rot);
     V3<P> vel = xyz(w.vel[i]);
     V3<P> ang = xyz(w.ang[i]);
     P dt = P(o.dt);
     V3<P> g{P(o.gx), P(o.gy), P(o.gz)};
-    w.init_pos[i] = pack(pos);
-    w.init_rot[i] = q4;
+    r.start_pos = pack(pos);
+    r.start_rot = r.rot;
     V3<P> ip = add(pos, scale(vel, dt));
     if (inv_mass > R(0)) ip = add(ip, scale(g, dt * dt));
-    w.inert_pos[i] = pack(ip);
+    w.inert_pos[at] = pack(ip);
     Q4<P> irot = quat_step(rot, scale(ang, dt));
-    w.inert_rot[i] = packq(irot);
+    w.inert_rot[at] = packq(irot);
     if (w.mdt2 && inv_mass != R(0)) {
         // the primal's diagonal, constant over the step (avbd/src/lib.rs:293-296)
-        const A4<R> inv = w.inv[i];
         const R mass = R(1) / inv.w;
         const V3<R> moment{R(1) / inv.x, R(1) / inv.y, R(1) / inv.z};
         const R dt2 = o.dt * o.dt;
         const V3<R> idt2 = divs(moment, dt2);
-        w.mdt2[i] = A4<R>{mass / dt2, idt2.x, idt2.y, idt2.z};
+        w.mdt2[at] = A4<R>{mass / dt2, idt2.x, idt2.y, idt2.z};
     }
     if (inv_mass > R(0)) {
         // adaptive gravity weight, clamped to [0, 1]: formed in R in the split
@@ -175,8 +175,31 @@ __device__ __forceinline__ void init_body(const DevWorld<P, R>& w, uint32_t i, c
             wgt = dot(accel, divs(gf, gm)) / gm;
             wgt = wgt < Fq(0) ? Fq(0) : (wgt > Fq(1) ? Fq(1) : wgt);
         }
-        w.pos[0][i] = pack(add(add(pos, scale(vel, dt)), scale(g, P(wgt) * dt * dt)));
-        w.rot[0][i] = packq(irot);  // the same quat_step(rot, ang dt)
+        r.pos = pack(add(add(pos, scale(vel, dt)), scale(g, P(wgt) * dt * dt)));
+        r.rot = packq(irot);  // the same quat_step(rot, ang dt)
+    }
+    return r;
+}
+
+// avbd_init with the poses in global memory (+ seeding buffer 1 with the
+// un-warm-started pose, render/gpu_physics.rs:479-482)
+template <class P, class R>
+__device__ __forceinline__ void init_body(const DevWorld<P, R>& w, uint32_t i, const SolveParams<R>& o) {
+    const A4<P> p4 = w.pos[0][i];
+    const InitPose<P> r = init_pose(w, i, i, o);
+    const R inv_mass = w.inv[i].w;
+    // buffer 1 holds the un-warm-started pose for bodies the primal never
+    // writes (static ones); a dynamic body's copy is overwritten by the first
+    // primal before anything reads it, unless there is no iteration at all
+    if (inv_mass == R(0) || o.iterations == 0) {
+        w.pos[1][i] = p4;
+        w.rot[1][i] = r.start_rot;
+    }
+    w.init_pos[i] = r.start_pos;
+    w.init_rot[i] = r.start_rot;
+    if (inv_mass > R(0)) {
+        w.pos[0][i] = r.pos;
+        w.rot[0][i] = r.rot;
     }
 }
 
@@ -221,28 +244,6 @@ struct TileFetch {
     __device__ __forceinline__ void store(uint32_t i, A4<P> p, A4<P> q) const {
         w.pos[1 - rd][i] = p;
         w.rot[1 - rd][i] = q;
-    }
-};
-
-// Poses of one scene chunk held in shared memory: bodies [lo, lo + count)
-// at index j - lo.  Every body a chunk's rows and joints touch lies in the
-// chunk (rows and joints never cross scenes).
-template <class P>
-struct SmemFetch {
-    const A4<P>* sp;  // snapshot (read) buffer
-    const A4<P>* sq;
-    const A4<P>* si;  // step-start pose
-    const A4<P>* sr;
-    A4<P>* wp;        // the primal's output buffer
-    A4<P>* wq;
-    uint32_t lo;
-    __device__ __forceinline__ A4<P> pos(uint32_t j) const { return sp[j - lo]; }
-    __device__ __forceinline__ A4<P> rot(uint32_t j) const { return sq[j - lo]; }
-    __device__ __forceinline__ A4<P> ipos(uint32_t j) const { return si[j - lo]; }
-    __device__ __forceinline__ A4<P> irot(uint32_t j) const { return sr[j - lo]; }
-    __device__ __forceinline__ void store(uint32_t i, A4<P> p, A4<P> q) const {
-        wp[i - lo] = p;
-        wq[i - lo] = q;
     }
 };
 
@@ -342,16 +343,6 @@ __device__ __forceinline__ void primal_row_f(const DevWorld<P, R>& w, uint32_t r
                                              Q4<R> sqr, V3<R> dqsl, V3<R> dqsa, R k_alpha, Block6<R>& B) {
     primal_row_core<P, R>(w.rs[r], w.rd[r], oth, fetch, sqr, dqsl, dqsa, k_alpha, B);
 }
-// The rows of a body read from the world's current row duals.
-struct RowsFromWorld {
-    template <class P, class R, class F>
-    __device__ __forceinline__ void operator()(const DevWorld<P, R>& w, uint32_t i, uint32_t r, uint32_t oth,
-                                               const F& fetch, Q4<R> sqr, V3<R> dqsl, V3<R> dqsa, R k_alpha,
-                                               Block6<R>& B) const {
-        primal_row_f(w, r, oth, fetch, sqr, dqsl, dqsa, k_alpha, B);
-    }
-};
-
 template <class P, class R>
 __device__ __forceinline__ void primal_row(const DevWorld<P, R>& w, uint32_t r, uint32_t oth, int rd, Q4<R> sqr,
                                            V3<R> dqsl, V3<R> dqsa, R k_alpha, Block6<R>& B) {
@@ -457,24 +448,21 @@ __device__ __forceinline__ void primal_jview_f(const JView& jv, const F& fetch, 
     primal_jview_p<P, R>(jv, fetch.pos(jv.other), fetch.rot(jv.other), sp, sq, sqr, B);
 }
 
-// The inertial start of body i's 6x6 system: diagonal M/dt^2, I/dt^2 and
-// the gradient toward the inertial pose.
+// What the primal of one body starts from besides its pose: its row list
+// [j0, j0 + n), the diagonal m / dt^2, I / dt^2 and the inertial target.
 template <class P, class R>
-__device__ __forceinline__ void primal_inertia(const DevWorld<P, R>& w, uint32_t i, const A4<R>& inv, V3<P> sp,
-                                               Q4<R> sqr, const SolveParams<R>& o, Block6<R>& B) {
-    R mdt2;
-    V3<R> idt2;
-    if (w.mdt2) {
-        const A4<R> d = w.mdt2[i];  // stored by init: the same divisions, once per step
-        mdt2 = d.x;
-        idt2 = V3<R>{d.y, d.z, d.w};
-    } else {
-        const R mass = R(1) / inv.w;
-        const V3<R> moment{R(1) / inv.x, R(1) / inv.y, R(1) / inv.z};
-        const R dt2 = o.dt * o.dt;
-        mdt2 = mass / dt2;
-        idt2 = divs(moment, dt2);
-    }
+struct BodyTask {
+    uint32_t i, j0, n;
+    A4<R> mdt2;
+    A4<P> ipos, irot;
+};
+
+// The inertial start of a body's 6x6 system: diagonal M/dt^2, I/dt^2 and the
+// gradient toward the inertial pose.
+template <class P, class R>
+__device__ __forceinline__ void primal_inertia(const BodyTask<P, R>& b, V3<P> sp, Q4<R> sqr, Block6<R>& B) {
+    const R mdt2 = b.mdt2.x;
+    const V3<R> idt2{b.mdt2.y, b.mdt2.z, b.mdt2.w};
 #pragma unroll
     for (int k = 0; k < 21; ++k) B.h[k] = R(0);
     B.h[tri(0, 0)] = mdt2;
@@ -483,8 +471,8 @@ __device__ __forceinline__ void primal_inertia(const DevWorld<P, R>& w, uint32_t
     B.h[tri(3, 3)] = idt2.x;
     B.h[tri(4, 4)] = idt2.y;
     B.h[tri(5, 5)] = idt2.z;
-    const V3<R> rl = mulv(V3<R>{mdt2, mdt2, mdt2}, cast3<R>(sub(sp, xyz(w.inert_pos[i]))));
-    const V3<R> ra = mulv(idt2, ang_diff(sqr, castq<R>(quat(w.inert_rot[i]))));
+    const V3<R> rl = mulv(V3<R>{mdt2, mdt2, mdt2}, cast3<R>(sub(sp, xyz(b.ipos))));
+    const V3<R> ra = mulv(idt2, ang_diff(sqr, castq<R>(quat(b.irot))));
     B.g[0] = rl.x;
     B.g[1] = rl.y;
     B.g[2] = rl.z;
@@ -493,13 +481,70 @@ __device__ __forceinline__ void primal_inertia(const DevWorld<P, R>& w, uint32_t
     B.g[5] = ra.z;
 }
 
+// Where the primal finds its bodies' constants and joints.  WorldBodies: by
+// body, through the row and joint CSRs.
+template <class P, class R>
+struct WorldBodies {
+    const DevWorld<P, R>& w;
+    const uint32_t* list;
+    __device__ __forceinline__ BodyTask<P, R> load(uint32_t t) const {
+        BodyTask<P, R> b;
+        b.i = list[t];
+        b.j0 = w.row_off[b.i];
+        b.n = w.row_off[b.i + 1] - b.j0;
+        b.mdt2 = w.mdt2[b.i];
+        b.ipos = w.inert_pos[b.i];
+        b.irot = w.inert_rot[b.i];
+        return b;
+    }
+    __device__ __forceinline__ uint32_t joints(uint32_t, uint32_t i) const {
+        return w.n_joints ? w.joint_off[i + 1] - w.joint_off[i] : 0u;
+    }
+    __device__ __forceinline__ JView joint(uint32_t, uint32_t i, uint32_t q) const {
+        return w.jview[w.joint_off[i] + q];
+    }
+};
+// ListBodies: by position in the dynamic-body list, where the scene-chunk
+// solve keeps them (SolveList): a warp's bodies are consecutive positions, so
+// all of a body's constants and its first two joints are coalesced loads
+// that depend on nothing but the position.
+template <class P, class R>
+struct ListBodies {
+    const DevWorld<P, R>& w;
+    __device__ __forceinline__ BodyTask<P, R> load(uint32_t t) const {
+        BodyTask<P, R> b;
+        b.i = w.dyn_list[t];
+        const uint2 r = w.solve.rows[t];
+        b.j0 = r.x;
+        b.n = r.y;
+        b.mdt2 = w.mdt2[t];
+        b.ipos = w.inert_pos[t];
+        b.irot = w.inert_rot[t];
+        return b;
+    }
+    __device__ __forceinline__ uint32_t joints(uint32_t t, uint32_t) const {
+        return w.n_joints ? w.solve.joints[t] : 0u;
+    }
+    __device__ __forceinline__ JView joint(uint32_t t, uint32_t i, uint32_t q) const {
+        if (q >= kListJoints) return w.jview[w.joint_off[i] + q];
+        JView v;
+        const uint2 m = w.solve.joint_meta[q * w.solve.stride + t];
+        v.self_anchor = w.solve.joint_self[q * w.solve.stride + t];
+        v.other_anchor = w.solve.joint_other[q * w.solve.stride + t];
+        v.other = m.x;
+        v.kind = m.y;
+        return v;
+    }
+};
+
 // Joint rows, the 6x6 solve and the pose update of body i (the tail of
-// avbd_primal)
-template <class P, class R, class F>
-__device__ __forceinline__ void primal_finish(const DevWorld<P, R>& w, uint32_t i, uint32_t k0, uint32_t k1,
-                                              const F& fetch, V3<P> sp, Q4<P> sq, Q4<R> sqr, Block6<R>& B) {
-    for (uint32_t k = k0; k < k1; ++k) {
-        const JView jv = w.jview[k];
+// avbd_primal); t: its position for `bodies`
+template <class P, class R, class F, class S>
+__device__ __forceinline__ void primal_finish(const S& bodies, uint32_t t, uint32_t i, const F& fetch, V3<P> sp,
+                                              Q4<P> sq, Q4<R> sqr, Block6<R>& B) {
+    const uint32_t nj = bodies.joints(t, i);
+    for (uint32_t k = 0; k < nj; ++k) {
+        const JView jv = bodies.joint(t, i, k);
         primal_jview_f<P, R>(jv, fetch, sp, sq, sqr, B);
     }
     R dx[6];
@@ -512,32 +557,32 @@ __device__ __forceinline__ void primal_finish(const DevWorld<P, R>& w, uint32_t 
 }
 
 // avbd_primal for one body: reads the snapshot through `fetch` and stores
-// the new pose through it.  [k0, k1) is the body's joint-view range.
-template <class P, class R, class F, class Rows = RowsFromWorld>
-__device__ __forceinline__ void primal_body_f(const DevWorld<P, R>& w, uint32_t i, uint32_t k0, uint32_t k1,
-                                              const SolveParams<R>& o, const F& fetch, const Rows& rows = Rows()) {
-    const A4<R> inv = w.inv[i];
-    if (inv.w == R(0)) return;
+// the new pose through it.
+template <class P, class R, class F>
+__device__ __forceinline__ void primal_body_f(const DevWorld<P, R>& w, uint32_t i, const SolveParams<R>& o,
+                                              const F& fetch) {
+    if (w.inv[i].w == R(0)) return;
+    const WorldBodies<P, R> bodies{w, &i};
+    const BodyTask<P, R> b = bodies.load(0);
     const V3<P> sp = xyz(fetch.pos(i));
     const Q4<P> sq = quat(fetch.rot(i));
     const Q4<R> sqr = castq<R>(sq);
     Block6<R> B;
-    primal_inertia(w, i, inv, sp, sqr, o, B);
-    const uint32_t j0 = w.row_off[i], j1 = w.row_off[i + 1];
-    if (j0 < j1) {
+    primal_inertia(b, sp, sqr, B);
+    if (b.n) {
         // displacement since the step start: read only by contact rows
         const V3<R> dqsl = cast3<R>(sub(sp, xyz(fetch.ipos(i))));
         const V3<R> dqsa = ang_diff(sqr, castq<R>(quat(fetch.irot(i))));
         const R k_alpha = R(1) - o.alpha;
-        for (uint32_t j = j0; j < j1; ++j) rows(w, i, w.row_idx[j], w.row_oth[j], fetch, sqr, dqsl, dqsa, k_alpha, B);
+        for (uint32_t j = b.j0; j < b.j0 + b.n; ++j)
+            primal_row_f(w, w.row_idx[j], w.row_oth[j], fetch, sqr, dqsl, dqsa, k_alpha, B);
     }
-    primal_finish(w, i, k0, k1, fetch, sp, sq, sqr, B);
+    primal_finish(bodies, 0u, i, fetch, sp, sq, sqr, B);
 }
 
 template <class P, class R>
 __device__ __forceinline__ void primal_body(const DevWorld<P, R>& w, uint32_t i, int rd, const SolveParams<R>& o) {
-    const uint32_t k0 = w.n_joints ? w.joint_off[i] : 0u, k1 = w.n_joints ? w.joint_off[i + 1] : 0u;
-    primal_body_f(w, i, k0, k1, o, GlobalFetch<P, R>{w, rd});
+    primal_body_f(w, i, o, GlobalFetch<P, R>{w, rd});
 }
 
 // Tile variant: the CTA's T consecutive bodies stage their snapshot and
@@ -558,8 +603,7 @@ __global__ void __launch_bounds__(T, MINB) k_primal_tile(DevWorld<P, R> w, int r
     }
     __syncthreads();
     if (i < w.n) {
-        const uint32_t k0 = w.n_joints ? w.joint_off[i] : 0u, k1 = w.n_joints ? w.joint_off[i + 1] : 0u;
-        primal_body_f(w, i, k0, k1, o, TileFetch<P, R, T>{w, rd, lo, s_pos, s_rot, s_ipos, s_irot});
+        primal_body_f(w, i, o, TileFetch<P, R, T>{w, rd, lo, s_pos, s_rot, s_ipos, s_irot});
     }
 }
 
@@ -574,6 +618,39 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_primal(DevWorld<P, R> w, int rd
         primal_body(w, w.dyn_list[t], rd, o);
 }
 
+// avbd_dual, avbd/src/lib.rs:565-663: the row's dual update from its bodies' new poses (a, and b unless the
+// row is against a container) and step-start poses.
+template <class P, class R>
+__device__ __forceinline__ RowDual<P, R> dual_update(const RowStatic<R>& rs, RowDual<P, R> du, A4<P> pa4, A4<P> qa4,
+                                                     A4<P> ia_p, A4<P> ia_q, bool has_b, A4<P> pb4, A4<P> qb4,
+                                                     A4<P> ib_p, A4<P> ib_q, const SolveParams<R>& o) {
+    V3<R> dal = cast3<R>(sub(xyz(pa4), xyz(ia_p)));
+    V3<R> daa = ang_diff(castq<R>(quat(qa4)), castq<R>(quat(ia_q)));
+    V3<R> dbl{R(0), R(0), R(0)}, dba{R(0), R(0), R(0)}, rbw{R(0), R(0), R(0)};
+    if (has_b) {
+        dbl = cast3<R>(sub(xyz(pb4), xyz(ib_p)));
+        dba = ang_diff(castq<R>(quat(qb4)), castq<R>(quat(ib_q)));
+        rbw = rotate(castq<R>(quat(qb4)), xyz(rs.rb));
+    }
+    V3<R> raw = rotate(castq<R>(quat(qa4)), xyz(rs.ra));
+    V3<R> r0 = xyz(rs.n), r1 = xyz(rs.t1), r2 = xyz(rs.t2);
+    const R k_alpha = R(1) - o.alpha;
+    R c0 = rs.ra.w * k_alpha, c1 = rs.rb.w * k_alpha, c2 = rs.t1.w * k_alpha;
+    c0 = c0 + (dot(r0, dal) + dot(cross(raw, r0), daa) - dot(r0, dbl) - dot(cross(rbw, r0), dba));
+    c1 = c1 + (dot(r1, dal) + dot(cross(raw, r1), daa) - dot(r1, dbl) - dot(cross(rbw, r1), dba));
+    c2 = c2 + (dot(r2, dal) + dot(cross(raw, r2), daa) - dot(r2, dbl) - dot(cross(rbw, r2), dba));
+    P f0, f1, f2, tm, bounds;
+    row_forces(du, rs.n.w, c0, c1, c2, f0, f1, f2, tm, bounds);
+    du.lambda.x = f0;
+    du.lambda.y = f1;
+    du.lambda.z = f2;
+    if (f0 < P(0)) du.penalty.x = fmin_(du.penalty.x + o.beta_lin * dabs(c0), o.penalty_max);
+    if (tm <= bounds) {
+        du.penalty.y = fmin_(du.penalty.y + o.beta_lin * dabs(c1), o.penalty_max);
+        du.penalty.z = fmin_(du.penalty.z + o.beta_lin * dabs(c2), o.penalty_max);
+    }
+    return du;
+}
 // A group of up to 32 bodies by one warp, for bodies with contact rows.  A
 // thread per body walks its rows one dependent gather and one chain of sums
 // after another (about 900 cycles a row), so the warp lasts as long as its
@@ -611,27 +688,28 @@ __host__ __device__ constexpr size_t primal_group_smem() {
     return (size_t)kPrimalGroupWarps * primal_group_words<R>() * sizeof(R);
 }
 
-// Bodies list[0 .. nb) (dynamic ones, nb <= 32), all lanes of the warp;
-// stage: the warp's primal_group_words<R>() words of shared memory.
-template <class P, class R, class F>
-__device__ __forceinline__ void primal_group(const DevWorld<P, R>& w, const uint32_t* list, uint32_t nb,
+// Bodies t0 .. t0 + nb of `bodies` (dynamic ones, nb <= 32), all lanes of the
+// warp; stage: the warp's primal_group_words<R>() words of shared memory
+// (kStaged false: none, rows always serial).
+template <bool kStaged, class P, class R, class F, class S>
+__device__ __forceinline__ void primal_group(const DevWorld<P, R>& w, const S& bodies, uint32_t t0, uint32_t nb,
                                              const SolveParams<R>& o, const F& fetch, R* stage, uint32_t lane) {
     constexpr uint32_t kAll = 0xFFFFFFFFu;
     R* const sums = stage + 32 * kGroupStage;  // [body][27]
     const bool live = lane < nb;
-    uint32_t i = 0, j0 = 0, n = 0;
+    BodyTask<P, R> task;
+    task.i = task.j0 = task.n = 0;
     V3<P> sp{P(0), P(0), P(0)};
     Q4<P> sq{P(0), P(0), P(0), P(1)};
     Block6<R> B;
     if (live) {
-        i = list[lane];
-        j0 = w.row_off[i];
-        n = w.row_off[i + 1] - j0;
-        sp = xyz(fetch.pos(i));
-        sq = quat(fetch.rot(i));
+        task = bodies.load(t0 + lane);
+        sp = xyz(fetch.pos(task.i));
+        sq = quat(fetch.rot(task.i));
     }
     const Q4<R> sqr = castq<R>(sq);
-    if (live) primal_inertia(w, i, A4<R>{}, sp, sqr, o, B);
+    if (live) primal_inertia(task, sp, sqr, B);
+    const uint32_t i = task.i, j0 = task.j0, n = task.n;
     uint32_t incl = n;  // inclusive sums of the row counts
 #pragma unroll
     for (int off = 1; off < 32; off <<= 1) {
@@ -646,7 +724,7 @@ __device__ __forceinline__ void primal_group(const DevWorld<P, R>& w, const uint
             dqsl = cast3<R>(sub(sp, xyz(fetch.ipos(i))));
             dqsa = ang_diff(sqr, castq<R>(quat(fetch.irot(i))));
         }
-        if (__reduce_max_sync(kAll, n) <= kGroupSerial * ((total + 31u) / 32u)) {
+        if (!kStaged || __reduce_max_sync(kAll, n) <= kGroupSerial * ((total + 31u) / 32u)) {
             for (uint32_t j = j0; j < j0 + n; ++j)
                 primal_row_f(w, w.row_idx[j], w.row_oth[j], fetch, sqr, dqsl, dqsa, k_alpha, B);
         } else {
@@ -656,9 +734,11 @@ __device__ __forceinline__ void primal_group(const DevWorld<P, R>& w, const uint
 #pragma unroll
                 for (int e = 0; e < 6; ++e) sums[lane * kGroupSums + 21 + e] = B.g[e];
             }
-            // lane e's entry: H[ra][rb] (product J[ra] J[rb] k) or g[ra] (J[ra] f)
+            // lane e's entry: H[ra][rb] (product J[ra] J[rb] k) or g[ra]
+            // (J[ra] f 1, the 1 at the stride's last word)
             const bool is_h = lane < 21u;
             uint32_t ra = 0, rb = 7;
+            stage[lane * kGroupStage + 24] = R(1);
             if (is_h) {
                 while ((ra + 1) * (ra + 2) / 2 <= lane) ++ra;
                 rb = lane - ra * (ra + 1) / 2;
@@ -701,14 +781,15 @@ __device__ __forceinline__ void primal_group(const DevWorld<P, R>& w, const uint
                     const uint32_t q0 = max(end - cb, base) - base, q1 = min(end - base, cnt);
                     if (cb && lane < (uint32_t)kGroupSums) {
                         R acc = sums[b * kGroupSums + lane];
+#pragma unroll 4
                         for (uint32_t t = q0; t < q1; ++t) {
                             const R* p = stage + t * kGroupStage;
+                            R v[3];
 #pragma unroll
-                            for (int u = 0; u < 3; ++u) {
-                                const R v = p[u * 8 + ra] * p[u * 8 + rb];
-                                const R vk = v * p[u * 8 + 6];
-                                acc = acc + (is_h ? vk : v);
-                            }
+                            for (uint32_t u = 0; u < 3; ++u)
+                                v[u] = p[u * 8 + ra] * p[u * 8 + rb] * p[is_h ? u * 8 + 6 : 24];
+#pragma unroll
+                            for (uint32_t u = 0; u < 3; ++u) acc = acc + v[u];
                         }
                         sums[b * kGroupSums + lane] = acc;
                     }
@@ -725,10 +806,15 @@ __device__ __forceinline__ void primal_group(const DevWorld<P, R>& w, const uint
         }
     }
     if (live) {
-        const uint32_t k0 = w.n_joints ? w.joint_off[i] : 0u, k1 = w.n_joints ? w.joint_off[i + 1] : 0u;
-        primal_finish(w, i, k0, k1, fetch, sp, sq, sqr, B);
+        primal_finish(bodies, t0 + lane, i, fetch, sp, sq, sqr, B);
     }
 }
+
+// Worlds of jointed bodies: they carry few rows, and their joints are spread
+// evenly by the list's order, so a thread per body is the better shape (the
+// 257-scene split batch: 2.21 ms a pass against 2.27 in groups).
+template <class P, class R>
+inline bool mostly_jointed(const DevWorld<P, R>& w) { return (uint64_t)w.n_joints * 2 > w.n_dyn; }
 
 // Bodies per warp: all 32 lanes once that gives every SM 12 warps, fewer
 // (down to one) in smaller worlds, which would leave SMs idle.
@@ -745,7 +831,7 @@ __device__ __forceinline__ void primal_groups(const DevWorld<P, R>& w, const uin
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     R* stage = reinterpret_cast<R*>(primal_group_smem_raw) + warp * primal_group_words<R>();
     for (uint32_t t = (blockIdx.x * kPrimalGroupWarps + warp) * g; t < n; t += gridDim.x * kPrimalGroupWarps * g)
-        primal_group(w, list + t, min(g, n - t), o, fetch, stage, lane);
+        primal_group<true>(w, WorldBodies<P, R>{w, list}, t, min(g, n - t), o, fetch, stage, lane);
 }
 template <class P, class R>
 __global__ void __launch_bounds__(kPrimalGroupWarps * 32, sizeof(R) == 4 ? 4 : 2)
@@ -783,10 +869,7 @@ inline void launch_primal(int variant, bool pdl, const DevWorld<P, R>& w, int rd
             launch_k(pdl, k_primal<P, R, 256, 3>, grid(256), 256, 0, s, w, rd, wr, o);
             break;
         case 5:
-            // jointed bodies carry few rows and their joints are spread
-            // evenly by the list's order: a thread per body with 20 warps an
-            // SM (the 257-scene split batch: 2.21 ms against 2.27 in groups)
-            if ((uint64_t)w.n_joints * 2 > nd)
+            if (mostly_jointed(w))
                 launch_k(pdl, k_primal<P, R, 64, 10>, grid(64), 64, 0, s, w, rd, wr, o);
             else
                 group(primal_group_size(nd, sms));
@@ -826,61 +909,35 @@ struct InPlaceFetch {
     }
 };
 
-// Coloured Gauss-Seidel sweep: bodies color_order[c0 .. c1) in place.
+// Coloured Gauss-Seidel sweep: bodies color_order[c0 .. c1) in place, grouped
+// or (worlds of jointed bodies, as in launch_primal) a thread each.
 template <class P, class R>
 __global__ void __launch_bounds__(kPrimalGroupWarps * 32, sizeof(R) == 4 ? 4 : 2)
     k_primal_color(DevWorld<P, R> w, uint32_t c0, uint32_t c1, uint32_t g, SolveParams<R> o) {
     primal_groups(w, w.color_order + c0, c1 - c0, g, o, InPlaceFetch<P, R>{w});
 }
-
-// avbd_dual, avbd/src/lib.rs:565-663: the row's dual update from its bodies' new poses (a, and b unless the
-// row is against a container) and step-start poses.
 template <class P, class R>
-__device__ __forceinline__ RowDual<P, R> dual_update(const RowStatic<R>& rs, RowDual<P, R> du, A4<P> pa4, A4<P> qa4,
-                                                     A4<P> ia_p, A4<P> ia_q, bool has_b, A4<P> pb4, A4<P> qb4,
-                                                     A4<P> ib_p, A4<P> ib_q, const SolveParams<R>& o) {
-    V3<R> dal = cast3<R>(sub(xyz(pa4), xyz(ia_p)));
-    V3<R> daa = ang_diff(castq<R>(quat(qa4)), castq<R>(quat(ia_q)));
-    V3<R> dbl{R(0), R(0), R(0)}, dba{R(0), R(0), R(0)}, rbw{R(0), R(0), R(0)};
-    if (has_b) {
-        dbl = cast3<R>(sub(xyz(pb4), xyz(ib_p)));
-        dba = ang_diff(castq<R>(quat(qb4)), castq<R>(quat(ib_q)));
-        rbw = rotate(castq<R>(quat(qb4)), xyz(rs.rb));
-    }
-    V3<R> raw = rotate(castq<R>(quat(qa4)), xyz(rs.ra));
-    V3<R> r0 = xyz(rs.n), r1 = xyz(rs.t1), r2 = xyz(rs.t2);
-    const R k_alpha = R(1) - o.alpha;
-    R c0 = rs.ra.w * k_alpha, c1 = rs.rb.w * k_alpha, c2 = rs.t1.w * k_alpha;
-    c0 = c0 + (dot(r0, dal) + dot(cross(raw, r0), daa) - dot(r0, dbl) - dot(cross(rbw, r0), dba));
-    c1 = c1 + (dot(r1, dal) + dot(cross(raw, r1), daa) - dot(r1, dbl) - dot(cross(rbw, r1), dba));
-    c2 = c2 + (dot(r2, dal) + dot(cross(raw, r2), daa) - dot(r2, dbl) - dot(cross(rbw, r2), dba));
-    P f0, f1, f2, tm, bounds;
-    row_forces(du, rs.n.w, c0, c1, c2, f0, f1, f2, tm, bounds);
-    du.lambda.x = f0;
-    du.lambda.y = f1;
-    du.lambda.z = f2;
-    if (f0 < P(0)) du.penalty.x = fmin_(du.penalty.x + o.beta_lin * dabs(c0), o.penalty_max);
-    if (tm <= bounds) {
-        du.penalty.y = fmin_(du.penalty.y + o.beta_lin * dabs(c1), o.penalty_max);
-        du.penalty.z = fmin_(du.penalty.z + o.beta_lin * dabs(c2), o.penalty_max);
-    }
-    return du;
+__global__ void __launch_bounds__(128)
+    k_primal_color_bodies(DevWorld<P, R> w, uint32_t c0, uint32_t c1, SolveParams<R> o) {
+    for (uint32_t t = c0 + blockIdx.x * blockDim.x + threadIdx.x; t < c1; t += gridDim.x * blockDim.x)
+        primal_body_f(w, w.color_order[t], o, InPlaceFetch<P, R>{w});
 }
-// avbd_dual, avbd/src/lib.rs:565-663, for row c of `rd`: new duals into
-// `out`; `fetch` reads the new state.
-template <class P, class R, class F>
-__device__ __forceinline__ void dual_row_io(const DevWorld<P, R>& w, uint32_t c, const F& fetch,
-                                            const RowDual<P, R>* rd, RowDual<P, R>* out, const SolveParams<R>& o) {
-    const uint2 ab = w.ab[c];
-    const bool has_b = ab.y != kContainer;
-    const uint32_t b = has_b ? ab.y : ab.x;
-    out[c] = dual_update<P, R>(w.rs[c], rd[c], fetch.pos(ab.x), fetch.rot(ab.x), fetch.ipos(ab.x),
-                               fetch.irot(ab.x), has_b, fetch.pos(b), fetch.rot(b), fetch.ipos(b), fetch.irot(b), o);
-}
+
+// avbd_dual, avbd/src/lib.rs:565-663, for row c; `fetch` reads the new state.
 template <class P, class R, class F>
 __device__ __forceinline__ void dual_row_f(const DevWorld<P, R>& w, uint32_t c, const F& fetch,
                                            const SolveParams<R>& o) {
-    dual_row_io(w, c, fetch, w.rd, w.rd, o);
+    const uint2 ab = w.ab[c];
+    const bool has_b = ab.y != kContainer;
+    A4<P> pb{}, qb{}, ib{}, jb{};
+    if (has_b) {
+        pb = fetch.pos(ab.y);
+        qb = fetch.rot(ab.y);
+        ib = fetch.ipos(ab.y);
+        jb = fetch.irot(ab.y);
+    }
+    w.rd.put(c, dual_update<P, R>(w.rs[c], w.rd[c], fetch.pos(ab.x), fetch.rot(ab.x), fetch.ipos(ab.x),
+                                  fetch.irot(ab.x), has_b, pb, qb, ib, jb, o));
 }
 template <class P, class R>
 __device__ __forceinline__ void dual_row(const DevWorld<P, R>& w, uint32_t c, int rd, const SolveParams<R>& o) {

@@ -1,5 +1,5 @@
-// k_chunk.cuh -- the whole AVBD solve of a step in one launch: one CTA per
-// chunk of consecutive scenes, poses resident in shared memory.
+// k_chunk.cuh -- the whole AVBD solve of a step in one launch: one cluster of
+// CTAs per chunk of consecutive scenes, poses resident in shared memory.
 //
 // The reference dispatches init, then (primal, dual) x iterations, then
 // recover as separate compute passes over every body and contact
@@ -7,25 +7,21 @@
 // every pose and row.  Scenes never couple -- rows and joints stay inside a
 // scene -- so a chunk of whole scenes can run its whole schedule alone: its
 // snapshot / new poses (both Jacobi parities) and step-start poses live in
-// shared memory, the phases are separated by __syncthreads, and only the
-// rows, joint views and per-body constants stream from L1 / L2 / HBM.  Each phase
-// evaluates exactly the expressions of the per-phase kernels (the same
-// device functions, reading shared instead of global memory), so the result
-// is bit-identical to init, 10 x (primal, dual), recover launched one by one.
+// the shared memory of the cluster's CTAs, the phases are separated by
+// cluster barriers, and only the rows, joint views and per-body constants
+// stream from L1 / L2 / HBM.  Each phase evaluates exactly the expressions of
+// the per-phase kernels, so the result is bit-identical to init, 10 x
+// (primal, dual), recover launched one by one.
 //
-// Shared memory per body: pos[2], rot[2], init pos, init rot = 6 x A4<P>
-// (96 B at FP32, 192 B at FP64 poses); a chunk holds at most
-// solve_chunk_cap<P>() bodies (2048 / 1024), one CTA per SM.  The host packs
-// scenes into chunks so that the chunks fill whole waves of the GPU's SMs.
-// (Measured and dropped: 64 B per body with the step-start poses read from
-// global memory, which let one wave of 152 chunks of up to 3391 bodies hold
-// the bench batch, ran the solve 0.48 -> 0.59 ms: the step-start reads of
-// contact rows and the smaller L1 cost more than the wave saved.  Also
-// measured and dropped: forming each row's dual inside the next iteration's
-// primal -- bit-identical, one barrier per iteration instead of two, duals
-// of pair rows formed by both endpoints, a second dual buffer -- which ran
-// 0.48 -> 0.59 ms (640 threads) and 0.50 -> 0.54 ms (512): the extra work
-// and spills in the primal cost more than the barrier saved.)
+// A chunk's bodies are dealt to its CTAs in blocks of 2^blk consecutive
+// bodies, round robin: chains and nearby boxes stay in one CTA for the most
+// part (their poses are read from its own shared memory, others' through
+// distributed shared memory), and a scene's loose boxes, which carry the
+// contact rows and follow its chains, are spread over all of them.  Rows are
+// dealt evenly for the dual.  One CTA for the whole chunk (the layout before)
+// bounded a step by its largest scene: 2,000 bodies are four rounds of 512
+// threads an iteration, whatever else the GPU has free; and a CTA that fills
+// an SM leaves it idle at every barrier.
 #pragma once
 
 #include "k_avbd.cuh"
@@ -33,22 +29,145 @@
 
 namespace dio {
 
-// threads per CTA: 512 (128 registers, no spill) or 640 (96 registers)
-constexpr int kChunkThreads = 512;
-constexpr int kChunkThreadsWide = 640;
+// Spread: a cluster of 256-thread CTAs a chunk, two CTAs an SM at 128
+// registers (FP64: one), rows staged (grouped primal).  Packed, for worlds
+// that fill the GPU several times over: one CTA a chunk, 512 threads (FP64
+// 256), the whole SM; a __syncthreads between phases keeps L1, which a
+// cluster barrier's acquire empties (measured: a dependent load after it
+// takes 266 cycles against 38, the barrier itself 500 cycles, 1,100-1,600
+// with a global store in flight).
+template <class R, bool kSpread>
+__host__ __device__ constexpr int chunk_threads() {
+    return sizeof(R) == 4 && !kSpread ? 512 : 256;
+}
+constexpr uint32_t kMaxClusterShift = 3;  // up to 8 CTAs (the portable cluster size)
 
-template <class P>
+// shared memory of a CTA holding `cap` bodies: pos[2], rot[2], step-start pos
+// and rot (spread: then each warp's staging of the grouped primal), and the
+// groups' first bodies
+template <class R>
+__host__ __device__ constexpr size_t spread_stage_words() {
+    return chunk_threads<R, true>() / 32 * primal_group_words<R>();
+}
+template <class P, class R, bool kSpread>
 __host__ __device__ constexpr size_t chunk_smem_bytes(uint32_t cap) {
-    return (size_t)6 * cap * sizeof(A4<P>);
+    return (size_t)6 * cap * sizeof(A4<P>) + (kSpread ? spread_stage_words<R>() * sizeof(R) : 0) + (size_t)cap * 2;
 }
-// bodies of a chunk: its poses fill at most 192 KB of shared memory
-template <class P>
-__host__ __device__ constexpr uint32_t solve_chunk_cap() {
-    return sizeof(P) == 4 ? 2048u : 1024u;
+// coloured: one pose buffer (the sweeps are in place), colour, order and
+// selection arrays
+template <class P, class R, bool kSpread>
+__host__ __device__ constexpr size_t chunk_colored_smem_bytes(uint32_t cap) {
+    return (size_t)4 * cap * sizeof(A4<P>) + (kSpread ? spread_stage_words<R>() * sizeof(R) : 0) + (size_t)cap * 12 +
+           (size_t)2 * (kMaxColors + 1) * 4;
 }
-static_assert(chunk_smem_bytes<float>(solve_chunk_cap<float>()) <= 200u * 1024u &&
-                  chunk_smem_bytes<double>(solve_chunk_cap<double>()) <= 200u * 1024u,
-              "scene-chunk poses must fit a CTA's shared memory");
+// bodies of a chunk over all its CTAs, and of a CTA at most
+constexpr uint32_t kSolveChunkCap = 2048;
+template <class P, bool kSpread>
+__host__ __device__ constexpr uint32_t solve_cta_cap() {
+    return (sizeof(P) == 4 ? 2048u : 1024u) / (kSpread ? 2u : 1u);
+}
+template <class P, class R, bool kSpread>
+constexpr bool chunk_fits() {
+    return chunk_smem_bytes<P, R, kSpread>(solve_cta_cap<P, kSpread>()) <= 227u * 1024u &&
+           chunk_colored_smem_bytes<P, R, kSpread>(solve_cta_cap<P, kSpread>()) <= 227u * 1024u &&
+           (solve_cta_cap<P, kSpread>() << kMaxClusterShift) >= kSolveChunkCap &&
+           solve_cta_cap<P, kSpread>() <= 4u * chunk_threads<R, kSpread>();  // cta_scan4
+}
+static_assert(chunk_fits<float, float, true>() && chunk_fits<float, float, false>() &&
+                  chunk_fits<double, float, true>() && chunk_fits<double, float, false>() &&
+                  chunk_fits<double, double, true>() && chunk_fits<double, double, false>(),
+              "scene-chunk poses must fit the CTAs' shared memory");
+
+// How a chunk is dealt: 2^cl CTAs, blocks of 2^blk bodies.
+struct SolveShape {
+    uint32_t cl, blk;
+    __host__ __device__ uint32_t owner(uint32_t d) const { return (d >> blk) & ((1u << cl) - 1u); }
+    __host__ __device__ uint32_t slot(uint32_t d) const {
+        return ((d >> (blk + cl)) << blk) | (d & ((1u << blk) - 1u));
+    }
+    // chunk position of slot s of CTA `rank`
+    __host__ __device__ uint32_t body(uint32_t s, uint32_t rank) const {
+        return ((s >> blk) << (blk + cl)) | (rank << blk) | (s & ((1u << blk) - 1u));
+    }
+    // slots of a CTA of a chunk of nb bodies
+    __host__ __device__ uint32_t slots(uint32_t nb) const {
+        return ((nb + (1u << (blk + cl)) - 1u) >> (blk + cl)) << blk;
+    }
+};
+
+__device__ __forceinline__ uint32_t cta_smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+// another CTA's shared memory at the address that p has in this CTA
+__device__ __forceinline__ uint32_t peer_addr(const void* p, uint32_t rank) {
+    uint32_t a;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(cta_smem_addr(p)), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ A4<float> peer_load(const A4<float>* p, uint32_t rank) {
+    A4<float> v;
+    asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                 : "r"(peer_addr(p, rank)));
+    return v;
+}
+__device__ __forceinline__ A4<double> peer_load(const A4<double>* p, uint32_t rank) {
+    A4<double> v;
+    const uint32_t a = peer_addr(p, rank);
+    asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "r"(a));
+    asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];" : "=d"(v.z), "=d"(v.w) : "r"(a + 16u));
+    return v;
+}
+__device__ __forceinline__ uint32_t peer_load(const uint32_t* p, uint32_t rank) {
+    uint32_t v;
+    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(peer_addr(p, rank)));
+    return v;
+}
+// barrier over the chunk's CTAs; orders their shared and global memory (the
+// rows' duals are written by one CTA and read by others)
+template <bool kCluster>
+__device__ __forceinline__ void chunk_sync() {
+    if constexpr (kCluster) {
+        asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+    } else {
+        __syncthreads();
+    }
+}
+
+// Poses of a chunk in its CTAs' shared memory.  Every body a chunk's rows and
+// joints touch lies in the chunk (rows and joints never cross scenes).
+template <class P, bool kCluster>
+struct ChunkFetch {
+    const A4<P>* sp;  // snapshot (read) buffer
+    const A4<P>* sq;
+    const A4<P>* si;  // step-start pose
+    const A4<P>* sr;
+    A4<P>* wp;        // the primal's output buffer
+    A4<P>* wq;
+    uint32_t lo, rank;
+    SolveShape shape;
+    template <class T>
+    __device__ __forceinline__ T get(const T* a, uint32_t j) const {
+        const uint32_t d = j - lo;
+        if constexpr (kCluster) {
+            const uint32_t own = shape.owner(d), s = shape.slot(d);
+            return own == rank ? a[s] : peer_load(a + s, own);
+        } else {
+            return a[d];
+        }
+    }
+    __device__ __forceinline__ A4<P> pos(uint32_t j) const { return get(sp, j); }
+    __device__ __forceinline__ A4<P> rot(uint32_t j) const { return get(sq, j); }
+    __device__ __forceinline__ A4<P> ipos(uint32_t j) const { return get(si, j); }
+    __device__ __forceinline__ A4<P> irot(uint32_t j) const { return get(sr, j); }
+    // a body of this CTA: its new pose, once stored
+    __device__ __forceinline__ A4<P> new_pos(uint32_t i) const { return wp[kCluster ? shape.slot(i - lo) : i - lo]; }
+    __device__ __forceinline__ A4<P> new_rot(uint32_t i) const { return wq[kCluster ? shape.slot(i - lo) : i - lo]; }
+    __device__ __forceinline__ void store(uint32_t i, A4<P> p, A4<P> q) const {
+        const uint32_t s = kCluster ? shape.slot(i - lo) : i - lo;
+        wp[s] = p;
+        wq[s] = q;
+    }
+};
 
 // First index r in [s0, s1) with ab[r].x >= key (ab sorted by .x there), or
 // s1; one warp, 32-way search (every lane must call it).
@@ -70,78 +189,229 @@ __device__ __forceinline__ uint32_t warp_lower_bound(const uint2* ab, uint32_t s
     return lo + __popc(__ballot_sync(0xFFFFFFFFu, less));
 }
 
-// One CTA per chunk (chunks[c] = scene range [x, y), bodies contiguous;
-// dyn_runs[c] = the chunk's run of the dynamic-body list, ordered by work
-// signature so a warp's bodies take the same code path).
-// `cap` is the shared-memory capacity in bodies (the largest chunk).  Rows of the chunk: its
-// pair rows are one range of the pair-row section (pairs sorted by body a,
-// scenes contiguous) and its container rows one range of the container
-// section (dynamic bodies in index order).
-template <class P, class R, int T>
-__global__ void __launch_bounds__(T, 1)
+// What a CTA of the solve works on: its chunk's bodies [lo, lo + nb) and its
+// run of the dynamic-body list, ordered by work signature (a warp's bodies
+// take the same code path).
+struct ChunkCta {
+    uint32_t lo, nb, rank;
+    uint2 dyn;
+    // the chunk's rows: a range of the pair-row section (pairs sorted by body
+    // a, scenes contiguous) and one of the container section (dynamic bodies
+    // in index order)
+    uint32_t p0, np, c0, rows;
+    __device__ __forceinline__ uint32_t row(uint32_t t) const { return t < np ? p0 + t : c0 + (t - np); }
+};
+__device__ __forceinline__ ChunkCta chunk_cta(const uint2* chunks, const uint2* dyn_runs, const SceneDesc* scenes,
+                                              const SolveShape& shape) {
+    ChunkCta c;
+    const uint2 ch = chunks[blockIdx.x >> shape.cl];
+    c.rank = blockIdx.x & ((1u << shape.cl) - 1u);  // clusters run along x
+    c.dyn = dyn_runs[blockIdx.x];
+    c.lo = scenes[ch.x].body_lo;
+    c.nb = scenes[ch.y - 1].body_hi - c.lo;
+    c.p0 = c.np = c.c0 = c.rows = 0;
+    return c;
+}
+// the rows' four bounds, a warp each, into s_rows (read after the next barrier)
+__device__ __forceinline__ void chunk_row_bounds(const uint2* ab, const Counters* ctr, const ChunkCta& c,
+                                                 uint32_t* s_rows) {
+    const uint32_t warp = threadIdx.x >> 5;
+    if (warp < 4) {
+        const uint32_t m = ctr->rows, split = min(ctr->pair_rows, m);
+        const uint32_t r = warp_lower_bound(ab, warp < 2 ? 0u : split, warp < 2 ? split : m,
+                                            (warp & 1) ? c.lo + c.nb : c.lo);
+        if ((threadIdx.x & 31) == 0) s_rows[warp] = r;
+    }
+}
+__device__ __forceinline__ void take_row_bounds(ChunkCta& c, const uint32_t* s_rows) {
+    c.p0 = s_rows[0];
+    c.np = s_rows[1] - s_rows[0];
+    c.c0 = s_rows[2];
+    c.rows = c.np + (s_rows[3] - s_rows[2]);
+}
+
+// Exclusive sums of four values a thread (thread-major order) over the CTA;
+// returns the total.  s_warp: a word a warp.
+__device__ __forceinline__ uint32_t cta_scan4(uint32_t (&v)[4], uint32_t* s_warp) {
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t mine = v[0] + v[1] + v[2] + v[3];
+    uint32_t x = mine;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, off);
+        if (lane >= (uint32_t)off) x += y;
+    }
+    __syncthreads();
+    if (lane == 31u) s_warp[warp] = x;
+    __syncthreads();
+    uint32_t before = 0, total = 0;
+    for (uint32_t k = 0; k < blockDim.x / 32u; ++k) {
+        if (k < warp) before += s_warp[k];
+        total += s_warp[k];
+    }
+    uint32_t run = before + x - mine;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const uint32_t t = v[k];
+        v[k] = run;
+        run += t;
+    }
+    return total;
+}
+
+// The CTA's bodies cut into groups for its warps: at most 32 bodies and
+// about `per` incidences -- as few as four when there are warps enough (each
+// body's rows are a chain of sums), twice as many until every warp has one
+// group.  Bodies without rows are not split up: they fill 32 lanes.  Packed
+// CTAs have more groups than warps anyway: 128 incidences, four a body.  The
+// cut is made once a step (the rows do not change within it).  first[k]: the
+// group's first body, from c.dyn.x; returns the number of groups.
+template <bool kSpread, class P, class R>
+__device__ __forceinline__ uint32_t chunk_groups(const DevWorld<P, R>& w, const ChunkCta& c, uint16_t* first,
+                                                 uint32_t* s_warp) {
+    const uint32_t n = c.dyn.y - c.dyn.x, warps = blockDim.x / 32u, u0 = threadIdx.x * 4u;
+    uint32_t rows[4];
+#pragma unroll
+    for (int k = 0; k < 4; ++k) rows[k] = u0 + k < n ? w.solve.rows[c.dyn.x + u0 + k].y : 0u;
+    // a body's share of a group in units of 1 / (32 per)
+    uint32_t per = kSpread ? 4u : 128u;
+    auto share = [&](uint32_t r) { return max(min(r, per) * 32u, per); };
+    uint32_t sums[4];
+    for (;; per *= 2u) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) sums[k] = u0 + k < n ? share(rows[k]) : 0u;
+        const uint32_t total = cta_scan4(sums, s_warp);
+        if (!kSpread || total <= warps * 32u * per || per >= 4096u) break;
+    }
+    // a body's group: its sum over 32 per
+    uint32_t starts[4], last = 0xFFFFFFFFu;
+    if (u0 && u0 <= n) {  // the body before this thread's first
+        const uint32_t r = w.solve.rows[c.dyn.x + u0 - 1u].y;
+        last = (sums[0] - share(r)) / (32u * per);
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        starts[k] = u0 + k < n && sums[k] / (32u * per) != last ? 1u : 0u;
+        last = sums[k] / (32u * per);
+    }
+    uint32_t at[4] = {starts[0], starts[1], starts[2], starts[3]};
+    const uint32_t groups = cta_scan4(at, s_warp);
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+        if (starts[k]) first[at[k]] = (uint16_t)(u0 + k);
+    return groups;
+}
+
+// The primal of `groups` groups by the CTA's warps, taken from the end
+// through a shared cursor: the end of a CTA's run holds the bodies without
+// joints, whose contact rows make them the longest.  range(k, t, n): group
+// k's first position and bodies.
+template <bool kSpread, class P, class R, class F, class S, class Range>
+__device__ __forceinline__ void chunk_primal(const DevWorld<P, R>& w, const S& bodies, uint32_t groups, Range&& range,
+                                             const SolveParams<R>& o, const F& fetch, R* stage, uint32_t* cursor) {
+    const uint32_t lane = threadIdx.x & 31u;
+    for (;;) {
+        uint32_t k = 0;
+        if (lane == 0) k = atomicAdd(cursor, 1u);
+        k = __shfl_sync(0xFFFFFFFFu, k, 0);
+        if (k >= groups) break;
+        uint32_t t, n;
+        range(groups - 1u - k, t, n);
+        primal_group<kSpread>(w, bodies, t, n, o, fetch, stage, lane);
+    }
+}
+
+// avbd_init for the CTA's bodies: `put(slot, InitPose)` for each.  Dynamic
+// bodies leave their constants and row lists at their list positions.
+template <class P, class R, class Put>
+__device__ __forceinline__ void chunk_init(const DevWorld<P, R>& w, const ChunkCta& c, const SolveShape& shape,
+                                           const SolveParams<R>& o, Put&& put) {
+    for (uint32_t s = threadIdx.x; s < shape.slots(c.nb); s += blockDim.x) {
+        const uint32_t d = shape.body(s, c.rank);
+        if (d >= c.nb) continue;
+        const uint32_t i = c.lo + d;
+        if (w.inv[i].w != R(0)) continue;
+        InitPose<P> r;
+        r.start_pos = r.pos = w.pos[0][i];
+        r.start_rot = r.rot = w.rot[0][i];
+        r.start_pos.w = P(0);
+        put(s, r);
+    }
+    for (uint32_t t = c.dyn.x + threadIdx.x; t < c.dyn.y; t += blockDim.x) {
+        const uint32_t i = w.dyn_list[t];
+        put(shape.slot(i - c.lo), init_pose(w, i, t, o));
+        const uint32_t j0 = w.row_off[i];
+        w.solve.rows[t] = make_uint2(j0, w.row_off[i + 1] - j0);
+    }
+}
+
+// One cluster per chunk (chunks[c] = scene range [x, y), bodies contiguous;
+// dyn_runs[c 2^cl + rank] = a CTA's run of the dynamic-body list).  `cap`:
+// bodies a CTA's shared memory holds (the largest chunk's slots).
+template <class P, class R, bool kSpread, bool kCluster>
+__global__ void __launch_bounds__(chunk_threads<R, kSpread>(), sizeof(R) == 4 && kSpread ? 2 : 1)
     k_solve_chunks(DevWorld<P, R> w, const uint2* chunks, const uint2* dyn_runs, const SceneDesc* scenes, uint32_t cap,
-                   SolveParams<R> o) {
+                   SolveShape shape, SolveParams<R> o) {
     extern __shared__ __align__(16) unsigned char chunk_smem[];
     __shared__ uint32_t s_rows[4];
+    __shared__ uint32_t s_cursor[2];
+    __shared__ uint32_t s_warp[chunk_threads<R, kSpread>() / 32];
     pdl_enter();
     // layout: pos parity 0, pos parity 1, rot parity 0, rot parity 1, step
-    // start pos, step start rot (parity b at s_pos + b * cap)
+    // start pos, step start rot (parity b at s_pos + b * cap), staging
     A4<P>* const s_pos = reinterpret_cast<A4<P>*>(chunk_smem);
     A4<P>* const s_rot = s_pos + 2 * cap;
     A4<P>* const s_ipos = s_pos + 4 * cap;
     A4<P>* const s_irot = s_pos + 5 * cap;
-    const uint2 ch = chunks[blockIdx.x];
-    const uint2 dr = dyn_runs[blockIdx.x];  // the chunk's dynamic bodies: w.dyn_list[dr.x, dr.y)
-    const uint32_t lo = scenes[ch.x].body_lo, hi = scenes[ch.y - 1].body_hi;
     const uint32_t tid = threadIdx.x, nt = blockDim.x;
-
-    // the chunk's row ranges, one warp per bound
-    const uint32_t warp = tid >> 5;
-    if (warp < 4) {
-        const uint32_t m = w.ctr->rows;
-        const uint32_t split = min(w.ctr->pair_rows, m);
-        const uint32_t s0 = warp < 2 ? 0u : split, s1 = warp < 2 ? split : m;
-        const uint32_t r = warp_lower_bound(w.ab, s0, s1, (warp & 1) ? hi : lo);
-        if ((tid & 31) == 0) s_rows[warp] = r;
-    }
-    // avbd_init for the chunk's bodies (global state as the per-phase kernel
-    // leaves it), then the poses of both parities and the step start into
-    // shared memory: the same thread writes and reads a body's records
-    for (uint32_t i = lo + tid; i < hi; i += nt) {
-        init_body(w, i, o);
-        s_pos[i - lo] = w.pos[0][i];
-        s_rot[i - lo] = w.rot[0][i];
-        s_pos[cap + i - lo] = w.pos[1][i];
-        s_rot[cap + i - lo] = w.rot[1][i];
-        s_ipos[i - lo] = w.init_pos[i];
-        s_irot[i - lo] = w.init_rot[i];
-    }
+    R* const stage0 = reinterpret_cast<R*>(s_pos + 6 * cap);
+    R* const stage = stage0 + (kSpread ? (tid >> 5) * primal_group_words<R>() : 0);
+    uint16_t* const s_first = reinterpret_cast<uint16_t*>(stage0 + (kSpread ? spread_stage_words<R>() : 0));
+    ChunkCta c = chunk_cta(chunks, dyn_runs, scenes, shape);
+    chunk_row_bounds(w.ab, w.ctr, c, s_rows);
+    if (tid < 2) s_cursor[tid] = 0u;
+    // the poses of both parities and the step start into shared memory
+    chunk_init(w, c, shape, o, [&](uint32_t s, const InitPose<P>& ip) {
+        s_pos[s] = ip.pos;
+        s_rot[s] = ip.rot;
+        s_pos[cap + s] = ip.start_pos;  // read for static bodies, and without any iteration
+        s_rot[cap + s] = ip.start_rot;
+        s_ipos[s] = ip.start_pos;
+        s_irot[s] = ip.start_rot;
+    });
+    chunk_sync<kCluster>();
+    take_row_bounds(c, s_rows);
+    const uint32_t groups = chunk_groups<kSpread>(w, c, s_first, s_warp);
     __syncthreads();
-    const uint32_t p0 = s_rows[0], p1 = s_rows[1], c0 = s_rows[2], c1 = s_rows[3];
-    const uint32_t np = p1 - p0, nrows = np + (c1 - c0);
+    auto range = [&](uint32_t k, uint32_t& t, uint32_t& n) {
+        const uint32_t u = s_first[k];
+        t = c.dyn.x + u;
+        n = (k + 1u < groups ? s_first[k + 1u] : c.dyn.y - c.dyn.x) - u;
+    };
+    using Fetch = ChunkFetch<P, kCluster>;
     for (uint32_t k = 0; k < o.iterations; ++k) {
         const uint32_t rd = (k & 1u) * cap, wr = cap - rd;
-        const SmemFetch<P> f{s_pos + rd, s_rot + rd, s_ipos, s_irot, s_pos + wr, s_rot + wr, lo};
-        for (uint32_t t = dr.x + tid; t < dr.y; t += nt) {
-            const uint32_t i = w.dyn_list[t];
-            const uint32_t k0 = w.n_joints ? w.joint_off[i] : 0u, k1 = w.n_joints ? w.joint_off[i + 1] : 0u;
-            primal_body_f(w, i, k0, k1, o, f);
-        }
-        __syncthreads();
-        const SmemFetch<P> fd{s_pos + wr, s_rot + wr, s_ipos, s_irot, nullptr, nullptr, lo};
-        for (uint32_t t = tid; t < nrows; t += nt) dual_row_f(w, t < np ? p0 + t : c0 + (t - np), fd, o);
-        __syncthreads();
+        if (tid == 0) s_cursor[(k + 1u) & 1u] = 0u;  // last used before the previous barrier
+        const Fetch f{s_pos + rd, s_rot + rd, s_ipos, s_irot, s_pos + wr, s_rot + wr, c.lo, c.rank, shape};
+        chunk_primal<kSpread>(w, ListBodies<P, R>{w}, groups, range, o, f, stage, &s_cursor[k & 1u]);
+        chunk_sync<kCluster>();
+        if (!c.rows) continue;  // the same for all CTAs of the chunk
+        const Fetch fd{s_pos + wr, s_rot + wr, s_ipos, s_irot, nullptr, nullptr, c.lo, c.rank, shape};
+        for (uint32_t t = c.rank * nt + tid; t < c.rows; t += nt << shape.cl) dual_row_f(w, c.row(t), fd, o);
+        chunk_sync<kCluster>();
     }
     // avbd_recover from the final parity, and the final pose into buffer 0
     const uint32_t fp = (o.iterations - 1u) % 2u;
     const uint32_t rb = fp == 0 ? 1u : 0u;
     const uint32_t fp_read = (o.iterations == 0 ? 0u : o.iterations - 1u) % 2u;
     const uint32_t final_buf = 1u - fp_read;
-    const SmemFetch<P> fr{s_pos + rb * cap, s_rot + rb * cap, s_ipos, s_irot, nullptr, nullptr, lo};
-    for (uint32_t i = lo + tid; i < hi; i += nt) {
-        recover_body_f(w, i, fr, o);
-        w.pos[0][i] = s_pos[final_buf * cap + i - lo];
-        w.rot[0][i] = s_rot[final_buf * cap + i - lo];
+    const Fetch fr{s_pos + rb * cap, s_rot + rb * cap, s_ipos, s_irot, nullptr, nullptr, c.lo, c.rank, shape};
+    for (uint32_t s = tid; s < shape.slots(c.nb); s += nt) {
+        const uint32_t d = shape.body(s, c.rank);
+        if (d >= c.nb) continue;
+        recover_body_f(w, c.lo + d, fr, o);
+        w.pos[0][c.lo + d] = s_pos[final_buf * cap + s];
+        w.rot[0][c.lo + d] = s_rot[final_buf * cap + s];
     }
 }
 
@@ -150,151 +420,176 @@ __global__ void __launch_bounds__(T, 1)
 // colours its own dynamic bodies (the Jones-Plassmann rounds of k_color.cuh
 // -- priority hash(index), ties by index, smallest colour free among the
 // coloured neighbours -- with the colours in shared memory and a barrier
-// between a round's selection and its assignment), sorts them by colour,
-// then runs init, per iteration one in-place primal sweep per colour
-// (barrier after each) and the dual, and recover.  One pose buffer (the
-// sweeps are in place): 4 x A4<P> per body plus colour, order and selection
-// arrays.  The colouring of a disconnected graph is the union of its
-// components' colourings, so per-chunk rounds give the colours of the
-// whole-world rounds; results equal the host-driven coloured step bit for
-// bit.
+// between a round's selection and its assignment); each CTA sorts its bodies
+// by colour, then the chunk runs init, per iteration one in-place primal
+// sweep per colour (barrier after each) and the dual, and recover.  One pose
+// buffer (the sweeps are in place).  The colouring of a disconnected graph is
+// the union of its components' colourings, so per-chunk rounds give the
+// colours of the whole-world rounds; results equal the host-driven coloured
+// step bit for bit.
 
-template <class P>
-__host__ __device__ constexpr size_t chunk_colored_smem_bytes(uint32_t cap) {
-    return (size_t)4 * cap * sizeof(A4<P>) + (size_t)cap * (4 + 4 + 4) + (size_t)2 * (kMaxColors + 1) * 4;
-}
+// list positions in the order of the colours
+template <class P, class R>
+struct OrderedBodies {
+    ListBodies<P, R> list;
+    const uint32_t* order;
+    __device__ __forceinline__ BodyTask<P, R> load(uint32_t k) const { return list.load(order[k]); }
+    __device__ __forceinline__ uint32_t joints(uint32_t k, uint32_t i) const { return list.joints(order[k], i); }
+    __device__ __forceinline__ JView joint(uint32_t k, uint32_t i, uint32_t q) const {
+        return list.joint(order[k], i, q);
+    }
+};
 
 constexpr uint32_t kChunkColorRounds = 4096;  // Jones-Plassmann rounds before giving up
 
-template <class P, class R, int T>
-__global__ void __launch_bounds__(T, 1)
+template <class P, class R, bool kSpread, bool kCluster>
+__global__ void __launch_bounds__(chunk_threads<R, kSpread>(), sizeof(R) == 4 && kSpread ? 2 : 1)
     k_solve_chunks_colored(DevWorld<P, R> w, const uint2* chunks, const uint2* dyn_runs, const SceneDesc* scenes,
-                           uint32_t cap, SolveParams<R> o) {
+                           uint32_t cap, SolveShape shape, SolveParams<R> o) {
     extern __shared__ __align__(16) unsigned char chunk_smem[];
     __shared__ uint32_t s_rows[4];
-    __shared__ uint32_t s_colored, s_ncolors;
+    __shared__ uint32_t s_cursor[2];
+    __shared__ uint32_t s_colored, s_ncolors, s_ndyn;
     pdl_enter();
     A4<P>* const s_pos = reinterpret_cast<A4<P>*>(chunk_smem);
     A4<P>* const s_rot = s_pos + cap;
     A4<P>* const s_ipos = s_pos + 2 * cap;
     A4<P>* const s_irot = s_pos + 3 * cap;
-    uint32_t* const s_color = reinterpret_cast<uint32_t*>(s_pos + 4 * cap);
+    const uint32_t tid = threadIdx.x, nt = blockDim.x;
+    R* const stage0 = reinterpret_cast<R*>(s_pos + 4 * cap);
+    R* const stage = stage0 + (kSpread ? (tid >> 5) * primal_group_words<R>() : 0);
+    uint32_t* const s_color =
+        reinterpret_cast<uint32_t*>(stage0 + (kSpread ? spread_stage_words<R>() : 0));
     uint32_t* const s_order = s_color + cap;
     uint32_t* const s_sel = s_order + cap;
-    uint32_t* const s_cstart = s_sel + cap;          // kMaxColors + 1
-    uint32_t* const s_cursor = s_cstart + kMaxColors + 1;
-    const uint2 ch = chunks[blockIdx.x];
-    const uint2 dr = dyn_runs[blockIdx.x];
-    const uint32_t lo = scenes[ch.x].body_lo, hi = scenes[ch.y - 1].body_hi;
-    const uint32_t tid = threadIdx.x, nt = blockDim.x;
-    const uint32_t warp = tid >> 5;
-    if (warp < 4) {
-        const uint32_t m = w.ctr->rows;
-        const uint32_t split = min(w.ctr->pair_rows, m);
-        const uint32_t s0 = warp < 2 ? 0u : split, s1 = warp < 2 ? split : m;
-        const uint32_t r = warp_lower_bound(w.ab, s0, s1, (warp & 1) ? hi : lo);
-        if ((tid & 31) == 0) s_rows[warp] = r;
-    }
+    uint32_t* const s_cstart = s_sel + cap;  // kMaxColors + 1
+    uint32_t* const s_next = s_cstart + kMaxColors + 1;
+    ChunkCta c = chunk_cta(chunks, dyn_runs, scenes, shape);
+    const uint32_t lo = c.lo, ndyn = c.dyn.y - c.dyn.x, ctas = 1u << shape.cl;
+    chunk_row_bounds(w.ab, w.ctr, c, s_rows);
     if (tid == 0) {
         s_colored = 0;
         s_ncolors = 0;
+        s_ndyn = ndyn;
     }
-    for (uint32_t c = tid; c <= kMaxColors; c += nt) {
-        s_cstart[c] = 0;
-        s_cursor[c] = 0;
+    if (tid < 2) s_cursor[tid] = 0u;
+    for (uint32_t q = tid; q <= kMaxColors; q += nt) {
+        s_cstart[q] = 0;
+        s_next[q] = 0;
     }
-    // init (the in-place schedule reads and writes buffer 0) and colours reset
-    for (uint32_t i = lo + tid; i < hi; i += nt) {
-        init_body(w, i, o);
-        s_pos[i - lo] = w.pos[0][i];
-        s_rot[i - lo] = w.rot[0][i];
-        s_ipos[i - lo] = w.init_pos[i];
-        s_irot[i - lo] = w.init_rot[i];
-        s_color[i - lo] = kNoColor;
-    }
-    __syncthreads();
+    // init (the in-place schedule reads and writes one buffer) and colours reset
+    chunk_init(w, c, shape, o, [&](uint32_t s, const InitPose<P>& ip) {
+        s_pos[s] = ip.pos;
+        s_rot[s] = ip.rot;
+        s_ipos[s] = ip.start_pos;
+        s_irot[s] = ip.start_rot;
+        s_color[s] = kNoColor;
+    });
+    chunk_sync<kCluster>();
+    const ChunkFetch<P, kCluster> f{s_pos, s_rot, s_ipos, s_irot, s_pos, s_rot, lo, c.rank, shape};  // in place
+    // a value that every CTA of the chunk keeps at the same address, over all of them
+    auto over = [&](const uint32_t* v, uint32_t start, auto&& join) {
+        uint32_t r = start;
+        if constexpr (kCluster)
+            for (uint32_t q = 0; q < ctas; ++q) r = join(r, peer_load(v, q));
+        else
+            r = join(r, *v);
+        return r;
+    };
+    auto sum = [](uint32_t a, uint32_t b) { return a + b; };
     // Jones-Plassmann rounds over the chunk's dynamic bodies
-    const uint32_t ndyn = dr.y - dr.x;
+    const uint32_t want = over(&s_ndyn, 0u, sum);
     uint32_t rounds = 0;
-    while (s_colored < ndyn) {
+    while (over(&s_colored, 0u, sum) < want) {
         if (++rounds > kChunkColorRounds) {
             if (tid == 0) atomicOr(&w.ctr->error_flags, kErrColorOverflow);
             break;
         }
-        for (uint32_t t = dr.x + tid; t < dr.y; t += nt) {
-            const uint32_t v = w.dyn_list[t];
+        for (uint32_t t = c.dyn.x + tid; t < c.dyn.y; t += nt) {
+            const uint32_t v = w.dyn_list[t], s = shape.slot(v - lo);
             bool sel = false;
-            if (s_color[v - lo] == kNoColor) {
+            if (s_color[s] == kNoColor) {
                 sel = true;
                 for_each_neighbour(w, v, [&](uint32_t u) {
-                    if (sel && s_color[u - lo] == kNoColor && !color_beats(v, u)) sel = false;
+                    if (sel && f.get(s_color, u) == kNoColor && !color_beats(v, u)) sel = false;
                 });
             }
-            s_sel[v - lo] = sel ? 1u : 0u;
+            s_sel[s] = sel ? 1u : 0u;
         }
-        __syncthreads();
-        for (uint32_t t = dr.x + tid; t < dr.y; t += nt) {
-            const uint32_t v = w.dyn_list[t];
-            if (!s_sel[v - lo]) continue;
+        chunk_sync<kCluster>();
+        for (uint32_t t = c.dyn.x + tid; t < c.dyn.y; t += nt) {
+            const uint32_t v = w.dyn_list[t], s = shape.slot(v - lo);
+            if (!s_sel[s]) continue;
             unsigned long long used[kMaxColors / 64] = {0ull, 0ull, 0ull, 0ull};
             for_each_neighbour(w, v, [&](uint32_t u) {
-                const uint32_t c = s_color[u - lo];
-                if (c < kMaxColors) used[c >> 6] |= 1ull << (c & 63);
+                const uint32_t q = f.get(s_color, u);
+                if (q < kMaxColors) used[q >> 6] |= 1ull << (q & 63);
             });
-            uint32_t c = kMaxColors;
-            for (uint32_t q = 0; q < kMaxColors / 64; ++q)
-                if (~used[q]) {
-                    c = q * 64 + (__ffsll(~used[q]) - 1);
+            uint32_t q = kMaxColors;
+            for (uint32_t k = 0; k < kMaxColors / 64; ++k)
+                if (~used[k]) {
+                    q = k * 64 + (__ffsll(~used[k]) - 1);
                     break;
                 }
-            if (c >= kMaxColors) {
+            if (q >= kMaxColors) {
                 atomicOr(&w.ctr->error_flags, kErrColorOverflow);
-                c = kMaxColors - 1;
+                q = kMaxColors - 1;
             }
-            s_color[v - lo] = c;
+            s_color[s] = q;
             atomicAdd(&s_colored, 1u);
-            atomicMax(&s_ncolors, c + 1);
+            atomicMax(&s_ncolors, q + 1);
         }
-        __syncthreads();
+        chunk_sync<kCluster>();
     }
-    const uint32_t ncolors = s_ncolors;
-    // colours out, and the chunk's dynamic bodies sorted by colour
-    for (uint32_t i = lo + tid; i < hi; i += nt) w.color[i] = s_color[i - lo];
+    const uint32_t ncolors = over(&s_ncolors, 0u, [](uint32_t a, uint32_t b) { return max(a, b); });
+    // colours out, and the CTA's dynamic bodies sorted by colour
+    for (uint32_t s = tid; s < shape.slots(c.nb); s += nt) {
+        const uint32_t d = shape.body(s, c.rank);
+        if (d < c.nb) w.color[lo + d] = s_color[s];
+    }
     if (tid == 0) atomicMax(&w.ctr->colors, ncolors);
-    for (uint32_t t = dr.x + tid; t < dr.y; t += nt) {
-        const uint32_t c = s_color[w.dyn_list[t] - lo];
-        if (c < kMaxColors) atomicAdd(&s_cstart[c + 1], 1u);
+    for (uint32_t t = c.dyn.x + tid; t < c.dyn.y; t += nt) {
+        const uint32_t q = s_color[shape.slot(w.dyn_list[t] - lo)];
+        if (q < kMaxColors) atomicAdd(&s_cstart[q + 1], 1u);
     }
     __syncthreads();
     if (tid == 0)
-        for (uint32_t c = 0; c < ncolors; ++c) s_cstart[c + 1] += s_cstart[c];
+        for (uint32_t q = 0; q < ncolors; ++q) s_cstart[q + 1] += s_cstart[q];
     __syncthreads();
-    for (uint32_t t = dr.x + tid; t < dr.y; t += nt) {
-        const uint32_t v = w.dyn_list[t];
-        const uint32_t c = s_color[v - lo];
-        if (c < kMaxColors) s_order[s_cstart[c] + atomicAdd(&s_cursor[c], 1u)] = v;
+    for (uint32_t t = c.dyn.x + tid; t < c.dyn.y; t += nt) {
+        const uint32_t q = s_color[shape.slot(w.dyn_list[t] - lo)];
+        if (q < kMaxColors) s_order[s_cstart[q] + atomicAdd(&s_next[q], 1u)] = t;
     }
     __syncthreads();
-    const uint32_t p0 = s_rows[0], p1 = s_rows[1], c0 = s_rows[2], c1 = s_rows[3];
-    const uint32_t np = p1 - p0, nrows = np + (c1 - c0);
-    const SmemFetch<P> f{s_pos, s_rot, s_ipos, s_irot, s_pos, s_rot, lo};  // in place
+    take_row_bounds(c, s_rows);
+    uint32_t turn = 0;  // alternates the group cursors
     for (uint32_t k = 0; k < o.iterations; ++k) {
-        for (uint32_t c = 0; c < ncolors; ++c) {
-            for (uint32_t t = s_cstart[c] + tid; t < s_cstart[c + 1]; t += nt) {
-                const uint32_t i = s_order[t];
-                const uint32_t k0 = w.n_joints ? w.joint_off[i] : 0u, k1 = w.n_joints ? w.joint_off[i + 1] : 0u;
-                primal_body_f(w, i, k0, k1, o, f);
-            }
-            __syncthreads();
+        for (uint32_t q = 0; q < ncolors; ++q, turn ^= 1u) {
+            if (tid == 0) s_cursor[turn ^ 1u] = 0u;  // last used before the previous barrier
+            // groups of 32 bodies, or fewer when the warps would not all get one
+            const uint32_t q0 = s_cstart[q], qn = s_cstart[q + 1] - q0;
+            uint32_t g = 32;
+            while (g > 1 && qn <= (g / 2) * (nt / 32u)) g /= 2;
+            auto range = [&](uint32_t e, uint32_t& t, uint32_t& n) {
+                t = q0 + e * g;
+                n = min(g, qn - e * g);
+            };
+            chunk_primal<kSpread>(w, OrderedBodies<P, R>{{w}, s_order}, (qn + g - 1) / g, range, o, f, stage,
+                                  &s_cursor[turn]);
+            chunk_sync<kCluster>();
         }
-        for (uint32_t t = tid; t < nrows; t += nt) dual_row_f(w, t < np ? p0 + t : c0 + (t - np), f, o);
-        __syncthreads();
+        if (!c.rows) continue;  // the same for all CTAs of the chunk
+        for (uint32_t t = c.rank * nt + tid; t < c.rows; t += nt << shape.cl) dual_row_f(w, c.row(t), f, o);
+        chunk_sync<kCluster>();
     }
-    for (uint32_t i = lo + tid; i < hi; i += nt) {
-        recover_body_f(w, i, f, o);
-        w.pos[0][i] = s_pos[i - lo];
-        w.rot[0][i] = s_rot[i - lo];
+    for (uint32_t s = tid; s < shape.slots(c.nb); s += nt) {
+        const uint32_t d = shape.body(s, c.rank);
+        if (d >= c.nb) continue;
+        recover_body_f(w, lo + d, f, o);
+        w.pos[0][lo + d] = s_pos[s];
+        w.rot[0][lo + d] = s_rot[s];
     }
+    chunk_sync<kCluster>();  // peers may still be reading this CTA's counts
 }
 
 }  // namespace dio

@@ -45,11 +45,11 @@ __device__ __forceinline__ void write_row(const DevWorld<P, R>& w, uint32_t r, u
     rs.t2 = pack(t2, R(0));
     rs.ra = pack(ra, c0.x);
     rs.rb = pack(rb, c0.y);
-    w.rs[r] = rs;
+    w.rs.put(r, rs);
     RowDual<P, R> du;
     du.penalty = A4<R>{kmin, kmin, kmin, R(0)};
     du.lambda = A4<P>{P(0), P(0), P(0), P(0)};
-    w.rd[r] = du;
+    w.rd.put(r, du);
     w.ab[r] = make_uint2(a, b);
 }
 
@@ -305,7 +305,7 @@ static __global__ void k_row_keys(const uint2* ab, const uint32_t* m_dev, uint32
 template <class P, class R>
 __global__ void k_warm(DevWorld<P, R> w, const uint32_t* m_dev, const unsigned long long* new_keys,
                        const uint32_t* new_ids, const unsigned long long* prev_keys, const uint32_t* prev_ids,
-                       uint32_t n_prev, const RowDual<P, R>* prev_dual, PrepParams<R> o) {
+                       uint32_t n_prev, RowDuals<P, R> prev_dual, PrepParams<R> o) {
     uint32_t m = *m_dev;
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < m; t += gridDim.x * blockDim.x) {
         unsigned long long key = new_keys[t];
@@ -336,7 +336,7 @@ __global__ void k_warm(DevWorld<P, R> w, const uint32_t* m_dev, const unsigned l
         du.penalty.x = fmin_(fmax_(kx, o.penalty_min), o.penalty_max);
         du.penalty.y = fmin_(fmax_(ky, o.penalty_min), o.penalty_max);
         du.penalty.z = fmin_(fmax_(kz, o.penalty_min), o.penalty_max);
-        w.rd[r] = du;
+        w.rd.put(r, du);
     }
 }
 
@@ -406,7 +406,7 @@ static __global__ void k_roll_counters(Counters* c, uint32_t* zero0, uint32_t* z
 }
 
 template <class P, class R>
-__global__ void k_warm_sections(DevWorld<P, R> w, const uint2* prev_ab, const RowDual<P, R>* prev_dual,
+__global__ void k_warm_sections(DevWorld<P, R> w, const uint2* prev_ab, RowDuals<P, R> prev_dual,
                                 PrepParams<R> o) {
     pdl_enter();
     const uint32_t m = w.ctr->rows, pair_rows = w.ctr->pair_rows;
@@ -441,7 +441,7 @@ __global__ void k_warm_sections(DevWorld<P, R> w, const uint2* prev_ab, const Ro
         du.penalty.x = fmin_(fmax_(kx, o.penalty_min), o.penalty_max);
         du.penalty.y = fmin_(fmax_(ky, o.penalty_min), o.penalty_max);
         du.penalty.z = fmin_(fmax_(kz, o.penalty_min), o.penalty_max);
-        w.rd[r] = du;
+        w.rd.put(r, du);
     }
 }
 

@@ -138,11 +138,11 @@ __global__ void k_na_rows(DevWorld<float, float> w, const DioContact* c, uint32_
         s.t2 = A4<float>{x.tangent2[0], x.tangent2[1], x.tangent2[2], 0.f};
         s.ra = A4<float>{x.r_a[0], x.r_a[1], x.r_a[2], x.c0[0]};
         s.rb = A4<float>{x.r_b[0], x.r_b[1], x.r_b[2], x.c0[1]};
-        w.rs[r] = s;
+        w.rs.put(r, s);
         RowDual<float, float> d;
         d.penalty = A4<float>{x.penalty[0], x.penalty[1], x.penalty[2], 0.f};
         d.lambda = A4<float>{x.lambda[0], x.lambda[1], x.lambda[2], 0.f};
-        w.rd[r] = d;
+        w.rd.put(r, d);
         w.ab[r] = make_uint2(x.a, x.b);
         if (x.a >= n || (x.b != kContainer && x.b >= n)) atomicOr(&w.ctr->error_flags, kErrBadIndex);
     }
@@ -284,8 +284,9 @@ extern "C" int dio_avbd_solve_noalloc(const DioBodyState* state, const float* po
     w.prev_vel = a4(10);
     w.inv = a4(11);
     w.friction = reinterpret_cast<float*>(base + kOffFric);
-    w.rs = reinterpret_cast<RowStatic<float>*>(base + kOffRs);
-    w.rd = reinterpret_cast<RowDual<float, float>*>(base + kOffRd);
+    w.rs = RowStatics<float>{reinterpret_cast<A4<float>*>(base + kOffRs), kNaMaxContacts};
+    w.rd.penalty = reinterpret_cast<A4<float>*>(base + kOffRd);
+    w.rd.lambda = w.rd.penalty + kNaMaxContacts;
     w.ab = reinterpret_cast<uint2*>(base + kOffAb);
     w.row_oth = reinterpret_cast<uint32_t*>(base + kOffOth);
     w.row_off = const_cast<uint32_t*>(offsets);

@@ -233,15 +233,17 @@ typedef struct DioConfig {
                                    (launch shape, body tiles, bodies per warp;
                                    every variant computes the same bits;
                                    autotuned)                             */
-    uint32_t block_size;        /* threads per CTA of the scene-chunk
-                                   solve: 0 (512) or 640 (autotuned)      */
+    uint32_t block_size;        /* CTA shape of the scene-chunk solve: 0 --
+                                   chosen by the scenes' sizes and number --
+                                   or 640, a whole SM for each chunk where
+                                   every scene fits one (autotuned)       */
     uint32_t batched_solver;    /* DioSolveLaunch: DIO_SOLVE_AUTO (0) runs
                                    a world step's whole solve (init, the
                                    iterations, recover) as one launch, a
-                                   CTA per chunk of whole scenes with the
-                                   poses in shared memory, when every
-                                   scene fits a chunk (2048 bodies, 1024
-                                   with FP64 poses) and no joint crosses
+                                   CTA or a cluster of CTAs per chunk of
+                                   whole scenes with the poses in shared
+                                   memory, when every scene fits a chunk
+                                   (2048 bodies) and no joint crosses
                                    scenes; DIO_SOLVE_PER_PHASE (1) always
                                    launches init / primal / dual / recover
                                    kernels.  Both give identical results. */
