@@ -62,11 +62,10 @@ constexpr int kMaskAxisX = (1 << 0) | (1 << 4) | (1 << 5);  // J = (s, 0, 0, 0, 
 constexpr int kMaskAxisY = (1 << 1) | (1 << 3) | (1 << 5);  // J = (0, s, 0, -s r.z, 0, s r.x)
 constexpr int kMaskAxisZ = (1 << 2) | (1 << 3) | (1 << 4);  // J = (0, 0, s, s r.y, -s r.x, 0)
 
-// solve6, avbd/src/lib.rs:107-180 (unpivoted LDL^T); solves H x = -g.  Each
-// quotient by a pivot is the IEEE quotient (div_rn.cuh: one reciprocal per
-// pivot, a correction step per quotient, one range test per pivot's column).
-template <class R>
-__device__ __forceinline__ void solve6(const Block6<R>& B, R x[6]) {
+// solve6, avbd/src/lib.rs:107-180 (unpivoted LDL^T); solves H x = -g.
+// div(p, a): the quotient of a by pivot p.
+template <class R, class Div>
+__device__ __forceinline__ void solve6_with(const Block6<R>& B, R x[6], Div&& div) {
     const R* H = B.h;
     R a11 = H[tri(0, 0)], a21 = H[tri(1, 0)], a31 = H[tri(2, 0)], a22 = H[tri(1, 1)], a32 = H[tri(2, 1)],
       a33 = H[tri(2, 2)];
@@ -75,32 +74,29 @@ __device__ __forceinline__ void solve6(const Block6<R>& B, R x[6]) {
     R a43 = H[tri(3, 2)], a53 = H[tri(4, 2)], a63 = H[tri(5, 2)];
     R a44 = H[tri(3, 3)], a54 = H[tri(4, 3)], a64 = H[tri(5, 3)], a55 = H[tri(4, 4)], a65 = H[tri(5, 4)],
       a66 = H[tri(5, 5)];
-    const Pivot<R> p1(a11);
-    R q1[5] = {a21, a31, a41, a51, a61};
-    divide_all(p1, q1);
-    const R l21 = q1[0], l31 = q1[1], l41 = q1[2], l51 = q1[3], l61 = q1[4];
+    const auto p1 = div.pivot(a11);
+    R l21 = div(p1, a21), l31 = div(p1, a31), l41 = div(p1, a41), l51 = div(p1, a51), l61 = div(p1, a61);
     R d1 = a11;
     R d2 = a22 - l21 * l21 * d1;
-    const Pivot<R> p2(d2);
-    R q2[4] = {a32 - l21 * l31 * d1, a42 - l21 * l41 * d1, a52 - l21 * l51 * d1, a62 - l21 * l61 * d1};
-    divide_all(p2, q2);
-    const R l32 = q2[0], l42 = q2[1], l52 = q2[2], l62 = q2[3];
+    const auto p2 = div.pivot(d2);
+    R l32 = div(p2, a32 - l21 * l31 * d1);
+    R l42 = div(p2, a42 - l21 * l41 * d1);
+    R l52 = div(p2, a52 - l21 * l51 * d1);
+    R l62 = div(p2, a62 - l21 * l61 * d1);
     R d3 = a33 - (l31 * l31 * d1 + l32 * l32 * d2);
-    const Pivot<R> p3(d3);
-    R q3[3] = {a43 - l31 * l41 * d1 - l32 * l42 * d2, a53 - l31 * l51 * d1 - l32 * l52 * d2,
-               a63 - l31 * l61 * d1 - l32 * l62 * d2};
-    divide_all(p3, q3);
-    const R l43 = q3[0], l53 = q3[1], l63 = q3[2];
+    const auto p3 = div.pivot(d3);
+    R l43 = div(p3, a43 - l31 * l41 * d1 - l32 * l42 * d2);
+    R l53 = div(p3, a53 - l31 * l51 * d1 - l32 * l52 * d2);
+    R l63 = div(p3, a63 - l31 * l61 * d1 - l32 * l62 * d2);
     R d4 = a44 - (l41 * l41 * d1 + l42 * l42 * d2 + l43 * l43 * d3);
-    const Pivot<R> p4(d4);
-    R q4[2] = {a54 - l41 * l51 * d1 - l42 * l52 * d2 - l43 * l53 * d3,
-               a64 - l41 * l61 * d1 - l42 * l62 * d2 - l43 * l63 * d3};
-    divide_all(p4, q4);
-    const R l54 = q4[0], l64 = q4[1];
+    const auto p4 = div.pivot(d4);
+    R l54 = div(p4, a54 - l41 * l51 * d1 - l42 * l52 * d2 - l43 * l53 * d3);
+    R l64 = div(p4, a64 - l41 * l61 * d1 - l42 * l62 * d2 - l43 * l63 * d3);
     R d5 = a55 - (l51 * l51 * d1 + l52 * l52 * d2 + l53 * l53 * d3 + l54 * l54 * d4);
-    const Divisor<R> p5(d5);
-    const R l65 = p5.div(a65 - l51 * l61 * d1 - l52 * l62 * d2 - l53 * l63 * d3 - l54 * l64 * d4);
+    const auto p5 = div.pivot(d5);
+    R l65 = div(p5, a65 - l51 * l61 * d1 - l52 * l62 * d2 - l53 * l63 * d3 - l54 * l64 * d4);
     R d6 = a66 - (l61 * l61 * d1 + l62 * l62 * d2 + l63 * l63 * d3 + l64 * l64 * d4 + l65 * l65 * d5);
+    const auto p6 = div.pivot(d6);
     R b0 = -B.g[0], b1 = -B.g[1], b2 = -B.g[2], b3 = -B.g[3], b4 = -B.g[4], b5 = -B.g[5];
     R y1 = b0;
     R y2 = b1 - l21 * y1;
@@ -108,22 +104,46 @@ __device__ __forceinline__ void solve6(const Block6<R>& B, R x[6]) {
     R y4 = b3 - l41 * y1 - l42 * y2 - l43 * y3;
     R y5 = b4 - l51 * y1 - l52 * y2 - l53 * y3 - l54 * y4;
     R y6 = b5 - l61 * y1 - l62 * y2 - l63 * y3 - l64 * y4 - l65 * y5;
-    Quotients<R> qz;
-    R z1 = qz.div(p1, y1), z2 = qz.div(p2, y2), z3 = qz.div(p3, y3), z4 = qz.div(p4, y4), z5 = qz.div(p5.p, y5);
-    if (!(qz.in_range() && p1.ok() && p2.ok() && p3.ok() && p4.ok() && p5.p.ok())) {
-        z1 = y1 / d1;
-        z2 = y2 / d2;
-        z3 = y3 / d3;
-        z4 = y4 / d4;
-        z5 = y5 / d5;
-    }
-    R z6 = y6 / d6;
+    R z1 = div(p1, y1), z2 = div(p2, y2), z3 = div(p3, y3), z4 = div(p4, y4), z5 = div(p5, y5), z6 = div(p6, y6);
     x[5] = z6;
     x[4] = z5 - l65 * x[5];
     x[3] = z4 - l54 * x[4] - l64 * x[5];
     x[2] = z3 - l43 * x[3] - l53 * x[4] - l63 * x[5];
     x[1] = z2 - l32 * x[2] - l42 * x[3] - l52 * x[4] - l62 * x[5];
     x[0] = z1 - l21 * x[1] - l31 * x[2] - l41 * x[3] - l51 * x[4] - l61 * x[5];
+}
+template <class R>
+struct PlainDiv {
+    __device__ __forceinline__ R pivot(R b) const { return b; }
+    __device__ __forceinline__ R operator()(R b, R a) const { return a / b; }
+};
+
+// Each quotient by a pivot is the IEEE quotient: one reciprocal per pivot and
+// a correction step per quotient (div_rn.cuh), with one range test for the
+// whole system; a system outside the range is solved again with IEEE
+// divisions (in line: through a call, the system goes to local memory on
+// every solve, and 1024 scenes take 2816 us a pass instead of 2610; with a
+// test per pivot's column 2658).
+template <class R>
+__device__ __forceinline__ void solve6(const Block6<R>& B, R x[6]) {
+    if constexpr (sizeof(R) == 4) {
+        struct Collect {
+            Quotients<R>& q;
+            bool& ok;
+            __device__ __forceinline__ Pivot<R> pivot(R b) const {
+                const Pivot<R> p(b);
+                ok = ok && p.ok();
+                return p;
+            }
+            __device__ __forceinline__ R operator()(const Pivot<R>& p, R a) const { return q.div(p, a); }
+        };
+        Quotients<R> q;
+        bool ok = true;
+        solve6_with(B, x, Collect{q, ok});
+        if (!(ok && q.in_range())) solve6_with(B, x, PlainDiv<R>());
+    } else {
+        solve6_with(B, x, PlainDiv<R>());
+    }
 }
 
 // avbd_init, avbd/src/lib.rs:202-254, for one body: the inertial target and
@@ -485,6 +505,7 @@ __device__ __forceinline__ void primal_inertia(const BodyTask<P, R>& b, V3<P> sp
 // body, through the row and joint CSRs.
 template <class P, class R>
 struct WorldBodies {
+    static constexpr bool kAhead = false;
     const DevWorld<P, R>& w;
     const uint32_t* list;
     __device__ __forceinline__ BodyTask<P, R> load(uint32_t t) const {
@@ -510,6 +531,7 @@ struct WorldBodies {
 // that depend on nothing but the position.
 template <class P, class R>
 struct ListBodies {
+    static constexpr bool kAhead = sizeof(P) == 4;
     const DevWorld<P, R>& w;
     __device__ __forceinline__ BodyTask<P, R> load(uint32_t t) const {
         BodyTask<P, R> b;
@@ -537,14 +559,27 @@ struct ListBodies {
     }
 };
 
+// A body's joints: their number and, where S::kAhead, the first of them
+// loaded ahead of the row terms (the scene-chunk solve: 1024 scenes 2610 ->
+// 2553 us a pass; elsewhere, and for two joints, its registers cost more).
+struct JointsAhead {
+    uint32_t n = 0;
+    JView first;
+    template <class S>
+    __device__ __forceinline__ void load(const S& bodies, uint32_t t, uint32_t i) {
+        n = bodies.joints(t, i);
+        if constexpr (S::kAhead)
+            if (n) first = bodies.joint(t, i, 0);
+    }
+};
+
 // Joint rows, the 6x6 solve and the pose update of body i (the tail of
 // avbd_primal); t: its position for `bodies`
 template <class P, class R, class F, class S>
 __device__ __forceinline__ void primal_finish(const S& bodies, uint32_t t, uint32_t i, const F& fetch, V3<P> sp,
-                                              Q4<P> sq, Q4<R> sqr, Block6<R>& B) {
-    const uint32_t nj = bodies.joints(t, i);
-    for (uint32_t k = 0; k < nj; ++k) {
-        const JView jv = bodies.joint(t, i, k);
+                                              Q4<P> sq, Q4<R> sqr, const JointsAhead& joints, Block6<R>& B) {
+    for (uint32_t k = 0; k < joints.n; ++k) {
+        const JView jv = S::kAhead && k == 0u ? joints.first : bodies.joint(t, i, k);
         primal_jview_f<P, R>(jv, fetch, sp, sq, sqr, B);
     }
     R dx[6];
@@ -577,7 +612,9 @@ __device__ __forceinline__ void primal_body_f(const DevWorld<P, R>& w, uint32_t 
         for (uint32_t j = b.j0; j < b.j0 + b.n; ++j)
             primal_row_f(w, w.row_idx[j], w.row_oth[j], fetch, sqr, dqsl, dqsa, k_alpha, B);
     }
-    primal_finish(bodies, 0u, i, fetch, sp, sq, sqr, B);
+    JointsAhead joints;
+    joints.load(bodies, 0u, i);
+    primal_finish(bodies, 0u, i, fetch, sp, sq, sqr, joints, B);
 }
 
 template <class P, class R>
@@ -702,8 +739,10 @@ __device__ __forceinline__ void primal_group(const DevWorld<P, R>& w, const S& b
     V3<P> sp{P(0), P(0), P(0)};
     Q4<P> sq{P(0), P(0), P(0), P(1)};
     Block6<R> B;
+    JointsAhead joints;
     if (live) {
         task = bodies.load(t0 + lane);
+        joints.load(bodies, t0 + lane, task.i);
         sp = xyz(fetch.pos(task.i));
         sq = quat(fetch.rot(task.i));
     }
@@ -806,7 +845,7 @@ __device__ __forceinline__ void primal_group(const DevWorld<P, R>& w, const S& b
         }
     }
     if (live) {
-        primal_finish(bodies, t0 + lane, i, fetch, sp, sq, sqr, B);
+        primal_finish(bodies, t0 + lane, i, fetch, sp, sq, sqr, joints, B);
     }
 }
 

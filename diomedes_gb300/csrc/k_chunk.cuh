@@ -431,6 +431,7 @@ __global__ void __launch_bounds__(chunk_threads<R, kSpread>(), sizeof(R) == 4 &&
 // list positions in the order of the colours
 template <class P, class R>
 struct OrderedBodies {
+    static constexpr bool kAhead = false;
     ListBodies<P, R> list;
     const uint32_t* order;
     __device__ __forceinline__ BodyTask<P, R> load(uint32_t k) const { return list.load(order[k]); }
