@@ -5,6 +5,8 @@
 //   bodies   pos[2], rot[2]       ping-pong pose buffers (Jacobi parity)
 //            init_pos, init_rot   pose at step start       (avbd_init)
 //            inert_pos, inert_rot inertial target           (avbd_init)
+//            rot_r, moved_l/a     R rotation and displacement since the step
+//                                 start, per pose buffer
 //            vel, ang, prev_vel   velocities
 //            inv                  inverse moment xyz, inverse mass in w
 //            shape                DioShape (80 B, the reference GpuShape)
@@ -24,6 +26,7 @@
 #include <utility>
 
 #include "../../include/dio_cuda.h"
+#include "cvt64.cuh"
 #include "dio_math.cuh"
 
 namespace dio {
@@ -97,12 +100,20 @@ template <class P, class R>
 struct RowDuals {
     A4<R>* penalty;
     A4<P>* lambda;
+    A4<R>* lambda_r;  // lambda rounded to R (lambda itself when P is R), as the primal takes it
     __device__ __forceinline__ RowDual<P, R> operator[](uint32_t r) const {
         return RowDual<P, R>{penalty[r], lambda[r]};
+    }
+    __device__ __forceinline__ RowDual<R, R> rounded(uint32_t r) const {
+        return RowDual<R, R>{penalty[r], lambda_r[r]};
     }
     __device__ __forceinline__ void put(uint32_t r, const RowDual<P, R>& d) const {
         penalty[r] = d.penalty;
         lambda[r] = d.lambda;
+        if constexpr (sizeof(P) != sizeof(R)) {
+            const V3<R> l = narrow3<R>(xyz(d.lambda));
+            lambda_r[r] = A4<R>{l.x, l.y, l.z, R(0)};
+        }
     }
 };
 
@@ -160,7 +171,13 @@ struct DevWorld {
     A4<P>* init_pos;
     A4<P>* init_rot;
     A4<P>* inert_pos;
-    A4<P>* inert_rot;
+    A4<R>* inert_rot;
+    // per pose buffer: the rotation rounded to R (rot itself when P is R) and
+    // the body's displacement since the step start, linear xyz and angular
+    // (x in moved_l.w, y and z in moved_a)
+    A4<R>* rot_r[2];
+    A4<R>* moved_l[2];
+    V2<R>* moved_a[2];
     A4<P>* vel;
     A4<P>* ang;
     A4<P>* prev_vel;

@@ -489,6 +489,14 @@ class Engine final : public EngineBase {
         DIO_TRY(alloc(&w_.init_rot, N));
         DIO_TRY(alloc(&w_.inert_pos, N));
         DIO_TRY(alloc(&w_.inert_rot, N));
+        for (int b = 0; b < 2; ++b) {
+            if constexpr (std::is_same<P, R>::value)
+                w_.rot_r[b] = w_.rot[b];
+            else
+                DIO_TRY(alloc(&w_.rot_r[b], N));
+            DIO_TRY(alloc(&w_.moved_l[b], N));
+            DIO_TRY(alloc(&w_.moved_a[b], N));
+        }
         DIO_TRY(alloc(&w_.vel, N));
         DIO_TRY(alloc(&w_.ang, N));
         DIO_TRY(alloc(&w_.prev_vel, N));
@@ -533,6 +541,10 @@ class Engine final : public EngineBase {
             rs_[b].stride = M;
             DIO_TRY(alloc(&rd_[b].penalty, M));
             DIO_TRY(alloc(&rd_[b].lambda, M));
+            if constexpr (std::is_same<P, R>::value)
+                rd_[b].lambda_r = rd_[b].lambda;
+            else
+                DIO_TRY(alloc(&rd_[b].lambda_r, M));
             DIO_TRY(alloc(&ab_[b], M));
             DIO_TRY(alloc(&keys_s_[b], M));
             DIO_TRY(alloc(&ids_s_[b], M));

@@ -173,7 +173,7 @@ __device__ __forceinline__ InitPose<P> init_pose(const DevWorld<P, R>& w, uint32
     if (inv_mass > R(0)) ip = add(ip, scale(g, dt * dt));
     w.inert_pos[at] = pack(ip);
     Q4<P> irot = quat_step(rot, scale(ang, dt));
-    w.inert_rot[at] = packq(irot);
+    w.inert_rot[at] = packq(narrowq<R>(irot));
     if (w.mdt2 && inv_mass != R(0)) {
         // the primal's diagonal, constant over the step (avbd/src/lib.rs:293-296)
         const R mass = R(1) / inv.w;
@@ -201,6 +201,33 @@ __device__ __forceinline__ InitPose<P> init_pose(const DevWorld<P, R>& w, uint32
     return r;
 }
 
+// What the rows of a body take from it: its rotation rounded to R and its
+// displacement since the step start, linear and angular, formed once per pose
+// (each row and dual formed them again from four pose records a body).
+template <class R>
+struct Moved {
+    V3<R> dl, da;
+    Q4<R> q;
+};
+template <class R, class P>
+__device__ __forceinline__ Moved<R> moved_from(A4<P> pos, Q4<R> q, A4<P> start_pos, A4<P> start_rot) {
+    Moved<R> m;
+    m.dl = narrow3<R>(sub(xyz(pos), xyz(start_pos)));
+    m.q = q;
+    m.da = ang_diff(q, narrowq<R>(quat(start_rot)));
+    return m;
+}
+template <class P, class R>
+__device__ __forceinline__ void put_moved(const DevWorld<P, R>& w, int buf, uint32_t i, const Moved<R>& m) {
+    if constexpr (sizeof(P) != sizeof(R)) w.rot_r[buf][i] = packq(m.q);
+    w.moved_l[buf][i] = pack(m.dl, m.da.x);
+    w.moved_a[buf][i] = V2<R>{m.da.y, m.da.z};
+}
+template <class R>
+__device__ __forceinline__ Moved<R> moved_of(A4<R> q, A4<R> l, V2<R> a) {
+    return Moved<R>{xyz(l), V3<R>{l.w, a.x, a.y}, quat(q)};
+}
+
 // avbd_init with the poses in global memory (+ seeding buffer 1 with the
 // un-warm-started pose, render/gpu_physics.rs:479-482)
 template <class P, class R>
@@ -221,6 +248,11 @@ __device__ __forceinline__ void init_body(const DevWorld<P, R>& w, uint32_t i, c
         w.pos[0][i] = r.pos;
         w.rot[0][i] = r.rot;
     }
+    if (w.moved_l[0]) {
+        const Moved<R> m = moved_from<R>(r.pos, narrowq<R>(quat(r.rot)), r.start_pos, r.start_rot);
+        put_moved(w, 0, i, m);
+        if (inv_mass == R(0)) put_moved(w, 1, i, m);
+    }
 }
 
 template <class P, class R>
@@ -230,82 +262,138 @@ __global__ void __launch_bounds__(256) k_init(DevWorld<P, R> w, uint32_t lo, uin
         init_body(w, i, o);
 }
 
-// Where the primal reads another body's snapshot / step-start pose: global
-// memory, or a shared-memory tile of consecutive bodies with a global
-// fallback.  Both return the same values.
-// `store` writes a body's new pose (the primal's output buffer).
+// Where the primal and the dual find poses.  pos: a position; rot: a body's
+// own rotation; rot_r: a rotation rounded to R; moved: what rows take; store:
+// a body's new pose.
+// PoseFetch: pose buffer rd in global memory, displacements formed here.
 template <class P, class R>
-struct GlobalFetch {
+struct PoseFetch {
     const DevWorld<P, R>& w;
     int rd;
     __device__ __forceinline__ A4<P> pos(uint32_t j) const { return w.pos[rd][j]; }
     __device__ __forceinline__ A4<P> rot(uint32_t j) const { return w.rot[rd][j]; }
+    __device__ __forceinline__ Q4<R> rot_r(uint32_t j) const { return narrowq<R>(quat(w.rot[rd][j])); }
     __device__ __forceinline__ A4<P> ipos(uint32_t j) const { return w.init_pos[j]; }
     __device__ __forceinline__ A4<P> irot(uint32_t j) const { return w.init_rot[j]; }
-    __device__ __forceinline__ void store(uint32_t i, A4<P> p, A4<P> q) const {
-        w.pos[1 - rd][i] = p;
-        w.rot[1 - rd][i] = q;
+    __device__ __forceinline__ Moved<R> moved(uint32_t j) const {
+        return moved_from<R>(w.pos[rd][j], rot_r(j), w.init_pos[j], w.init_rot[j]);
     }
 };
-
+// GlobalFetch: buffer rd read and wr written (the same buffer: in place, the
+// coloured sweeps), displacements kept with the poses.
+template <class P, class R>
+struct GlobalFetch {
+    const DevWorld<P, R>& w;
+    int rd, wr;
+    __device__ __forceinline__ A4<P> pos(uint32_t j) const { return w.pos[rd][j]; }
+    __device__ __forceinline__ A4<P> rot(uint32_t j) const { return w.rot[rd][j]; }
+    __device__ __forceinline__ Q4<R> rot_r(uint32_t j) const { return quat(w.rot_r[rd][j]); }
+    __device__ __forceinline__ Moved<R> moved(uint32_t j) const {
+        return moved_of(w.rot_r[rd][j], w.moved_l[rd][j], w.moved_a[rd][j]);
+    }
+    __device__ __forceinline__ void store(uint32_t i, A4<P> p, A4<P> q) const {
+        const Moved<R> m = moved_from<R>(p, narrowq<R>(quat(q)), w.init_pos[i], w.init_rot[i]);
+        w.pos[wr][i] = p;
+        w.rot[wr][i] = q;
+        put_moved(w, wr, i, m);
+    }
+};
+// TileFetch: a shared-memory tile of consecutive bodies' poses, the others
+// from global memory.
 template <class P, class R, int T>
 struct TileFetch {
-    const DevWorld<P, R>& w;
-    int rd;
+    GlobalFetch<P, R> g;
     uint32_t lo;
     const A4<P>* sp;
     const A4<P>* sq;
     const A4<P>* si;
     const A4<P>* sr;
-    __device__ __forceinline__ A4<P> pos(uint32_t j) const { return j - lo < (uint32_t)T ? sp[j - lo] : w.pos[rd][j]; }
-    __device__ __forceinline__ A4<P> rot(uint32_t j) const { return j - lo < (uint32_t)T ? sq[j - lo] : w.rot[rd][j]; }
-    __device__ __forceinline__ A4<P> ipos(uint32_t j) const { return j - lo < (uint32_t)T ? si[j - lo] : w.init_pos[j]; }
-    __device__ __forceinline__ A4<P> irot(uint32_t j) const { return j - lo < (uint32_t)T ? sr[j - lo] : w.init_rot[j]; }
-    __device__ __forceinline__ void store(uint32_t i, A4<P> p, A4<P> q) const {
-        w.pos[1 - rd][i] = p;
-        w.rot[1 - rd][i] = q;
+    __device__ __forceinline__ bool in(uint32_t j) const { return j - lo < (uint32_t)T; }
+    __device__ __forceinline__ A4<P> pos(uint32_t j) const { return in(j) ? sp[j - lo] : g.pos(j); }
+    __device__ __forceinline__ A4<P> rot(uint32_t j) const { return in(j) ? sq[j - lo] : g.rot(j); }
+    __device__ __forceinline__ Q4<R> rot_r(uint32_t j) const {
+        return in(j) ? narrowq<R>(quat(sq[j - lo])) : g.rot_r(j);
     }
+    __device__ __forceinline__ Moved<R> moved(uint32_t j) const {
+        return in(j) ? moved_from<R>(sp[j - lo], rot_r(j), si[j - lo], sr[j - lo]) : g.moved(j);
+    }
+    __device__ __forceinline__ void store(uint32_t i, A4<P> p, A4<P> q) const { g.store(i, p, q); }
 };
 
 // Clamped row forces shared by avbd_primal and avbd_dual (avbd/src/lib.rs:
 // 380-406, 606-631): normal f0 <= 0, friction (f1, f2) scaled back onto the
 // cone |f_t| <= mu |f0|; `tm` (unclamped friction magnitude) and `bounds`
 // feed the dual's penalty rule.
-template <class P, class R>
-__device__ __forceinline__ void row_forces(const RowDual<P, R>& du, R mu, R c0, R c1, R c2, P& f0, P& f1, P& f2,
+template <class P>
+__device__ __forceinline__ void row_forces(const RowDual<P, P>& du, P mu, P c0, P c1, P c2, P& f0, P& f1, P& f2,
                                            P& tm, P& bounds) {
-    f0 = fmin_(P(du.penalty.x * c0) + du.lambda.x, P(0));
-    const P f1r = P(du.penalty.y * c1) + du.lambda.y;
-    const P f2r = P(du.penalty.z * c2) + du.lambda.z;
-    bounds = dabs(f0) * P(mu);
+    f0 = fmin_(du.penalty.x * c0 + du.lambda.x, P(0));
+    const P f1r = du.penalty.y * c1 + du.lambda.y;
+    const P f2r = du.penalty.z * c2 + du.lambda.z;
+    bounds = dabs(f0) * mu;
     f1 = f1r;
     f2 = f2r;
-    if constexpr (std::is_same<P, R>::value) {
-        tm = dsqrt(f1r * f1r + f2r * f2r);
-        if (tm > bounds && tm > P(0)) {
-            const P s = bounds / tm;
-            f1 = f1r * s;
-            f2 = f2r * s;
-        }
+    tm = dsqrt(f1r * f1r + f2r * f2r);
+    if (tm > bounds && tm > P(0)) {
+        const P s = bounds / tm;
+        f1 = f1r * s;
+        f2 = f2r * s;
+    }
+}
+
+// The same in the split mode (FP64 forces, FP32 elsewhere): the cone
+// magnitude tm and its scale factor in FP32, applied to the FP64 forces
+// (lambda accumulates in FP64).  f0_neg: f0 < 0; inside: tm <= mu |f0|.
+// FP64 instructions are few: the sign of f0 and the cone test are decided on
+// bits and in FP32 (the rounded bound is within 2^-22 of the FP64 one)
+// unless they are too close, tiny, or not finite.
+__device__ __forceinline__ void row_forces_split(const RowDual<double, float>& du, float mu, float c0, float c1,
+                                                 float c2, double& f0, double& f1, double& f2, bool& f0_neg,
+                                                 bool& inside) {
+    const double g0 = widen(du.penalty.x * c0) + du.lambda.x;
+    const uint32_t hi = (uint32_t)__double2hiint(g0), lo = (uint32_t)__double2loint(g0), m = hi & 0x7FFFFFFFu;
+    if (m >= 0x7FF00000u || (m | lo) == 0u) {  // infinite, NaN or zero
+        f0 = fmin(g0, 0.0);
+        f0_neg = f0 < 0.0;
     } else {
-        // split mode: the cone magnitude and its scale factor in R, applied to
-        // the P forces (lambda still accumulates in P)
-        const R f1q = R(f1r), f2q = R(f2r);
-        const R tmr = dsqrt(f1q * f1q + f2q * f2q);
-        tm = P(tmr);
-        if (tm > bounds && tm > P(0)) {
-            const R sr = R(bounds) / tmr;
-            f1 = f1r * P(sr);
-            f2 = f2r * P(sr);
-        }
+        f0_neg = hi >> 31;
+        f0 = f0_neg ? g0 : 0.0;
+    }
+    const double f1r = widen(du.penalty.y * c1) + du.lambda.y;
+    const double f2r = widen(du.penalty.z * c2) + du.lambda.z;
+    f1 = f1r;
+    f2 = f2r;
+    const float f1q = to_float(f1r), f2q = to_float(f2r);
+    const float tm = dsqrt(f1q * f1q + f2q * f2q);
+    const float f0q = to_float(f0);
+    const float bound = fabsf(f0q) * mu;
+    bool outside;
+    if (!f0_neg && f0q == 0.f && isfinite(mu) && !isnan(tm)) {  // f0 is a zero: so is the bound
+        outside = tm > 0.f;
+        inside = !outside;
+    } else if (bound >= 1e-30f && bound <= 1e30f && tm >= bound * 1.000001f) {
+        outside = true;
+        inside = false;
+    } else if (bound >= 1e-30f && bound <= 1e30f && tm <= bound * 0.999999f) {
+        outside = false;
+        inside = true;
+    } else {
+        const double b = fabs(f0) * (double)mu, t = (double)tm;
+        outside = t > b && t > 0.0;
+        inside = t <= b;
+    }
+    if (outside) {
+        const float s = to_float(fabs(f0) * widen(mu)) / tm;
+        f1 = f1r * widen(s);
+        f2 = f2r * widen(s);
     }
 }
 
 // One contact row seen from body i (avbd/src/lib.rs:321-418): its three
 // stamps (normal, tangent 1, tangent 2) as Jacobian rows (jl, ja), stiffness
 // k and force f.
-template <class P, class R, class F>
-__device__ __forceinline__ void primal_row_terms(const RowStatic<R>& rs, const RowDual<P, R>& du, uint32_t oth,
+template <class R, class F>
+__device__ __forceinline__ void primal_row_terms(const RowStatic<R>& rs, const RowDual<R, R>& du, uint32_t oth,
                                                  const F& fetch, Q4<R> sqr, V3<R> dqsl, V3<R> dqsa, R k_alpha,
                                                  V3<R> jl[3], V3<R> ja[3], R k[3], R f[3]) {
     const bool container = oth == kContainer;
@@ -318,11 +406,10 @@ __device__ __forceinline__ void primal_row_terms(const RowStatic<R>& rs, const R
     V3<R> rw = rotate(sqr, is_a ? xyz(rs.ra) : xyz(rs.rb));
     V3<R> dol{R(0), R(0), R(0)}, doa{R(0), R(0), R(0)}, rot_other{R(0), R(0), R(0)};
     if (!container) {
-        A4<P> op = fetch.pos(other);
-        A4<P> oq = fetch.rot(other);
-        dol = cast3<R>(sub(xyz(op), xyz(fetch.ipos(other))));
-        doa = ang_diff(castq<R>(quat(oq)), castq<R>(quat(fetch.irot(other))));
-        rot_other = rotate(castq<R>(quat(oq)), is_a ? xyz(rs.rb) : xyz(rs.ra));
+        const Moved<R> m = fetch.moved(other);
+        dol = m.dl;
+        doa = m.da;
+        rot_other = rotate(m.q, is_a ? xyz(rs.rb) : xyz(rs.ra));
     }
     V3<R> j0 = cross(rw, r0), j1 = cross(rw, r1), j2 = cross(rw, r2);
     R c0 = rs.ra.w * k_alpha, c1 = rs.rb.w * k_alpha, c2 = rs.t1.w * k_alpha;
@@ -330,11 +417,9 @@ __device__ __forceinline__ void primal_row_terms(const RowStatic<R>& rs, const R
     c1 = c1 + (dot(r1, dqsl) + dot(j1, dqsa) - dot(r1, dol) - dot(cross(rot_other, r1), doa));
     c2 = c2 + (dot(r2, dqsl) + dot(j2, dqsa) - dot(r2, dol) - dot(cross(rot_other, r2), doa));
     // the forces only feed the R Hessian: in the split mode they are formed
-    // in R from the P lambda (the dual accumulates lambda in P)
-    using Fq = std::conditional_t<std::is_same<P, R>::value, P, R>;
-    const RowDual<Fq, R> dv{du.penalty, A4<Fq>{Fq(du.lambda.x), Fq(du.lambda.y), Fq(du.lambda.z), Fq(0)}};
-    Fq f0, f1, f2, tm, bounds;
-    row_forces(dv, rs.n.w, c0, c1, c2, f0, f1, f2, tm, bounds);
+    // in R from the rounded lambda (the dual accumulates lambda in P)
+    R tm, bounds;
+    row_forces(du, rs.n.w, c0, c1, c2, f[0], f[1], f[2], tm, bounds);
     jl[0] = r0;
     jl[1] = r1;
     jl[2] = r2;
@@ -344,29 +429,15 @@ __device__ __forceinline__ void primal_row_terms(const RowStatic<R>& rs, const R
     k[0] = du.penalty.x;
     k[1] = du.penalty.y;
     k[2] = du.penalty.z;
-    f[0] = R(f0);
-    f[1] = R(f1);
-    f[2] = R(f2);
-}
-template <class P, class R, class F>
-__device__ __forceinline__ void primal_row_core(const RowStatic<R>& rs, const RowDual<P, R>& du, uint32_t oth,
-                                                const F& fetch, Q4<R> sqr, V3<R> dqsl, V3<R> dqsa, R k_alpha,
-                                                Block6<R>& B) {
-    V3<R> jl[3], ja[3];
-    R k[3], f[3];
-    primal_row_terms<P, R>(rs, du, oth, fetch, sqr, dqsl, dqsa, k_alpha, jl, ja, k, f);
-#pragma unroll
-    for (int s = 0; s < 3; ++s) stamp(B, jl[s], ja[s], k[s], f[s]);
 }
 template <class P, class R, class F>
 __device__ __forceinline__ void primal_row_f(const DevWorld<P, R>& w, uint32_t r, uint32_t oth, const F& fetch,
                                              Q4<R> sqr, V3<R> dqsl, V3<R> dqsa, R k_alpha, Block6<R>& B) {
-    primal_row_core<P, R>(w.rs[r], w.rd[r], oth, fetch, sqr, dqsl, dqsa, k_alpha, B);
-}
-template <class P, class R>
-__device__ __forceinline__ void primal_row(const DevWorld<P, R>& w, uint32_t r, uint32_t oth, int rd, Q4<R> sqr,
-                                           V3<R> dqsl, V3<R> dqsa, R k_alpha, Block6<R>& B) {
-    primal_row_f(w, r, oth, GlobalFetch<P, R>{w, rd}, sqr, dqsl, dqsa, k_alpha, B);
+    V3<R> jl[3], ja[3];
+    R k[3], f[3];
+    primal_row_terms<R>(w.rs[r], w.rd.rounded(r), oth, fetch, sqr, dqsl, dqsa, k_alpha, jl, ja, k, f);
+#pragma unroll
+    for (int s = 0; s < 3; ++s) stamp(B, jl[s], ja[s], k[s], f[s]);
 }
 
 // One joint seen from body i (avbd/src/lib.rs:425-537).
@@ -410,11 +481,11 @@ __device__ __forceinline__ void primal_joint(const DevWorld<P, R>& w, const DioC
 }
 
 // The same joint row from a JView: p_a - p_b is formed exactly as the
-// reference forms it (joint a's anchor point minus joint b's).  `op4`/`oq4`
+// reference forms it (joint a's anchor point minus joint b's).  `op4`/`oq`
 // are the other body's snapshot pose, loaded by the caller.
 template <class P, class R>
-__device__ __forceinline__ void primal_jview_p(const JView& jv, A4<P> op4, A4<P> oq4, V3<P> sp, Q4<P> sq,
-                                               Q4<R> sqr, Block6<R>& B) {
+__device__ __forceinline__ void primal_jview_p(const JView& jv, A4<P> op4, Q4<R> oq, V3<P> sp, Q4<R> sqr,
+                                               Block6<R>& B) {
     const bool is_a = !(jv.kind & kIsB);
     const uint32_t kind = jv.kind & ~kIsB;
     const V3<R> anc_s{R(jv.self_anchor.x), R(jv.self_anchor.y), R(jv.self_anchor.z)};
@@ -423,14 +494,14 @@ __device__ __forceinline__ void primal_jview_p(const JView& jv, A4<P> op4, A4<P>
     V3<R> delta;  // joint a's anchor point minus joint b's
     if constexpr (std::is_same<P, R>::value) {
         const V3<P> p_self = add(sp, r_self);
-        const V3<P> p_other = add(xyz(op4), rotate(quat(oq4), anc_o));
+        const V3<P> p_other = add(xyz(op4), rotate(oq, anc_o));
         delta = is_a ? sub(p_self, p_other) : sub(p_other, p_self);
     } else {
         // split mode: the position difference in P, the anchor offsets (small
         // body-frame vectors) rotated and differenced in R
-        const V3<R> r_other = rotate(castq<R>(quat(oq4)), anc_o);
-        delta = is_a ? add(cast3<R>(sub(sp, xyz(op4))), sub(r_self, r_other))
-                     : add(cast3<R>(sub(xyz(op4), sp)), sub(r_other, r_self));
+        const V3<R> r_other = rotate(oq, anc_o);
+        delta = is_a ? add(narrow3<R>(sub(sp, xyz(op4))), sub(r_self, r_other))
+                     : add(narrow3<R>(sub(xyz(op4), sp)), sub(r_other, r_self));
     }
     const R sign = is_a ? R(1) : R(-1);
     const R stiff = R(jv.other_anchor.w);
@@ -463,9 +534,8 @@ __device__ __forceinline__ void primal_jview_p(const JView& jv, A4<P> op4, A4<P>
 }
 
 template <class P, class R, class F>
-__device__ __forceinline__ void primal_jview_f(const JView& jv, const F& fetch, V3<P> sp, Q4<P> sq, Q4<R> sqr,
-                                               Block6<R>& B) {
-    primal_jview_p<P, R>(jv, fetch.pos(jv.other), fetch.rot(jv.other), sp, sq, sqr, B);
+__device__ __forceinline__ void primal_jview_f(const JView& jv, const F& fetch, V3<P> sp, Q4<R> sqr, Block6<R>& B) {
+    primal_jview_p<P, R>(jv, fetch.pos(jv.other), fetch.rot_r(jv.other), sp, sqr, B);
 }
 
 // What the primal of one body starts from besides its pose: its row list
@@ -474,7 +544,8 @@ template <class P, class R>
 struct BodyTask {
     uint32_t i, j0, n;
     A4<R> mdt2;
-    A4<P> ipos, irot;
+    A4<P> ipos;
+    A4<R> irot;
 };
 
 // The inertial start of a body's 6x6 system: diagonal M/dt^2, I/dt^2 and the
@@ -491,8 +562,8 @@ __device__ __forceinline__ void primal_inertia(const BodyTask<P, R>& b, V3<P> sp
     B.h[tri(3, 3)] = idt2.x;
     B.h[tri(4, 4)] = idt2.y;
     B.h[tri(5, 5)] = idt2.z;
-    const V3<R> rl = mulv(V3<R>{mdt2, mdt2, mdt2}, cast3<R>(sub(sp, xyz(b.ipos))));
-    const V3<R> ra = mulv(idt2, ang_diff(sqr, castq<R>(quat(b.irot))));
+    const V3<R> rl = mulv(V3<R>{mdt2, mdt2, mdt2}, narrow3<R>(sub(sp, xyz(b.ipos))));
+    const V3<R> ra = mulv(idt2, ang_diff(sqr, quat(b.irot)));
     B.g[0] = rl.x;
     B.g[1] = rl.y;
     B.g[2] = rl.z;
@@ -580,15 +651,24 @@ __device__ __forceinline__ void primal_finish(const S& bodies, uint32_t t, uint3
                                               Q4<P> sq, Q4<R> sqr, const JointsAhead& joints, Block6<R>& B) {
     for (uint32_t k = 0; k < joints.n; ++k) {
         const JView jv = S::kAhead && k == 0u ? joints.first : bodies.joint(t, i, k);
-        primal_jview_f<P, R>(jv, fetch, sp, sq, sqr, B);
+        primal_jview_f<P, R>(jv, fetch, sp, sqr, B);
     }
     R dx[6];
     solve6(B, dx);
-    const A4<P> np = pack(add(sp, cast3<P>(V3<R>{dx[0], dx[1], dx[2]})));
+    const A4<P> np = pack(add(sp, widen3<P>(V3<R>{dx[0], dx[1], dx[2]})));
     if constexpr (std::is_same<P, R>::value)
         fetch.store(i, np, packq(quat_step(sq, V3<P>{dx[3], dx[4], dx[5]})));
     else
-        fetch.store(i, np, packq(quat_step_split<P, R>(sq, V3<R>{dx[3], dx[4], dx[5]})));
+        fetch.store(i, np, packq(quat_step_split<P, R>(sq, sqr, V3<R>{dx[3], dx[4], dx[5]})));
+}
+
+// a body's own rotation rounded to R
+template <class R, class P, class F>
+__device__ __forceinline__ Q4<R> own_rot_r(const F& fetch, uint32_t i, Q4<P> q) {
+    if constexpr (std::is_same<P, R>::value)
+        return q;
+    else
+        return fetch.rot_r(i);
 }
 
 // avbd_primal for one body: reads the snapshot through `fetch` and stores
@@ -601,16 +681,15 @@ __device__ __forceinline__ void primal_body_f(const DevWorld<P, R>& w, uint32_t 
     const BodyTask<P, R> b = bodies.load(0);
     const V3<P> sp = xyz(fetch.pos(i));
     const Q4<P> sq = quat(fetch.rot(i));
-    const Q4<R> sqr = castq<R>(sq);
+    const Q4<R> sqr = own_rot_r<R>(fetch, i, sq);
     Block6<R> B;
     primal_inertia(b, sp, sqr, B);
     if (b.n) {
         // displacement since the step start: read only by contact rows
-        const V3<R> dqsl = cast3<R>(sub(sp, xyz(fetch.ipos(i))));
-        const V3<R> dqsa = ang_diff(sqr, castq<R>(quat(fetch.irot(i))));
+        const Moved<R> m = fetch.moved(i);
         const R k_alpha = R(1) - o.alpha;
         for (uint32_t j = b.j0; j < b.j0 + b.n; ++j)
-            primal_row_f(w, w.row_idx[j], w.row_oth[j], fetch, sqr, dqsl, dqsa, k_alpha, B);
+            primal_row_f(w, w.row_idx[j], w.row_oth[j], fetch, sqr, m.dl, m.da, k_alpha, B);
     }
     JointsAhead joints;
     joints.load(bodies, 0u, i);
@@ -619,7 +698,7 @@ __device__ __forceinline__ void primal_body_f(const DevWorld<P, R>& w, uint32_t 
 
 template <class P, class R>
 __device__ __forceinline__ void primal_body(const DevWorld<P, R>& w, uint32_t i, int rd, const SolveParams<R>& o) {
-    primal_body_f(w, i, o, GlobalFetch<P, R>{w, rd});
+    primal_body_f(w, i, o, GlobalFetch<P, R>{w, rd, 1 - rd});
 }
 
 // Tile variant: the CTA's T consecutive bodies stage their snapshot and
@@ -640,7 +719,7 @@ __global__ void __launch_bounds__(T, MINB) k_primal_tile(DevWorld<P, R> w, int r
     }
     __syncthreads();
     if (i < w.n) {
-        primal_body_f(w, i, o, TileFetch<P, R, T>{w, rd, lo, s_pos, s_rot, s_ipos, s_irot});
+        primal_body_f(w, i, o, TileFetch<P, R, T>{{w, rd, wr}, lo, s_pos, s_rot, s_ipos, s_irot});
     }
 }
 
@@ -658,31 +737,36 @@ __global__ void __launch_bounds__(BLOCK, MINB) k_primal(DevWorld<P, R> w, int rd
 // avbd_dual, avbd/src/lib.rs:565-663: the row's dual update from its bodies' new poses (a, and b unless the
 // row is against a container) and step-start poses.
 template <class P, class R>
-__device__ __forceinline__ RowDual<P, R> dual_update(const RowStatic<R>& rs, RowDual<P, R> du, A4<P> pa4, A4<P> qa4,
-                                                     A4<P> ia_p, A4<P> ia_q, bool has_b, A4<P> pb4, A4<P> qb4,
-                                                     A4<P> ib_p, A4<P> ib_q, const SolveParams<R>& o) {
-    V3<R> dal = cast3<R>(sub(xyz(pa4), xyz(ia_p)));
-    V3<R> daa = ang_diff(castq<R>(quat(qa4)), castq<R>(quat(ia_q)));
+__device__ __forceinline__ RowDual<P, R> dual_update(const RowStatic<R>& rs, RowDual<P, R> du, const Moved<R>& a,
+                                                     bool has_b, const Moved<R>& b, const SolveParams<R>& o) {
     V3<R> dbl{R(0), R(0), R(0)}, dba{R(0), R(0), R(0)}, rbw{R(0), R(0), R(0)};
     if (has_b) {
-        dbl = cast3<R>(sub(xyz(pb4), xyz(ib_p)));
-        dba = ang_diff(castq<R>(quat(qb4)), castq<R>(quat(ib_q)));
-        rbw = rotate(castq<R>(quat(qb4)), xyz(rs.rb));
+        dbl = b.dl;
+        dba = b.da;
+        rbw = rotate(b.q, xyz(rs.rb));
     }
-    V3<R> raw = rotate(castq<R>(quat(qa4)), xyz(rs.ra));
+    V3<R> raw = rotate(a.q, xyz(rs.ra));
     V3<R> r0 = xyz(rs.n), r1 = xyz(rs.t1), r2 = xyz(rs.t2);
     const R k_alpha = R(1) - o.alpha;
     R c0 = rs.ra.w * k_alpha, c1 = rs.rb.w * k_alpha, c2 = rs.t1.w * k_alpha;
-    c0 = c0 + (dot(r0, dal) + dot(cross(raw, r0), daa) - dot(r0, dbl) - dot(cross(rbw, r0), dba));
-    c1 = c1 + (dot(r1, dal) + dot(cross(raw, r1), daa) - dot(r1, dbl) - dot(cross(rbw, r1), dba));
-    c2 = c2 + (dot(r2, dal) + dot(cross(raw, r2), daa) - dot(r2, dbl) - dot(cross(rbw, r2), dba));
-    P f0, f1, f2, tm, bounds;
-    row_forces(du, rs.n.w, c0, c1, c2, f0, f1, f2, tm, bounds);
-    du.lambda.x = f0;
-    du.lambda.y = f1;
-    du.lambda.z = f2;
-    if (f0 < P(0)) du.penalty.x = fmin_(du.penalty.x + o.beta_lin * dabs(c0), o.penalty_max);
-    if (tm <= bounds) {
+    c0 = c0 + (dot(r0, a.dl) + dot(cross(raw, r0), a.da) - dot(r0, dbl) - dot(cross(rbw, r0), dba));
+    c1 = c1 + (dot(r1, a.dl) + dot(cross(raw, r1), a.da) - dot(r1, dbl) - dot(cross(rbw, r1), dba));
+    c2 = c2 + (dot(r2, a.dl) + dot(cross(raw, r2), a.da) - dot(r2, dbl) - dot(cross(rbw, r2), dba));
+    bool f0_neg, inside;
+    if constexpr (std::is_same<P, R>::value) {
+        P f0, f1, f2, tm, bounds;
+        row_forces(du, rs.n.w, c0, c1, c2, f0, f1, f2, tm, bounds);
+        du.lambda.x = f0;
+        du.lambda.y = f1;
+        du.lambda.z = f2;
+        f0_neg = f0 < P(0);
+        inside = tm <= bounds;
+    } else {
+        const RowDual<P, R> old = du;
+        row_forces_split(old, rs.n.w, c0, c1, c2, du.lambda.x, du.lambda.y, du.lambda.z, f0_neg, inside);
+    }
+    if (f0_neg) du.penalty.x = fmin_(du.penalty.x + o.beta_lin * dabs(c0), o.penalty_max);
+    if (inside) {
         du.penalty.y = fmin_(du.penalty.y + o.beta_lin * dabs(c1), o.penalty_max);
         du.penalty.z = fmin_(du.penalty.z + o.beta_lin * dabs(c2), o.penalty_max);
     }
@@ -746,7 +830,7 @@ __device__ __forceinline__ void primal_group(const DevWorld<P, R>& w, const S& b
         sp = xyz(fetch.pos(task.i));
         sq = quat(fetch.rot(task.i));
     }
-    const Q4<R> sqr = castq<R>(sq);
+    const Q4<R> sqr = live ? own_rot_r<R>(fetch, task.i, sq) : Q4<R>{R(0), R(0), R(0), R(1)};
     if (live) primal_inertia(task, sp, sqr, B);
     const uint32_t i = task.i, j0 = task.j0, n = task.n;
     uint32_t incl = n;  // inclusive sums of the row counts
@@ -760,8 +844,9 @@ __device__ __forceinline__ void primal_group(const DevWorld<P, R>& w, const S& b
         const R k_alpha = R(1) - o.alpha;
         V3<R> dqsl{R(0), R(0), R(0)}, dqsa{R(0), R(0), R(0)};
         if (n) {
-            dqsl = cast3<R>(sub(sp, xyz(fetch.ipos(i))));
-            dqsa = ang_diff(sqr, castq<R>(quat(fetch.irot(i))));
+            const Moved<R> m = fetch.moved(i);
+            dqsl = m.dl;
+            dqsa = m.da;
         }
         if (!kStaged || __reduce_max_sync(kAll, n) <= kGroupSerial * ((total + 31u) / 32u)) {
             for (uint32_t j = j0; j < j0 + n; ++j)
@@ -799,7 +884,8 @@ __device__ __forceinline__ void primal_group(const DevWorld<P, R>& w, const S& b
                     const uint32_t r = w.row_idx[j];
                     V3<R> jl[3], ja[3];
                     R k[3], ff[3];
-                    primal_row_terms<P, R>(w.rs[r], w.rd[r], w.row_oth[j], fetch, q, dl, da, k_alpha, jl, ja, k, ff);
+                    primal_row_terms<R>(w.rs[r], w.rd.rounded(r), w.row_oth[j], fetch, q, dl, da, k_alpha, jl, ja, k,
+                                        ff);
                     R* mine = stage + lane * kGroupStage;
 #pragma unroll
                     for (int t = 0; t < 3; ++t) {
@@ -876,7 +962,7 @@ template <class P, class R>
 __global__ void __launch_bounds__(kPrimalGroupWarps * 32, sizeof(R) == 4 ? 4 : 2)
     k_primal_group(DevWorld<P, R> w, int rd, uint32_t g, SolveParams<R> o) {
     pdl_enter();
-    primal_groups(w, w.dyn_list, w.n_dyn, g, o, GlobalFetch<P, R>{w, rd});
+    primal_groups(w, w.dyn_list, w.n_dyn, g, o, GlobalFetch<P, R>{w, rd, 1 - rd});
 }
 
 // variants: 0-4 k_primal over the dynamic-body list with {threads per CTA,
@@ -934,32 +1020,18 @@ inline void launch_primal(int variant, bool pdl, const DevWorld<P, R>& w, int rd
     }
 }
 
-// Buffer 0 read and written in place (the coloured Gauss-Seidel sweeps).
-template <class P, class R>
-struct InPlaceFetch {
-    const DevWorld<P, R>& w;
-    __device__ __forceinline__ A4<P> pos(uint32_t j) const { return w.pos[0][j]; }
-    __device__ __forceinline__ A4<P> rot(uint32_t j) const { return w.rot[0][j]; }
-    __device__ __forceinline__ A4<P> ipos(uint32_t j) const { return w.init_pos[j]; }
-    __device__ __forceinline__ A4<P> irot(uint32_t j) const { return w.init_rot[j]; }
-    __device__ __forceinline__ void store(uint32_t i, A4<P> p, A4<P> q) const {
-        w.pos[0][i] = p;
-        w.rot[0][i] = q;
-    }
-};
-
 // Coloured Gauss-Seidel sweep: bodies color_order[c0 .. c1) in place, grouped
 // or (worlds of jointed bodies, as in launch_primal) a thread each.
 template <class P, class R>
 __global__ void __launch_bounds__(kPrimalGroupWarps * 32, sizeof(R) == 4 ? 4 : 2)
     k_primal_color(DevWorld<P, R> w, uint32_t c0, uint32_t c1, uint32_t g, SolveParams<R> o) {
-    primal_groups(w, w.color_order + c0, c1 - c0, g, o, InPlaceFetch<P, R>{w});
+    primal_groups(w, w.color_order + c0, c1 - c0, g, o, GlobalFetch<P, R>{w, 0, 0});
 }
 template <class P, class R>
 __global__ void __launch_bounds__(128)
     k_primal_color_bodies(DevWorld<P, R> w, uint32_t c0, uint32_t c1, SolveParams<R> o) {
     for (uint32_t t = c0 + blockIdx.x * blockDim.x + threadIdx.x; t < c1; t += gridDim.x * blockDim.x)
-        primal_body_f(w, w.color_order[t], o, InPlaceFetch<P, R>{w});
+        primal_body_f(w, w.color_order[t], o, GlobalFetch<P, R>{w, 0, 0});
 }
 
 // avbd_dual, avbd/src/lib.rs:565-663, for row c; `fetch` reads the new state.
@@ -968,19 +1040,13 @@ __device__ __forceinline__ void dual_row_f(const DevWorld<P, R>& w, uint32_t c, 
                                            const SolveParams<R>& o) {
     const uint2 ab = w.ab[c];
     const bool has_b = ab.y != kContainer;
-    A4<P> pb{}, qb{}, ib{}, jb{};
-    if (has_b) {
-        pb = fetch.pos(ab.y);
-        qb = fetch.rot(ab.y);
-        ib = fetch.ipos(ab.y);
-        jb = fetch.irot(ab.y);
-    }
-    w.rd.put(c, dual_update<P, R>(w.rs[c], w.rd[c], fetch.pos(ab.x), fetch.rot(ab.x), fetch.ipos(ab.x),
-                                  fetch.irot(ab.x), has_b, pb, qb, ib, jb, o));
+    Moved<R> b{};
+    if (has_b) b = fetch.moved(ab.y);
+    w.rd.put(c, dual_update<P, R>(w.rs[c], w.rd[c], fetch.moved(ab.x), has_b, b, o));
 }
 template <class P, class R>
 __device__ __forceinline__ void dual_row(const DevWorld<P, R>& w, uint32_t c, int rd, const SolveParams<R>& o) {
-    dual_row_f(w, c, GlobalFetch<P, R>{w, rd}, o);
+    dual_row_f(w, c, GlobalFetch<P, R>{w, rd, rd}, o);
 }
 
 template <class P, class R>
@@ -1023,7 +1089,7 @@ __device__ __forceinline__ void recover_body_f(const DevWorld<P, R>& w, uint32_t
 }
 template <class P, class R>
 __device__ __forceinline__ void recover_body(const DevWorld<P, R>& w, uint32_t i, int rb, const SolveParams<R>& o) {
-    recover_body_f(w, i, GlobalFetch<P, R>{w, rb}, o);
+    recover_body_f(w, i, PoseFetch<P, R>{w, rb}, o);
 }
 
 template <class P, class R>

@@ -42,22 +42,69 @@ __host__ __device__ constexpr int chunk_threads() {
 }
 constexpr uint32_t kMaxClusterShift = 3;  // up to 8 CTAs (the portable cluster size)
 
-// shared memory of a CTA holding `cap` bodies: pos[2], rot[2], step-start pos
-// and rot (spread: then each warp's staging of the grouped primal), and the
-// groups' first bodies
+// Poses of a chunk in its CTAs' shared memory.  Every body a chunk's rows and
+// joints touch lies in the chunk (rows and joints never cross scenes).  With
+// one pose type: both pose buffers and the step start, displacements formed
+// here.  Split (P wider than R): what other bodies read -- positions, R
+// rotations and displacements, per buffer; a body's own P rotation and step
+// start stay in global memory.
+template <class P, class R>
+struct ChunkPoses {
+    static constexpr bool kSplit = sizeof(P) != sizeof(R);
+    // buffer b of an array at b * step
+    A4<P>* pos;
+    A4<P>* rot;
+    A4<P>* ipos;
+    A4<P>* irot;
+    A4<R>* rot_r;
+    A4<R>* moved_l;
+    V2<R>* moved_a;
+    uint32_t step;
+    // bytes a body; buffers: 2, or 1 in place (buffer 1 is buffer 0)
+    __host__ __device__ static constexpr size_t body_bytes(int buffers) {
+        return kSplit ? buffers * (sizeof(A4<P>) + 2 * sizeof(A4<R>) + sizeof(V2<R>))
+                      : (2 * buffers + 2) * sizeof(A4<P>);
+    }
+    // lays the arrays out from `base`; returns what follows them
+    __device__ __forceinline__ unsigned char* place(unsigned char* base, uint32_t cap, uint32_t buffers) {
+        auto take = [&](auto*& p, uint32_t n) {
+            p = reinterpret_cast<std::remove_reference_t<decltype(p)>>(base);
+            base += (size_t)n * cap * sizeof(*p);
+        };
+        step = buffers > 1u ? cap : 0u;
+        take(pos, buffers);
+        if constexpr (kSplit) {
+            take(rot_r, buffers);
+            take(moved_l, buffers);
+            take(moved_a, buffers);
+        } else {
+            take(rot, buffers);
+            take(ipos, 1u);
+            take(irot, 1u);
+        }
+        return base;
+    }
+    __device__ __forceinline__ void put_moved(uint32_t at, const Moved<R>& m) const {
+        rot_r[at] = packq(m.q);
+        moved_l[at] = pack(m.dl, m.da.x);
+        moved_a[at] = V2<R>{m.da.y, m.da.z};
+    }
+};
+// shared memory of a CTA holding `cap` bodies: the poses (spread: then each
+// warp's staging of the grouped primal), and the groups' first bodies
 template <class R>
 __host__ __device__ constexpr size_t spread_stage_words() {
     return chunk_threads<R, true>() / 32 * primal_group_words<R>();
 }
 template <class P, class R, bool kSpread>
 __host__ __device__ constexpr size_t chunk_smem_bytes(uint32_t cap) {
-    return (size_t)6 * cap * sizeof(A4<P>) + (kSpread ? spread_stage_words<R>() * sizeof(R) : 0) + (size_t)cap * 2;
+    return cap * ChunkPoses<P, R>::body_bytes(2) + (kSpread ? spread_stage_words<R>() * sizeof(R) : 0) + (size_t)cap * 2;
 }
 // coloured: one pose buffer (the sweeps are in place), colour, order and
 // selection arrays
 template <class P, class R, bool kSpread>
 __host__ __device__ constexpr size_t chunk_colored_smem_bytes(uint32_t cap) {
-    return (size_t)4 * cap * sizeof(A4<P>) + (kSpread ? spread_stage_words<R>() * sizeof(R) : 0) + (size_t)cap * 12 +
+    return cap * ChunkPoses<P, R>::body_bytes(1) + (kSpread ? spread_stage_words<R>() * sizeof(R) : 0) + (size_t)cap * 12 +
            (size_t)2 * (kMaxColors + 1) * 4;
 }
 // bodies of a chunk over all its CTAs, and of a CTA at most
@@ -116,6 +163,11 @@ __device__ __forceinline__ A4<double> peer_load(const A4<double>* p, uint32_t ra
     asm volatile("ld.shared::cluster.v2.f64 {%0, %1}, [%2];" : "=d"(v.z), "=d"(v.w) : "r"(a + 16u));
     return v;
 }
+__device__ __forceinline__ V2<float> peer_load(const V2<float>* p, uint32_t rank) {
+    V2<float> v;
+    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(peer_addr(p, rank)));
+    return v;
+}
 __device__ __forceinline__ uint32_t peer_load(const uint32_t* p, uint32_t rank) {
     uint32_t v;
     asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(peer_addr(p, rank)));
@@ -133,16 +185,12 @@ __device__ __forceinline__ void chunk_sync() {
     }
 }
 
-// Poses of a chunk in its CTAs' shared memory.  Every body a chunk's rows and
-// joints touch lies in the chunk (rows and joints never cross scenes).
-template <class P, bool kCluster>
+template <class P, class R, bool kCluster>
 struct ChunkFetch {
-    const A4<P>* sp;  // snapshot (read) buffer
-    const A4<P>* sq;
-    const A4<P>* si;  // step-start pose
-    const A4<P>* sr;
-    A4<P>* wp;        // the primal's output buffer
-    A4<P>* wq;
+    static constexpr bool kSplit = ChunkPoses<P, R>::kSplit;
+    const DevWorld<P, R>& w;
+    const ChunkPoses<P, R>& c;
+    uint32_t rd, wr;  // snapshot and output buffer, as offsets
     uint32_t lo, rank;
     SolveShape shape;
     template <class T>
@@ -155,17 +203,77 @@ struct ChunkFetch {
             return a[d];
         }
     }
-    __device__ __forceinline__ A4<P> pos(uint32_t j) const { return get(sp, j); }
-    __device__ __forceinline__ A4<P> rot(uint32_t j) const { return get(sq, j); }
-    __device__ __forceinline__ A4<P> ipos(uint32_t j) const { return get(si, j); }
-    __device__ __forceinline__ A4<P> irot(uint32_t j) const { return get(sr, j); }
-    // a body of this CTA: its new pose, once stored
-    __device__ __forceinline__ A4<P> new_pos(uint32_t i) const { return wp[kCluster ? shape.slot(i - lo) : i - lo]; }
-    __device__ __forceinline__ A4<P> new_rot(uint32_t i) const { return wq[kCluster ? shape.slot(i - lo) : i - lo]; }
-    __device__ __forceinline__ void store(uint32_t i, A4<P> p, A4<P> q) const {
-        const uint32_t s = kCluster ? shape.slot(i - lo) : i - lo;
-        wp[s] = p;
-        wq[s] = q;
+    __device__ __forceinline__ uint32_t slot(uint32_t i) const { return kCluster ? shape.slot(i - lo) : i - lo; }
+    __device__ __forceinline__ A4<P> pos(uint32_t j) const { return get(c.pos + rd, j); }
+    __device__ __forceinline__ A4<P> rot(uint32_t i) const {  // a body of this CTA
+        if constexpr (kSplit)
+            return w.rot[0][i];
+        else
+            return c.rot[rd + slot(i)];
+    }
+    __device__ __forceinline__ Q4<R> rot_r(uint32_t j) const {
+        if constexpr (kSplit)
+            return quat(get(c.rot_r + rd, j));
+        else
+            return quat(get(c.rot + rd, j));
+    }
+    __device__ __forceinline__ Moved<R> moved(uint32_t j) const {
+        if constexpr (kSplit)
+            return moved_of(get(c.rot_r + rd, j), get(c.moved_l + rd, j), get(c.moved_a + rd, j));
+        else
+            return moved_from<R>(get(c.pos + rd, j), quat(get(c.rot + rd, j)), get(c.ipos, j), get(c.irot, j));
+    }
+    __device__ __forceinline__ void store(uint32_t i, A4<P> p, A4<P> q) const {  // a body of this CTA
+        const uint32_t at = wr + slot(i);
+        c.pos[at] = p;
+        if constexpr (kSplit) {
+            w.rot[0][i] = q;
+            c.put_moved(at, moved_from<R>(p, narrowq<R>(quat(q)), w.init_pos[i], w.init_rot[i]));
+        } else {
+            c.rot[at] = q;
+        }
+    }
+    // avbd_init's result for slot s; buffer 1 holds the step start, read for
+    // static bodies and without any iteration
+    __device__ __forceinline__ void put(uint32_t i, uint32_t s, const InitPose<P>& p) const {
+        if (c.step) c.pos[c.step + s] = p.start_pos;
+        c.pos[s] = p.pos;
+        if constexpr (kSplit) {
+            w.rot[0][i] = p.rot;
+            w.init_pos[i] = p.start_pos;
+            w.init_rot[i] = p.start_rot;
+            const Moved<R> m = moved_from<R>(p.pos, narrowq<R>(quat(p.rot)), p.start_pos, p.start_rot);
+            if (c.step) c.put_moved(c.step + s, m);
+            c.put_moved(s, m);
+        } else {
+            if (c.step) c.rot[c.step + s] = p.start_rot;
+            c.rot[s] = p.rot;
+            c.ipos[s] = p.start_pos;
+            c.irot[s] = p.start_rot;
+        }
+    }
+    // the step-start pose of a body of this CTA
+    __device__ __forceinline__ A4<P> ipos(uint32_t i) const {
+        if constexpr (kSplit)
+            return w.init_pos[i];
+        else
+            return c.ipos[slot(i)];
+    }
+    __device__ __forceinline__ A4<P> irot(uint32_t i) const {
+        if constexpr (kSplit)
+            return w.init_rot[i];
+        else
+            return c.irot[slot(i)];
+    }
+    // avbd_recover, then the final pose (buffer offset `fin`) into global buffer 0
+    __device__ __forceinline__ void recover(uint32_t i, uint32_t fin, const SolveParams<R>& o) const {
+        recover_body_f(w, i, *this, o);
+        w.pos[0][i] = c.pos[fin + slot(i)];
+        if constexpr (kSplit) {
+            if (o.iterations == 0) w.rot[0][i] = w.init_rot[i];  // the pose before the warm start
+        } else {
+            w.rot[0][i] = c.rot[fin + slot(i)];
+        }
     }
 };
 
@@ -321,11 +429,11 @@ __device__ __forceinline__ void chunk_primal(const DevWorld<P, R>& w, const S& b
     }
 }
 
-// avbd_init for the CTA's bodies: `put(slot, InitPose)` for each.  Dynamic
-// bodies leave their constants and row lists at their list positions.
-template <class P, class R, class Put>
+// avbd_init for the CTA's bodies.  Dynamic bodies leave their constants and
+// row lists at their list positions.
+template <class P, class R, class F>
 __device__ __forceinline__ void chunk_init(const DevWorld<P, R>& w, const ChunkCta& c, const SolveShape& shape,
-                                           const SolveParams<R>& o, Put&& put) {
+                                           const SolveParams<R>& o, const F& fetch) {
     for (uint32_t s = threadIdx.x; s < shape.slots(c.nb); s += blockDim.x) {
         const uint32_t d = shape.body(s, c.rank);
         if (d >= c.nb) continue;
@@ -335,11 +443,11 @@ __device__ __forceinline__ void chunk_init(const DevWorld<P, R>& w, const ChunkC
         r.start_pos = r.pos = w.pos[0][i];
         r.start_rot = r.rot = w.rot[0][i];
         r.start_pos.w = P(0);
-        put(s, r);
+        fetch.put(i, s, r);
     }
     for (uint32_t t = c.dyn.x + threadIdx.x; t < c.dyn.y; t += blockDim.x) {
         const uint32_t i = w.dyn_list[t];
-        put(shape.slot(i - c.lo), init_pose(w, i, t, o));
+        fetch.put(i, shape.slot(i - c.lo), init_pose(w, i, t, o));
         const uint32_t j0 = w.row_off[i];
         w.solve.rows[t] = make_uint2(j0, w.row_off[i + 1] - j0);
     }
@@ -357,28 +465,17 @@ __global__ void __launch_bounds__(chunk_threads<R, kSpread>(), sizeof(R) == 4 &&
     __shared__ uint32_t s_cursor[2];
     __shared__ uint32_t s_warp[chunk_threads<R, kSpread>() / 32];
     pdl_enter();
-    // layout: pos parity 0, pos parity 1, rot parity 0, rot parity 1, step
-    // start pos, step start rot (parity b at s_pos + b * cap), staging
-    A4<P>* const s_pos = reinterpret_cast<A4<P>*>(chunk_smem);
-    A4<P>* const s_rot = s_pos + 2 * cap;
-    A4<P>* const s_ipos = s_pos + 4 * cap;
-    A4<P>* const s_irot = s_pos + 5 * cap;
+    // layout: poses, staging, the groups' first bodies
     const uint32_t tid = threadIdx.x, nt = blockDim.x;
-    R* const stage0 = reinterpret_cast<R*>(s_pos + 6 * cap);
+    ChunkPoses<P, R> poses;
+    R* const stage0 = reinterpret_cast<R*>(poses.place(chunk_smem, cap, 2));
     R* const stage = stage0 + (kSpread ? (tid >> 5) * primal_group_words<R>() : 0);
     uint16_t* const s_first = reinterpret_cast<uint16_t*>(stage0 + (kSpread ? spread_stage_words<R>() : 0));
     ChunkCta c = chunk_cta(chunks, dyn_runs, scenes, shape);
     chunk_row_bounds(w.ab, w.ctr, c, s_rows);
     if (tid < 2) s_cursor[tid] = 0u;
-    // the poses of both parities and the step start into shared memory
-    chunk_init(w, c, shape, o, [&](uint32_t s, const InitPose<P>& ip) {
-        s_pos[s] = ip.pos;
-        s_rot[s] = ip.rot;
-        s_pos[cap + s] = ip.start_pos;  // read for static bodies, and without any iteration
-        s_rot[cap + s] = ip.start_rot;
-        s_ipos[s] = ip.start_pos;
-        s_irot[s] = ip.start_rot;
-    });
+    using Fetch = ChunkFetch<P, R, kCluster>;
+    chunk_init(w, c, shape, o, Fetch{w, poses, 0u, cap, c.lo, c.rank, shape});
     chunk_sync<kCluster>();
     take_row_bounds(c, s_rows);
     const uint32_t groups = chunk_groups<kSpread>(w, c, s_first, s_warp);
@@ -388,30 +485,24 @@ __global__ void __launch_bounds__(chunk_threads<R, kSpread>(), sizeof(R) == 4 &&
         t = c.dyn.x + u;
         n = (k + 1u < groups ? s_first[k + 1u] : c.dyn.y - c.dyn.x) - u;
     };
-    using Fetch = ChunkFetch<P, kCluster>;
     for (uint32_t k = 0; k < o.iterations; ++k) {
         const uint32_t rd = (k & 1u) * cap, wr = cap - rd;
         if (tid == 0) s_cursor[(k + 1u) & 1u] = 0u;  // last used before the previous barrier
-        const Fetch f{s_pos + rd, s_rot + rd, s_ipos, s_irot, s_pos + wr, s_rot + wr, c.lo, c.rank, shape};
-        chunk_primal<kSpread>(w, ListBodies<P, R>{w}, groups, range, o, f, stage, &s_cursor[k & 1u]);
+        chunk_primal<kSpread>(w, ListBodies<P, R>{w}, groups, range, o, Fetch{w, poses, rd, wr, c.lo, c.rank, shape},
+                              stage, &s_cursor[k & 1u]);
         chunk_sync<kCluster>();
         if (!c.rows) continue;  // the same for all CTAs of the chunk
-        const Fetch fd{s_pos + wr, s_rot + wr, s_ipos, s_irot, nullptr, nullptr, c.lo, c.rank, shape};
+        const Fetch fd{w, poses, wr, wr, c.lo, c.rank, shape};
         for (uint32_t t = c.rank * nt + tid; t < c.rows; t += nt << shape.cl) dual_row_f(w, c.row(t), fd, o);
         chunk_sync<kCluster>();
     }
-    // avbd_recover from the final parity, and the final pose into buffer 0
-    const uint32_t fp = (o.iterations - 1u) % 2u;
-    const uint32_t rb = fp == 0 ? 1u : 0u;
-    const uint32_t fp_read = (o.iterations == 0 ? 0u : o.iterations - 1u) % 2u;
-    const uint32_t final_buf = 1u - fp_read;
-    const Fetch fr{s_pos + rb * cap, s_rot + rb * cap, s_ipos, s_irot, nullptr, nullptr, c.lo, c.rank, shape};
+    // avbd_recover from the last written buffer (none: the warm start), and
+    // the final pose
+    const uint32_t rb = (o.iterations & 1u) * cap, fin = o.iterations ? rb : cap;
+    const Fetch fr{w, poses, rb, rb, c.lo, c.rank, shape};
     for (uint32_t s = tid; s < shape.slots(c.nb); s += nt) {
         const uint32_t d = shape.body(s, c.rank);
-        if (d >= c.nb) continue;
-        recover_body_f(w, c.lo + d, fr, o);
-        w.pos[0][c.lo + d] = s_pos[final_buf * cap + s];
-        w.rot[0][c.lo + d] = s_rot[final_buf * cap + s];
+        if (d < c.nb) fr.recover(c.lo + d, fin, o);
     }
 }
 
@@ -452,12 +543,9 @@ __global__ void __launch_bounds__(chunk_threads<R, kSpread>(), sizeof(R) == 4 &&
     __shared__ uint32_t s_cursor[2];
     __shared__ uint32_t s_colored, s_ncolors, s_ndyn;
     pdl_enter();
-    A4<P>* const s_pos = reinterpret_cast<A4<P>*>(chunk_smem);
-    A4<P>* const s_rot = s_pos + cap;
-    A4<P>* const s_ipos = s_pos + 2 * cap;
-    A4<P>* const s_irot = s_pos + 3 * cap;
     const uint32_t tid = threadIdx.x, nt = blockDim.x;
-    R* const stage0 = reinterpret_cast<R*>(s_pos + 4 * cap);
+    ChunkPoses<P, R> poses;
+    R* const stage0 = reinterpret_cast<R*>(poses.place(chunk_smem, cap, 1));
     R* const stage = stage0 + (kSpread ? (tid >> 5) * primal_group_words<R>() : 0);
     uint32_t* const s_color =
         reinterpret_cast<uint32_t*>(stage0 + (kSpread ? spread_stage_words<R>() : 0));
@@ -479,15 +567,10 @@ __global__ void __launch_bounds__(chunk_threads<R, kSpread>(), sizeof(R) == 4 &&
         s_next[q] = 0;
     }
     // init (the in-place schedule reads and writes one buffer) and colours reset
-    chunk_init(w, c, shape, o, [&](uint32_t s, const InitPose<P>& ip) {
-        s_pos[s] = ip.pos;
-        s_rot[s] = ip.rot;
-        s_ipos[s] = ip.start_pos;
-        s_irot[s] = ip.start_rot;
-        s_color[s] = kNoColor;
-    });
+    const ChunkFetch<P, R, kCluster> f{w, poses, 0u, 0u, lo, c.rank, shape};
+    chunk_init(w, c, shape, o, f);
+    for (uint32_t s = tid; s < shape.slots(c.nb); s += nt) s_color[s] = kNoColor;
     chunk_sync<kCluster>();
-    const ChunkFetch<P, kCluster> f{s_pos, s_rot, s_ipos, s_irot, s_pos, s_rot, lo, c.rank, shape};  // in place
     // a value that every CTA of the chunk keeps at the same address, over all of them
     auto over = [&](const uint32_t* v, uint32_t start, auto&& join) {
         uint32_t r = start;
@@ -586,9 +669,7 @@ __global__ void __launch_bounds__(chunk_threads<R, kSpread>(), sizeof(R) == 4 &&
     for (uint32_t s = tid; s < shape.slots(c.nb); s += nt) {
         const uint32_t d = shape.body(s, c.rank);
         if (d >= c.nb) continue;
-        recover_body_f(w, lo + d, f, o);
-        w.pos[0][lo + d] = s_pos[s];
-        w.rot[0][lo + d] = s_rot[s];
+        f.recover(lo + d, 0u, o);
     }
     chunk_sync<kCluster>();  // peers may still be reading this CTA's counts
 }

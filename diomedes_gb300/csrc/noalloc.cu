@@ -206,7 +206,7 @@ __global__ void __launch_bounds__(128) k_na_primal(DevWorld<float, float> w, uin
         const V3<float> dqsa = ang_diff(sq, quat(w.init_rot[i]));
         const float k_alpha = 1.f - o.alpha;
         for (uint32_t j = w.row_off[i]; j < w.row_off[i + 1]; ++j)
-            primal_row(w, w.row_idx[j], w.row_oth[j], rd, sq, dqsl, dqsa, k_alpha, B);
+            primal_row_f(w, w.row_idx[j], w.row_oth[j], PoseFetch<float, float>{w, rd}, sq, dqsl, dqsa, k_alpha, B);
         for (uint32_t k = 0; k < w.n_joints; ++k) {
             const DioConstraint jt = w.joints[k];
             if (jt.a == i || jt.b == i) primal_joint(w, jt, i, rd, sp, sq, sq, B);
@@ -216,6 +216,11 @@ __global__ void __launch_bounds__(128) k_na_primal(DevWorld<float, float> w, uin
         w.pos[wr][i] = pack(add(sp, V3<float>{dx[0], dx[1], dx[2]}));
         w.rot[wr][i] = packq(quat_step(sq, V3<float>{dx[3], dx[4], dx[5]}));
     }
+}
+
+__global__ void __launch_bounds__(256) k_na_dual(DevWorld<float, float> w, uint32_t m, int rd, SolveParams<float> o) {
+    for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < m; c += gridDim.x * blockDim.x)
+        dual_row_f(w, c, PoseFetch<float, float>{w, rd}, o);
 }
 
 __global__ void k_na_pack(DevWorld<float, float> w, uint32_t n, int buf, const DioBodyState* st_in, float* pos3,
@@ -286,7 +291,7 @@ extern "C" int dio_avbd_solve_noalloc(const DioBodyState* state, const float* po
     w.friction = reinterpret_cast<float*>(base + kOffFric);
     w.rs = RowStatics<float>{reinterpret_cast<A4<float>*>(base + kOffRs), kNaMaxContacts};
     w.rd.penalty = reinterpret_cast<A4<float>*>(base + kOffRd);
-    w.rd.lambda = w.rd.penalty + kNaMaxContacts;
+    w.rd.lambda = w.rd.lambda_r = w.rd.penalty + kNaMaxContacts;
     w.ab = reinterpret_cast<uint2*>(base + kOffAb);
     w.row_oth = reinterpret_cast<uint32_t*>(base + kOffOth);
     w.row_off = const_cast<uint32_t*>(offsets);
@@ -320,7 +325,7 @@ extern "C" int dio_avbd_solve_noalloc(const DioBodyState* state, const float* po
     for (uint32_t k = 0; k < o.iterations; ++k) {
         int par = (int)(k % 2);
         k_na_primal<<<grid_for(n, 128), 128, 0, s>>>(w, n, par, 1 - par, o);
-        if (m) k_dual<float, float><<<grid_for(m, 256), 256, 0, s>>>(w, 0, m, nullptr, 1 - par, o);
+        if (m) k_na_dual<<<grid_for(m, 256), 256, 0, s>>>(w, m, 1 - par, o);
     }
     uint32_t fp = (o.iterations - 1u) % 2u;
     int rb = fp == 0 ? 1 : 0;
