@@ -688,7 +688,7 @@ class Engine final : public EngineBase {
     // fitted to measured solves (us for 10 iterations of the jointed batches
     // of scenes.batched, 2 to 1024 scenes): a cluster costs 56 plus 47 per
     // round of 256 bodies of a CTA and a little per body (coloured 139 more;
-    // FP64 poses 1.7 times that) whatever the number of scenes, until the clusters exceed what the
+    // split precision 1.35 times that, FP64 three times) whatever the number of scenes, until the clusters exceed what the
     // GPU holds; a packed CTA 18 plus 0.092 a body (coloured 1.6 times), the
     // SMs taking the next largest chunk as they fall free; packed only when
     // there are more chunks than SMs (contact-dense scenes are twice as slow
@@ -708,7 +708,7 @@ class Engine final : public EngineBase {
         solve_estimate_ = 0.0;
         if (scenes_host_.empty() || largest == 0 || largest > kSolveChunkCap) return 0;
         const bool colored = cfg_.solver_mode == DIO_SOLVER_COLORED;
-        const double wide = sizeof(P) == 4 ? 1.0 : 1.7;
+        const double wide = sizeof(P) == sizeof(R) ? (sizeof(P) == 4 ? 1.0 : 3.0) : 1.35;
         double best = 1e300;
         std::vector<uint2> chunks;
         auto consider = [&](bool spread, SolveShape sh, double us) {
@@ -1478,14 +1478,13 @@ class Engine final : public EngineBase {
         return true;
     }
     // the whole solve of a world step as one launch (k_solve_chunks)
-    // unless, with FP64 poses (half the bodies a CTA), the per-phase launches
-    // are the faster: 297 us plus 2 per 1,000 bodies (coloured 670 plus 3.1),
-    // measured as above
+    // unless, with FP64 poses, the per-phase launches are the faster: 285 us
+    // plus 1.5 per 1,000 bodies (coloured 500 plus 2.3), measured as above
     bool use_chunk_solve() const {
         if (!chunk_world_ || cfg_.batched_solver != DIO_SOLVE_AUTO) return false;
         if (sizeof(P) == 4) return true;
-        return solve_estimate_ <= (cfg_.solver_mode == DIO_SOLVER_COLORED ? 670.0 + 3.1e-3 * solve_total_
-                                                                           : 297.0 + 2.0e-3 * solve_total_);
+        return solve_estimate_ <= (cfg_.solver_mode == DIO_SOLVER_COLORED ? 500.0 + 2.3e-3 * solve_total_
+                                                                           : 285.0 + 1.5e-3 * solve_total_);
     }
     bool chunk_solve_possible() const override { return chunk_world_; }
     int solve_chunks(const SolveParams<R>& o) {

@@ -89,6 +89,38 @@ __device__ __forceinline__ V3<R> support(const ShapeR<R>& s, V3<R> d, const A4<R
     }
 }
 
+// Warp minimum / maximum of the finite values of the lanes with `has`, ties to
+// the lowest index: the index (0xFFFFFFFF: no lane has one).  FP32: the
+// values as ordered integers through two redux instructions (five rounds of
+// two shuffles took ten times as long); -0 is taken as +0, as a comparison
+// takes it.
+__device__ __forceinline__ uint32_t order_bits(float x) {
+    const uint32_t u = __float_as_uint(x + 0.f);
+    return u & 0x80000000u ? ~u : u | 0x80000000u;
+}
+template <bool kMax, class R>
+__device__ __forceinline__ uint32_t warp_best(bool has, R v, uint32_t index) {
+    constexpr uint32_t kAll = 0xFFFFFFFFu;
+    if constexpr (sizeof(R) == 4) {
+        // ordered bits of a number lie strictly between 0 and 2^32 - 1
+        const uint32_t key = order_bits(v);
+        const uint32_t best = kMax ? __reduce_max_sync(kAll, has ? key : 0u) : __reduce_min_sync(kAll, has ? key : kAll);
+        return __reduce_min_sync(kAll, has && key == best ? index : kAll);
+    } else {
+        uint32_t bi = has ? index : kAll;
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) {
+            const R ov = __shfl_xor_sync(kAll, v, off);
+            const uint32_t oi = __shfl_xor_sync(kAll, bi, off);
+            if (oi != kAll && (bi == kAll || (kMax ? ov > v : ov < v) || (ov == v && oi < bi))) {
+                v = ov;
+                bi = oi;
+            }
+        }
+        return bi;
+    }
+}
+
 // support() of a hull with the 32 lanes of a warp over its vertices (every
 // lane calls it with the same arguments and gets the same vertex): each
 // lane keeps its first maximum over vertices lane, lane + 32, ..., then the
@@ -109,15 +141,7 @@ __device__ __forceinline__ V3<R> support_warp(const ShapeR<R>& s, V3<R> d, const
             bi = i;
         }
     }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-        const R ov = __shfl_xor_sync(0xFFFFFFFFu, bv, off);
-        const uint32_t oi = __shfl_xor_sync(0xFFFFFFFFu, bi, off);
-        if (oi != 0xFFFFFFFFu && (bi == 0xFFFFFFFFu || ov > bv || (ov == bv && oi < bi))) {
-            bv = ov;
-            bi = oi;
-        }
-    }
+    bi = warp_best<true>(bi != 0xFFFFFFFFu, bv, bi);
     return xyz(hull[s.hf + bi]);
 }
 
@@ -481,6 +505,7 @@ __device__ bool gjk(const NB<R>& a, const NB<R>& b, const A4<R>* hull, Simplex<R
 constexpr int kEpaV = 68;   // 4 simplex points + one per iteration (64)
 constexpr int kEpaF = 256;  // face capacity (reference: 512; overflow flagged)
 constexpr int kEpaH = 256;  // horizon capacity (reference: 512; overflow flagged)
+constexpr int kEpaE = kEpaV * (kEpaV - 1) / 2;  // vertex pairs
 template <class R>
 __host__ __device__ constexpr int epa_warps() { return sizeof(R) == 8 ? 2 : 4; }  // FP64 polytopes are twice the size
 
@@ -490,17 +515,19 @@ struct EpaSmem {
     A4<R> w[kEpaV];
     A4<R> fnd[kEpaF];      // face normal xyz, distance w
     uint32_t fabc[kEpaF];  // a | b << 8 | c << 16
+    uint32_t vis[kEpaF];   // the faces that see the new vertex, in order
     uint32_t hor[kEpaH];   // a | b << 8
+    uint32_t edge[(kEpaE + 3) / 4];  // visible faces at each vertex pair (a byte each; zero between uses)
 };
 
 __device__ __forceinline__ uint32_t fa_(uint32_t f) { return f & 0xFF; }
 __device__ __forceinline__ uint32_t fb_(uint32_t f) { return (f >> 8) & 0xFF; }
 __device__ __forceinline__ uint32_t fc_(uint32_t f) { return (f >> 16) & 0xFF; }
 
-__device__ __forceinline__ bool edge_in_face(uint32_t a, uint32_t b, uint32_t f) {
-    uint32_t x = fa_(f), y = fb_(f), z = fc_(f);
-    return (x == a && y == b) || (y == a && z == b) || (z == a && x == b) || (x == b && y == a) ||
-           (y == b && z == a) || (z == b && x == a);
+// place of the unordered vertex pair (a, b), a != b, in the edge bytes
+__device__ __forceinline__ uint32_t edge_at(uint32_t a, uint32_t b) {
+    const uint32_t hi = max(a, b), lo = min(a, b);
+    return hi * (hi - 1u) / 2u + lo;
 }
 
 // add_face arithmetic, epa.rs:58-85.  Returns false for a degenerate face.
@@ -568,23 +595,36 @@ __device__ void face_contact(const EpaSmem<R>& S, A4<R> nd, uint32_t abc, V3<R>&
 }
 
 // Warp-cooperative epa, epa.rs:89-189.  All lanes of the warp call it with
-// the same arguments; returns true (uniformly) on convergence.
+// the same arguments; returns true (uniformly) on convergence.  One pass over
+// the faces per new vertex: faces that see it move to the visible list, the
+// others close up in place, both in order.  An edge of a visible face is on
+// the horizon when no other visible face has it (in either direction): the
+// visible faces are counted at each vertex pair, where testing each edge
+// against every visible face took most of an iteration.
+// Measured per iteration of one warp: about 4,700 cycles before (hull pairs),
+// bound by latency; see k_epa for whole launches.
 template <class R>
 __device__ bool epa_warp(EpaSmem<R>& S, const NB<R>& a, const NB<R>& b, const A4<R>* simplex, const A4<R>* hull,
                          uint32_t* err, V3<R>& normal, R& depth, V3<R>& pa, V3<R>& pb) {
+    constexpr uint32_t kAll = 0xFFFFFFFFu;
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t lt_mask = (1u << lane) - 1u;
     if (lane < 4) {
         S.v[lane] = simplex[lane];
         S.w[lane] = simplex[4 + lane];
     }
-    if (lane == 0) {
-        S.fnd[0] = A4<R>{R(0), R(0), R(0), R(0)};
-        S.fabc[0] = 0;
-    }
     __syncwarp();
     uint32_t nf = 0;
     uint32_t nv = 4;
+    // the lane's nearest face among those it wrote: first minimum in index order
+    R near_d = R(0);
+    uint32_t near_i = kAll;
+    auto wrote = [&](R d, uint32_t pos) {
+        if (!isnan(d) && (near_i == kAll || d < near_d)) {
+            near_d = d;
+            near_i = pos;
+        }
+    };
     {
         // the four initial faces, epa.rs:97-100, added in order
         const uint32_t init[4] = {0u | (1u << 8) | (2u << 16), 0u | (3u << 8) | (1u << 16),
@@ -593,12 +633,12 @@ __device__ bool epa_warp(EpaSmem<R>& S, const NB<R>& a, const NB<R>& b, const A4
         uint32_t abc;
         bool ok = false;
         if (lane < 4) ok = make_face(S, fa_(init[lane]), fb_(init[lane]), fc_(init[lane]), nd, abc);
-        uint32_t okm = __ballot_sync(0xFFFFFFFFu, ok);
-        __syncwarp();
+        const uint32_t okm = __ballot_sync(kAll, ok);
         if (ok) {
-            uint32_t pos = __popc(okm & lt_mask);
+            const uint32_t pos = __popc(okm & lt_mask);
             S.fnd[pos] = nd;
             S.fabc[pos] = abc;
+            wrote(nd.w, pos);
         }
         nf = __popc(okm);
         __syncwarp();
@@ -608,44 +648,20 @@ __device__ bool epa_warp(EpaSmem<R>& S, const NB<R>& a, const NB<R>& b, const A4
         // where the reference would emit its zero default face (a zero normal
         // at zero depth, whose tangents are NaN)
         if (nf == 0) return false;  // warp-uniform
-        // closest face: first minimum in index order (strict <)
-        uint32_t mi = 0;
-        {
-            R d0 = S.fnd[0].w;
-            if (nf > 0 && !isnan(d0)) {
-                R bv = R(0);
-                uint32_t bi = 0xFFFFFFFFu;
-                for (uint32_t i = lane; i < nf; i += 32) {
-                    R d = S.fnd[i].w;
-                    if (isnan(d)) continue;
-                    if (bi == 0xFFFFFFFFu || d < bv) {
-                        bv = d;
-                        bi = i;
-                    }
-                }
-#pragma unroll
-                for (int off = 16; off > 0; off >>= 1) {
-                    R ov = __shfl_xor_sync(0xFFFFFFFFu, bv, off);
-                    uint32_t oi = __shfl_xor_sync(0xFFFFFFFFu, bi, off);
-                    bool take = oi != 0xFFFFFFFFu && (bi == 0xFFFFFFFFu || ov < bv || (ov == bv && oi < bi));
-                    if (take) {
-                        bv = ov;
-                        bi = oi;
-                    }
-                }
-                mi = bi;
-            }
-        }
-        A4<R> mnd = S.fnd[mi];
-        uint32_t mabc = S.fabc[mi];
+        // closest face: first minimum in index order (strict <); the serial
+        // scan starts from face 0, which a NaN distance there keeps
+        uint32_t mi = warp_best<false>(near_i != kAll, near_d, near_i);
+        if (isnan(S.fnd[0].w)) mi = 0;
+        const A4<R> mnd = S.fnd[mi];
+        const uint32_t mabc = S.fabc[mi];
         V3<R> sp, sw;
         support_witness_warp(a, b, xyz(mnd), hull, sp, sw, lane);
-        R sd = dot(xyz(mnd), sp);
+        const R sd = dot(xyz(mnd), sp);
         if (sd - mnd.w < R(1e-4)) {
             face_contact(S, mnd, mabc, normal, depth, pa, pb);
             return true;
         }
-        uint32_t ni = nv;
+        const uint32_t ni = nv;
         if (ni >= 256u) {
             face_contact(S, mnd, mabc, normal, depth, pa, pb);
             return true;
@@ -655,115 +671,104 @@ __device__ bool epa_warp(EpaSmem<R>& S, const NB<R>& a, const NB<R>& b, const A4
             S.w[ni] = pack(sw);
         }
         nv += 1;
-        __syncwarp();
-        // visibility masks (one 32-bit ballot per chunk of faces)
-        uint32_t vm[kEpaF / 32];
-#pragma unroll
-        for (int c = 0; c < kEpaF / 32; ++c) {
-            vm[c] = 0u;
-            if (c * 32 >= (int)nf) continue;  // warp-uniform
-            uint32_t i = c * 32 + lane;
-            bool vis = false;
+        // faces that see the vertex, and the others closed up
+        near_i = kAll;
+        uint32_t kept = 0, nvis = 0;
+        for (uint32_t c = 0; c < nf; c += 32u) {
+            const uint32_t i = c + lane;
+            A4<R> f{};
+            uint32_t abc = 0;
+            bool vis = false, keep = false;
             if (i < nf) {
-                A4<R> f = S.fnd[i];
-                vis = dot(xyz(f), sub(sp, xyz(S.v[fa_(S.fabc[i])]))) > R(0);
+                f = S.fnd[i];
+                abc = S.fabc[i];
+                vis = dot(xyz(f), sub(sp, xyz(S.v[fa_(abc)]))) > R(0);
+                keep = !vis;
             }
-            vm[c] = __ballot_sync(0xFFFFFFFFu, vis);
+            const uint32_t vm = __ballot_sync(kAll, vis), km = __ballot_sync(kAll, keep);  // all have read
+            if (vis) S.vis[nvis + __popc(vm & lt_mask)] = abc;
+            if (keep) {
+                const uint32_t pos = kept + __popc(km & lt_mask);
+                S.fnd[pos] = f;
+                S.fabc[pos] = abc;
+                wrote(f.w, pos);
+            }
+            nvis += __popc(vm);
+            kept += __popc(km);
+            __syncwarp();
         }
-        // horizon: edges of visible faces not shared with another visible face
+        nf = kept;
+        // visible faces at each of their edges
+        for (uint32_t c = lane; c < nvis; c += 32u) {
+            const uint32_t f = S.vis[c], x = fa_(f), y = fb_(f), z = fc_(f);
+            const uint32_t e[3] = {edge_at(x, y), edge_at(y, z), edge_at(z, x)};
+#pragma unroll
+            for (int k = 0; k < 3; ++k) atomicAdd(&S.edge[e[k] >> 2], 1u << (8u * (e[k] & 3u)));
+        }
+        __syncwarp();
+        // horizon: edges of one visible face, in face and edge order
         uint32_t hc = 0;
-        for (int c = 0; c < kEpaF / 32; ++c) {
-            if (c * 32 >= (int)nf) break;
-            uint32_t i = c * 32 + lane;
+        for (uint32_t c = 0; c < nvis; c += 32u) {
             uint32_t my[3];
             uint32_t k = 0;
-            if ((vm[c] >> lane) & 1u) {
-                uint32_t f = S.fabc[i];
-                uint32_t e[3][2] = {{fa_(f), fb_(f)}, {fb_(f), fc_(f)}, {fc_(f), fa_(f)}};
-                for (int ee = 0; ee < 3; ++ee) {
-                    bool shared = false;
-                    for (int cc = 0; cc < kEpaF / 32 && !shared; ++cc) {
-                        uint32_t m = vm[cc];
-                        while (m) {
-                            uint32_t bit = __ffs(m) - 1;
-                            m &= m - 1;
-                            uint32_t j = cc * 32 + bit;
-                            if (j == i) continue;
-                            if (edge_in_face(e[ee][0], e[ee][1], S.fabc[j])) {
-                                shared = true;
-                                break;
-                            }
-                        }
-                    }
-                    if (!shared) my[k++] = e[ee][0] | (e[ee][1] << 8);
+            if (c + lane < nvis) {
+                const uint32_t f = S.vis[c + lane], v[4] = {fa_(f), fb_(f), fc_(f), fa_(f)};
+#pragma unroll
+                for (int q = 0; q < 3; ++q) {
+                    const uint32_t e = edge_at(v[q], v[q + 1]);
+                    my[q] = v[q] | (v[q + 1] << 8);
+                    if (((S.edge[e >> 2] >> (8u * (e & 3u))) & 0xFFu) == 1u) k |= 1u << q;
                 }
             }
-            // order-preserving append (inclusive warp scan of k)
-            uint32_t incl = k;
+            // order-preserving append: one ballot per edge
+            const uint32_t b0 = __ballot_sync(kAll, k & 1u), b1 = __ballot_sync(kAll, k & 2u),
+                           b2 = __ballot_sync(kAll, k & 4u);
+            uint32_t at = hc + __popc(b0 & lt_mask) + __popc(b1 & lt_mask) + __popc(b2 & lt_mask);
 #pragma unroll
-            for (int off = 1; off < 32; off <<= 1) {
-                uint32_t t = __shfl_up_sync(0xFFFFFFFFu, incl, off);
-                if (lane >= (uint32_t)off) incl += t;
-            }
-            uint32_t total = __shfl_sync(0xFFFFFFFFu, incl, 31);
-            uint32_t base = hc + incl - k;
-            for (uint32_t t = 0; t < k; ++t)
-                if (base + t < (uint32_t)kEpaH) S.hor[base + t] = my[t];
-            hc += total;
+            for (int q = 0; q < 3; ++q)
+                if ((k >> q) & 1u) {
+                    if (at < (uint32_t)kEpaH) S.hor[at] = my[q];
+                    ++at;
+                }
+            hc += __popc(b0) + __popc(b1) + __popc(b2);
         }
         if (hc > (uint32_t)kEpaH) {
             if (lane == 0) atomicOr(err, kErrEpaHorizon);
             hc = kEpaH;
         }
         __syncwarp();
-        // compact the kept (invisible) faces in place, preserving order
-        uint32_t wr = 0;
-        for (int c = 0; c < kEpaF / 32; ++c) {
-            if (c * 32 >= (int)nf) break;
-            uint32_t i = c * 32 + lane;
-            bool keep = i < nf && !((vm[c] >> lane) & 1u);
-            A4<R> f;
-            uint32_t fabc = 0;
-            if (keep) {
-                f = S.fnd[i];
-                fabc = S.fabc[i];
-            }
-            uint32_t km = __ballot_sync(0xFFFFFFFFu, keep);
-            __syncwarp();
-            if (keep) {
-                uint32_t pos = wr + __popc(km & lt_mask);
-                S.fnd[pos] = f;
-                S.fabc[pos] = fabc;
-            }
-            wr += __popc(km);
-            __syncwarp();
+        for (uint32_t c = lane; c < nvis; c += 32u) {
+            const uint32_t f = S.vis[c], x = fa_(f), y = fb_(f), z = fc_(f);
+            S.edge[edge_at(x, y) >> 2] = 0u;
+            S.edge[edge_at(y, z) >> 2] = 0u;
+            S.edge[edge_at(z, x) >> 2] = 0u;
         }
-        nf = wr;
         // stitch the horizon to the new vertex (degenerate faces dropped)
-        for (uint32_t c = 0; c * 32 < hc; ++c) {
-            uint32_t h = c * 32 + lane;
+        for (uint32_t c = 0; c < hc; c += 32u) {
+            const uint32_t h = c + lane;
             A4<R> nd;
             uint32_t abc = 0;
             bool ok = false;
             if (h < hc) {
-                uint32_t e = S.hor[h];
+                const uint32_t e = S.hor[h];
                 ok = make_face(S, ni, e & 0xFF, (e >> 8) & 0xFF, nd, abc);
             }
-            uint32_t okm = __ballot_sync(0xFFFFFFFFu, ok);
-            uint32_t pos = nf + __popc(okm & lt_mask);
+            const uint32_t okm = __ballot_sync(kAll, ok);
+            const uint32_t pos = nf + __popc(okm & lt_mask);
             if (ok && pos < (uint32_t)kEpaF) {
                 S.fnd[pos] = nd;
                 S.fabc[pos] = abc;
+                wrote(nd.w, pos);
             }
-            uint32_t add_n = __popc(okm);
+            const uint32_t add_n = __popc(okm);
             if (nf + add_n > (uint32_t)kEpaF) {
                 if (lane == 0) atomicOr(err, kErrEpaFaces);
                 nf = kEpaF;
             } else {
                 nf += add_n;
             }
-            __syncwarp();
         }
+        __syncwarp();
     }
     return false;
 }

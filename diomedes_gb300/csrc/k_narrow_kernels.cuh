@@ -152,6 +152,7 @@ __global__ void __launch_bounds__(32 * epa_warps<R>(), 4) k_epa(DevWorld<P, R> w
     const uint32_t lane = threadIdx.x & 31;
     EpaSmem<R>& S = smem[warp];
     if (lane == 0) mbar_init(&mbar[warp], 1);
+    for (uint32_t e = lane; e < sizeof(S.edge) / 4; e += 32) S.edge[e] = 0u;
     __syncwarp();
     uint32_t parity = 0;
     uint32_t nw = w.ctr->epa_work;
