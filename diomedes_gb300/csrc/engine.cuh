@@ -189,6 +189,7 @@ struct DevWorld {
     A4<P>* origin;  // per-scene detection origin (split precision rebase)
     const A4<R>* walls;  // per scene, 6 container walls: outward normal xyz, plane offset w
     const A4<R>* hull;  // hull vertex pool
+    const R* hull_bound;  // L1 bounding radius of each hull body, or null
     // broad phase
     A4<R>* aabb_min;
     A4<R>* aabb_max;
@@ -283,10 +284,10 @@ __device__ __forceinline__ uint32_t warp_append(uint32_t* cursor) {
 
 // cluster: CTAs per thread-block cluster (0: none)
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_clusters(bool pdl, uint32_t cluster, void (*kern)(KArgs...), int grid, int block, size_t smem,
-                                   cudaStream_t s, Args&&... args) {
+inline cudaError_t launch_clusters(bool pdl, uint32_t cluster, void (*kern)(KArgs...), dim3 grid, int block,
+                                   size_t smem, cudaStream_t s, Args&&... args) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)grid);
+    cfg.gridDim = grid;
     cfg.blockDim = dim3((unsigned)block);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
@@ -309,7 +310,11 @@ inline cudaError_t launch_clusters(bool pdl, uint32_t cluster, void (*kern)(KArg
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_k(bool pdl, void (*kern)(KArgs...), int grid, int block, size_t smem, cudaStream_t s,
                             Args&&... args) {
-    return launch_clusters(pdl, 0u, kern, grid, block, smem, s, std::forward<Args>(args)...);
+    return launch_clusters(pdl, 0u, kern, dim3((unsigned)grid), block, smem, s, std::forward<Args>(args)...);
+}
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_grid(bool pdl, void (*kern)(KArgs...), dim3 grid, int block, cudaStream_t s, Args&&... args) {
+    return launch_clusters(pdl, 0u, kern, grid, block, 0, s, std::forward<Args>(args)...);
 }
 
 }  // namespace dio

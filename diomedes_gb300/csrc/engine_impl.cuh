@@ -38,14 +38,6 @@ namespace dio {
 // small kernels used by the pipeline ------------------------------------
 static __global__ void k_set_u32(uint32_t* dst, uint32_t v) { *dst = v; }
 static __global__ void k_copy_u32(uint32_t* dst, const uint32_t* src) { *dst = *src; }
-static __global__ void k_sum_rows(Counters* c, const uint32_t* pair_rows, const uint32_t* cont_rows, uint32_t max_rows) {
-    pdl_enter();
-    c->pair_rows = *pair_rows;
-    c->container_rows = *cont_rows;
-    uint64_t t = (uint64_t)*pair_rows + *cont_rows;
-    c->rows = t > max_rows ? max_rows : (uint32_t)t;
-    if (t > max_rows) c->error_flags |= kErrRowOverflow;
-}
 static __global__ void k_pairs_total(Counters* c, const uint32_t* total, uint32_t max_pairs) {
     pdl_enter();
     c->pairs = *total;
@@ -505,6 +497,7 @@ class Engine final : public EngineBase {
         DIO_TRY(alloc(&w_.friction, N));
         DIO_TRY(alloc(&w_.shape, N));
         DIO_TRY(alloc(&w_.scene, N));
+        DIO_TRY(alloc(&hull_bound_, N));
         DIO_TRY(alloc(&origin_, S));
         DIO_TRY(alloc(&walls_, 6ull * S));
         w_.walls = walls_;
@@ -577,6 +570,7 @@ class Engine final : public EngineBase {
         DIO_TRY(alloc(&counts_, CNT));
         DIO_TRY(alloc(&offsets_, CNT));
         DIO_TRY(alloc(&counts2_, (size_t)N + 2));
+        DIO_TRY(alloc(&incident_, (size_t)N + 2));
         DIO_TRY(alloc(&offsets2_, (size_t)N + 2));
         DIO_TRY(alloc(&scenes_, S));
         DIO_TRY(alloc(&chunks_, S));
@@ -946,7 +940,7 @@ class Engine final : public EngineBase {
             if (n_slots)
                 DIO_CK(cudaMemcpyAsync(w_.slots, slots, (size_t)n_slots * sizeof(DioContactOut), cudaMemcpyHostToDevice,
                                        stream_));
-            DIO_TRY(build_rows(opts_prep(*options), n_slots, 1, nullptr, n));
+            DIO_TRY(build_rows(opts_prep(*options), n_slots, 1, nullptr, n, WarmStart<P, R>{}, nullptr));
             DIO_TRY(pull_counters());
             uint32_t M = hctr_->rows;
             *m = M;
@@ -1109,6 +1103,8 @@ class Engine final : public EngineBase {
             DIO_CK(cudaStreamSynchronize(stream_));
         }
         w_.n = n;
+        if (n) k_hull_bounds<P, R><<<grid_for(n, 128), 128, 0, stream_>>>(w_, n, hull_bound_);
+        w_.hull_bound = hull_bound_;  // read for hull bodies only
         DIO_CK(cudaMemsetAsync(ctr_, 0, sizeof(Counters), stream_));
         DIO_TRY(upload_joints(d->constraints, d->n_constraints, n));
         // the scene-chunk solve needs every scene in a chunk and every joint
@@ -1718,35 +1714,26 @@ class Engine final : public EngineBase {
 
     // Rows from `groups` groups of `per` slots (+ container rows for bodies).
     // src: the narrow slots the pair rows come from (w_.slots, or the
-    // previous step's with contact_lag)
+    // previous step's with contact_lag); incident: CSR counters (k_rows)
     int build_rows(const PrepParams<R>& o, uint32_t groups, uint32_t per, const uint32_t* groups_dev, uint32_t n,
-                   const Slot<R>* src = nullptr) {
-        uint32_t G = groups;
+                   const WarmStart<P, R>& warm, uint32_t* incident, const Slot<R>* src = nullptr) {
+        const uint32_t G = groups;
         if (!src) src = w_.slots;
+        // a thread a body or group, or (a device count) strided over a fixed grid
+        const uint64_t items = (uint64_t)n + (groups_dev ? std::min<uint64_t>(G, (uint64_t)sms_ * 1024u) : G);
+        DIO_CK(launch_k(pdl(), k_row_counts<P, R>, grid_for(items, 128), 128, 0, stream_, w_, src, per, groups_dev, G, n,
+                        o, counts_, counts2_, incident));
         if (G) {
-            // grid-stride over the live groups (a device count: fixed grids)
-            DIO_CK(launch_k(pdl(), k_slot_count<R>, std::min(grid_for(G, 256), sms_ * 8), 256, 0, stream_, src, per,
-                            groups_dev, G, counts_));
             // offsets of the live groups, the total at offsets_[G]
-            DIO_CK(ss_.scan(counts_, offsets_, G, pdl(), stream_, groups_dev, offsets_ + G));
-            DIO_CK(launch_k(pdl(), k_slot_rows<P, R>, std::min(grid_for(G, 128), sms_ * 16), 128, 0, stream_, w_, src,
-                            per, groups_dev, G, (const uint32_t*)offsets_, o));
+            DIO_CK(ss_.scan_both(ScanJob{counts_, offsets_, G, groups_dev, nullptr, offsets_ + G},
+                                 ScanJob{counts2_, offsets2_, n + 1, nullptr, nullptr, nullptr}, pdl(), stream_));
         } else {
             DIO_CK(cudaMemsetAsync(offsets_, 0, 4, stream_));
+            DIO_CK(ss_.scan(counts2_, offsets2_, n + 1, false, stream_));
         }
-        const uint32_t* pair_rows = offsets_ + G;
-        if (n) {
-            DIO_CK(launch_k(pdl() && G, k_cont_count<P, R>, grid_for(n, 128), 128, 0, stream_, w_, 0u, n, o, counts2_));
-            DIO_CK(ss_.scan(counts2_, offsets2_, n + 1, pdl(), stream_));
-            // clears counts2_ for the CSR count of finish_rows_world
-            DIO_CK(launch_k(pdl(), k_cont_rows<P, R>, grid_for(n, 128), 128, 0, stream_, w_, 0u, n, o,
-                            (const uint32_t*)offsets2_, pair_rows, counts2_));
-        } else {
-            DIO_CK(cudaMemsetAsync(offsets2_, 0, 4, stream_));
-        }
-        DIO_CK(launch_k(pdl() && n, k_sum_rows, 1, 1, 0, stream_, ctr_, pair_rows, (const uint32_t*)(offsets2_ + n),
-                        w_.max_rows));
-        launches_ += 5;
+        DIO_CK(launch_k(pdl(), k_rows<P, R>, grid_for(items, 128), 128, 0, stream_, w_, src, per, groups_dev, G, n, o,
+                        (const uint32_t*)offsets_, (const uint32_t*)offsets2_, warm, incident));
+        launches_ += 2;
         return DIO_OK;
     }
 
@@ -2134,9 +2121,10 @@ class Engine final : public EngineBase {
     // the pair rows), alternating with the row buffers
     void set_slots() { w_.slots = cfg_.contact_lag && slots_[1] ? slots_[cur_] : slots_[0]; }
     int build_world_rows(const PrepParams<R>& pp, uint32_t n) {
-        if (cfg_.contact_lag && slots_[1])
-            return build_rows(pp, cap_.max_pairs, cfg_.contacts_per_pair, &ctr_->prev_pairs, n, slots_[1 - cur_]);
-        return build_rows(pp, cap_.max_pairs, cfg_.contacts_per_pair, &ctr_->pairs, n);
+        const bool lag = cfg_.contact_lag && slots_[1];
+        const WarmStart<P, R> warm{true, ab_[1 - cur_], rd_[1 - cur_], ctr_};
+        return build_rows(pp, cap_.max_pairs, cfg_.contacts_per_pair, lag ? &ctr_->prev_pairs : &ctr_->pairs, n, warm,
+                          incident_, lag ? slots_[1 - cur_] : w_.slots);
     }
     int step_body_dev(const DioAvbdOptions& opt) {
         struct WorldStep {  // the flag holds for this step's launches only
@@ -2161,7 +2149,7 @@ class Engine final : public EngineBase {
         span_end(e, 3);
         e = span_begin();
         DIO_TRY(build_world_rows(pp, n));
-        DIO_TRY(finish_rows_world(pp, n));
+        DIO_TRY(finish_rows_world(n));
         span_end(e, 4);
         SolveParams<R> so = solve_params(opt.dt, opt.gravity, opt.alpha, opt.beta_lin, opt.penalty_max, opt.iterations);
         e = span_begin();
@@ -2190,7 +2178,7 @@ class Engine final : public EngineBase {
         span_end(e, 3);
         e = span_begin();
         DIO_TRY(build_world_rows(pp, n));
-        DIO_TRY(finish_rows_world(pp, n));
+        DIO_TRY(finish_rows_world(n));
         span_end(e, 4);
         DIO_TRY(color_world(n));
         SolveParams<R> so = solve_params(opt.dt, opt.gravity, opt.alpha, opt.beta_lin, opt.penalty_max, opt.iterations);
@@ -2281,25 +2269,18 @@ class Engine final : public EngineBase {
         return DIO_OK;
     }
 
-    // warm start + decay + dynamic-body CSR, all bounded by device counts
-    int finish_rows_world(const PrepParams<R>& o, uint32_t n) {
-        int pb = 1 - cur_;
+    // dynamic-body CSR, bounded by device counts; incident_ holds each body's
+    // rows (k_rows)
+    int finish_rows_world(uint32_t n) {
         const int gf = std::min(grid_for(cap_.max_contacts, 256), sms_ * 8);
-        DIO_CK(launch_k(pdl(), k_warm_sections<P, R>, gf, 256, 0, stream_, w_, (const uint2*)ab_[pb],
-                        rd_[pb], o));
-        // counts2_ was cleared by k_cont_rows (build_rows, bodies [0, n))
-        if (!n) DIO_CK(cudaMemsetAsync(counts2_, 0, 4, stream_));
-        DIO_CK(launch_k(pdl() && n, k_csr_count_dyn<P, R>, gf, 256, 0, stream_, w_, counts2_));
-        DIO_CK(ss_.scan(counts2_, w_.row_off, n + 1, pdl(), stream_));
+        DIO_CK(ss_.scan(incident_, w_.row_off, n + 1, pdl(), stream_));
         // takes the counts back to zero
-        DIO_CK(launch_k(pdl(), k_csr_scatter_dyn<P, R>, gf, 256, 0, stream_, w_, counts2_));
-        int gn = grid_for(n, 256);
-        DIO_CK(launch_k(pdl(), k_sort_segments, gn, 256, 0, stream_, (const uint32_t*)w_.row_off, n, w_.max_incid,
-                        w_.row_idx, lb_long_, &ctr_->long_count));
-        DIO_CK(launch_k(pdl(), k_sort_long, sms_, 512, 0, stream_, (const uint32_t*)w_.row_off, w_.row_idx,
-                        (const uint32_t*)lb_long_, (const uint32_t*)&ctr_->long_count, &ctr_->error_flags));
-        DIO_CK(launch_k(pdl(), k_csr_other_dyn<P, R>, gn, 256, 0, stream_, w_));
-        launches_ += 6;
+        DIO_CK(launch_k(pdl(), k_csr_scatter_dyn<P, R>, gf, 256, 0, stream_, w_, incident_));
+        DIO_CK(launch_k(pdl(), k_csr_finish_dyn<P, R>, grid_for(n, 128), 128, 0, stream_, w_, lb_long_,
+                        &ctr_->long_count));
+        DIO_CK(launch_k(pdl(), k_csr_finish_long<P, R>, sms_, 512, 0, stream_, w_, (const uint32_t*)lb_long_,
+                        (const uint32_t*)&ctr_->long_count));
+        launches_ += 3;
         return DIO_OK;
     }
 
@@ -2424,6 +2405,7 @@ class Engine final : public EngineBase {
     uint32_t ncolors_ = 0;
     uint32_t color_off_h_[kMaxColors + 1] = {};
     uint32_t *counts_ = nullptr, *offsets_ = nullptr, *counts2_ = nullptr, *offsets2_ = nullptr;
+    uint32_t* incident_ = nullptr;  // rows of each dynamic body
     SceneDesc* scenes_ = nullptr;
     std::vector<SceneDesc> scenes_host_;
     bool chunk_world_ = false;  // every scene in a solve chunk, joints inside scenes
@@ -2461,6 +2443,7 @@ class Engine final : public EngineBase {
     A4<P>* origin_ = nullptr;
     A4<R>* walls_ = nullptr;
     A4<R>* hull_ = nullptr;
+    R* hull_bound_ = nullptr;
     Counters* ctr_ = nullptr;
     Counters* hctr_ = nullptr;
     ScanSort ss_;  // prefix sums and radix sorts

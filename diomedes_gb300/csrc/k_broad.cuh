@@ -22,7 +22,19 @@ __device__ __forceinline__ void body_aabb(const NB<R>& b, const A4<R>* hull, V3<
     const V3<R> X{R(1), R(0), R(0)}, Y{R(0), R(1), R(0)}, Z{R(0), R(0), R(1)};
     mn = b.pos;
     mx = b.pos;
-    V3<R> sx = ws(X), snx = ws(neg(X)), sy = ws(Y), sny = ws(neg(Y)), sz = ws(Z), snz = ws(neg(Z));
+    V3<R> sx, snx, sy, sny, sz, snz;
+    if (b.shape.tag == DIO_SHAPE_HULL && b.shape.hc && hull) {
+        // the six queries in one pass over the vertices
+        const Q4<R> qc = conj(b.rot);
+        const V3<R> d[6] = {rotate(qc, X), rotate(qc, neg(X)), rotate(qc, Y), rotate(qc, neg(Y)), rotate(qc, Z),
+                            rotate(qc, neg(Z))};
+        uint32_t best[6];
+        hull_supports<6>(hull + b.shape.hf, b.shape.hc, d, best);
+        auto at = [&](int k) { return add(rotate(b.rot, xyz(hull[b.shape.hf + best[k]])), b.pos); };
+        sx = at(0), snx = at(1), sy = at(2), sny = at(3), sz = at(4), snz = at(5);
+    } else {
+        sx = ws(X), snx = ws(neg(X)), sy = ws(Y), sny = ws(neg(Y)), sz = ws(Z), snz = ws(neg(Z));
+    }
     if (sx.x > mx.x) mx.x = sx.x;
     if (snx.x < mn.x) mn.x = snx.x;
     if (sy.y > mx.y) mx.y = sy.y;

@@ -1023,42 +1023,16 @@ static __global__ void k_sort_segments(const uint32_t* offsets, uint32_t n, uint
     }
 }
 
-constexpr int kLongSort = 4096;
-
 static __global__ void __launch_bounds__(512) k_sort_long(const uint32_t* offsets, uint32_t* pb, const uint32_t* long_list,
                                                    const uint32_t* long_count, uint32_t* err) {
     pdl_enter();
     __shared__ uint32_t s[kLongSort];
-    uint32_t cnt = *long_count;
+    const uint32_t cnt = *long_count;
     for (uint32_t q = blockIdx.x; q < cnt; q += gridDim.x) {
-        uint32_t i = long_list[q];
-        uint32_t a = offsets[i], len = offsets[i + 1] - a;
-        if (len > (uint32_t)kLongSort) {
-            if (threadIdx.x == 0) atomicOr(err, kErrIndexOverflow);
-            continue;
-        }
-        uint32_t p2 = 1;
-        while (p2 < len) p2 <<= 1;
-        for (uint32_t k = threadIdx.x; k < p2; k += blockDim.x) s[k] = k < len ? pb[a + k] : 0xFFFFFFFFu;
-        __syncthreads();
-        for (uint32_t size = 2; size <= p2; size <<= 1) {
-            for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
-                for (uint32_t t = threadIdx.x; t < p2; t += blockDim.x) {
-                    uint32_t u = t ^ stride;
-                    if (u > t) {
-                        bool up = (t & size) == 0;
-                        uint32_t x = s[t], y = s[u];
-                        if ((x > y) == up) {
-                            s[t] = y;
-                            s[u] = x;
-                        }
-                    }
-                }
-                __syncthreads();
-            }
-        }
-        for (uint32_t k = threadIdx.x; k < len; k += blockDim.x) pb[a + k] = s[k];
-        __syncthreads();
+        const uint32_t i = long_list[q];
+        if (!sort_segment(pb + offsets[i], offsets[i + 1] - offsets[i], s) && threadIdx.x == 0)
+            atomicOr(err, kErrIndexOverflow);
+        __syncthreads();  // the next segment's sort
     }
 }
 

@@ -46,6 +46,60 @@ struct NB {
     ShapeR<R> shape;
 };
 
+// The first maximum of dot(vertex, d[k]) over a hull's n > 0 vertices, for N
+// directions at once: what scanning the list with a strict comparison finds
+// (a NaN product never wins, a NaN first product keeps vertex 0).  Each
+// direction keeps four running maxima, over every fourth vertex, so four
+// loads and comparisons are in flight instead of one chain of them.
+template <int N, class R>
+__device__ __forceinline__ void hull_supports(const A4<R>* hull, uint32_t n, const V3<R> (&d)[N], uint32_t (&best)[N]) {
+    constexpr uint32_t kNone = 0xFFFFFFFFu;
+    R bd[N][4];
+    uint32_t bi[N][4];
+    const V3<R> v0 = xyz(hull[0]);
+    bool first_nan[N];
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        const R d0 = dot(v0, d[k]);
+        first_nan[k] = isnan(d0);
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            bd[k][q] = q ? -R(INFINITY) : d0;
+            bi[k][q] = q ? kNone : 0u;
+        }
+    }
+    auto visit = [&](uint32_t i, int q) {
+        const V3<R> v = xyz(hull[i]);
+#pragma unroll
+        for (int k = 0; k < N; ++k) {
+            const R dd = dot(v, d[k]);
+            if (dd > bd[k][q]) {
+                bd[k][q] = dd;
+                bi[k][q] = i;
+            }
+        }
+    };
+    uint32_t i = 0;
+    for (; i + 4u <= n; i += 4u)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) visit(i + q, q);
+#pragma unroll
+    for (int q = 0; q < 3; ++q)
+        if (i + q < n) visit(i + q, q);
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+        R b = bd[k][0];
+        uint32_t at = bi[k][0];
+#pragma unroll
+        for (int q = 1; q < 4; ++q)
+            if (bi[k][q] != kNone && (bd[k][q] > b || (bd[k][q] == b && bi[k][q] < at))) {
+                b = bd[k][q];
+                at = bi[k][q];
+            }
+        best[k] = first_nan[k] ? 0u : at;
+    }
+}
+
 // support, support.rs:21-61 (first max wins ties); BOX shares the cube's sign
 // select, HULL scans its vertex list with the same first-max rule.
 template <class R>
@@ -72,17 +126,10 @@ __device__ __forceinline__ V3<R> support(const ShapeR<R>& s, V3<R> d, const A4<R
         }
         case DIO_SHAPE_HULL: {
             if (s.hc == 0 || hull == nullptr) return {R(0), R(0), R(0)};
-            V3<R> best = xyz(hull[s.hf]);
-            R bd = dot(best, d);
-            for (uint32_t i = 1; i < s.hc; ++i) {
-                V3<R> v = xyz(hull[s.hf + i]);
-                R dd = dot(v, d);
-                if (dd > bd) {
-                    bd = dd;
-                    best = v;
-                }
-            }
-            return best;
+            const V3<R> dirs[1] = {d};
+            uint32_t best[1];
+            hull_supports<1>(hull + s.hf, s.hc, dirs, best);
+            return xyz(hull[s.hf + best[0]]);
         }
         default:
             return {R(0), R(0), R(0)};

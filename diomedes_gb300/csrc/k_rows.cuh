@@ -4,12 +4,14 @@
 // (engine/src/physics/gpu.rs:239-264), container_contacts (:352-404),
 // finalize_contacts (:266-311: warm start by (a, b), decay, CSR).  Here each
 // piece is a kernel over slots / bodies / rows:
-//   k_slot_count + scan  -> k_slot_rows      rows from valid narrow slots
-//   k_cont_count + scan  -> k_cont_rows      container (wall / floor) rows
+//   k_row_counts + scans -> k_rows           rows from valid narrow slots and
+//                                            container (wall / floor) rows
 //   k_row_keys                               64-bit (a, b) keys + incidences
 //   (radix sorts of keys / incidences)
 //   k_warm                                   warm start + decay
 //   k_csr_fill                               CSR idx / other-body arrays
+// A world's rows are in canonical order, so k_rows warm-starts them as it
+// writes them and counts the CSR's incidences on the way.
 #pragma once
 
 #include "k_narrow.cuh"
@@ -38,7 +40,8 @@ __device__ __forceinline__ void tangents(V3<R> n, V3<R>& t1, V3<R>& t2) {
 
 template <class P, class R>
 __device__ __forceinline__ void write_row(const DevWorld<P, R>& w, uint32_t r, uint32_t a, uint32_t b, V3<R> n,
-                                          V3<R> t1, V3<R> t2, V3<R> ra, V3<R> rb, V3<R> c0, R friction, R kmin) {
+                                          V3<R> t1, V3<R> t2, V3<R> ra, V3<R> rb, V3<R> c0, R friction,
+                                          const RowDual<P, R>& du) {
     RowStatic<R> rs;
     rs.n = pack(n, friction);
     rs.t1 = pack(t1, c0.z);
@@ -46,60 +49,106 @@ __device__ __forceinline__ void write_row(const DevWorld<P, R>& w, uint32_t r, u
     rs.ra = pack(ra, c0.x);
     rs.rb = pack(rb, c0.y);
     w.rs.put(r, rs);
-    RowDual<P, R> du;
-    du.penalty = A4<R>{kmin, kmin, kmin, R(0)};
-    du.lambda = A4<P>{P(0), P(0), P(0), P(0)};
     w.rd.put(r, du);
     w.ab[r] = make_uint2(a, b);
 }
-
-// Valid slots of each live group of `per` slots (the first min(*n_groups_dev,
-// n_groups) groups); the scan that follows stops at the same count.
-template <class R>
-__global__ void k_slot_count(const Slot<R>* slots, uint32_t per, const uint32_t* n_groups_dev, uint32_t n_groups,
-                             uint32_t* counts) {
-    pdl_enter();
-    const uint32_t ng = n_groups_dev ? min(*n_groups_dev, n_groups) : n_groups;
-    for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < ng; p += gridDim.x * blockDim.x) {
-        uint32_t c = 0;
-        for (uint32_t k = 0; k < per; ++k) c += slots[p * per + k].valid ? 1u : 0u;
-        counts[p] = c;
-    }
+template <class P, class R>
+__device__ __forceinline__ RowDual<P, R> fresh_dual(R kmin) {
+    return RowDual<P, R>{A4<R>{kmin, kmin, kmin, R(0)}, A4<P>{P(0), P(0), P(0), P(0)}};
+}
+// the decay of finalize_contacts (gpu.rs:266-283)
+template <class P, class R>
+__device__ __forceinline__ RowDual<P, R> decay(RowDual<P, R> du, const PrepParams<R>& o) {
+    P ag = P(o.alpha_gamma);
+    du.lambda.x = du.lambda.x * ag;
+    du.lambda.y = du.lambda.y * ag;
+    du.lambda.z = du.lambda.z * ag;
+    R kx = du.penalty.x * o.gamma, ky = du.penalty.y * o.gamma, kz = du.penalty.z * o.gamma;
+    du.penalty.x = fmin_(fmax_(kx, o.penalty_min), o.penalty_max);
+    du.penalty.y = fmin_(fmax_(ky, o.penalty_min), o.penalty_max);
+    du.penalty.z = fmin_(fmax_(kz, o.penalty_min), o.penalty_max);
+    return du;
 }
 
-// raw_contact for every valid slot, rows at `offsets[group]` in slot order.
+__device__ __forceinline__ bool key_less(uint2 a, uint2 b) { return a.x < b.x || (a.x == b.x && a.y < b.y); }
+__device__ __forceinline__ bool key_eq(uint2 a, uint2 b) { return a.x == b.x && a.y == b.y; }
+
+// Where a new row's dual comes from (finalize_contacts, gpu.rs:266-283).  A
+// world's rows are in canonical order: pair rows follow the pair list, which
+// is sorted by (a, b), and container rows the body index, so each section is
+// sorted by key with equal keys adjacent.  The first row of a key takes
+// (lambda, penalty) of the last previous row with it, found by binary search
+// in the previous step's section; every row then decays.  Without `on` (rows
+// prepared for a caller) the duals start fresh and k_warm follows.
 template <class P, class R>
-__global__ void k_slot_rows(DevWorld<P, R> w, const Slot<R>* slots, uint32_t per, const uint32_t* n_groups_dev,
-                            uint32_t n_groups, const uint32_t* offsets, PrepParams<R> o) {
-    pdl_enter();
-    const uint32_t ng = n_groups_dev ? min(*n_groups_dev, n_groups) : n_groups;
-    for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < ng; p += gridDim.x * blockDim.x) {
-        uint32_t r = offsets[p];
-        // a group without valid slots (a box overlap without contact) is
-        // skipped unread; the last live group ends at the total, offsets[n_groups]
-        const uint32_t r_end = p + 1 < ng ? offsets[p + 1] : offsets[n_groups];
-        if (r_end == r) continue;
-        for (uint32_t k = 0; k < per; ++k) {
-            const Slot<R> s = slots[p * per + k];
-            if (!s.valid) continue;
-            if (s.a >= w.n || s.b >= w.n) {
-                atomicOr(&w.ctr->error_flags, kErrBadIndex);
-                continue;
+struct WarmStart {
+    bool on;
+    const uint2* prev_ab;
+    RowDuals<P, R> prev;
+    const Counters* ctr;
+    __device__ __forceinline__ RowDual<P, R> dual(uint2 key, bool first, const PrepParams<R>& o) const {
+        RowDual<P, R> du = fresh_dual<P, R>(o.penalty_min);
+        if (!on) return du;
+        if (first) {
+            const bool cont = key.y == kContainer;
+            const uint32_t base = cont ? ctr->prev_pair_rows : 0u;
+            uint32_t lo = base, hi = cont ? ctr->prev_rows : ctr->prev_pair_rows;
+            while (lo < hi) {  // upper bound of key
+                const uint32_t mid = (lo + hi) >> 1;
+                if (!key_less(key, prev_ab[mid]))
+                    lo = mid + 1;
+                else
+                    hi = mid;
             }
-            if (r >= w.max_rows) {
-                atomicOr(&w.ctr->error_flags, kErrRowOverflow);
-                return;
+            if (lo > base && key_eq(prev_ab[lo - 1], key)) {
+                const RowDual<P, R> pd = prev[lo - 1];
+                du.lambda = pd.lambda;
+                du.penalty = pd.penalty;
             }
-            NB<R> A = load_nb(w, s.a), B = load_nb(w, s.b);
-            V3<R> nrm = xyz(s.normal);
-            V3<R> t1, t2;
-            tangents(nrm, t1, t2);
-            V3<R> ra = rotate(conj(A.rot), sub(xyz(s.pa), A.pos));
-            V3<R> rb = rotate(conj(B.rot), sub(xyz(s.pb), B.pos));
-            write_row(w, r, s.a, s.b, neg(nrm), t1, t2, ra, rb, V3<R>{o.margin - s.depth, R(0), R(0)}, o.friction,
-                      o.penalty_min);
-            ++r;
         }
+        return decay(du, o);
+    }
+};
+
+// raw_contact for the valid slots of group p, from row r on in slot order.
+template <class P, class R>
+__device__ __forceinline__ void slot_rows(const DevWorld<P, R>& w, const Slot<R>* slots, uint32_t per, uint32_t p,
+                                          uint32_t r, const PrepParams<R>& o, const WarmStart<P, R>& warm,
+                                          uint32_t* incident) {
+    bool first = true;
+    uint32_t rows = 0, sa = 0, sb = 0;
+    NB<R> A, B;
+    for (uint32_t k = 0; k < per; ++k) {
+        const Slot<R> s = slots[(size_t)p * per + k];
+        if (!s.valid) continue;
+        if (s.a >= w.n || s.b >= w.n) {
+            atomicOr(&w.ctr->error_flags, kErrBadIndex);
+            continue;
+        }
+        if (r >= w.max_rows) {
+            atomicOr(&w.ctr->error_flags, kErrRowOverflow);
+            break;
+        }
+        if (first || s.a != sa || s.b != sb) {  // a group's slots are one pair's
+            A = load_nb(w, s.a);
+            B = load_nb(w, s.b);
+            sa = s.a;
+            sb = s.b;
+        }
+        V3<R> nrm = xyz(s.normal);
+        V3<R> t1, t2;
+        tangents(nrm, t1, t2);
+        V3<R> ra = rotate(conj(A.rot), sub(xyz(s.pa), A.pos));
+        V3<R> rb = rotate(conj(B.rot), sub(xyz(s.pb), B.pos));
+        write_row(w, r, s.a, s.b, neg(nrm), t1, t2, ra, rb, V3<R>{o.margin - s.depth, R(0), R(0)}, o.friction,
+                  warm.dual(make_uint2(s.a, s.b), first, o));
+        first = false;
+        ++rows;
+        ++r;
+    }
+    if (incident && rows) {
+        if (w.inv[sa].w != R(0)) atomicAdd(&incident[sa], rows);
+        if (w.inv[sb].w != R(0)) atomicAdd(&incident[sb], rows);
     }
 }
 
@@ -126,8 +175,8 @@ __device__ __forceinline__ void support_face(const NB<R>& b, V3<R> outward, V3<R
 // container_contacts for one body (engine/src/physics/gpu.rs:352-404):
 // counts (write == false) or writes rows starting at `r`.
 template <class P, class R>
-__device__ __forceinline__ uint32_t container_rows(const DevWorld<P, R>& w, uint32_t i, const SceneDesc& sc,
-                                                   const PrepParams<R>& o, bool write_out, uint32_t r) {
+__device__ __forceinline__ uint32_t container_rows(const DevWorld<P, R>& w, uint32_t i, const PrepParams<R>& o,
+                                                   bool write_out, uint32_t r, const WarmStart<P, R>& warm) {
     const A4<R>* walls = w.walls + 6 * (size_t)w.scene[i];
     V3<R> vel = cast3<R>(xyz(w.vel[i]));
     // Quick reject: every support point lies within an L1 bounding radius of
@@ -144,7 +193,9 @@ __device__ __forceinline__ uint32_t container_rows(const DevWorld<P, R>& w, uint
     const V3<R> pos = cast3<R>(sub(xyz(w.pos[0][i]), org));  // as load_nb forms it
     const bool boxy = tag == DIO_SHAPE_CUBE || tag == DIO_SHAPE_BOX;
     R rbound = R(-1);
-    if (boxy) {
+    if (tag == DIO_SHAPE_HULL && w.hull_bound) {
+        rbound = w.hull_bound[i];  // over its vertices, kept from the upload
+    } else if (boxy) {
         rbound = dabs(R(c0.x)) + dabs(R(c0.y)) + dabs(R(c0.z));
     } else if (tag == DIO_SHAPE_SPHERE) {
         rbound = dabs(R(c0.x));
@@ -198,7 +249,8 @@ __device__ __forceinline__ uint32_t container_rows(const DevWorld<P, R>& w, uint
                     if (r + count < w.max_rows) {
                         V3<R> ra = rotate(conj(b.rot), sub(cp, b.pos));
                         write_row(w, r + count, i, kContainer, normal, t1, t2, ra, V3<R>{R(0), R(0), R(0)},
-                                  V3<R>{o.margin - depth, R(0), R(0)}, o.friction, o.penalty_min);
+                                  V3<R>{o.margin - depth, R(0), R(0)}, o.friction,
+                                  warm.dual(make_uint2(i, kContainer), count == 0, o));
                     } else {
                         atomicOr(&w.ctr->error_flags, kErrRowOverflow);
                     }
@@ -208,6 +260,25 @@ __device__ __forceinline__ uint32_t container_rows(const DevWorld<P, R>& w, uint
         }
     }
     return count;
+}
+
+// An L1 bounding radius of each hull body's vertices (a little over, for the
+// rounding of their rotation), once per upload.
+template <class P, class R>
+__global__ void k_hull_bounds(DevWorld<P, R> w, uint32_t n, R* bound) {
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const uint4 h = *reinterpret_cast<const uint4*>(&w.shape[i]);
+        if (h.x != DIO_SHAPE_HULL) continue;
+        R b = R(0);
+        bool finite = true;
+        for (uint32_t k = 0; k < h.z; ++k) {
+            const V3<R> v = xyz(w.hull[h.y + k]);
+            const R l = dabs(v.x) + dabs(v.y) + dabs(v.z);
+            finite = finite && finite_(l);
+            b = fmax_(b, l);
+        }
+        bound[i] = finite ? b * R(1.0001) : R(-1);  // -1: no bound, the full test
+    }
 }
 
 // The six walls of each scene's container (container_collide,
@@ -231,33 +302,71 @@ __global__ void k_scene_walls(DevWorld<P, R> w, const SceneDesc* scenes, uint32_
     }
 }
 
-// counts[hi - lo] is set to 0 for the exclusive scan over hi - lo + 1 entries
+// Valid slots of each live group of `per` slots (the first min(*ng_dev, ng)
+// groups) and container rows of each of the bodies [0, n); counts2[n] is set
+// to 0 for the exclusive scan over n + 1 entries, and so is incident[0 .. n]
+// (if given).
 template <class P, class R>
-__global__ void k_cont_count(DevWorld<P, R> w, uint32_t lo, uint32_t hi, PrepParams<R> o, uint32_t* counts) {
+__global__ void k_row_counts(DevWorld<P, R> w, const Slot<R>* slots, uint32_t per, const uint32_t* ng_dev, uint32_t ng,
+                             uint32_t n, PrepParams<R> o, uint32_t* counts, uint32_t* counts2, uint32_t* incident) {
     pdl_enter();
-    if (blockIdx.x == 0 && threadIdx.x == 0) counts[hi - lo] = 0u;
-    for (uint32_t i = lo + blockIdx.x * blockDim.x + threadIdx.x; i < hi; i += gridDim.x * blockDim.x) {
+    if (ng_dev) ng = min(*ng_dev, ng);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        counts2[n] = 0u;
+        if (incident) incident[n] = 0u;
+    }
+    const WarmStart<P, R> none{};
+    // bodies first: they are known to be there, and the longer work
+    const uint64_t items = (uint64_t)n + ng;
+    for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < items; t += (uint64_t)gridDim.x * blockDim.x) {
         uint32_t c = 0;
-        const SceneDesc sc = w.scenes[w.scene[i]];
-        if (w.inv[i].w != R(0) && sc.has_container) c = container_rows(w, i, sc, o, false, 0);
-        counts[i - lo] = c;
+        if (t < n) {
+            const uint32_t i = (uint32_t)t;
+            if (w.inv[i].w != R(0) && w.scenes[w.scene[i]].has_container) c = container_rows(w, i, o, false, 0, none);
+            counts2[i] = c;
+            if (incident) incident[i] = 0u;
+        } else {
+            const uint32_t p = (uint32_t)(t - n);
+            for (uint32_t k = 0; k < per; ++k) c += slots[(size_t)p * per + k].valid ? 1u : 0u;
+            counts[p] = c;
+        }
     }
 }
 
-// zero (may be null): hi - lo + 1 per-body counters cleared on the way, for
-// the dynamic-body CSR count that follows
+// The rows: pair rows at off[group] (total at off[ng], the capacity), then
+// container rows at off2[body].  incident (may be null, zero on entry): the
+// dynamic-body CSR's counters, each body's rows counted.
 template <class P, class R>
-__global__ void k_cont_rows(DevWorld<P, R> w, uint32_t lo, uint32_t hi, PrepParams<R> o, const uint32_t* offsets,
-                            const uint32_t* base_dev, uint32_t* zero) {
+__global__ void k_rows(DevWorld<P, R> w, const Slot<R>* slots, uint32_t per, const uint32_t* ng_dev, uint32_t ng,
+                       uint32_t n, PrepParams<R> o, const uint32_t* off, const uint32_t* off2, WarmStart<P, R> warm,
+                       uint32_t* incident) {
     pdl_enter();
-    uint32_t base = *base_dev;
-    if (zero && blockIdx.x == 0 && threadIdx.x == 0) zero[hi - lo] = 0u;
-    for (uint32_t i = lo + blockIdx.x * blockDim.x + threadIdx.x; i < hi; i += gridDim.x * blockDim.x) {
-        if (zero) zero[i - lo] = 0u;
-        const uint32_t r = offsets[i - lo];
-        if (offsets[i - lo + 1] == r) continue;  // no rows: nothing to recompute
-        const SceneDesc sc = w.scenes[w.scene[i]];
-        if (w.inv[i].w != R(0) && sc.has_container) container_rows(w, i, sc, o, true, base + r);
+    const uint32_t live = ng_dev ? min(*ng_dev, ng) : ng;
+    const uint32_t pair_rows = off[ng], cont_rows = off2[n];
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        w.ctr->pair_rows = pair_rows;
+        w.ctr->container_rows = cont_rows;
+        const uint64_t t = (uint64_t)pair_rows + cont_rows;
+        w.ctr->rows = t > w.max_rows ? w.max_rows : (uint32_t)t;
+        if (t > w.max_rows) atomicOr(&w.ctr->error_flags, kErrRowOverflow);
+    }
+    const uint64_t items = (uint64_t)live + n;
+    for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < items; t += (uint64_t)gridDim.x * blockDim.x) {
+        if (t < live) {
+            const uint32_t p = (uint32_t)t, r = off[p];
+            // a group without valid slots (a box overlap without contact) is
+            // skipped unread; the last live group ends at the total
+            if ((p + 1 < live ? off[p + 1] : pair_rows) != r) slot_rows(w, slots, per, p, r, o, warm, incident);
+        } else {
+            const uint32_t i = (uint32_t)(t - live), r = off2[i], rows = off2[i + 1] - r;
+            if (!rows) continue;  // nothing to recompute
+            container_rows(w, i, o, true, pair_rows + r, warm);
+            if (incident) {  // rows that were kept
+                const uint64_t at = (uint64_t)pair_rows + r;
+                const uint32_t kept = at >= w.max_rows ? 0u : (uint32_t)min((uint64_t)rows, w.max_rows - at);
+                if (kept) atomicAdd(&incident[i], kept);
+            }
+        }
     }
 }
 
@@ -328,15 +437,7 @@ __global__ void k_warm(DevWorld<P, R> w, const uint32_t* m_dev, const unsigned l
                 du.penalty = pd.penalty;
             }
         }
-        P ag = P(o.alpha_gamma);
-        du.lambda.x = du.lambda.x * ag;
-        du.lambda.y = du.lambda.y * ag;
-        du.lambda.z = du.lambda.z * ag;
-        R kx = du.penalty.x * o.gamma, ky = du.penalty.y * o.gamma, kz = du.penalty.z * o.gamma;
-        du.penalty.x = fmin_(fmax_(kx, o.penalty_min), o.penalty_max);
-        du.penalty.y = fmin_(fmax_(ky, o.penalty_min), o.penalty_max);
-        du.penalty.z = fmin_(fmax_(kz, o.penalty_min), o.penalty_max);
-        w.rd.put(r, du);
+        w.rd.put(r, decay(du, o));
     }
 }
 
@@ -374,16 +475,6 @@ __global__ void k_csr_fill(DevWorld<P, R> w, const uint32_t* inc_body_sorted, co
 }
 
 // ---- device-driven variants for the resident world (no host-known counts)
-//
-// The world's rows are in canonical order: pair rows follow the pair list,
-// which is sorted by (a, b), and container rows follow the body index, so
-// each section of the row list is sorted by key with equal keys adjacent.
-// The warm start therefore needs no sort: a row is the first of its key when
-// its predecessor in the section has another key, and the last previous row
-// with that key is found by binary search in the previous step's section.
-
-__device__ __forceinline__ bool key_less(uint2 a, uint2 b) { return a.x < b.x || (a.x == b.x && a.y < b.y); }
-__device__ __forceinline__ bool key_eq(uint2 a, uint2 b) { return a.x == b.x && a.y == b.y; }
 
 // roll the per-step counters: the finished step's row counts become the
 // warm-start source, the per-step counts restart at zero (and up to two
@@ -405,63 +496,12 @@ static __global__ void k_roll_counters(Counters* c, uint32_t* zero0, uint32_t* z
     c->traverse_pairs = 0;
 }
 
-template <class P, class R>
-__global__ void k_warm_sections(DevWorld<P, R> w, const uint2* prev_ab, RowDuals<P, R> prev_dual,
-                                PrepParams<R> o) {
-    pdl_enter();
-    const uint32_t m = w.ctr->rows, pair_rows = w.ctr->pair_rows;
-    const uint32_t prev_m = w.ctr->prev_rows, prev_pair = w.ctr->prev_pair_rows;
-    for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < m; r += gridDim.x * blockDim.x) {
-        const uint2 key = w.ab[r];
-        const bool cont = key.y == kContainer;
-        const uint32_t sec_lo = cont ? pair_rows : 0;
-        RowDual<P, R> du = w.rd[r];
-        bool first = r == sec_lo || !key_eq(w.ab[r - 1], key);
-        if (first) {
-            uint32_t lo = cont ? prev_pair : 0, hi = cont ? prev_m : prev_pair;
-            const uint32_t base = lo;
-            while (lo < hi) {  // upper bound of key
-                uint32_t mid = (lo + hi) >> 1;
-                if (!key_less(key, prev_ab[mid]))
-                    lo = mid + 1;
-                else
-                    hi = mid;
-            }
-            if (lo > base && key_eq(prev_ab[lo - 1], key)) {
-                const RowDual<P, R> pd = prev_dual[lo - 1];
-                du.lambda = pd.lambda;
-                du.penalty = pd.penalty;
-            }
-        }
-        P ag = P(o.alpha_gamma);
-        du.lambda.x = du.lambda.x * ag;
-        du.lambda.y = du.lambda.y * ag;
-        du.lambda.z = du.lambda.z * ag;
-        R kx = du.penalty.x * o.gamma, ky = du.penalty.y * o.gamma, kz = du.penalty.z * o.gamma;
-        du.penalty.x = fmin_(fmax_(kx, o.penalty_min), o.penalty_max);
-        du.penalty.y = fmin_(fmax_(ky, o.penalty_min), o.penalty_max);
-        du.penalty.z = fmin_(fmax_(kz, o.penalty_min), o.penalty_max);
-        w.rd.put(r, du);
-    }
-}
-
 // CSR of the dynamic bodies only (the primal never visits a static body):
-// counts, then an atomic scatter (each body's count taken down to zero),
-// then each segment sorted by row index,
-// which restores the reference's fill order (finalize_contacts, gpu.rs:
-// 286-310) without a sort over all incidences.
-template <class P, class R>
-__global__ void k_csr_count_dyn(DevWorld<P, R> w, uint32_t* counts) {
-    pdl_enter();
-    const uint32_t m = w.ctr->rows;
-    for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < m; r += gridDim.x * blockDim.x) {
-        uint2 ab = w.ab[r];
-        if (w.inv[ab.x].w != R(0)) atomicAdd(&counts[ab.x], 1u);
-        if (ab.y != kContainer && w.inv[ab.y].w != R(0)) atomicAdd(&counts[ab.y], 1u);
-    }
-}
-
-// remaining: each body's incidence count (k_csr_count_dyn), consumed here
+// counts from k_rows, then an atomic scatter (each body's count taken down to
+// zero), then each segment sorted by row index, which restores the
+// reference's fill order (finalize_contacts, gpu.rs:286-310) without a sort
+// over all incidences, with the other-body array.
+// remaining: each body's incidence count (k_rows), consumed here
 template <class P, class R>
 __global__ void k_csr_scatter_dyn(DevWorld<P, R> w, uint32_t* remaining) {
     pdl_enter();
@@ -479,15 +519,84 @@ __global__ void k_csr_scatter_dyn(DevWorld<P, R> w, uint32_t* remaining) {
     }
 }
 
+constexpr uint32_t kLongSort = 4096;
+// A segment of up to kLongSort words sorted ascending by the CTA through s
+// (kLongSort words), where it stays too; false (nothing done) when longer.
+__device__ __forceinline__ bool sort_segment(uint32_t* seg, uint32_t len, uint32_t* s) {
+    if (len > kLongSort) return false;
+    uint32_t p2 = 1;
+    while (p2 < len) p2 <<= 1;
+    for (uint32_t k = threadIdx.x; k < p2; k += blockDim.x) s[k] = k < len ? seg[k] : 0xFFFFFFFFu;
+    __syncthreads();
+    for (uint32_t size = 2; size <= p2; size <<= 1) {
+        for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
+            for (uint32_t t = threadIdx.x; t < p2; t += blockDim.x) {
+                const uint32_t u = t ^ stride;
+                if (u > t) {
+                    const bool up = (t & size) == 0;
+                    const uint32_t x = s[t], y = s[u];
+                    if ((x > y) == up) {
+                        s[t] = y;
+                        s[u] = x;
+                    }
+                }
+            }
+            __syncthreads();
+        }
+    }
+    for (uint32_t k = threadIdx.x; k < len; k += blockDim.x) seg[k] = s[k];
+    return true;
+}
+
+// the other body of row `row` seen from body i
+__device__ __forceinline__ uint32_t other_body(const uint2* ab, uint32_t row, uint32_t i) {
+    const uint2 v = ab[row];
+    return v.y == kContainer ? kContainer : (v.x == i ? v.y : (v.x | kIsB));
+}
+constexpr uint32_t kShortRows = 32;  // segments up to this sorted by a thread
 template <class P, class R>
-__global__ void k_csr_other_dyn(DevWorld<P, R> w) {
+__global__ void k_csr_finish_dyn(DevWorld<P, R> w, uint32_t* long_list, uint32_t* long_count) {
     pdl_enter();
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < w.n; i += gridDim.x * blockDim.x) {
-        uint32_t j0 = w.row_off[i], j1 = min(w.row_off[i + 1], w.max_incid);
-        for (uint32_t j = j0; j < j1; ++j) {
-            uint2 v = w.ab[w.row_idx[j]];
-            w.row_oth[j] = v.y == kContainer ? kContainer : (v.x == i ? v.y : (v.x | kIsB));
+        const uint32_t j0 = w.row_off[i], j1 = min(w.row_off[i + 1], w.max_incid);
+        if (j0 >= j1) continue;
+        const uint32_t len = j1 - j0;
+        if (len > kShortRows) {
+            long_list[warp_append(long_count)] = i;
+            continue;
         }
+        uint32_t v[kShortRows];
+        for (uint32_t k = 0; k < len; ++k) {
+            const uint32_t x = w.row_idx[j0 + k];
+            int m = (int)k - 1;
+            while (m >= 0 && v[m] > x) {
+                v[m + 1] = v[m];
+                --m;
+            }
+            v[m + 1] = x;
+        }
+        for (uint32_t k = 0; k < len; ++k) {
+            w.row_idx[j0 + k] = v[k];
+            w.row_oth[j0 + k] = other_body(w.ab, v[k], i);
+        }
+    }
+}
+// the long segments, a CTA each
+template <class P, class R>
+__global__ void __launch_bounds__(512) k_csr_finish_long(DevWorld<P, R> w, const uint32_t* long_list,
+                                                         const uint32_t* long_count) {
+    pdl_enter();
+    __shared__ uint32_t s[kLongSort];
+    const uint32_t cnt = *long_count;
+    for (uint32_t q = blockIdx.x; q < cnt; q += gridDim.x) {
+        const uint32_t i = long_list[q];
+        const uint32_t j0 = w.row_off[i], len = min(w.row_off[i + 1], w.max_incid) - j0;
+        if (sort_segment(w.row_idx + j0, len, s)) {
+            for (uint32_t k = threadIdx.x; k < len; k += blockDim.x) w.row_oth[j0 + k] = other_body(w.ab, s[k], i);
+        } else if (threadIdx.x == 0) {
+            atomicOr(&w.ctr->error_flags, kErrIndexOverflow);
+        }
+        __syncthreads();  // the next segment's sort
     }
 }
 

@@ -323,51 +323,61 @@ __device__ __forceinline__ uint32_t block_sum_scan(uint32_t v, uint32_t* s_warp,
     *total = all;
     return wofs + x - v;
 }
-static __global__ void __launch_bounds__(kScanThreads)
-    k_scan_partials(const uint32_t* in, uint32_t n, const uint32_t* n_dev, uint32_t* partials) {
+// One scan of a launch: n entries of `in`, or the first *n_dev of them; total
+// (optional) receives the sum; partials: a word a tile.
+struct ScanJob {
+    const uint32_t* in;
+    uint32_t* out;
+    uint32_t n;
+    const uint32_t* n_dev;
+    uint32_t* partials;
+    uint32_t* total;
+};
+// two independent scans share the launches, blockIdx.y telling them apart
+static __global__ void __launch_bounds__(kScanThreads) k_scan_partials(ScanJob j0, ScanJob j1) {
     pdl_enter();
     __shared__ uint32_t s_warp[kScanThreads / 32];
-    if (n_dev) n = min(*n_dev, n);
-    const bool in16 = (reinterpret_cast<uintptr_t>(in) & 15u) == 0u;
+    const ScanJob j = blockIdx.y ? j1 : j0;
+    const uint32_t n = j.n_dev ? min(*j.n_dev, j.n) : j.n;
+    const bool in16 = (reinterpret_cast<uintptr_t>(j.in) & 15u) == 0u;
     const uint32_t tiles = (uint32_t)(((size_t)n + kScanTile - 1) / kScanTile);
     for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         uint32_t v[kScanItems];
-        scan_load_tile(in, n, (size_t)tile * kScanTile + (size_t)threadIdx.x * kScanItems, in16, v);
+        scan_load_tile(j.in, n, (size_t)tile * kScanTile + (size_t)threadIdx.x * kScanItems, in16, v);
         uint32_t sum = 0;
 #pragma unroll
-        for (int j = 0; j < kScanItems; ++j) sum += v[j];
+        for (int k = 0; k < kScanItems; ++k) sum += v[k];
         uint32_t all = 0;
         block_sum_scan(sum, s_warp, &all);
-        if (threadIdx.x == 0) partials[tile] = all;
+        if (threadIdx.x == 0) j.partials[tile] = all;
     }
 }
-static __global__ void __launch_bounds__(kScanThreads)
-    k_scan_apply(const uint32_t* in, uint32_t* out, uint32_t n, const uint32_t* n_dev, const uint32_t* partials,
-                 uint32_t* total) {
+static __global__ void __launch_bounds__(kScanThreads) k_scan_apply(ScanJob j0, ScanJob j1) {
     pdl_enter();
     __shared__ uint32_t s_warp[kScanThreads / 32];
-    if (n_dev) n = min(*n_dev, n);
-    if (n == 0u && total && blockIdx.x == 0 && threadIdx.x == 0) *total = 0u;
-    const bool in16 = (reinterpret_cast<uintptr_t>(in) & 15u) == 0u;
-    const bool out16 = (reinterpret_cast<uintptr_t>(out) & 15u) == 0u;
+    const ScanJob j = blockIdx.y ? j1 : j0;
+    const uint32_t n = j.n_dev ? min(*j.n_dev, j.n) : j.n;
+    if (n == 0u && j.total && blockIdx.x == 0 && threadIdx.x == 0) *j.total = 0u;
+    const bool in16 = (reinterpret_cast<uintptr_t>(j.in) & 15u) == 0u;
+    const bool out16 = (reinterpret_cast<uintptr_t>(j.out) & 15u) == 0u;
     const uint32_t tiles = (uint32_t)(((size_t)n + kScanTile - 1) / kScanTile);
     for (uint32_t tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
         const size_t base = (size_t)tile * kScanTile + (size_t)threadIdx.x * kScanItems;
         uint32_t v[kScanItems];
-        scan_load_tile(in, n, base, in16, v);
+        scan_load_tile(j.in, n, base, in16, v);
         // partials of the lower tiles, one or more a thread
         uint32_t low = 0;
-        for (uint32_t t = threadIdx.x; t < tile; t += kScanThreads) low += partials[t];
+        for (uint32_t t = threadIdx.x; t < tile; t += kScanThreads) low += j.partials[t];
         uint32_t sum = 0;
 #pragma unroll
-        for (int j = 0; j < kScanItems; ++j) sum += v[j];
+        for (int k = 0; k < kScanItems; ++k) sum += v[k];
         // one pass: the tile's own thread sums and the lower partials
         uint32_t lowall = 0, tileall = 0;
         block_sum_scan(low, s_warp, &lowall);
         uint32_t run = lowall + block_sum_scan(sum, s_warp, &tileall);
-        if (total && tile + 1u == tiles && threadIdx.x == 0) *total = lowall + tileall;
+        if (j.total && tile + 1u == tiles && threadIdx.x == 0) *j.total = lowall + tileall;
         if (base + kScanItems <= n && out16) {
-            uint4* d4 = reinterpret_cast<uint4*>(out + base);
+            uint4* d4 = reinterpret_cast<uint4*>(j.out + base);
 #pragma unroll
             for (int k = 0; k < kScanItems / 4; ++k) {
                 uint4 q;
@@ -383,9 +393,9 @@ static __global__ void __launch_bounds__(kScanThreads)
             }
         } else {
 #pragma unroll
-            for (int j = 0; j < kScanItems; ++j) {
-                if (base + j < n) out[base + j] = run;
-                run += v[j];
+            for (int k = 0; k < kScanItems; ++k) {
+                if (base + k < n) j.out[base + k] = run;
+                run += v[k];
             }
         }
     }
@@ -670,7 +680,7 @@ struct ScanSort {
         if ((e = cudaMalloc(&hist, kRadixMaxPasses * 256 * 4)) != cudaSuccess) return e;
         if ((e = cudaMalloc(&done, 4)) != cudaSuccess) return e;
         if ((e = cudaMalloc(&bases, kRadixMaxPasses * 256 * 4)) != cudaSuccess) return e;
-        if ((e = cudaMalloc(&partials, (((size_t)max_scan + kScanTile - 1) / kScanTile + 1) * 4)) != cudaSuccess)
+        if ((e = cudaMalloc(&partials, 2 * (((size_t)max_scan + kScanTile - 1) / kScanTile + 1) * 4)) != cudaSuccess)
             return e;
         if ((e = cudaMalloc(&kalt, std::max<size_t>(1, max_sort) * 8)) != cudaSuccess) return e;
         if ((e = cudaMalloc(&valt, std::max<size_t>(1, max_sort) * 4)) != cudaSuccess) return e;
@@ -700,11 +710,26 @@ struct ScanSort {
             counted(1);
             return launch_k(pdl, k_scan_excl, 1, kScanThreads, 0, s, in, out, n, n_dev, total, lookback());
         }
-        counted(2);
-        cudaError_t e = launch_k(pdl, k_scan_partials, g, kScanThreads, 0, s, in, n, n_dev, partials);
-        if (e != cudaSuccess) return e;
-        return launch_k(true, k_scan_apply, g, kScanThreads, 0, s, in, out, n, n_dev, (const uint32_t*)partials,
-                        total);
+        const ScanJob j{in, out, n, n_dev, partials, total};
+        return scan_jobs(j, j, 1, g, pdl, s);
+    }
+    // two scans at once (each n <= max_scan, n > 0): half the launches
+    cudaError_t scan_both(ScanJob a, ScanJob b, bool pdl, cudaStream_t s) {
+        if (a.n > max_scan || b.n > max_scan || !a.n || !b.n) return cudaErrorInvalidValue;
+        auto tiles = [](uint32_t n) { return (int)(((size_t)n + kScanTile - 1) / kScanTile); };
+        a.partials = partials;
+        b.partials = partials + tiles(a.n);
+        return scan_jobs(a, b, 2, std::max(tiles(a.n), tiles(b.n)), pdl, s);
+    }
+    cudaError_t scan_jobs(const ScanJob& a, const ScanJob& b, int jobs, int tiles, bool pdl, cudaStream_t s) {
+        if (tiles > 1) {  // else no tile has lower ones
+            counted(1);
+            const cudaError_t e = launch_grid(pdl, k_scan_partials, dim3(tiles, jobs), kScanThreads, s, a, b);
+            if (e != cudaSuccess) return e;
+            pdl = true;
+        }
+        counted(1);
+        return launch_grid(pdl, k_scan_apply, dim3(tiles, jobs), kScanThreads, s, a, b);
     }
 
     // stable sort of n pairs by key bits [begin_bit, end_bit) (n <= max_sort);
