@@ -519,6 +519,7 @@ class Engine final : public EngineBase {
         DIO_TRY(alloc(&lb_vals_, N));
         DIO_TRY(alloc(&lb_leaf_, N));
         DIO_TRY(alloc(&lb_children_, N));
+        DIO_TRY(alloc(&lb_range_, N));
         DIO_TRY(alloc(&lb_parent_, 2ull * N));
         DIO_TRY(alloc(&lb_visits_, N));
         DIO_TRY(alloc(&lb_leaf_min_, N));
@@ -1597,7 +1598,7 @@ class Engine final : public EngineBase {
                         (const uint32_t*)w_.scene, n, (const uint32_t*)lb_bounds_, sbits, abits, lb_keys_, lb_vals_));
         DIO_CK(ss_.sort_pairs(lb_keys_, lb_keys_s_, lb_vals_, lb_leaf_, n, 0u, sbits + 3u * abits, pdl(), stream_));
         DIO_CK(launch_k(pdl(), k_karras, g, 256, 0, stream_, (const uint32_t*)lb_keys_s_, (const SceneDesc*)scenes_,
-                        (const uint32_t*)w_.scene, n, lb_children_, lb_parent_));
+                        (const uint32_t*)w_.scene, n, lb_children_, lb_parent_, lb_range_));
         launches_ += 4;
         return run_lbvh_refit(n, g);
     }
@@ -1638,8 +1639,6 @@ class Engine final : public EngineBase {
         // offsets, sorts the partner lists and emits the pairs
         ta.fused = (nchunks && !global_path) ? 1u : 0u;
         ta.nchunks = nchunks;
-        ta.pairs = w_.pairs;
-        ta.ctr = ctr_;
         auto scene_tree = [&](bool write) -> cudaError_t {
             if (!nchunks) return cudaSuccess;
             ++launches_;
@@ -1660,15 +1659,15 @@ class Engine final : public EngineBase {
         if (global_path) {
             DIO_CK(cudaMemsetAsync(lb_visits_, 0, (size_t)n * 4, stream_));
             if (!world_step_) DIO_CK(cudaMemsetAsync(&ctr_->traverse_pairs, 0, 4, stream_));  // else k_roll_counters
-            k_refit<R><<<g, 256, 0, stream_>>>(w_.aabb_min, w_.aabb_max, lb_leaf_, scenes_, w_.scene, n,
-                                               lb_children_, lb_parent_, lb_leaf_min_, lb_leaf_max_, lb_node_min_,
-                                               lb_node_max_, lb_visits_, tcap_skip, counts_);
+            k_refit<R><<<grid_for(n, kRefitLeaves), kRefitLeaves, 0, stream_>>>(
+                w_.aabb_min, w_.aabb_max, lb_leaf_, scenes_, w_.scene, n, lb_children_, lb_parent_, lb_range_,
+                lb_leaf_min_, lb_leaf_max_, lb_node_min_, lb_node_max_, lb_visits_, tcap_skip, counts_);
             // a walk per leaf fills the SMs from about 512 leaves per SM; fewer
             // leaves split each walk over four threads
             const uint32_t split = (uint64_t)n < (uint64_t)sms_ * 512u ? kWalkSplit : 1u;
             k_traverse_count<R><<<grid_for((uint64_t)n * split, 128), 128, 0, stream_>>>(
-                lb_leaf_, scenes_, w_.scene, n, lb_children_, lb_leaf_min_, lb_leaf_max_, lb_node_min_, lb_node_max_,
-                counts_, lb_gscratch_, w_.max_pairs, &ctr_->traverse_pairs, &ctr_->error_flags, tcap_skip, split);
+                scenes_, w_.scene, n, lb_leaf_min_, lb_leaf_max_, lb_node_min_, lb_node_max_, counts_, lb_gscratch_,
+                w_.max_pairs, &ctr_->traverse_pairs, &ctr_->error_flags, tcap_skip, split);
             launches_ += 2;
         }
         if (!world_step_) DIO_CK(cudaMemsetAsync(counts_ + n, 0, 4, stream_));  // else k_roll_counters
@@ -2469,7 +2468,7 @@ class Engine final : public EngineBase {
     uint32_t* lb_bounds_ = nullptr;
     uint32_t *lb_keys_ = nullptr, *lb_keys_s_ = nullptr;
     uint32_t *lb_vals_ = nullptr, *lb_leaf_ = nullptr, *lb_parent_ = nullptr, *lb_visits_ = nullptr;
-    uint2* lb_children_ = nullptr;
+    uint2 *lb_children_ = nullptr, *lb_range_ = nullptr;
     A4<R>*lb_leaf_min_ = nullptr, *lb_leaf_max_ = nullptr, *lb_node_min_ = nullptr, *lb_node_max_ = nullptr;
     uint32_t *lb_pb_ = nullptr, *lb_long_ = nullptr, *lb_long_count_ = nullptr;
     uint2* lb_gscratch_ = nullptr;  // pairs of the global trees' count pass

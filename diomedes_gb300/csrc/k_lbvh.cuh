@@ -159,9 +159,10 @@ __device__ __forceinline__ double tag_bits<double>(uint32_t v) { return __longlo
 // Internal node k of a scene whose sorted keys are seg[0, ns) and whose
 // slots start at global slot lo: node k lives at slot lo + k; child codes
 // are global slots, leaves flagged with kLeafFlag (leaf = sorted position);
-// parents of internal slots in [0, n), of leaves in [n, 2n)
+// parents of internal slots in [0, n), of leaves in [n, 2n); range (optional):
+// the first and last leaf position below the node
 __device__ __forceinline__ void karras_node(const uint32_t* seg, uint32_t lo, int ns, int k, uint32_t n,
-                                            uint2* children, uint32_t* parent) {
+                                            uint2* children, uint32_t* parent, uint2* range) {
     int d = (kdelta(seg, ns, k, k + 1) - kdelta(seg, ns, k, k - 1)) >= 0 ? 1 : -1;
     int dmin = kdelta(seg, ns, k, k - d);
     int lmax = 2;
@@ -181,13 +182,14 @@ __device__ __forceinline__ void karras_node(const uint32_t* seg, uint32_t lo, in
     uint32_t left = (min(k, j) == gamma) ? ((lo + gamma) | kLeafFlag) : (lo + gamma);
     uint32_t right = (max(k, j) == gamma + 1) ? ((lo + gamma + 1) | kLeafFlag) : (lo + gamma + 1);
     children[lo + k] = make_uint2(left, right);
+    if (range) range[lo + k] = make_uint2(lo + min(k, j), lo + max(k, j));
     parent[(left & kLeafFlag) ? n + (left & ~kLeafFlag) : left] = lo + k;
     parent[(right & kLeafFlag) ? n + (right & ~kLeafFlag) : right] = lo + k;
 }
 
 // binary radix tree per scene (Karras 2012) over the globally sorted keys
 static __global__ void k_karras(const uint32_t* keys, const SceneDesc* scenes, const uint32_t* scene_of_pos,
-                                uint32_t n, uint2* children, uint32_t* parent) {
+                                uint32_t n, uint2* children, uint32_t* parent, uint2* range) {
     pdl_enter();
     for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
         const SceneDesc sc = scenes[scene_of_pos[p]];
@@ -195,46 +197,89 @@ static __global__ void k_karras(const uint32_t* keys, const SceneDesc* scenes, c
         const int ns = (int)(sc.body_hi - sc.body_lo);
         const int k = (int)(p - lo);
         if (k >= ns - 1) continue;  // ns - 1 internal nodes
-        karras_node(keys + lo, lo, ns, k, n, children, parent);
+        karras_node(keys + lo, lo, ns, k, n, children, parent, range);
     }
 }
 
-// leaf boxes in sorted order, then bottom-up unions; a node's max corner
-// carries in w its highest leaf position (as bits).  counts: the per-body
-// pair counters of the count pass, cleared here.
+// A node's two children in one word (the w of its min corner): Karras' left
+// and right child lie at slots g and g + 1, each a leaf or an internal node.
+constexpr uint32_t kLeftLeaf = 0x80000000u, kRightLeaf = 0x40000000u, kChildSlot = 0x3FFFFFFFu;
+__device__ __forceinline__ uint32_t tree_word(uint2 c) {
+    return (c.x & ~kLeafFlag) | ((c.x & kLeafFlag) ? kLeftLeaf : 0u) | ((c.y & kLeafFlag) ? kRightLeaf : 0u);
+}
+
+// Leaf boxes in sorted order, then bottom-up unions.  The w slots: a leaf's
+// min corner its body; a node's min corner its children (tree_word), its max
+// corner its highest leaf position.  Each path climbs with its subtree's box
+// in registers; at a node both arrivals leave their boxes, the first one stops
+// and the second unites them.  A CTA's leaves are kRefitLeaves consecutive positions,
+// so the nodes over them alone (about log2(kRefitLeaves) levels of the tree)
+// meet in shared memory; only the levels above pay for global atomics, fences
+// and L2 reads, and each level's records are loaded during the exchange of the
+// level below (all levels through L2, a level at a time: 33 us cold for 8,192
+// leaves, now 15).  counts: the per-body pair counters of the count pass,
+// cleared here.
+constexpr int kRefitLeaves = 256;
 template <class R>
-__global__ void k_refit(const A4<R>* mn, const A4<R>* mx, const uint32_t* leaf_body, const SceneDesc* scenes,
-                        const uint32_t* scene_of_pos, uint32_t n, const uint2* children, const uint32_t* parent,
-                        A4<R>* leaf_min, A4<R>* leaf_max, A4<R>* node_min, A4<R>* node_max, uint32_t* visits,
-                        uint32_t skip_max, uint32_t* counts) {
-    for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < n; p += gridDim.x * blockDim.x) {
-        const SceneDesc sc = scenes[scene_of_pos[p]];
-        if (sc.body_hi - sc.body_lo <= skip_max) continue;  // k_scene_tree's scene
-        uint32_t b = leaf_body[p];
-        counts[b] = 0u;
-        leaf_min[p] = mn[b];
-        leaf_max[p] = mx[b];
-        if (sc.body_hi - sc.body_lo < 2) continue;
-        __threadfence();
-        uint32_t node = parent[n + p];
-        while (true) {
-            if (atomicAdd(&visits[node], 1u) == 0) break;  // first arrival stops
+__global__ void __launch_bounds__(kRefitLeaves)
+    k_refit(const A4<R>* mn, const A4<R>* mx, const uint32_t* leaf_body, const SceneDesc* scenes,
+            const uint32_t* scene_of_pos, uint32_t n, const uint2* children, const uint32_t* parent, const uint2* range,
+            A4<R>* leaf_min, A4<R>* leaf_max, A4<R>* node_min, A4<R>* node_max, uint32_t* visits, uint32_t skip_max,
+            uint32_t* counts) {
+    __shared__ A4<R> s_min[2][kRefitLeaves], s_max[2][kRefitLeaves];
+    __shared__ uint32_t s_visits[kRefitLeaves];
+    const uint32_t c0 = blockIdx.x * kRefitLeaves, p = c0 + threadIdx.x;
+    s_visits[threadIdx.x] = 0u;
+    __syncthreads();
+    if (p >= n) return;
+    const SceneDesc sc = scenes[scene_of_pos[p]];
+    if (sc.body_hi - sc.body_lo <= skip_max) return;  // k_scene_tree's scene
+    const uint32_t b = leaf_body[p];
+    counts[b] = 0u;
+    A4<R> bmin = mn[b], bmax = mx[b];
+    bmin.w = tag_bits<R>(b);
+    leaf_min[p] = bmin;
+    leaf_max[p] = bmax;
+    if (sc.body_hi - sc.body_lo < 2) return;
+    uint32_t node = parent[n + p], self = p | kLeafFlag;
+    uint2 c = children[node], rg = range[node];
+    uint32_t up = parent[node];  // the root's is not read as a node
+    while (true) {
+        // the next level's records, in flight during this level's exchange
+        const bool root = node == sc.body_lo;
+        const uint32_t next = root ? node : up;
+        const uint2 nc = children[next], nrg = range[next];
+        const uint32_t nup = parent[next];
+        A4<R> omin, omax;
+        if (rg.x >= c0 && rg.y < c0 + kRefitLeaves) {
+            const uint32_t s = node - c0;  // a node's slot is one end of its range
+            const uint32_t side = c.x == self ? 0u : 1u;
+            s_min[side][s] = bmin;
+            s_max[side][s] = bmax;
+            __threadfence_block();
+            if (atomicAdd(&s_visits[s], 1u) == 0u) break;  // first arrival stops
+            __threadfence_block();
+            omin = s_min[1u - side][s];
+            omax = s_max[1u - side][s];
+        } else {
             __threadfence();
-            uint2 c = children[node];
-            const A4<R>* lmn = (c.x & kLeafFlag) ? leaf_min : node_min;
-            const A4<R>* lmx = (c.x & kLeafFlag) ? leaf_max : node_max;
-            const A4<R>* rmn = (c.y & kLeafFlag) ? leaf_min : node_min;
-            const A4<R>* rmx = (c.y & kLeafFlag) ? leaf_max : node_max;
-            uint32_t li = c.x & ~kLeafFlag, ri = c.y & ~kLeafFlag;
-            // boxes written by other CTAs in this launch: read through L2
-            A4<R> a0 = ldcg4(&lmn[li]), a1 = ldcg4(&lmx[li]), b0 = ldcg4(&rmn[ri]), b1 = ldcg4(&rmx[ri]);
-            const uint32_t hi = max((c.x & kLeafFlag) ? li : tag_of(a1), (c.y & kLeafFlag) ? ri : tag_of(b1));
-            node_min[node] = A4<R>{fmin_(a0.x, b0.x), fmin_(a0.y, b0.y), fmin_(a0.z, b0.z), R(0)};
-            node_max[node] = A4<R>{fmax_(a1.x, b1.x), fmax_(a1.y, b1.y), fmax_(a1.z, b1.z), tag_bits<R>(hi)};
+            if (atomicAdd(&visits[node], 1u) == 0u) break;  // first arrival stops
             __threadfence();
-            if (node == sc.body_lo) break;  // scene root
-            node = parent[node];
+            // the sibling's box, written by another CTA in this launch: read through L2
+            const uint32_t sib = c.x == self ? c.y : c.x, si = sib & ~kLeafFlag;
+            omin = ldcg4(&((sib & kLeafFlag) ? leaf_min : node_min)[si]);
+            omax = ldcg4(&((sib & kLeafFlag) ? leaf_max : node_max)[si]);
         }
+        bmin = A4<R>{fmin_(bmin.x, omin.x), fmin_(bmin.y, omin.y), fmin_(bmin.z, omin.z), tag_bits<R>(tree_word(c))};
+        bmax = A4<R>{fmax_(bmax.x, omax.x), fmax_(bmax.y, omax.y), fmax_(bmax.z, omax.z), tag_bits<R>(rg.y)};
+        node_min[node] = bmin;
+        node_max[node] = bmax;
+        if (root) break;
+        self = node;
+        node = next;
+        c = nc;
+        rg = nrg;
+        up = nup;
     }
 }
 
@@ -244,19 +289,43 @@ constexpr int kStack = 64;
 // the leaf at position p visits only the subtrees holding positions above
 // p (a node's highest leaf position is its max corner's w), so each
 // overlapping pair is found once, by its lower position; it is counted for
-// body a = min(i, j) and appended as (a, b) to the pair scratch through a
-// warp-aggregated cursor, from which the write pass places it without
-// walking the trees again.  With split = kWalkSplit each leaf's walk is
+// body a = min(i, j) and appended as (a, b) to the CTA's buffer (both children's
+// hits of a warp by one shared atomic; a cursor in global memory put its round
+// trip into every step that found a pair), which goes to the pair scratch in one
+// piece, from which the write pass places it without walking the trees again.
+// A step of a walk is one round of loads: a node's word names both children,
+// and their boxes hold the next words (children read first, then their boxes:
+// 8,192 stacked cubes 130 us a step cold, now 47).  With split = kWalkSplit each leaf's walk is
 // split over 4 threads, one per subtree two levels below the root (a leaf at
 // that depth is tested directly), so a scene of a few thousand bodies still
 // fills the SMs with walks; with split = 1 a thread walks from the root.
-constexpr uint32_t kWalkSplit = 4;
+constexpr uint32_t kWalkSplit = 4, kWalkBuffer = 2048;
+// slots for the active lanes' hits: all the a, then all the b
+struct Slots2 {
+    uint32_t a, b;
+};
+__device__ __forceinline__ Slots2 warp_append2(uint32_t* cursor, bool a, bool b) {
+    uint32_t lane, lt;
+    asm("mov.u32 %0, %%laneid;" : "=r"(lane));
+    asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
+    const uint32_t m = __activemask();
+    const uint32_t ma = __ballot_sync(m, a), mb = __ballot_sync(m, b), na = (uint32_t)__popc(ma);
+    const int leader = __ffs(m) - 1;
+    uint32_t base = 0;
+    if ((int)lane == leader) base = atomicAdd(cursor, na + (uint32_t)__popc(mb));
+    base = __shfl_sync(m, base, leader);
+    return {base + (uint32_t)__popc(ma & lt), base + na + (uint32_t)__popc(mb & lt)};
+}
 template <class R>
 __global__ void __launch_bounds__(128)
-    k_traverse_count(const uint32_t* leaf_body, const SceneDesc* scenes, const uint32_t* scene_of_pos, uint32_t n,
-                     const uint2* children, const A4<R>* leaf_min, const A4<R>* leaf_max, const A4<R>* node_min,
-                     const A4<R>* node_max, uint32_t* counts, uint2* scratch, uint32_t scratch_cap,
-                     uint32_t* scratch_n, uint32_t* err, uint32_t skip_max, uint32_t split) {
+    k_traverse_count(const SceneDesc* scenes, const uint32_t* scene_of_pos, uint32_t n, const A4<R>* leaf_min,
+                     const A4<R>* leaf_max, const A4<R>* node_min, const A4<R>* node_max, uint32_t* counts,
+                     uint2* scratch, uint32_t scratch_cap, uint32_t* scratch_n, uint32_t* err, uint32_t skip_max,
+                     uint32_t split) {
+    __shared__ uint2 s_pairs[kWalkBuffer];
+    __shared__ uint32_t s_n, s_base;
+    if (threadIdx.x == 0) s_n = 0u;
+    __syncthreads();
     const uint64_t total = (uint64_t)n * split;
     for (uint64_t u = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; u < total;
          u += (uint64_t)gridDim.x * blockDim.x) {
@@ -264,79 +333,80 @@ __global__ void __launch_bounds__(128)
         const SceneDesc sc = scenes[scene_of_pos[p]];
         if (sc.body_hi - sc.body_lo <= skip_max) continue;  // k_scene_tree's scene
         if (sc.body_hi - sc.body_lo < 2) continue;
-        // the root (split 1), or its children, each replaced by its own
-        // children when internal
-        uint32_t items[kWalkSplit];
-        uint32_t ni = 0;
-        if (split == 1u) {
-            items[ni++] = sc.body_lo;
-        } else {
-            const uint2 rc = children[sc.body_lo];
-            const uint32_t top[2] = {rc.x, rc.y};
-#pragma unroll
-            for (int k = 0; k < 2; ++k) {
-                if (top[k] & kLeafFlag) {
-                    items[ni++] = top[k];
-                } else {
-                    const uint2 gc = children[top[k]];
-                    items[ni++] = gc.x;
-                    items[ni++] = gc.y;
-                }
-            }
-        }
-        if (part >= ni) continue;
-        const uint32_t i = leaf_body[p];
         const A4<R> qmn = leaf_min[p], qmx = leaf_max[p];
-        auto emit = [&](uint32_t idx) {
-            const uint32_t j = leaf_body[idx];
-            const uint32_t a = min(i, j), b = max(i, j);
-            atomicAdd(&counts[a], 1u);
-            const uint32_t slot = warp_append(scratch_n);
-            if (slot < scratch_cap) scratch[slot] = make_uint2(a, b);
-        };
-        const uint32_t first = items[part];
-        const uint32_t fidx = first & ~kLeafFlag;
-        if (first & kLeafFlag) {
-            if (fidx > p && overlap(qmn, qmx, leaf_min[fidx], leaf_max[fidx])) emit(fidx);
-            continue;
-        }
-        {
-            const A4<R> fmx = node_max[fidx];
-            if (!(tag_of(fmx) > p && overlap(qmn, qmx, node_min[fidx], fmx))) continue;
-        }
-        uint32_t stack[kStack];
-        int sp = 0;
-        uint32_t node = fidx;
-        while (true) {
-            const uint2 c = children[node];
-            const uint32_t ch[2] = {c.x, c.y};
-            uint32_t push = 0;
-            uint32_t next[2];
-#pragma unroll
-            for (int k = 0; k < 2; ++k) {
-                const uint32_t x = ch[k];
-                const uint32_t idx = x & ~kLeafFlag;
-                if (x & kLeafFlag) {
-                    if (idx > p && overlap(qmn, qmx, leaf_min[idx], leaf_max[idx])) emit(idx);
-                } else {
-                    const A4<R> bmx = node_max[idx];
-                    if (tag_of(bmx) > p && overlap(qmn, qmx, node_min[idx], bmx)) next[push++] = idx;
-                }
+        const uint32_t i = tag_of(qmn);
+        auto keep = [&](uint32_t slot, uint32_t j) {
+            const uint2 ab = make_uint2(min(i, j), max(i, j));
+            atomicAdd(&counts[ab.x], 1u);
+            if (slot < kWalkBuffer) {
+                s_pairs[slot] = ab;
+            } else {  // a denser neighbourhood than the buffer: straight to the scratch
+                const uint32_t at = atomicAdd(scratch_n, 1u);
+                if (at < scratch_cap) scratch[at] = ab;
             }
-            if (push == 0) {
-                if (sp == 0) break;
-                node = stack[--sp];
-            } else {
-                node = next[0];
-                if (push == 2) {
+        };
+        // the root's children (split 1), or one of its grandchildren (a leaf
+        // at that depth is tested directly)
+        uint32_t word = tag_of(node_min[sc.body_lo]);
+        if (split > 1u) {
+            const uint32_t side = part >> 1, half = part & 1u;
+            uint32_t s = (word & kChildSlot) + side;
+            bool leaf = word & (side ? kRightLeaf : kLeftLeaf);
+            if (leaf && half) continue;  // the leaf is the other half's
+            if (!leaf) {
+                word = tag_of(node_min[s]);
+                leaf = word & (half ? kRightLeaf : kLeftLeaf);
+                s = (word & kChildSlot) + half;
+            }
+            if (leaf) {
+                const A4<R> lmn = leaf_min[s];
+                if (s > p && overlap(qmn, qmx, lmn, leaf_max[s])) keep(atomicAdd(&s_n, 1u), tag_of(lmn));
+                continue;
+            }
+            const A4<R> bmn = node_min[s], bmx = node_max[s];
+            if (!(tag_of(bmx) > p && overlap(qmn, qmx, bmn, bmx))) continue;
+            word = tag_of(bmn);
+        }
+        uint32_t stack[kStack];  // words of the nodes still to visit
+        int sp = 0;
+        while (true) {
+            const uint32_t g = word & kChildSlot;
+            const bool ll = word & kLeftLeaf, rl = word & kRightLeaf;
+            // both children's boxes before either is tested: a step is one
+            // round of loads
+            const A4<R> amn = (ll ? leaf_min : node_min)[g], amx = (ll ? leaf_max : node_max)[g];
+            const A4<R> bmn = (rl ? leaf_min : node_min)[g + 1u], bmx = (rl ? leaf_max : node_max)[g + 1u];
+            const bool a = (ll ? g : tag_of(amx)) > p && overlap(qmn, qmx, amn, amx);
+            const bool b = (rl ? g + 1u : tag_of(bmx)) > p && overlap(qmn, qmx, bmn, bmx);
+            const bool ha = a && ll, hb = b && rl;
+            if (ha || hb) {
+                const Slots2 at = warp_append2(&s_n, ha, hb);
+                if (ha) keep(at.a, tag_of(amn));
+                if (hb) keep(at.b, tag_of(bmn));
+            }
+            const bool na = a && !ll, nb = b && !rl;
+            if (na) {
+                word = tag_of(amn);
+                if (nb) {
                     if (sp < kStack)
-                        stack[sp++] = next[1];
+                        stack[sp++] = tag_of(bmn);
                     else
                         atomicOr(err, kErrIndexOverflow);
                 }
+            } else if (nb) {
+                word = tag_of(bmn);
+            } else {
+                if (sp == 0) break;
+                word = stack[--sp];
             }
         }
     }
+    __syncthreads();
+    const uint32_t kept = min(s_n, kWalkBuffer);
+    if (threadIdx.x == 0 && kept) s_base = atomicAdd(scratch_n, kept);
+    __syncthreads();
+    for (uint32_t e = threadIdx.x; e < kept; e += blockDim.x)
+        if (s_base + e < scratch_cap) scratch[s_base + e] = s_pairs[e];
 }
 
 // Write pass of the global trees from the count pass's scratch: pair (a, b)
@@ -983,7 +1053,7 @@ __global__ void __launch_bounds__(kSceneTreeThreads)
         const int ns = (int)(sc.body_hi - sc.body_lo);
         const int k = (int)(lo + p - sc.body_lo);
         if (k >= ns - 1) continue;  // ns - 1 internal nodes
-        karras_node(s_key + (sc.body_lo - lo), sc.body_lo, ns, k, n, children, parent);
+        karras_node(s_key + (sc.body_lo - lo), sc.body_lo, ns, k, n, children, parent, nullptr);
     }
 }
 
