@@ -578,11 +578,10 @@ class Engine final : public EngineBase {
         DIO_TRY(alloc(&solve_chunks_, S));
         DIO_TRY(alloc(&chunk_dyn_, (size_t)S << kMaxClusterShift));
         DIO_TRY(alloc(&scene_chunk_, S));
-        DIO_TRY(alloc(&chunk_n_, S));
-        DIO_TRY(alloc(&chunk_ovf_, S));
-        DIO_TRY(alloc(&chunk_tot_, S));
+        DIO_TRY(alloc(&chunk_tot_, (size_t)S * kTreeParts));
         // pair scratch of the shared-memory trees: scratch_k_ slots per body
-        scratch_k_ = (uint32_t)std::min<uint64_t>(8, std::max<uint64_t>(2, 2 * ((uint64_t)PP + N - 1) / N));
+        // (at most 16: the write pass stages a chunk's pairs in its boxes' space)
+        scratch_k_ = (uint32_t)std::min<uint64_t>(16, std::max<uint64_t>(2, 2 * ((uint64_t)PP + N - 1) / N));
         DIO_TRY(alloc(&tree_scratch_, (size_t)N * scratch_k_));
         DIO_TRY(alloc(&hull_, H));
         DIO_TRY(alloc(&ctr_, 1));
@@ -1631,14 +1630,17 @@ class Engine final : public EngineBase {
         ta.cap = w_.max_pairs;
         ta.scratch = tree_scratch_;
         ta.scratch_k = scratch_k_;
-        ta.chunk_n = chunk_n_;
-        ta.chunk_ovf = chunk_ovf_;
         ta.chunk_tot = chunk_tot_;
         ta.err = &ctr_->error_flags;
         // every scene in a shared-memory tree: the write pass also forms the
         // offsets, sorts the partner lists and emits the pairs
         ta.fused = (nchunks && !global_path) ? 1u : 0u;
         ta.nchunks = nchunks;
+        // several CTAs a chunk while they fit the SMs (each refits the whole
+        // trees: more would only repeat that)
+        ta.parts = ta.fused ? std::max(1u, std::min({kTreeParts, (uint32_t)sms_ / nchunks, chunk_max_ / kPartLeaves})) : 1u;
+        ta.pairs = w_.pairs;
+        ta.ctr = ctr_;
         auto scene_tree = [&](bool write) -> cudaError_t {
             if (!nchunks) return cudaSuccess;
             ++launches_;
@@ -1646,7 +1648,7 @@ class Engine final : public EngineBase {
                 return launch_k(pdl(), k_scene_tree<R, true>, (int)nchunks, kSceneTreeThreads, tbytes, stream_,
                                 (const A4<R>*)w_.aabb_min, (const A4<R>*)w_.aabb_max, lb_leaf_min_, lb_leaf_max_,
                                 lb_node_min_, lb_node_max_, ta);
-            return launch_k(pdl(), k_scene_tree<R, false>, (int)nchunks, kSceneTreeThreads, tbytes, stream_,
+            return launch_k(pdl(), k_scene_tree<R, false>, (int)(nchunks * ta.parts), kSceneTreeThreads, tbytes, stream_,
                             (const A4<R>*)w_.aabb_min, (const A4<R>*)w_.aabb_max, lb_leaf_min_, lb_leaf_max_,
                             lb_node_min_, lb_node_max_, ta);
         };
@@ -2434,8 +2436,6 @@ class Engine final : public EngineBase {
     bool pdl() const { return world_step_ && !cfg_.profile; }
     int state_pending_ = 0;    // set_state_begin left: 1 the dynamic-set check, 2 a list rebuild
     bool lag_primed_ = false;  // the previous step's slots are this mode's
-    uint32_t* chunk_n_ = nullptr;
-    uint32_t* chunk_ovf_ = nullptr;
     uint32_t* chunk_tot_ = nullptr;
     uint2* tree_scratch_ = nullptr;
     uint32_t scratch_k_ = 2;

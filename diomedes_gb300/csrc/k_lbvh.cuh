@@ -488,13 +488,17 @@ __global__ void __launch_bounds__(128) k_traverse(const uint32_t* leaf_body, con
 // ---- one CTA per chunk of scenes, trees in shared memory ----
 // Consecutive scenes of at most scene_tree_cap<R>() bodies are packed into
 // chunks of at most that many bodies (a chunk's bodies and sorted positions
-// are both the index range [lo, hi)).  One CTA stages its chunk's trees (leaf
-// and node boxes, children, parents) in shared memory.
+// are both the index range [lo, hi)).  A CTA stages its chunk's trees (leaf
+// and node boxes, children, parents) in shared memory.  The count pass is
+// bound by the longest walk's serial steps, so up to kTreeParts CTAs take a
+// chunk's leaves where SMs are free: each refits the whole trees and walks its
+// share (33 scenes in 8 chunks: 32 us cold with one CTA a chunk, 23 with 8;
+// 1,617 bodies of 13 pairs each: 92 and 48).
 //   count pass  refit with shared-memory atomics (also each node's highest
 //               leaf position), then traverse: the leaf at position p visits
 //               only subtrees holding positions > p, so each overlapping pair
-//               is found once, by its lower position; it is counted for body
-//               a = min(i, j) and appended as (a, b) to the chunk's scratch
+//               is found once, by its lower position, and appended as (a, b),
+//               a = min(i, j), to the part's share of the chunk's scratch
 //               region (scratch_k slots per body of the chunk).  The w slots
 //               of the box corners carry what a traversal step needs next: a
 //               leaf's min corner its body; a node's min corner its two
@@ -502,7 +506,7 @@ __global__ void __launch_bounds__(128) k_traverse(const uint32_t* leaf_body, con
 //               its max corner its highest leaf position.  A step therefore
 //               loads only the two children's boxes, and the stack holds
 //               children words
-//   write pass  places the scratch pairs at the scanned per-body offsets; a
+//   write pass  counts the scratch pairs per body, places and orders them; a
 //               chunk whose scratch overflowed is traversed again and written
 //               directly (body i's partners j > i)
 // Per-body partner sets equal those of the global kernels (same trees, same
@@ -513,7 +517,7 @@ __host__ __device__ constexpr uint32_t scene_tree_cap() { return sizeof(R) == 4 
 template <class R>
 __host__ __device__ constexpr size_t scene_tree_bytes(uint32_t cap) {
     // leaf min/max, node min/max, children, leaf parent, node parent, visit
-    // flag (then per-body count), leaf's scene root
+    // flag (then per-body count), leaf's scene root; the write pass's space
     return (size_t)cap * (4 * sizeof(A4<R>) + sizeof(uint2) + 4 * sizeof(uint32_t)) + 16;
 }
 // a node's children (chunk positions with leaf flags) as one 24-bit word
@@ -543,21 +547,33 @@ struct TreeArgs {
     uint32_t cap;
     uint2* scratch;
     uint32_t scratch_k;
-    uint32_t* chunk_n;
-    uint32_t* chunk_ovf;
-    uint32_t* chunk_tot;  // pairs found per chunk (count pass)
+    // per chunk and part: the pairs found (count pass); the part's scratch
+    // holds them all if they are at most tree_part_slots
+    uint32_t* chunk_tot;
     uint32_t* err;
     // write pass of a world whose scenes all have shared-memory trees: it
-    // also forms the offsets, sorts each body's partners and emits the pairs
+    // also forms the counts and offsets, sorts each body's partners and emits
+    // the pairs
     uint32_t fused;
     uint32_t nchunks;
+    uint32_t parts;  // CTAs a chunk in the count pass (1 unless fused)
     DioPair* pairs;
     Counters* ctr;
 };
 
+// The CTAs that walk a chunk of nb bodies (of t.parts launched): at least four
+// warps of leaves each, so that equal shares of the scratch suit their pairs.
+constexpr uint32_t kTreeParts = 8, kPartLeaves = 128;
+__device__ __forceinline__ uint32_t tree_parts(const TreeArgs& t, uint32_t nb) {
+    return min(t.parts, max(1u, nb / kPartLeaves));
+}
+__device__ __forceinline__ uint32_t tree_part_slots(const TreeArgs& t, uint32_t nb) {
+    return nb * t.scratch_k / tree_parts(t, nb);
+}
+
 // Count-pass traversal from the leaf at chunk position p: pairs with leaves at
-// higher positions, counted for the lower body and appended (warp-aggregated) to the chunk's
-// scratch.  Both children's boxes (and their tags) are loaded before either
+// higher positions, counted for the lower body (if vis is given) and appended
+// (warp-aggregated) to the part's scratch.  Both children's boxes (and their tags) are loaded before either
 // is tested, so the loads of one step overlap.
 template <class R>
 __device__ __forceinline__ void tree_count_leaf(uint32_t p, uint32_t root, const A4<R>* lmn, const A4<R>* lmx,
@@ -570,46 +586,38 @@ __device__ __forceinline__ void tree_count_leaf(uint32_t p, uint32_t root, const
     int sp = 0;
     uint32_t cw = tag_of(nmn[root]);
     while (true) {
-        uint32_t idx[2], leaf[2];
-        A4<R> bmn[2], bmx[2];
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            const uint32_t c = k ? cw >> 12 : cw;
-            idx[k] = c & kCwIndex;
-            leaf[k] = c & kCwLeaf;
-            bmn[k] = (leaf[k] ? lmn : nmn)[idx[k]];
-            bmx[k] = (leaf[k] ? lmx : nmx)[idx[k]];
+        const uint32_t g = cw & kCwIndex, h = (cw >> 12) & kCwIndex;
+        const bool ll = cw & kCwLeaf, rl = (cw >> 12) & kCwLeaf;
+        const A4<R> amn = (ll ? lmn : nmn)[g], amx = (ll ? lmx : nmx)[g];
+        const A4<R> bmn = (rl ? lmn : nmn)[h], bmx = (rl ? lmx : nmx)[h];
+        // highest leaf position below: the leaf itself, or the node's tag
+        const bool a = (ll ? g : tag_of(amx)) > p && overlap(qmn, qmx, amn, amx);
+        const bool b = (rl ? h : tag_of(bmx)) > p && overlap(qmn, qmx, bmn, bmx);
+        const bool ha = a && ll, hb = b && rl;
+        if (ha || hb) {
+            const Slots2 at = warp_append2(s_cursor, ha, hb);
+            auto keep = [&](uint32_t slot, uint32_t j) {
+                const uint2 ab = make_uint2(min(i, j), max(i, j));
+                if (vis) atomicAdd(&vis[ab.x - lo], 1u);
+                if (slot < region) dst[slot] = ab;
+            };
+            if (ha) keep(at.a, tag_of(amn));
+            if (hb) keep(at.b, tag_of(bmn));
         }
-        uint32_t w0 = 0, w1 = 0, push = 0;
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            // highest leaf position below: the leaf itself, or the node's tag
-            if (!((leaf[k] ? idx[k] : tag_of(bmx[k])) > p && overlap(qmn, qmx, bmn[k], bmx[k]))) continue;
-            if (leaf[k]) {
-                const uint32_t j = tag_of(bmn[k]);
-                const uint32_t a = min(i, j), b = max(i, j);
-                atomicAdd(&vis[a - lo], 1u);
-                const uint32_t slot = warp_append(s_cursor);
-                if (slot < region) dst[slot] = make_uint2(a, b);
-            } else {
-                if (push == 0)
-                    w0 = tag_of(bmn[k]);
-                else
-                    w1 = tag_of(bmn[k]);
-                ++push;
-            }
-        }
-        if (push == 0) {
-            if (sp == 0) break;
-            cw = stack[--sp];
-        } else {
-            cw = w0;
-            if (push == 2) {
+        const bool na = a && !ll, nb = b && !rl;
+        if (na) {
+            cw = tag_of(amn);
+            if (nb) {
                 if (sp < kStack)
-                    stack[sp++] = w1;
+                    stack[sp++] = tag_of(bmn);
                 else
                     atomicOr(err, kErrIndexOverflow);
             }
+        } else if (nb) {
+            cw = tag_of(bmn);
+        } else {
+            if (sp == 0) break;
+            cw = stack[--sp];
         }
     }
 }
@@ -669,15 +677,16 @@ static_assert(scene_tree_cap<float>() <= 2u * kSceneTreeThreads && scene_tree_ca
               "the fused offsets scan takes two bodies a thread");
 // Fused write pass, part 1: the chunk's pair offsets.  base = pairs of the
 // chunks whose bodies come first (chunks are contiguous body ranges),
-// then a CTA-wide exclusive sum of the per-body counts: offsets[lo + p],
-// the scan's prefix in excl[p], the count in cnt[p].  CTA 0 also stores the
+// then a CTA-wide exclusive sum of the per-body counts cnt[p]: offsets[lo + p],
+// the scan's prefix in excl[p]; returns base.  CTA 0 also stores the
 // world's pair count (and the overflow flag), as k_pairs_total does.
-__device__ __forceinline__ void fused_offsets(const TreeArgs& t, uint32_t lo, uint32_t nb, uint32_t* excl,
-                                             uint32_t* cnt, uint32_t* s_red) {
+__device__ __forceinline__ uint32_t fused_offsets(const TreeArgs& t, uint32_t lo, uint32_t nb, uint32_t* excl,
+                                                 const uint32_t* cnt, uint32_t* s_red) {
     const uint32_t tid = threadIdx.x, nt = blockDim.x, lane = tid & 31u, warp = tid >> 5;
     unsigned long long before = 0, grand = 0;
     for (uint32_t c = tid; c < t.nchunks; c += nt) {
-        const uint32_t tot = t.chunk_tot[c];
+        unsigned long long tot = 0;
+        for (uint32_t k = 0; k < t.parts; ++k) tot += t.chunk_tot[c * t.parts + k];
         grand += tot;
         if (t.scenes[t.chunks[c].x].body_lo < lo) before += tot;
     }
@@ -704,7 +713,7 @@ __device__ __forceinline__ void fused_offsets(const TreeArgs& t, uint32_t lo, ui
     }
     // per-body counts, two consecutive bodies a thread
     const uint32_t p0 = 2u * tid;
-    const uint32_t c0 = p0 < nb ? t.counts[lo + p0] : 0u, c1 = p0 + 1u < nb ? t.counts[lo + p0 + 1u] : 0u;
+    const uint32_t c0 = p0 < nb ? cnt[p0] : 0u, c1 = p0 + 1u < nb ? cnt[p0 + 1u] : 0u;
     uint32_t x = c0 + c1;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -719,24 +728,117 @@ __device__ __forceinline__ void fused_offsets(const TreeArgs& t, uint32_t lo, ui
     const uint32_t b32 = (uint32_t)before;
     if (p0 < nb) {
         excl[p0] = e0;
-        cnt[p0] = c0;
         t.offsets[lo + p0] = b32 + e0;
     }
     if (p0 + 1u < nb) {
         excl[p0 + 1u] = e0 + c0;
-        cnt[p0 + 1u] = c1;
         t.offsets[lo + p0 + 1u] = b32 + e0 + c0;
     }
     __syncthreads();
+    return b32;
 }
 
-// Fused write pass, part 2: each body's partners (placed at its offsets in
-// pb) sorted ascending -- up to 32 in registers by the body's thread, longer
-// lists by the whole CTA (bitonic in `scratch`, the shared tree space) --
-// then the pairs (body, partner) in (a, b) order.
+// `len` words of s sorted ascending by the whole CTA (a bitonic network over
+// the next power of two, which s has room for)
+__device__ __forceinline__ void cta_sort(uint32_t* s, uint32_t len) {
+    const uint32_t tid = threadIdx.x, nt = blockDim.x;
+    uint32_t p2 = 1;
+    while (p2 < len) p2 <<= 1;
+    for (uint32_t k = len + tid; k < p2; k += nt) s[k] = 0xFFFFFFFFu;
+    __syncthreads();
+    for (uint32_t size = 2; size <= p2; size <<= 1) {
+        for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
+            for (uint32_t u = tid; u < p2 / 2u; u += nt) {
+                const uint32_t i = 2u * u - (u & (stride - 1u)), j = i + stride;
+                const uint32_t x = s[i], y = s[j];
+                if ((x > y) == ((i & size) == 0u)) {
+                    s[i] = y;
+                    s[j] = x;
+                }
+            }
+            __syncthreads();
+        }
+    }
+}
+
+// Fused write pass, part 2, from the chunk's scratch (all its pairs): the
+// partners go to their body's segment in shared memory, a thread per pair;
+// then each pair's place is its partner's rank in the segment, counted by the
+// same thread, and the pair goes straight to the list.  Lists beyond
+// kRankList, where counting costs more than sorting, are sorted by the CTA.
+// (A thread per body with an insertion sort in local memory over lists in
+// global memory, and a second walk for more than 8 pairs a body: 198 us cold
+// for 1,617 bodies with 13 pairs each, now 44.)
+constexpr uint32_t kRankList = 64;
+// A chunk's pairs in the parts of its scratch, as one list.
+struct ChunkPairs {
+    const uint2* scratch;
+    uint32_t slots, total;
+    uint32_t end[kTreeParts];  // of each part's pairs in the list
+    bool held;                 // every part's scratch has all its pairs
+    __device__ __forceinline__ ChunkPairs(const TreeArgs& t, uint32_t cidx, uint32_t lo, uint32_t nb)
+        : scratch(t.scratch + (size_t)lo * t.scratch_k), slots(tree_part_slots(t, nb)), total(0u), held(true) {
+#pragma unroll
+        for (uint32_t k = 0; k < kTreeParts; ++k) {
+            const uint32_t found = k < t.parts ? t.chunk_tot[cidx * t.parts + k] : 0u;
+            held = held && found <= slots;
+            end[k] = total += found;
+        }
+    }
+    __device__ __forceinline__ uint2 pair(uint32_t e) const {
+        uint32_t part = 0, first = 0;
+#pragma unroll
+        for (uint32_t k = 0; k + 1 < kTreeParts; ++k)
+            if (e >= end[k]) {
+                part = k + 1;
+                first = end[k];
+            }
+        return scratch[part * slots + (e - first)];
+    }
+};
+__device__ __forceinline__ void fused_ranks(const TreeArgs& t, const ChunkPairs& src, uint32_t lo, uint32_t nb,
+                                           uint32_t base, const uint32_t* excl, const uint32_t* cnt, uint32_t* fill,
+                                           uint32_t* seg, uint32_t* sort, uint32_t* long_list, uint32_t* s_nlong) {
+    const uint32_t tid = threadIdx.x, nt = blockDim.x;
+    if (tid == 0) *s_nlong = 0u;
+    for (uint32_t p = tid; p < nb; p += nt) fill[p] = 0u;
+    __syncthreads();
+    for (uint32_t e = tid; e < src.total; e += nt) {
+        const uint2 ab = src.pair(e);
+        seg[excl[ab.x - lo] + atomicAdd(&fill[ab.x - lo], 1u)] = ab.y;
+    }
+    for (uint32_t p = tid; p < nb; p += nt)
+        if (cnt[p] > kRankList) long_list[atomicAdd(s_nlong, 1u)] = p;
+    __syncthreads();
+    for (uint32_t e = tid; e < src.total; e += nt) {
+        const uint2 ab = src.pair(e);
+        const uint32_t len = cnt[ab.x - lo], first = excl[ab.x - lo];
+        if (len > kRankList) continue;
+        uint32_t rank = 0;
+        for (uint32_t q = 0; q < len; ++q) rank += seg[first + q] < ab.y ? 1u : 0u;
+        const uint32_t at = base + first + rank;
+        if (at < t.cap) t.pairs[at] = DioPair{ab.x, ab.y};
+    }
+    const uint32_t nlong = *s_nlong;
+    for (uint32_t q = 0; q < nlong; ++q) {
+        const uint32_t p = long_list[q], len = cnt[p];
+        for (uint32_t k = tid; k < len; k += nt) sort[k] = seg[excl[p] + k];
+        cta_sort(sort, len);
+        for (uint32_t k = tid; k < len; k += nt) {
+            const uint32_t at = base + excl[p] + k;
+            if (at < t.cap) t.pairs[at] = DioPair{lo + p, sort[k]};
+        }
+        __syncthreads();
+    }
+}
+
+// The same for a chunk whose scratch overflowed (the partners were written to
+// pb by the walks): each body's partners sorted ascending -- up to 32 in
+// registers by the body's thread, longer lists by the whole CTA (bitonic in
+// `scratch`, the shared tree space) -- then the pairs (body, partner) in
+// (a, b) order.
 __device__ __forceinline__ void fused_emit(const TreeArgs& t, uint32_t lo, uint32_t nb, const uint32_t* cnt,
-                                          uint32_t* long_list, uint32_t* s_nlong, uint32_t* scratch,
-                                          uint32_t scratch_words) {
+                                          uint32_t* long_list, uint32_t* s_nlong, uint32_t* scratch) {
     const uint32_t tid = threadIdx.x, nt = blockDim.x;
     if (tid == 0) *s_nlong = 0u;
     __syncthreads();
@@ -765,27 +867,8 @@ __device__ __forceinline__ void fused_emit(const TreeArgs& t, uint32_t lo, uint3
     for (uint32_t q = 0; q < nlong; ++q) {
         const uint32_t p = long_list[q];
         const uint32_t a = t.offsets[lo + p], len = cnt[p];
-        uint32_t p2 = 1;
-        while (p2 < len) p2 <<= 1;
-        if (p2 > scratch_words) {  // cannot happen: a list is shorter than the chunk
-            if (tid == 0) atomicOr(t.err, kErrIndexOverflow);
-            continue;
-        }
-        for (uint32_t k = tid; k < p2; k += nt) scratch[k] = k < len ? t.pb[a + k] : 0xFFFFFFFFu;
-        __syncthreads();
-        for (uint32_t size = 2; size <= p2; size <<= 1) {
-            for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
-                for (uint32_t u = tid; u < p2 / 2u; u += nt) {
-                    const uint32_t i = 2u * u - (u & (stride - 1u)), j = i + stride;
-                    const uint32_t x = scratch[i], y = scratch[j];
-                    if ((x > y) == ((i & size) == 0u)) {
-                        scratch[i] = y;
-                        scratch[j] = x;
-                    }
-                }
-                __syncthreads();
-            }
-        }
+        for (uint32_t k = tid; k < len; k += nt) scratch[k] = t.pb[a + k];
+        cta_sort(scratch, len);
         for (uint32_t k = tid; k < len; k += nt) t.pb[a + k] = scratch[k];
         __syncthreads();
     }
@@ -801,7 +884,10 @@ __global__ void __launch_bounds__(kSceneTreeThreads)
                  A4<R>* g_node_min, A4<R>* g_node_max, TreeArgs t) {
     pdl_enter();
     extern __shared__ __align__(16) unsigned char tree_smem[];
-    const uint32_t cidx = blockIdx.x;
+    // count pass: `parts` CTAs a chunk, each with the whole trees, walk the
+    // leaves of every parts-th warp
+    const uint32_t cidx = WRITE ? blockIdx.x : blockIdx.x / t.parts;
+    const uint32_t part = WRITE ? 0u : blockIdx.x % t.parts;
     const uint2 chunk = t.chunks[cidx];  // scenes [x, y)
     const uint32_t lo = t.scenes[chunk.x].body_lo;
     const uint32_t nb = t.scenes[chunk.y - 1].body_hi - lo;
@@ -821,28 +907,35 @@ __global__ void __launch_bounds__(kSceneTreeThreads)
     uint32_t* npar = lpar + cb;
     uint32_t* vis = npar + cb;  // visit flags, then per-body pair counts
     uint32_t* lroot = vis + cb;
-    // fused write pass: per-body prefix in lpar, count in npar (both unused
-    // by the write pass), the long list in lroot once the trees are walked
+    // write pass: per-body prefix in lpar, fill in npar (both unused by its
+    // walks), the long list in lroot once the trees are walked
     __shared__ uint32_t s_red[128];
     __shared__ uint32_t s_nlong;
-    const bool fused = WRITE && t.fused;
-    if (fused) fused_offsets(t, lo, nb, lpar, npar, s_red);
-    if (WRITE && !t.chunk_ovf[cidx]) {
-        // place the scratch pairs: body a's segment starts at offsets[a]
-        for (uint32_t p = tid; p < nb; p += nt) vis[p] = 0u;
-        __syncthreads();
-        const uint32_t np = t.chunk_n[cidx];
-        const uint2* src = t.scratch + (size_t)lo * t.scratch_k;
-        for (uint32_t k = tid; k < np; k += nt) {
-            const uint2 ab = src[k];
-            const uint32_t pos = t.offsets[ab.x] + atomicAdd(&vis[ab.x - lo], 1u);
-            if (pos < t.cap) t.pb[pos] = ab.y;
-        }
-        if (fused) {
+    if (WRITE) {
+        const ChunkPairs src(t, cidx, lo, nb);
+        if (src.held) {
+            for (uint32_t p = tid; p < nb; p += nt) vis[p] = 0u;
             __syncthreads();
-            fused_emit(t, lo, nb, npar, lroot, &s_nlong, reinterpret_cast<uint32_t*>(lmn),
-                       (uint32_t)(cb * 2u * sizeof(A4<R>) / 4u));
+            if (t.fused) {
+                for (uint32_t e = tid; e < src.total; e += nt) atomicAdd(&vis[src.pair(e).x - lo], 1u);
+                __syncthreads();
+                const uint32_t base = fused_offsets(t, lo, nb, lpar, vis, s_red);
+                // the segments take the boxes' space, 16 words a body (32 in FP64)
+                fused_ranks(t, src, lo, nb, base, lpar, vis, npar, reinterpret_cast<uint32_t*>(lmn),
+                            reinterpret_cast<uint32_t*>(ch), lroot, &s_nlong);
+                return;
+            }
+            // body a's segment starts at offsets[a]
+            for (uint32_t e = tid; e < src.total; e += nt) {
+                const uint2 ab = src.pair(e);
+                const uint32_t pos = t.offsets[ab.x] + atomicAdd(&vis[ab.x - lo], 1u);
+                if (pos < t.cap) t.pb[pos] = ab.y;
+            }
+            return;
         }
+    }
+    if (!WRITE && part >= tree_parts(t, nb)) {
+        if (tid == 0) t.chunk_tot[cidx * t.parts + part] = 0u;
         return;
     }
     // slot p is leaf p of its scene and, except for a scene's last slot,
@@ -861,8 +954,10 @@ __global__ void __launch_bounds__(kSceneTreeThreads)
             a.w = tag_bits<R>(b);
             lmn[p] = a;
             lmx[p] = c;
-            g_leaf_min[lo + p] = a;
-            g_leaf_max[lo + p] = c;
+            if (part == 0u) {
+                g_leaf_min[lo + p] = a;
+                g_leaf_max[lo + p] = c;
+            }
             lpar[p] = ns >= 2 ? t.parent[t.n + lo + p] - lo : 0u;
         }
         if (lo + p + 1 < sc.body_hi) {  // internal node
@@ -878,7 +973,7 @@ __global__ void __launch_bounds__(kSceneTreeThreads)
             }
         }
     }
-    if (!WRITE && tid == 0) *s_cursor = 0u;
+    if (tid == 0) *s_cursor = 0u;
     __syncthreads();
     if (!WRITE) {
         // bottom-up unions and highest leaf positions: the second arrival at
@@ -907,37 +1002,44 @@ __global__ void __launch_bounds__(kSceneTreeThreads)
         __syncthreads();
         for (uint32_t p = tid; p < nb; p += nt) {
             vis[p] = 0u;  // per-body pair counts from here on
-            if (lroot[p] != kNoRoot && lo + p + 1 < t.scenes[t.scene_of_pos[lo + p]].body_hi) {
+            if (part == 0u && lroot[p] != kNoRoot && lo + p + 1 < t.scenes[t.scene_of_pos[lo + p]].body_hi) {
                 g_node_min[lo + p] = nmn[p];
                 g_node_max[lo + p] = nmx[p];
             }
         }
         __syncthreads();
     }
-    const uint32_t region = nb * t.scratch_k;
-    uint2* dst = t.scratch + (size_t)lo * t.scratch_k;
-    for (uint32_t p = tid; p < nb; p += nt) {
-        const uint32_t root = lroot[p];
-        if (root == kNoRoot) continue;
-        if (WRITE)
-            tree_write_leaf<R>(p, root, lmn, lmx, nmn, nmx, ch, t);
-        else
-            tree_count_leaf<R>(p, root, lmn, lmx, nmn, nmx, vis, s_cursor, dst, region, lo, t.err);
-    }
     if (!WRITE) {
-        __syncthreads();
-        for (uint32_t p = tid; p < nb; p += nt) t.counts[lo + p] = vis[p];
-        if (tid == 0) {
-            const uint32_t total = *s_cursor;
-            t.chunk_n[cidx] = min(total, region);
-            t.chunk_ovf[cidx] = total > region ? 1u : 0u;
-            t.chunk_tot[cidx] = total;
+        const uint32_t parts = tree_parts(t, nb), slots = tree_part_slots(t, nb);
+        uint2* dst = t.scratch + (size_t)lo * t.scratch_k + part * slots;
+        for (uint32_t u = tid;; u += nt) {
+            const uint32_t p = ((u >> 5) * parts + part) * 32u + (u & 31u);
+            if (p >= nb) break;
+            if (lroot[p] != kNoRoot)
+                tree_count_leaf<R>(p, lroot[p], lmn, lmx, nmn, nmx, t.fused ? nullptr : vis, s_cursor, dst, slots, lo,
+                                   t.err);
         }
-    }
-    if (fused) {
         __syncthreads();
-        fused_emit(t, lo, nb, npar, lroot, &s_nlong, reinterpret_cast<uint32_t*>(lmn),
-                   (uint32_t)(cb * 2u * sizeof(A4<R>) / 4u));
+        if (!t.fused)
+            for (uint32_t p = tid; p < nb; p += nt) t.counts[lo + p] = vis[p];
+        if (tid == 0) t.chunk_tot[cidx * t.parts + part] = *s_cursor;
+        return;
+    }
+    // the scratch overflowed: walk the trees again
+    if (t.fused) {
+        for (uint32_t p = tid; p < nb; p += nt) vis[p] = 0u;
+        __syncthreads();
+        for (uint32_t p = tid; p < nb; p += nt)
+            if (lroot[p] != kNoRoot)
+                tree_count_leaf<R>(p, lroot[p], lmn, lmx, nmn, nmx, vis, s_cursor, nullptr, 0u, lo, t.err);
+        __syncthreads();
+        fused_offsets(t, lo, nb, lpar, vis, s_red);
+    }
+    for (uint32_t p = tid; p < nb; p += nt)
+        if (lroot[p] != kNoRoot) tree_write_leaf<R>(p, lroot[p], lmn, lmx, nmn, nmx, ch, t);
+    if (t.fused) {
+        __syncthreads();
+        fused_emit(t, lo, nb, vis, lroot, &s_nlong, reinterpret_cast<uint32_t*>(lmn));
     }
 }
 
