@@ -60,7 +60,6 @@ struct Counters {
     uint32_t scene_cursor;
     uint32_t prev_rows;       // rows of the previous step (warm-start source)
     uint32_t prev_pair_rows;  // of which from narrow-phase slots
-    uint32_t long_count;      // CSR segments too long for the in-thread sort
     uint32_t dyn_changed;     // a state update turned a body static or dynamic
     uint32_t prev_pairs;      // pairs of the previous step (contact-lag rows)
     uint32_t traverse_pairs;  // pairs appended by the global trees' count pass

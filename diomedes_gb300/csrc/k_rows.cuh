@@ -77,8 +77,10 @@ __device__ __forceinline__ bool key_eq(uint2 a, uint2 b) { return a.x == b.x && 
 // world's rows are in canonical order: pair rows follow the pair list, which
 // is sorted by (a, b), and container rows the body index, so each section is
 // sorted by key with equal keys adjacent.  The first row of a key takes
-// (lambda, penalty) of the last previous row with it, found by binary search
-// in the previous step's section; every row then decays.  Without `on` (rows
+// (lambda, penalty) of the last previous row with it, found from where the new
+// row stands in its section (`rank`: of the key's last new row): contacts come
+// and go slowly, so the search gallops out from there, and for a section that
+// kept its rows it ends at once.  Every row then decays.  Without `on` (rows
 // prepared for a caller) the duals start fresh and k_warm follows.
 template <class P, class R>
 struct WarmStart {
@@ -86,17 +88,46 @@ struct WarmStart {
     const uint2* prev_ab;
     RowDuals<P, R> prev;
     const Counters* ctr;
-    __device__ __forceinline__ RowDual<P, R> dual(uint2 key, bool first, const PrepParams<R>& o) const {
+    __device__ __forceinline__ RowDual<P, R> dual(uint2 key, bool first, uint32_t rank, const PrepParams<R>& o) const {
         RowDual<P, R> du = fresh_dual<P, R>(o.penalty_min);
         if (!on) return du;
         if (first) {
             const bool cont = key.y == kContainer;
             const uint32_t base = cont ? ctr->prev_pair_rows : 0u;
             uint32_t lo = base, hi = cont ? ctr->prev_rows : ctr->prev_pair_rows;
-            while (lo < hi) {  // upper bound of key
-                const uint32_t mid = (lo + hi) >> 1;
-                if (!key_less(key, prev_ab[mid]))
-                    lo = mid + 1;
+            // upper bound of key: rows before lo are at most key, rows from hi on above it
+            auto above = [&](uint32_t at) { return key_less(key, prev_ab[at]); };
+            if (lo < hi) {
+                const uint32_t at = rank < hi - base ? base + rank : hi - 1u;
+                uint32_t step = 1u;
+                if (above(at)) {
+                    hi = at;
+                    while (lo < hi) {
+                        const uint32_t g = hi - lo > step ? hi - step : lo;
+                        if (!above(g)) {
+                            lo = g + 1u;
+                            break;
+                        }
+                        hi = g;
+                        step <<= 1;
+                    }
+                } else {
+                    lo = at + 1u;
+                    while (lo < hi) {
+                        const uint32_t g = hi - lo > step ? lo + step - 1u : hi - 1u;
+                        if (above(g)) {
+                            hi = g;
+                            break;
+                        }
+                        lo = g + 1u;
+                        step <<= 1;
+                    }
+                }
+            }
+            while (lo < hi) {
+                const uint32_t mid = lo + ((hi - lo) >> 1);
+                if (!above(mid))
+                    lo = mid + 1u;
                 else
                     hi = mid;
             }
@@ -110,46 +141,24 @@ struct WarmStart {
     }
 };
 
-// raw_contact for the valid slots of group p, from row r on in slot order.
+// The lanes of this lane's group of `per` slots (per divides 32) among `m`.
+__device__ __forceinline__ uint32_t group_lanes(uint32_t m, uint32_t lane, uint32_t per) {
+    return m & ((per == 32u ? 0xFFFFFFFFu : (1u << per) - 1u) << (lane & ~(per - 1u)));
+}
+
+// raw_contact for one valid slot, as row r; `first` of its group, which ends
+// with row `last`.
 template <class P, class R>
-__device__ __forceinline__ void slot_rows(const DevWorld<P, R>& w, const Slot<R>* slots, uint32_t per, uint32_t p,
-                                          uint32_t r, const PrepParams<R>& o, const WarmStart<P, R>& warm,
-                                          uint32_t* incident) {
-    bool first = true;
-    uint32_t rows = 0, sa = 0, sb = 0;
-    NB<R> A, B;
-    for (uint32_t k = 0; k < per; ++k) {
-        const Slot<R> s = slots[(size_t)p * per + k];
-        if (!s.valid) continue;
-        if (s.a >= w.n || s.b >= w.n) {
-            atomicOr(&w.ctr->error_flags, kErrBadIndex);
-            continue;
-        }
-        if (r >= w.max_rows) {
-            atomicOr(&w.ctr->error_flags, kErrRowOverflow);
-            break;
-        }
-        if (first || s.a != sa || s.b != sb) {  // a group's slots are one pair's
-            A = load_nb(w, s.a);
-            B = load_nb(w, s.b);
-            sa = s.a;
-            sb = s.b;
-        }
-        V3<R> nrm = xyz(s.normal);
-        V3<R> t1, t2;
-        tangents(nrm, t1, t2);
-        V3<R> ra = rotate(conj(A.rot), sub(xyz(s.pa), A.pos));
-        V3<R> rb = rotate(conj(B.rot), sub(xyz(s.pb), B.pos));
-        write_row(w, r, s.a, s.b, neg(nrm), t1, t2, ra, rb, V3<R>{o.margin - s.depth, R(0), R(0)}, o.friction,
-                  warm.dual(make_uint2(s.a, s.b), first, o));
-        first = false;
-        ++rows;
-        ++r;
-    }
-    if (incident && rows) {
-        if (w.inv[sa].w != R(0)) atomicAdd(&incident[sa], rows);
-        if (w.inv[sb].w != R(0)) atomicAdd(&incident[sb], rows);
-    }
+__device__ __forceinline__ void slot_row(const DevWorld<P, R>& w, const Slot<R>& s, uint32_t r, bool first,
+                                         uint32_t last, const PrepParams<R>& o, const WarmStart<P, R>& warm) {
+    const RowDual<P, R> du = warm.dual(make_uint2(s.a, s.b), first, last, o);
+    const NB<R> A = load_nb(w, s.a), B = load_nb(w, s.b);
+    V3<R> nrm = xyz(s.normal);
+    V3<R> t1, t2;
+    tangents(nrm, t1, t2);
+    V3<R> ra = rotate(conj(A.rot), sub(xyz(s.pa), A.pos));
+    V3<R> rb = rotate(conj(B.rot), sub(xyz(s.pb), B.pos));
+    write_row(w, r, s.a, s.b, neg(nrm), t1, t2, ra, rb, V3<R>{o.margin - s.depth, R(0), R(0)}, o.friction, du);
 }
 
 // cube_support_face, engine/src/physics/gpu.rs:314-350 (per-axis for BOX)
@@ -173,10 +182,12 @@ __device__ __forceinline__ void support_face(const NB<R>& b, V3<R> outward, V3<R
 }
 
 // container_contacts for one body (engine/src/physics/gpu.rs:352-404):
-// counts (write == false) or writes rows starting at `r`.
+// counts (write == false) or writes rows starting at `r`; `last`: its last
+// row's place among the container rows.
 template <class P, class R>
 __device__ __forceinline__ uint32_t container_rows(const DevWorld<P, R>& w, uint32_t i, const PrepParams<R>& o,
-                                                   bool write_out, uint32_t r, const WarmStart<P, R>& warm) {
+                                                   bool write_out, uint32_t r, uint32_t last,
+                                                   const WarmStart<P, R>& warm) {
     const A4<R>* walls = w.walls + 6 * (size_t)w.scene[i];
     V3<R> vel = cast3<R>(xyz(w.vel[i]));
     // Quick reject: every support point lies within an L1 bounding radius of
@@ -250,7 +261,7 @@ __device__ __forceinline__ uint32_t container_rows(const DevWorld<P, R>& w, uint
                         V3<R> ra = rotate(conj(b.rot), sub(cp, b.pos));
                         write_row(w, r + count, i, kContainer, normal, t1, t2, ra, V3<R>{R(0), R(0), R(0)},
                                   V3<R>{o.margin - depth, R(0), R(0)}, o.friction,
-                                  warm.dual(make_uint2(i, kContainer), count == 0, o));
+                                  warm.dual(make_uint2(i, kContainer), count == 0, last, o));
                     } else {
                         atomicOr(&w.ctr->error_flags, kErrRowOverflow);
                     }
@@ -316,19 +327,24 @@ __global__ void k_row_counts(DevWorld<P, R> w, const Slot<R>* slots, uint32_t pe
         if (incident) incident[n] = 0u;
     }
     const WarmStart<P, R> none{};
-    // bodies first: they are known to be there, and the longer work
-    const uint64_t items = (uint64_t)n + ng;
-    for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < items; t += (uint64_t)gridDim.x * blockDim.x) {
-        uint32_t c = 0;
-        if (t < n) {
+    // bodies first (up to a warp's multiple, so that a group's slots are one
+    // warp's): they are known to be there, and the longer work
+    const uint32_t nw = (n + 31u) & ~31u, lane = threadIdx.x & 31u;
+    const uint64_t items = (uint64_t)nw + (uint64_t)ng * per;
+    for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t - lane < items;
+         t += (uint64_t)gridDim.x * blockDim.x) {
+        if (t < nw) {
             const uint32_t i = (uint32_t)t;
-            if (w.inv[i].w != R(0) && w.scenes[w.scene[i]].has_container) c = container_rows(w, i, o, false, 0, none);
+            if (i >= n) continue;
+            uint32_t c = 0;
+            if (w.inv[i].w != R(0) && w.scenes[w.scene[i]].has_container) c = container_rows(w, i, o, false, 0, 0, none);
             counts2[i] = c;
             if (incident) incident[i] = 0u;
         } else {
-            const uint32_t p = (uint32_t)(t - n);
-            for (uint32_t k = 0; k < per; ++k) c += slots[(size_t)p * per + k].valid ? 1u : 0u;
-            counts[p] = c;
+            const uint64_t k = t - nw;
+            const uint32_t valid = __ballot_sync(0xFFFFFFFFu, t < items && slots[k].valid);
+            if (t < items && (lane & (per - 1u)) == 0u)
+                counts[k / per] = (uint32_t)__popc(group_lanes(valid, lane, per));
         }
     }
 }
@@ -350,17 +366,48 @@ __global__ void k_rows(DevWorld<P, R> w, const Slot<R>* slots, uint32_t per, con
         w.ctr->rows = t > w.max_rows ? w.max_rows : (uint32_t)t;
         if (t > w.max_rows) atomicOr(&w.ctr->error_flags, kErrRowOverflow);
     }
-    const uint64_t items = (uint64_t)live + n;
-    for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < items; t += (uint64_t)gridDim.x * blockDim.x) {
-        if (t < live) {
-            const uint32_t p = (uint32_t)t, r = off[p];
+    // a thread a slot: the rows of a contact-dense pair are written together
+    // (a thread a group wrote up to eight in turn: 20 us cold for 90 pairs of
+    // cubes, now 8; 200,000-body wall 94 and 74, with the galloping warm start)
+    const uint64_t nslots = (uint64_t)live * per, sw = (nslots + 31u) & ~31ull, items = sw + n;
+    const uint32_t lane = threadIdx.x & 31u;
+    for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t - lane < items;
+         t += (uint64_t)gridDim.x * blockDim.x) {
+        if (t < sw) {
+            const uint32_t p = (uint32_t)(t / per);
+            uint32_t r = 0;
+            bool good = false;
+            Slot<R> s;
             // a group without valid slots (a box overlap without contact) is
             // skipped unread; the last live group ends at the total
-            if ((p + 1 < live ? off[p + 1] : pair_rows) != r) slot_rows(w, slots, per, p, r, o, warm, incident);
+            if (t < nslots && (p + 1 < live ? off[p + 1] : pair_rows) != (r = off[p])) {
+                s = slots[t];
+                good = s.valid;
+                if (good && (s.a >= w.n || s.b >= w.n)) {
+                    atomicOr(&w.ctr->error_flags, kErrBadIndex);
+                    good = false;
+                }
+            }
+            const uint32_t rows = group_lanes(__ballot_sync(0xFFFFFFFFu, good), lane, per);
+            r += (uint32_t)__popc(rows & ((1u << lane) - 1u));
+            if (good && r >= w.max_rows) {
+                atomicOr(&w.ctr->error_flags, kErrRowOverflow);
+                good = false;
+            }
+            const uint32_t kept = group_lanes(__ballot_sync(0xFFFFFFFFu, good), lane, per);
+            if (!good) continue;
+            const bool first = !(kept & ((1u << lane) - 1u));
+            if (incident && first) {  // a group's slots are one pair's
+                if (w.inv[s.a].w != R(0)) atomicAdd(&incident[s.a], (uint32_t)__popc(kept));
+                if (w.inv[s.b].w != R(0)) atomicAdd(&incident[s.b], (uint32_t)__popc(kept));
+            }
+            slot_row(w, s, r, first, r + (uint32_t)__popc(kept) - 1u, o, warm);
         } else {
-            const uint32_t i = (uint32_t)(t - live), r = off2[i], rows = off2[i + 1] - r;
+            const uint64_t b = t - sw;
+            if (b >= n) continue;
+            const uint32_t i = (uint32_t)b, r = off2[i], rows = off2[i + 1] - r;
             if (!rows) continue;  // nothing to recompute
-            container_rows(w, i, o, true, pair_rows + r, warm);
+            container_rows(w, i, o, true, pair_rows + r, r + rows - 1u, warm);
             if (incident) {  // rows that were kept
                 const uint64_t at = (uint64_t)pair_rows + r;
                 const uint32_t kept = at >= w.max_rows ? 0u : (uint32_t)min((uint64_t)rows, w.max_rows - at);
@@ -491,112 +538,62 @@ static __global__ void k_roll_counters(Counters* c, uint32_t* zero0, uint32_t* z
     c->container_rows = 0;
     c->gjk_work = 0;
     c->epa_work = 0;
-    c->long_count = 0;
     c->colors = 0;
     c->traverse_pairs = 0;
 }
 
 // CSR of the dynamic bodies only (the primal never visits a static body):
-// counts from k_rows, then an atomic scatter (each body's count taken down to
-// zero), then each segment sorted by row index, which restores the
-// reference's fill order (finalize_contacts, gpu.rs:286-310) without a sort
-// over all incidences, with the other-body array.
+// counts from k_rows, an atomic scatter (each body's count taken down to
+// zero) into `loose`, then each row's place in its body's segment by its rank
+// there, which restores the reference's fill order (finalize_contacts,
+// gpu.rs:286-310) without a sort over all incidences, with the other-body
+// array.
 // remaining: each body's incidence count (k_rows), consumed here
 template <class P, class R>
-__global__ void k_csr_scatter_dyn(DevWorld<P, R> w, uint32_t* remaining) {
+__global__ void k_csr_scatter_dyn(DevWorld<P, R> w, uint32_t* remaining, uint32_t* loose) {
     pdl_enter();
     const uint32_t m = w.ctr->rows;
     for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < m; r += gridDim.x * blockDim.x) {
         uint2 ab = w.ab[r];
         if (w.inv[ab.x].w != R(0)) {
             uint32_t j = w.row_off[ab.x] + atomicSub(&remaining[ab.x], 1u) - 1u;
-            if (j < w.max_incid) w.row_idx[j] = r;
+            if (j < w.max_incid) loose[j] = r;
         }
         if (ab.y != kContainer && w.inv[ab.y].w != R(0)) {
             uint32_t j = w.row_off[ab.y] + atomicSub(&remaining[ab.y], 1u) - 1u;
-            if (j < w.max_incid) w.row_idx[j] = r;
+            if (j < w.max_incid) loose[j] = r;
         }
     }
 }
 
-constexpr uint32_t kLongSort = 4096;
-// A segment of up to kLongSort words sorted ascending by the CTA through s
-// (kLongSort words), where it stays too; false (nothing done) when longer.
-__device__ __forceinline__ bool sort_segment(uint32_t* seg, uint32_t len, uint32_t* s) {
-    if (len > kLongSort) return false;
-    uint32_t p2 = 1;
-    while (p2 < len) p2 <<= 1;
-    for (uint32_t k = threadIdx.x; k < p2; k += blockDim.x) s[k] = k < len ? seg[k] : 0xFFFFFFFFu;
-    __syncthreads();
-    for (uint32_t size = 2; size <= p2; size <<= 1) {
-        for (uint32_t stride = size >> 1; stride > 0; stride >>= 1) {
-            for (uint32_t t = threadIdx.x; t < p2; t += blockDim.x) {
-                const uint32_t u = t ^ stride;
-                if (u > t) {
-                    const bool up = (t & size) == 0;
-                    const uint32_t x = s[t], y = s[u];
-                    if ((x > y) == up) {
-                        s[t] = y;
-                        s[u] = x;
-                    }
-                }
-            }
-            __syncthreads();
-        }
-    }
-    for (uint32_t k = threadIdx.x; k < len; k += blockDim.x) seg[k] = s[k];
-    return true;
-}
-
-// the other body of row `row` seen from body i
-__device__ __forceinline__ uint32_t other_body(const uint2* ab, uint32_t row, uint32_t i) {
-    const uint2 v = ab[row];
-    return v.y == kContainer ? kContainer : (v.x == i ? v.y : (v.x | kIsB));
-}
-constexpr uint32_t kShortRows = 32;  // segments up to this sorted by a thread
+constexpr uint32_t kLongRows = 4096;
+// A thread per end of a row counts the smaller rows of its body's segment: the
+// loads do not wait for one another, and the threads of a pair's rows read the
+// same ones.  (A thread per body with an insertion sort in local memory, longer
+// segments by a CTA each: 15 us cold a step for 8,192 stacked cubes, 13.5 for a
+// 55-cube pyramid of 8-contact pairs; now 6 and 5.)  A segment beyond kLongRows
+// rows is reported and left as it is.
 template <class P, class R>
-__global__ void k_csr_finish_dyn(DevWorld<P, R> w, uint32_t* long_list, uint32_t* long_count) {
+__global__ void k_csr_finish_dyn(DevWorld<P, R> w, const uint32_t* loose) {
     pdl_enter();
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < w.n; i += gridDim.x * blockDim.x) {
+    const uint64_t items = 2ull * w.ctr->rows;
+    for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < items; t += (uint64_t)gridDim.x * blockDim.x) {
+        const uint32_t r = (uint32_t)(t >> 1);
+        const uint2 ab = w.ab[r];
+        const uint32_t i = (t & 1u) ? ab.y : ab.x;
+        if (i == kContainer || w.inv[i].w == R(0)) continue;
         const uint32_t j0 = w.row_off[i], j1 = min(w.row_off[i + 1], w.max_incid);
         if (j0 >= j1) continue;
-        const uint32_t len = j1 - j0;
-        if (len > kShortRows) {
-            long_list[warp_append(long_count)] = i;
+        if (j1 - j0 > kLongRows) {
+            atomicOr(&w.ctr->error_flags, kErrIndexOverflow);
             continue;
         }
-        uint32_t v[kShortRows];
-        for (uint32_t k = 0; k < len; ++k) {
-            const uint32_t x = w.row_idx[j0 + k];
-            int m = (int)k - 1;
-            while (m >= 0 && v[m] > x) {
-                v[m + 1] = v[m];
-                --m;
-            }
-            v[m + 1] = x;
-        }
-        for (uint32_t k = 0; k < len; ++k) {
-            w.row_idx[j0 + k] = v[k];
-            w.row_oth[j0 + k] = other_body(w.ab, v[k], i);
-        }
-    }
-}
-// the long segments, a CTA each
-template <class P, class R>
-__global__ void __launch_bounds__(512) k_csr_finish_long(DevWorld<P, R> w, const uint32_t* long_list,
-                                                         const uint32_t* long_count) {
-    pdl_enter();
-    __shared__ uint32_t s[kLongSort];
-    const uint32_t cnt = *long_count;
-    for (uint32_t q = blockIdx.x; q < cnt; q += gridDim.x) {
-        const uint32_t i = long_list[q];
-        const uint32_t j0 = w.row_off[i], len = min(w.row_off[i + 1], w.max_incid) - j0;
-        if (sort_segment(w.row_idx + j0, len, s)) {
-            for (uint32_t k = threadIdx.x; k < len; k += blockDim.x) w.row_oth[j0 + k] = other_body(w.ab, s[k], i);
-        } else if (threadIdx.x == 0) {
-            atomicOr(&w.ctr->error_flags, kErrIndexOverflow);
-        }
-        __syncthreads();  // the next segment's sort
+        uint32_t j = j0;
+#pragma unroll 8
+        for (uint32_t q = j0; q < j1; ++q) j += loose[q] < r ? 1u : 0u;
+        if (j >= j1) continue;
+        w.row_idx[j] = r;
+        w.row_oth[j] = ab.y == kContainer ? kContainer : ((t & 1u) ? (ab.x | kIsB) : ab.y);
     }
 }
 
