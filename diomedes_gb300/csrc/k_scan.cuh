@@ -7,8 +7,9 @@
 // scanned with the lower tiles' sums; one k_scan_excl launch, a single-pass
 // look-back scan, for a single tile); every sort (LBVH Morton keys of worlds
 // with scenes beyond the shared-memory trees, the dynamic-body work order,
-// warm-start row keys, incidence lists) is one k_radix_hist launch plus one
-// k_radix_pass launch per 8-bit digit, each pass with decoupled look-back.
+// warm-start row keys, incidence lists) is one k_rank_sort launch for up to
+// kRankSortMax keys, else one k_radix_hist launch plus one k_radix_pass
+// launch per 8-bit digit, each pass with decoupled look-back.
 // All of them open with griddepcontrol.wait and so chain with programmatic
 // dependent launch.
 //
@@ -618,6 +619,60 @@ __global__ void __launch_bounds__(kRadixThreads)
     if (tid == 0) lb_done(lb.ctl);
 }
 
+// ---- small sorts ----------------------------------------------------------
+// Stable sort by rank: a key's place is the number of smaller keys, and of
+// equal ones before it.  A CTA ranks 32 keys, a lane each; its eight warps share
+// the counting and read a staged tile four (two) keys a load, one address a
+// warp.  n / 32 CTAs spread the n^2 comparisons (two instructions each; four for
+// 64-bit keys) over the SMs, where the digit passes of a small sort are one to
+// three CTAs' serial chain.  Cold, one launch against the passes and their
+// histogram: 8,192 keys of 32 bits 19 us (one digit 25, four 55), 4,096 of
+// 64 bits 12 us (80); for twice 8,192 the squared work passes one digit's time.
+constexpr int kRankThreads = 256, kRankTile = 1024;
+template <class K>
+__global__ void __launch_bounds__(kRankThreads)
+    k_rank_sort(const K* __restrict__ kin, const uint32_t* __restrict__ vin, K* __restrict__ kout,
+                uint32_t* __restrict__ vout, uint32_t n, uint32_t begin_bit, K mask) {
+    pdl_enter();
+    __shared__ __align__(16) K s_key[kRankTile];
+    __shared__ uint32_t s_rank[32];
+    const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+    constexpr uint32_t kSlice = kRankTile / (kRankThreads / 32);
+    const uint32_t e0 = blockIdx.x * 32u, me = e0 + lane;
+    const K key = me < n ? kin[me] : K(0);
+    const K mine = (key >> begin_bit) & mask;
+    uint32_t rank = 0;
+    if (tid < 32u) s_rank[tid] = 0u;
+    for (uint32_t t0 = 0; t0 < n; t0 += kRankTile) {
+        __syncthreads();
+        // past the end: never below a key, and counted only by `<`
+        for (uint32_t k = tid; k < (uint32_t)kRankTile; k += kRankThreads)
+            s_key[k] = t0 + k < n ? (kin[t0 + k] >> begin_bit) & mask : ~K(0);
+        __syncthreads();
+        const uint32_t q0 = t0 + warp * kSlice;  // a slice is before, after or around the CTA's keys
+        const K* s = s_key + warp * kSlice;
+        if (q0 >= n) continue;
+        if (q0 + kSlice <= e0) {
+#pragma unroll 16
+            for (uint32_t q = 0; q < kSlice; ++q) rank += s[q] <= mine ? 1u : 0u;
+        } else if (q0 > e0) {
+#pragma unroll 16
+            for (uint32_t q = 0; q < kSlice; ++q) rank += s[q] < mine ? 1u : 0u;
+        } else {
+            for (uint32_t q = 0; q < kSlice; ++q) rank += s[q] < mine || (s[q] == mine && q0 + q < me) ? 1u : 0u;
+        }
+    }
+    atomicAdd(&s_rank[lane], rank);
+    __syncthreads();
+    if (warp == 0 && me < n) {
+        kout[s_rank[lane]] = key;
+        vout[s_rank[lane]] = vin[me];
+    }
+}
+static_assert(kRankTile % 32 == 0 && (kRankTile / (kRankThreads / 32)) % 32 == 0,
+              "a CTA's 32 keys lie in one slice");
+constexpr uint32_t kRankSortMax = 8192;  // the largest sort by rank
+
 // ---- host side ----------------------------------------------------------
 // Buffers of the scan and sort kernels for one stream: the look-back control
 // word and status array, the digit histograms, and the sort's ping-pong
@@ -745,7 +800,14 @@ struct ScanSort {
                 return e;
             return cudaMemcpyAsync(vout, vin, (size_t)n * 4, cudaMemcpyDeviceToDevice, s);
         }
-        const uint32_t passes = (end_bit - begin_bit + 7u) / 8u;
+        const uint32_t bits = end_bit - begin_bit;
+        if (n <= kRankSortMax) {
+            counted(1);
+            const K mask = bits < 8 * sizeof(K) ? (K(1) << bits) - K(1) : ~K(0);
+            return launch_k(pdl, k_rank_sort<K>, (int)((n + 31u) / 32u), kRankThreads, 0, s, kin, vin, kout, vout, n,
+                            begin_bit, mask);
+        }
+        const uint32_t passes = (bits + 7u) / 8u;
         const int gh = std::max(1, std::min((int)((n + 4095u) / 4096u), 2 * sms));
         if ((e = launch_k(pdl, k_radix_hist<K>, gh, kRadixHistThreads, 0, s, kin, n, begin_bit, end_bit, hist, done,
                           bases)) != cudaSuccess)
