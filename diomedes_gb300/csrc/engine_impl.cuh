@@ -586,6 +586,7 @@ class Engine final : public EngineBase {
         DIO_TRY(alloc(&hull_, H));
         DIO_TRY(alloc(&ctr_, 1));
         DIO_CK(cudaMallocHost(&hctr_, sizeof(Counters)));
+        DIO_CK(cudaEventCreateWithFlags(&copied_, cudaEventDisableTiming));
         // prefix sums and radix sorts: up to CNT scanned counts, and sorts of
         // row keys (M), incidences (INC) and per-body keys (N)
         DIO_CK(ss_.init((uint32_t)std::max<size_t>(std::max<size_t>(M, N), INC),
@@ -842,7 +843,15 @@ class Engine final : public EngineBase {
         DIO_CK(cudaMemsetAsync(ctr_, 0, sizeof(Counters), stream_));
         rebuild_now_ = true;
         lbvh_valid_ = false;
-        return run_broad(0, n);
+        DIO_TRY(run_broad(0, n));
+        return inputs_read();
+    }
+    // The caller's bodies or states have been copied (upload_bodies,
+    // upload_state): theirs again when the call returns, with the kernels
+    // still running.
+    int inputs_read() {
+        DIO_CK(cudaEventSynchronize(copied_));
+        return DIO_OK;
     }
     int pair_count(uint32_t* count) override {
         if (!count) return inval("null count");
@@ -872,7 +881,8 @@ class Engine final : public EngineBase {
         DIO_TRY(single_scene(n, nullptr));
         DIO_CK(cudaMemcpyAsync(w_.pairs, pairs, (size_t)np * sizeof(DioPair), cudaMemcpyHostToDevice, stream_));
         DIO_CK(cudaMemsetAsync(ctr_, 0, sizeof(Counters), stream_));
-        return run_narrow(np, nullptr);
+        DIO_TRY(run_narrow(np, nullptr));
+        return inputs_read();
     }
     int narrow_submit(uint32_t np) override {
         if (np > cap_.max_pairs) return cap_err("too many pairs for the compute buffers");
@@ -892,8 +902,7 @@ class Engine final : public EngineBase {
         } else {
             return inval("narrow_read needs an FP32 engine");
         }
-        DIO_CK(cudaStreamSynchronize(stream_));
-        DIO_TRY(check_flags());
+        DIO_TRY(check_flags());  // one wait for both
         return DIO_OK;
     }
     int set_hull(const float* xyzw, uint32_t count) override {
@@ -923,7 +932,7 @@ class Engine final : public EngineBase {
             return inval("prepare_contacts needs an FP32 engine");
         } else {
             DIO_TRY(upload_bodies(bodies, n, n_hull_));
-            DIO_TRY(upload_state(state, n));
+            DIO_TRY(upload_state(state, n, false));
             DIO_TRY(single_scene(n, container));
             DIO_CK(cudaMemsetAsync(ctr_, 0, sizeof(Counters), stream_));
             // previous rows into the "previous" buffer, then their sorted keys
@@ -947,8 +956,7 @@ class Engine final : public EngineBase {
             DIO_TRY(finish_rows(opts_prep(*options), M, n));
             uint32_t ninc = 0;
             DIO_CK(cudaMemcpyAsync(&ninc, w_.row_off + n, 4, cudaMemcpyDeviceToHost, stream_));
-            DIO_CK(cudaStreamSynchronize(stream_));
-            DIO_TRY(check_flags());
+            DIO_TRY(check_flags());  // one wait for both
             if (M > cap || ninc > index_cap) return cap_err("output buffers smaller than the rows / CSR");
             DioContact* dout = reinterpret_cast<DioContact*>(dstage_);
             k_pack_contacts<P, R><<<grid_for(M, 256), 256, 0, stream_>>>(w_.rs, w_.rd, w_.ab, dout, &ctr_->rows);
@@ -979,7 +987,7 @@ class Engine final : public EngineBase {
         if (ninc > 2ull * cap_.max_contacts) return cap_err("too many CSR indices");
         if (ninc && !indices) return inval("null indices");
         w_.n_joints = 0;  // this call's joints are uploaded below
-        DIO_TRY(upload_state(state, n));
+        DIO_TRY(upload_state(state, n, false));
         // poses
         char* st = reinterpret_cast<char*>(dstage_);
         float* dpos = reinterpret_cast<float*>(st);
@@ -1005,7 +1013,7 @@ class Engine final : public EngineBase {
         SolveParams<R> o = solve_params(options->dt, options->gravity, options->alpha, options->beta_lin,
                                         options->penalty_max, options->iterations);
         DIO_TRY(solve(o, n, m));
-        return DIO_OK;
+        return inputs_read();
     }
 
     int avbd_read(const DioAvbdResult* out) override {
@@ -1022,8 +1030,7 @@ class Engine final : public EngineBase {
         k_pack_result<P, R><<<grid_for(n, 256), 256, 0, stream_>>>(w_, n, buf, dp, dqq, dv, da, dpv);
         if (m) k_pack_dual<P, R><<<grid_for(m, 256), 256, 0, stream_>>>(w_.rd, m, dl, dk);
         DIO_CK(cudaMemcpyAsync(hstage_, d, nb + mb, cudaMemcpyDeviceToHost, stream_));
-        DIO_CK(cudaStreamSynchronize(stream_));
-        DIO_TRY(check_flags());
+        DIO_TRY(check_flags());  // one wait for both
         const float* h = reinterpret_cast<const float*>(hstage_);
         const float *hp = h, *hq = hp + 3 * (size_t)n, *hv = hq + 4 * (size_t)n, *ha = hv + 3 * (size_t)n,
                     *hpv = ha + 3 * (size_t)n, *hl = hpv + 3 * (size_t)n, *hk = hl + 3 * (size_t)m;
@@ -1316,6 +1323,8 @@ class Engine final : public EngineBase {
         allocs_.clear();
         ss_.release();
         if (dstage_) cudaFree(dstage_);
+        if (copied_) cudaEventDestroy(copied_);
+        copied_ = nullptr;
         if (hstage_) cudaFreeHost(hstage_);
         if (hctr_) cudaFreeHost(hctr_);
         dstage_ = nullptr;
@@ -1383,33 +1392,46 @@ class Engine final : public EngineBase {
         if (!hull_ranges_ok(bodies, n, n_hull)) return inval("hull vertex range beyond the hull-vertex pool");
         DioGpuBody* db = reinterpret_cast<DioGpuBody*>(dstage_);
         DIO_CK(cudaMemcpyAsync(db, bodies, (size_t)n * sizeof(DioGpuBody), cudaMemcpyHostToDevice, stream_));
+        DIO_CK(cudaEventRecord(copied_, stream_));
         k_unpack_bodies<P, R><<<grid_for(n, 256), 256, 0, stream_>>>(w_, db, n);
         w_.n = n;
         return DIO_OK;
     }
-    int upload_state(const DioBodyState* state, uint32_t n) {
+    // order: the dynamic list in the solve's order (a caller whose joints order
+    // it again, or that does not solve, goes without)
+    int upload_state(const DioBodyState* state, uint32_t n, bool order = true) {
         if (!n) return DIO_OK;
         if (!state) return inval("null state");
         DioBodyState* ds = reinterpret_cast<DioBodyState*>(reinterpret_cast<char*>(dstage_) +
                                                            align256((size_t)n * sizeof(DioGpuBody)));
         DIO_CK(cudaMemcpyAsync(ds, state, (size_t)n * sizeof(DioBodyState), cudaMemcpyHostToDevice, stream_));
+        DIO_CK(cudaEventRecord(copied_, stream_));
         k_unpack_state<P, R><<<grid_for(n, 256), 256, 0, stream_>>>(w_, ds, n);
-        return build_dyn_list(n);
+        return build_dyn_list(n, state, order);
     }
-    // compacted list of dynamic bodies (inverse mass != 0), index order
-    int build_dyn_list(uint32_t n) {
+    // compacted list of dynamic bodies (inverse mass != 0), index order.
+    // state (if given): the states it is built from, in host memory; a short
+    // list is counted there while the kernels run, which costs less than
+    // waiting for them (a 5,005-body solve, its list ordered once: 446 us a pass
+    // and 404)
+    static constexpr uint32_t kHostCount = 8192;
+    int build_dyn_list(uint32_t n, const DioBodyState* state = nullptr, bool order = true) {
         dyn_list_n_ = n;
         k_dyn_flags<P, R><<<grid_for(n, 256), 256, 0, stream_>>>(w_, n, counts2_, dyn_keep_);
         DIO_CK(cudaMemsetAsync(counts2_ + n, 0, 4, stream_));
         DIO_CK(ss_.scan(counts2_, offsets2_, n + 1, false, stream_));
         k_dyn_fill<<<grid_for(n, 256), 256, 0, stream_>>>(counts2_, offsets2_, n, dyn_list_);
         uint32_t nd = 0;
-        DIO_CK(cudaMemcpyAsync(&nd, offsets2_ + n, 4, cudaMemcpyDeviceToHost, stream_));
-        DIO_CK(cudaStreamSynchronize(stream_));
+        if (state && n <= kHostCount) {
+            for (uint32_t i = 0; i < n; ++i) nd += state[i].inv_mass != 0.0f ? 1u : 0u;
+        } else {
+            DIO_CK(cudaMemcpyAsync(&nd, offsets2_ + n, 4, cudaMemcpyDeviceToHost, stream_));
+            DIO_CK(cudaStreamSynchronize(stream_));
+        }
         if (w_.n_dyn != nd) drop_graphs();  // launch shapes depend on it
         w_.n_dyn = nd;
         w_.dyn_list = dyn_list_;
-        return order_dyn_list();
+        return order || chunked_scenes_ ? order_dyn_list() : DIO_OK;
     }
     // stable sort of the dynamic-body list by work signature (k_dyn_keys);
     // index order is kept inside a signature
@@ -1446,17 +1468,19 @@ class Engine final : public EngineBase {
             x.half_extent = c->half_extent;
             std::memcpy(x.rotation, c->rotation, 16);
         }
-        DIO_CK(cudaMemcpyAsync(scenes_, &x, sizeof x, cudaMemcpyHostToDevice, stream_));
         DIO_CK(cudaMemsetAsync(w_.scene, 0, (size_t)std::max(n, 1u) * 4, stream_));
         w_.n_scenes = 1;
         w_.origin = nullptr;
-        k_scene_walls<P, R><<<1, 32, 0, stream_>>>(w_, scenes_, 1u, walls_);
         w_.n = n;
         // the API path is single-scene FP32; keep host scene table in sync
         scenes_host_.assign(1, x);
-        DIO_TRY(note_scene_sizes());
-        chunked_scenes_ = false;  // these calls solve per phase: the list needs no CTA order
-        DIO_CK(cudaStreamSynchronize(stream_));
+        scene_max_ = n;
+        chunk_max_ = pack_chunks(scene_tree_cap<R>(), chunks_host_);
+        // these calls solve per phase: no solve chunks, and the list needs no CTA order
+        solve_chunks_host_.clear();
+        chunked_scenes_ = chunk_world_ = false;
+        k_single_scene<P, R><<<1, 32, 0, stream_>>>(x, !chunks_host_.empty(), scenes_, chunks_, walls_);
+        DIO_CK(cudaGetLastError());
         return DIO_OK;
     }
     // every joint's two bodies in one scene of the uploaded world
@@ -2449,6 +2473,7 @@ class Engine final : public EngineBase {
     Counters* hctr_ = nullptr;
     ScanSort ss_;  // prefix sums and radix sorts
     void* dstage_ = nullptr;
+    cudaEvent_t copied_ = nullptr;  // after the last upload_bodies / upload_state copy
     void* hstage_ = nullptr;
     size_t stage_bytes_ = 0;
     int cur_ = 0;

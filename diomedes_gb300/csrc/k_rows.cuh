@@ -292,24 +292,39 @@ __global__ void k_hull_bounds(DevWorld<P, R> w, uint32_t n, R* bound) {
     }
 }
 
-// The six walls of each scene's container (container_collide,
+// Wall k of a scene's container (container_collide,
 // engine/src/physics/gpu.rs): outward normal = rotation * (+-axis), plane
 // offset = centre . outward + half extent; centre rebased to the scene's
-// detection origin.  Computed once per upload.
+// detection origin.
+template <class P, class R>
+__device__ __forceinline__ A4<R> scene_wall(const SceneDesc& sc, V3<P> org, uint32_t k) {
+    const V3<R> center = cast3<R>(sub(V3<P>{P(sc.center[0]), P(sc.center[1]), P(sc.center[2])}, org));
+    const Q4<R> crot{R(sc.rotation[0]), R(sc.rotation[1]), R(sc.rotation[2]), R(sc.rotation[3])};
+    const R half = R(sc.half_extent);
+    const V3<R> axis = k < 2 ? V3<R>{R(1), R(0), R(0)} : (k < 4 ? V3<R>{R(0), R(1), R(0)} : V3<R>{R(0), R(0), R(1)});
+    const R sign = (k & 1) ? R(-1) : R(1);
+    const V3<R> outward = rotate(crot, scale(axis, sign));
+    return A4<R>{outward.x, outward.y, outward.z, dot(center, outward) + half};
+}
+// every scene's walls, once per upload
 template <class P, class R>
 __global__ void k_scene_walls(DevWorld<P, R> w, const SceneDesc* scenes, uint32_t ns, A4<R>* walls) {
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < 6 * ns; t += gridDim.x * blockDim.x) {
         const uint32_t s = t / 6, k = t % 6;
-        const SceneDesc sc = scenes[s];
         V3<P> org{P(0), P(0), P(0)};
         if (w.origin) org = xyz(w.origin[s]);
-        const V3<R> center = cast3<R>(sub(V3<P>{P(sc.center[0]), P(sc.center[1]), P(sc.center[2])}, org));
-        const Q4<R> crot{R(sc.rotation[0]), R(sc.rotation[1]), R(sc.rotation[2]), R(sc.rotation[3])};
-        const R half = R(sc.half_extent);
-        const V3<R> axis = k < 2 ? V3<R>{R(1), R(0), R(0)} : (k < 4 ? V3<R>{R(0), R(1), R(0)} : V3<R>{R(0), R(0), R(1)});
-        const R sign = (k & 1) ? R(-1) : R(1);
-        const V3<R> outward = rotate(crot, scale(axis, sign));
-        walls[t] = A4<R>{outward.x, outward.y, outward.z, dot(center, outward) + half};
+        walls[t] = scene_wall<P, R>(scenes[s], org, k);
+    }
+}
+// The scene table of a caller's single scene: given by value, so that the host
+// waits for no copy (chunk: it is one of the shared-memory trees).
+template <class P, class R>
+__global__ void k_single_scene(const SceneDesc sc, bool chunk, SceneDesc* scenes, uint2* chunks, A4<R>* walls) {
+    const uint32_t k = threadIdx.x;
+    if (k < 6u) walls[k] = scene_wall<P, R>(sc, V3<P>{P(0), P(0), P(0)}, k);
+    if (k == 0u) {
+        scenes[0] = sc;
+        if (chunk) chunks[0] = make_uint2(0u, 1u);
     }
 }
 
