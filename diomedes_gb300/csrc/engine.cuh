@@ -54,6 +54,7 @@ struct Counters {
     uint32_t container_rows;  // rows against containers
     uint32_t gjk_work;        // pairs routed to GJK
     uint32_t epa_work;        // pairs routed to EPA
+    uint32_t epa_next;        // of which taken by a warp after its first
     uint32_t error_flags;
     uint32_t colors;
     uint32_t color_remaining;

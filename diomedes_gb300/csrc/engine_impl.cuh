@@ -888,7 +888,7 @@ class Engine final : public EngineBase {
         if (np > cap_.max_pairs) return cap_err("too many pairs for the compute buffers");
         last_np_ = np;
         if (np == 0) return DIO_OK;
-        DIO_CK(cudaMemsetAsync(&ctr_->gjk_work, 0, 2 * sizeof(uint32_t), stream_));
+        DIO_CK(cudaMemsetAsync(&ctr_->gjk_work, 0, 3 * sizeof(uint32_t), stream_));
         return run_narrow(np, nullptr);
     }
     int narrow_read(DioContactOut* out, uint32_t cap, uint32_t* n) override {

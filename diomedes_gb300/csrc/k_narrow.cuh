@@ -136,8 +136,8 @@ __device__ __forceinline__ V3<R> support(const ShapeR<R>& s, V3<R> d, const A4<R
     }
 }
 
-// Warp minimum / maximum of the finite values of the lanes with `has`, ties to
-// the lowest index: the index (0xFFFFFFFF: no lane has one).  FP32: the
+// Minimum / maximum of the finite values of the lanes with `has`, among the
+// lanes of the mask (an aligned group of kLanes), ties to the lowest index: the index (0xFFFFFFFF: no lane has one).  FP32: the
 // values as ordered integers through two redux instructions (five rounds of
 // two shuffles took ten times as long); -0 is taken as +0, as a comparison
 // takes it.
@@ -145,20 +145,20 @@ __device__ __forceinline__ uint32_t order_bits(float x) {
     const uint32_t u = __float_as_uint(x + 0.f);
     return u & 0x80000000u ? ~u : u | 0x80000000u;
 }
-template <bool kMax, class R>
-__device__ __forceinline__ uint32_t warp_best(bool has, R v, uint32_t index) {
+template <bool kMax, int kLanes, class R>
+__device__ __forceinline__ uint32_t lanes_best(bool has, R v, uint32_t index, uint32_t mask) {
     constexpr uint32_t kAll = 0xFFFFFFFFu;
     if constexpr (sizeof(R) == 4) {
         // ordered bits of a number lie strictly between 0 and 2^32 - 1
         const uint32_t key = order_bits(v);
-        const uint32_t best = kMax ? __reduce_max_sync(kAll, has ? key : 0u) : __reduce_min_sync(kAll, has ? key : kAll);
-        return __reduce_min_sync(kAll, has && key == best ? index : kAll);
+        const uint32_t best = kMax ? __reduce_max_sync(mask, has ? key : 0u) : __reduce_min_sync(mask, has ? key : kAll);
+        return __reduce_min_sync(mask, has && key == best ? index : kAll);
     } else {
         uint32_t bi = has ? index : kAll;
 #pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-            const R ov = __shfl_xor_sync(kAll, v, off);
-            const uint32_t oi = __shfl_xor_sync(kAll, bi, off);
+        for (int off = kLanes / 2; off > 0; off >>= 1) {
+            const R ov = __shfl_xor_sync(mask, v, off);
+            const uint32_t oi = __shfl_xor_sync(mask, bi, off);
             if (oi != kAll && (bi == kAll || (kMax ? ov > v : ov < v) || (ov == v && oi < bi))) {
                 v = ov;
                 bi = oi;
@@ -166,6 +166,10 @@ __device__ __forceinline__ uint32_t warp_best(bool has, R v, uint32_t index) {
         }
         return bi;
     }
+}
+template <bool kMax, class R>
+__device__ __forceinline__ uint32_t warp_best(bool has, R v, uint32_t index) {
+    return lanes_best<kMax, 32>(has, v, index, 0xFFFFFFFFu);
 }
 
 // support() of a hull with the 32 lanes of a warp over its vertices (every
@@ -192,13 +196,33 @@ __device__ __forceinline__ V3<R> support_warp(const ShapeR<R>& s, V3<R> d, const
     return xyz(hull[s.hf + bi]);
 }
 
-template <class R>
+// The same with an aligned group of kG lanes (mask: theirs); kG = 1: support().
+template <int kG, class R>
+__device__ __forceinline__ V3<R> support_group(const ShapeR<R>& s, V3<R> d, const A4<R>* hull, uint32_t lane,
+                                               uint32_t mask) {
+    if (kG == 1 || s.tag != DIO_SHAPE_HULL || s.hc == 0 || hull == nullptr) return support(s, d, hull);
+    const V3<R> v0 = xyz(hull[s.hf]);
+    if (isnan(dot(v0, d))) return v0;
+    R bv = R(0);
+    uint32_t bi = 0xFFFFFFFFu;
+    for (uint32_t i = lane & (kG - 1); i < s.hc; i += kG) {
+        const R dd = dot(xyz(hull[s.hf + i]), d);
+        if (!isnan(dd) && (bi == 0xFFFFFFFFu || dd > bv)) {
+            bv = dd;
+            bi = i;
+        }
+    }
+    bi = lanes_best<true, kG>(bi != 0xFFFFFFFFu, bv, bi, mask);
+    return xyz(hull[s.hf + bi]);
+}
+
+template <int kG, class R>
 __device__ __forceinline__ void support_witness(const NB<R>& a, const NB<R>& b, V3<R> d, const A4<R>* hull,
-                                                V3<R>& point, V3<R>& wit) {
+                                                V3<R>& point, V3<R>& wit, uint32_t lane, uint32_t mask) {
     V3<R> al = rotate(conj(a.rot), d);
-    V3<R> ap = add(rotate(a.rot, support(a.shape, al, hull)), a.pos);
+    V3<R> ap = add(rotate(a.rot, support_group<kG>(a.shape, al, hull, lane, mask)), a.pos);
     V3<R> bl = rotate(conj(b.rot), neg(d));
-    V3<R> bp = add(rotate(b.rot, support(b.shape, bl, hull)), b.pos);
+    V3<R> bp = add(rotate(b.rot, support_group<kG>(b.shape, bl, hull, lane, mask)), b.pos);
     point = sub(ap, bp);
     wit = ap;
 }
@@ -528,18 +552,19 @@ __device__ bool contains_origin(Simplex<R>& s, V3<R>& d) {
     return false;
 }
 
-// gjk, gjk.rs:77-109
-template <class R>
-__device__ bool gjk(const NB<R>& a, const NB<R>& b, const A4<R>* hull, Simplex<R>& s) {
+// gjk, gjk.rs:77-109, by an aligned group of kG lanes (mask: theirs; every lane
+// the same simplex)
+template <int kG, class R>
+__device__ bool gjk(const NB<R>& a, const NB<R>& b, const A4<R>* hull, Simplex<R>& s, uint32_t lane, uint32_t mask) {
     V3<R> d = sub(a.pos, b.pos);
     if (d.x == R(0) && d.y == R(0) && d.z == R(0)) d = {R(1), R(0), R(0)};
     s.len = 0;
     V3<R> pt, wt;
-    support_witness(a, b, d, hull, pt, wt);
+    support_witness<kG>(a, b, d, hull, pt, wt, lane, mask);
     s.push_front(pt, wt);
     d = neg(s.p[0]);
     for (int it = 0; it < 64; ++it) {
-        support_witness(a, b, d, hull, pt, wt);
+        support_witness<kG>(a, b, d, hull, pt, wt, lane, mask);
         if (dot(pt, d) < R(0)) return false;
         s.push_front(pt, wt);
         if (contains_origin(s, d)) return true;

@@ -553,6 +553,7 @@ static __global__ void k_roll_counters(Counters* c, uint32_t* zero0, uint32_t* z
     c->container_rows = 0;
     c->gjk_work = 0;
     c->epa_work = 0;
+    c->epa_next = 0;
     c->colors = 0;
     c->traverse_pairs = 0;
 }
