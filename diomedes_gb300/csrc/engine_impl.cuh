@@ -1733,7 +1733,8 @@ class Engine final : public EngineBase {
     int run_narrow(uint32_t np, const uint32_t* np_dev) {
         uint32_t per = cfg_.contacts_per_pair;
         w_.per_pair = per;
-        int g = np_dev ? sms_ * 8 : grid_for(np, 128);
+        int g = np_dev ? sms_ * 8
+                       : std::min(grid_for((uint64_t)np * kManifoldLanes, 128), std::max(sms_ * 8, grid_for(np, 128)));
         DIO_CK(launch_k(pdl(), k_narrow_main<P, R>, g, 128, 0, stream_, w_, np_dev, np));
         DIO_CK(launch_k(pdl(), k_gjk<P, R>, sms_ * 4, 128, 0, stream_, w_));
         DIO_CK(launch_k(pdl(), k_epa<P, R>, sms_ * 4, 32 * epa_warps<R>(), 0, stream_, w_));

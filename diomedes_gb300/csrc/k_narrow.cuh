@@ -432,6 +432,136 @@ __device__ bool collide_manifold(const NB<R>& a, const NB<R>& b, uint32_t max_co
     return true;
 }
 
+// collide_manifold by an aligned group of eight lanes (mask: theirs, `lane` this
+// one's place in it): an axis or two, then a vertex of the clipped polygon, a
+// lane.  Same tests on the same values, so the same result: the least overlap
+// with the lowest axis on a tie, vertices and contacts at their place in the
+// serial order.  The lane with `emit` has contact `at` of `count`.  poly: two
+// buffers of eight vertices in shared memory.
+constexpr uint32_t kManifoldLanes = 8;
+template <class R>
+struct GroupContact {
+    V3<R> normal, pa, pb;
+    R depth;
+    uint32_t count, at;
+    bool emit;
+};
+template <class R>
+__device__ __forceinline__ V3<R> pick(const V3<R> ax[3], uint32_t i) {
+    return i == 0 ? ax[0] : (i == 1 ? ax[1] : ax[2]);
+}
+template <class R>
+__device__ __forceinline__ V3<R> shfl3(uint32_t mask, V3<R> v, uint32_t src) {
+    return {__shfl_sync(mask, v.x, (int)src), __shfl_sync(mask, v.y, (int)src), __shfl_sync(mask, v.z, (int)src)};
+}
+template <class R>
+__device__ __forceinline__ void manifold_group(const NB<R>& a, const NB<R>& b, uint32_t max_contacts, uint32_t lane,
+                                               uint32_t mask, V3<R> (*poly)[kManifoldLanes], GroupContact<R>& out) {
+    constexpr uint32_t kNone = 0xFFFFFFFFu;
+    const uint32_t base = (threadIdx.x & 31u) - lane, below = (1u << lane) - 1u;
+    out.count = 0;
+    out.emit = false;
+    const bool per_axis = !(a.shape.tag == DIO_SHAPE_CUBE && b.shape.tag == DIO_SHAPE_CUBE);
+    V3<R> aax[3], bax[3];
+    axes_of(a.rot, aax);
+    axes_of(b.rot, bax);
+    const V3<R> ha = box_half(a.shape), hb = box_half(b.shape);
+    const V3<R> delta = sub(b.pos, a.pos);
+    R best_ov = 3.402823466e+38f;
+    if (sizeof(R) == 8) best_ov = R(1.7976931348623157e308);
+    V3<R> best_n{R(1), R(0), R(0)};
+    uint32_t best_kind = 0, best_t = kNone;
+    bool apart = false;
+#pragma unroll 1
+    for (uint32_t t = lane; t < 15u; t += kManifoldLanes) {
+        const uint32_t e = t - 6u;
+        const V3<R> raw = t < 3u ? pick(aax, t) : (t < 6u ? pick(bax, t - 3u) : cross(pick(aax, e / 3u), pick(bax, e % 3u)));
+        apart = apart || !test_axis(raw, 0u, t, ha, aax, hb, bax, delta, per_axis, best_ov, best_n, best_kind, best_t);
+    }
+    if (__any_sync(mask, apart)) return;
+    const uint32_t t = lanes_best<false, (int)kManifoldLanes>(best_t != kNone, best_ov, best_t, mask);
+    const uint32_t owner = base + (t == kNone ? 0u : t & (kManifoldLanes - 1u));  // no axis: the initial values
+    const V3<R> normal = shfl3(mask, best_n, owner);
+    const R depth = __shfl_sync(mask, best_ov, (int)owner);
+    out.normal = normal;
+    out.depth = depth;
+    auto centered = [&] {
+        out.pa = add(a.pos, scale(normal, box_radius(ha, aax, normal, per_axis)));
+        out.pb = sub(b.pos, scale(normal, box_radius(hb, bax, normal, per_axis)));
+        out.count = 1;
+        out.at = 0;
+        out.emit = lane == 0;
+    };
+    if (t != kNone && t >= 6u) {
+        centered();
+        return;
+    }
+    const bool ref_a = t == kNone || t < 3u;
+    const uint32_t best_idx = t == kNone ? 0u : (ref_a ? t : t - 3u);
+    const V3<R> rn = ref_a ? normal : neg(normal);
+    V3<R> rax[3], iax[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        rax[k] = ref_a ? aax[k] : bax[k];
+        iax[k] = ref_a ? bax[k] : aax[k];
+    }
+    uint32_t inc_axis = 0;  // incident_axis, cuboid.rs:198-214
+    R bdot = dabs(dot(iax[0], rn));
+#pragma unroll
+    for (uint32_t i = 1; i < 3; ++i) {
+        const R d = dabs(dot(iax[i], rn));
+        if (d > bdot) {
+            bdot = d;
+            inc_axis = i;
+        }
+    }
+    V3<R> center, u, v, c2, u2, v2, verts[4];
+    R eu, ev, eu2, ev2;
+    face_frame(ref_a ? a.pos : b.pos, rax, ref_a ? ha : hb, best_idx, rn, (V3<R>*)nullptr, center, u, v, eu, ev);
+    face_frame(ref_a ? b.pos : a.pos, iax, ref_a ? hb : ha, inc_axis, neg(rn), verts, c2, u2, v2, eu2, ev2);
+    uint32_t n = 4;
+    V3<R> cur = lane == 0 ? verts[0] : (lane == 1 ? verts[1] : (lane == 2 ? verts[2] : verts[3]));
+#pragma unroll 1
+    for (uint32_t plane = 0; plane < 4u && n; ++plane) {
+        const V3<R> axis = plane < 2u ? u : v;
+        const V3<R> pn = (plane & 1u) ? neg(axis) : axis;
+        const R offset = dot(pn, center) + (plane < 2u ? eu : ev);
+        const uint32_t from = base + (lane == 0 ? n - 1u : lane - 1u);
+        const R cur_d = dot(pn, cur) - offset;
+        const V3<R> prev = shfl3(mask, cur, from);
+        const R prev_d = __shfl_sync(mask, cur_d, (int)from);
+        const bool live = lane < n, pin = prev_d <= R(1.0e-5), cin = cur_d <= R(1.0e-5);
+        const R den = prev_d - cur_d;
+        const bool cross_ = live && pin != cin && dabs(den) > R(1.0e-8), keep = live && cin;
+        const uint32_t bc = __ballot_sync(mask, cross_) >> base, bk = __ballot_sync(mask, keep) >> base;
+        const uint32_t at = (uint32_t)__popc(bc & below) + (uint32_t)__popc(bk & below);
+        V3<R>* dst = poly[plane & 1u];
+        if (cross_ && at < kManifoldLanes) {
+            R s = prev_d / den;
+            s = s < R(0) ? R(0) : (s > R(1) ? R(1) : s);
+            dst[at] = add(prev, scale(sub(cur, prev), s));
+        }
+        if (keep && at + (cross_ ? 1u : 0u) < kManifoldLanes) dst[at + (cross_ ? 1u : 0u)] = cur;
+        const uint32_t group = (1u << kManifoldLanes) - 1u;
+        n = min((uint32_t)__popc(bc & group) + (uint32_t)__popc(bk & group), kManifoldLanes);
+        __syncwarp(mask);
+        if (lane < n) cur = dst[lane];
+    }
+    const R pd = dot(rn, center) - dot(rn, cur);
+    const uint32_t on = __ballot_sync(mask, lane < n && !(pd < R(-1.0e-5))) >> base;
+    const uint32_t all = (uint32_t)__popc(on & ((1u << kManifoldLanes) - 1u));
+    if (all == 0) {
+        centered();
+        return;
+    }
+    out.count = min(all, max_contacts);
+    out.at = (uint32_t)__popc(on & below);
+    out.emit = ((on >> lane) & 1u) && out.at < max_contacts;
+    const V3<R> rp = add(cur, scale(rn, pd > R(0) ? pd : R(0)));
+    out.pa = ref_a ? rp : cur;
+    out.pb = ref_a ? cur : rp;
+}
+
 // ---------------------------------------------------------------- GJK
 template <class R>
 struct Simplex {
