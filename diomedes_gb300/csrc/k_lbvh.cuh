@@ -895,7 +895,7 @@ __global__ void __launch_bounds__(kSceneTreeThreads)
     uint32_t* lroot = vis + cb;
     // write pass: per-body prefix in lpar, fill in npar (both unused by its
     // walks), the long list in lroot once the trees are walked
-    __shared__ uint32_t s_red[128];
+    __shared__ __align__(16) uint32_t s_red[128];  // also 64-bit sums
     __shared__ uint32_t s_nlong;
     if (WRITE) {
         const ChunkPairs src(t, cidx, lo, nb);
