@@ -275,12 +275,21 @@ int dio_world_set_state(DioCtx* ctx, const DioGpuBody* bodies, const DioBodyStat
 int dio_world_download(DioCtx* ctx, DioGpuBody* bodies, DioBodyState* state) {
     return with_world(ctx, false, [&](dio::EngineBase* e) { return e->download(bodies, state); });
 }
+// worlds that step together lay their launches out for a part of the GPU each
+static void share_gpu(DioCtx* const* ctxs, uint32_t count) {
+    for (uint32_t g = 0; g < count; ++g)
+        with_world(ctxs[g], false, [&](dio::EngineBase* e) {
+            e->share_gpu(count);
+            return DIO_OK;
+        });
+}
 int dio_worlds_step_host(DioCtx* const* ctxs, uint32_t count, DioGpuBody* const* bodies,
                          DioBodyState* const* states, const DioAvbdOptions* options, uint32_t steps) {
     if (!count) return DIO_OK;
     if (!ctxs || !bodies || !states || !options) return DIO_ERR_INVALID;
     for (uint32_t g = 0; g < count; ++g)
         if (!ctxs[g] || !bodies[g] || !states[g]) return DIO_ERR_INVALID;
+    share_gpu(ctxs, count);
     int rc = DIO_OK;
     // every world's state copy is queued (behind that world's previous
     // read-back) before the host waits on any of them; world g is stepped as
@@ -325,6 +334,7 @@ int dio_worlds_step_motion_host(DioCtx* const* ctxs, uint32_t count, DioBodyMoti
     if (!ctxs || !motions || !options) return DIO_ERR_INVALID;
     for (uint32_t g = 0; g < count; ++g)
         if (!ctxs[g] || !motions[g]) return DIO_ERR_INVALID;
+    share_gpu(ctxs, count);
     int rc = DIO_OK;
     // each world's chain (upload, step, read-back) is stream-ordered; the
     // worlds' chains are queued in turn, so one world's copies run beside
@@ -389,7 +399,7 @@ std::string tune_key(DioCtx* ctx, dio::EngineBase* e) {
 }
 
 // cache lines: key, primal variant, LBVH rebuild period, solve launch,
-// chunk-solve CTA size, ms
+// chunk-solve CTA shape, ms
 bool cache_lookup(const char* path, const std::string& key, uint32_t* variant, uint32_t* period, uint32_t* solve,
                   uint32_t* block) {
     if (!path) return false;

@@ -700,6 +700,8 @@ class Engine final : public EngineBase {
         solve_chunks_host_.clear();
         shape_mode_ = cfg_.solver_mode;
         shape_block_ = cfg_.block_size;
+        shape_sharers_ = sharers_;
+        const int sms = sms_share();
         solve_estimate_ = 0.0;
         if (scenes_host_.empty() || largest == 0 || largest > kSolveChunkCap) return 0;
         const bool colored = cfg_.solver_mode == DIO_SOLVER_COLORED;
@@ -720,9 +722,9 @@ class Engine final : public EngineBase {
                 while (sh.blk && (most >> sh.blk) < (1u << cl)) --sh.blk;
                 const uint32_t slots = sh.slots(most);
                 if (slots > solve_cta_cap<P, true>() || (cl && most < (4u << cl))) continue;
-                const int held = std::max(1, clusters_held(sh, slots, colored));
+                const int held = std::max(1, clusters_held(sh, slots, colored) / (int)sharers_);
                 const uint64_t waves = (chunks.size() + held - 1) / held;
-                const double over = double(chunks.size() << cl) / sms_ - 1.0;  // CTAs beyond one an SM
+                const double over = double(chunks.size() << cl) / sms - 1.0;  // CTAs beyond one an SM
                 const double share = 1.0 + 0.25 * std::min(1.0, std::max(0.0, over));
                 const uint32_t rounds = (slots + 255u) / 256u;
                 consider(true, sh,
@@ -732,9 +734,9 @@ class Engine final : public EngineBase {
         if (largest <= solve_cta_cap<P, false>())
             for (uint32_t target : {512u, 768u, 1024u}) {
                 pack_solve(std::min(target, solve_cta_cap<P, false>()), chunks);
-                if (chunks.size() <= (size_t)sms_ && !solve_chunks_host_.empty()) continue;
+                if (chunks.size() <= (size_t)sms && !solve_chunks_host_.empty()) continue;
                 // longest first over the SMs
-                std::vector<double> sm(std::min<size_t>((size_t)sms_, chunks.size()), 0.0);
+                std::vector<double> sm(std::min<size_t>((size_t)sms, chunks.size()), 0.0);
                 auto later = [](double x, double y) { return x > y; };
                 for (const uint2& c : chunks) {
                     const uint32_t bodies = scenes_host_[c.y - 1].body_hi - scenes_host_[c.x].body_lo;
@@ -742,7 +744,7 @@ class Engine final : public EngineBase {
                     sm.back() += 18.0 + 0.092 * bodies;
                     std::push_heap(sm.begin(), sm.end(), later);
                 }
-                const double us = *std::max_element(sm.begin(), sm.end()) * (chunks.size() > (size_t)sms_ ? 1.35 : 1.0);
+                const double us = *std::max_element(sm.begin(), sm.end()) * (chunks.size() > (size_t)sms ? 1.35 : 1.0);
                 consider(false, SolveShape{0, 5}, us * wide * (colored ? 1.6 : 1.0));
             }
         solve_estimate_ = best;
@@ -751,6 +753,16 @@ class Engine final : public EngineBase {
         for (const uint2& c : solve_chunks_host_)
             most = std::max(most, scenes_host_[c.y - 1].body_hi - scenes_host_[c.x].body_lo);
         return most;
+    }
+    // The SMs that this world counts on: worlds stepped together on their
+    // streams take a part each.  Eight 128-scene worlds, frames with motion
+    // records: 6.7e8 body-steps/s so, 5.6e8 with the tree count laid out for a
+    // whole GPU by each, 4.4e8 with the solve too.
+    int sms_share() const { return std::max(1, sms_ / (int)sharers_); }
+    void share_gpu(uint32_t worlds) override {
+        if (sharers_ == worlds || !world_ready_) return;
+        sharers_ = worlds;
+        drop_graphs();  // the next step packs its solve again
     }
     // clusters of the spread solve that the GPU holds at once
     int clusters_held(const SolveShape& sh, uint32_t slots, bool colored) const {
@@ -787,7 +799,9 @@ class Engine final : public EngineBase {
     // the solve's shape follows the solver mode and the CTA shape asked for;
     // both may change after the upload
     int reshape_solve() {
-        if (!chunk_world_ || (shape_mode_ == cfg_.solver_mode && shape_block_ == cfg_.block_size)) return DIO_OK;
+        if (!chunk_world_ || (shape_mode_ == cfg_.solver_mode && shape_block_ == cfg_.block_size &&
+                              shape_sharers_ == sharers_))
+            return DIO_OK;
         drop_graphs();
         DIO_TRY(note_scene_sizes());
         return order_dyn_list();
@@ -1060,6 +1074,7 @@ class Engine final : public EngineBase {
         drop_graphs();
         lbvh_valid_ = false;
         w_.n_joints = 0;  // the world's joints are uploaded below
+        sharers_ = 1;
         DIO_TRY(upload_bodies(d->bodies, n, d->n_hull_vertices));
         if (d->positions_f64 || d->orientations_f64) {
             double* dp = reinterpret_cast<double*>(dstage_);
@@ -1503,8 +1518,8 @@ class Engine final : public EngineBase {
     bool use_chunk_solve() const {
         if (!chunk_world_ || cfg_.batched_solver != DIO_SOLVE_AUTO) return false;
         if (sizeof(P) == 4) return true;
-        return solve_estimate_ <= (cfg_.solver_mode == DIO_SOLVER_COLORED ? 500.0 + 2.3e-3 * solve_total_
-                                                                           : 285.0 + 1.5e-3 * solve_total_);
+        return solve_estimate_ <= sharers_ * (cfg_.solver_mode == DIO_SOLVER_COLORED ? 500.0 + 2.3e-3 * solve_total_
+                                                                                     : 285.0 + 1.5e-3 * solve_total_);
     }
     bool chunk_solve_possible() const override { return chunk_world_; }
     int solve_chunks(const SolveParams<R>& o) {
@@ -1666,7 +1681,7 @@ class Engine final : public EngineBase {
         ta.nchunks = nchunks;
         // several CTAs a chunk while they fit the SMs (each refits the whole
         // trees: more would only repeat that)
-        ta.parts = ta.fused ? std::max(1u, std::min({kTreeParts, (uint32_t)sms_ / nchunks, chunk_max_ / kPartLeaves})) : 1u;
+        ta.parts = ta.fused ? std::max(1u, std::min({kTreeParts, (uint32_t)sms_share() / nchunks, chunk_max_ / kPartLeaves})) : 1u;
         ta.pairs = w_.pairs;
         ta.ctr = ctr_;
         auto scene_tree = [&](bool write) -> cudaError_t {
@@ -2484,6 +2499,7 @@ class Engine final : public EngineBase {
     uint32_t api_bodies_ = 0, api_n_ = 0, api_m_ = 0, api_iters_ = 0, last_np_ = 0;
     uint64_t steps_ = 0;
     bool world_ready_ = false;
+    uint32_t sharers_ = 1, shape_sharers_ = 1;  // worlds stepped together, now and when the solve was packed
     struct Span {
         cudaEvent_t a, b;
         int kind;

@@ -62,8 +62,8 @@ __device__ __forceinline__ void sphere_or_queue(const DevWorld<P, R>& w, uint32_
 // are a serial chain of some 40,000 cycles in one thread, so eight lanes share
 // a pair (narrow phase of a 55-cube pyramid 22 us a step and now 14, of 1,024
 // scenes 19 and 15) up to kGroupedPairs.  They execute more instructions in all:
-// 28,000 pairs of stacked cubes, nearly all in contact, are a tie (34.5 and
-// 35.1), and with several times as many a thread a pair keeps the chip as busy.
+// 38,000 pairs of a mixed pile are a tie (183 and 182), and 90,000 of stacked
+// cubes, nearly all in contact, take 47 against 35 with a thread a pair.
 constexpr uint32_t kGroupedPairs = 65536;
 template <class P, class R>
 __device__ __forceinline__ void narrow_grouped(const DevWorld<P, R>& w, uint32_t np) {
@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(128) k_narrow_main(DevWorld<P, R> w, const uin
 // empty: kGjkLanes lanes share a pair's scans while the grid has that many
 // threads (cold, 648 pairs of a mixed pile 35 us with one lane, 22 with eight).
 // Beyond, a group's pairs queue behind one another, and one lane a pair is the
-// faster (16,000 pairs 36 and 37 us, 28,000 pairs 60 and 80).
+// faster (13,000 pairs 36 and 37 us, 32,000 pairs 60 and 80).
 constexpr int kGjkLanes = 8;
 template <int kG, class P, class R>
 __device__ __forceinline__ void gjk_pairs(const DevWorld<P, R>& w, uint32_t nw) {
@@ -211,7 +211,7 @@ constexpr uint32_t kEpaWaitPolls = 1u << 20;  // rounds of the bounded waits for
 // warp's shared memory with bulk TMA copies, so the support queries of the
 // expansion read shared memory.  A warp takes the next pair that is left: a
 // pair's expansion takes 4 to 64 iterations, and with a fixed share the longest
-// sum of a warp's pairs set the time (15,000 pairs of a mixed pile 134 us cold,
+// sum of a warp's pairs set the time (a 50,000-body mixed pile 134 us cold,
 // now 114).
 template <class P, class R>
 __global__ void __launch_bounds__(32 * epa_warps<R>(), 4) k_epa(DevWorld<P, R> w) {
