@@ -92,7 +92,8 @@ def parse():
     ap.add_argument("--no-per-phase", action="store_true")
     ap.add_argument("--no-tune", action="store_true", help="keep the default configuration (profiling runs)")
     ap.add_argument("--block-size", type=int, default=None, choices=[0, 640],
-                    help="threads per CTA of the scene-chunk solve (0: 512); default: the autotuner's choice")
+                    help="CTA shape of the scene-chunk solve (0: by the scenes' sizes; 640: a whole SM for each "
+                         "chunk); default: the autotuner's choice")
     ap.add_argument("--primal-variant", type=int, default=None,
                     help="primal kernel variant of the per-phase solve; default: the autotuner's choice")
     ap.add_argument("--colored", action="store_true",
