@@ -687,10 +687,13 @@ class Engine final : public EngineBase {
     // GPU holds; a packed CTA 18 plus 0.092 a body (coloured 1.6 times), the
     // SMs taking the next largest chunk as they fall free; packed only when
     // there are more chunks than SMs (contact-dense scenes are twice as slow
-    // packed: the 901-body pile 225 against 127).  33 scenes: 104
-    // spread over 8 CTAs, 148 over 4, 203 packed; 257: 244, 193, 209; 1024:
-    // 850, 585, 413.  Returns the largest chunk's bodies (0: some scene
-    // exceeds the cap).
+    // packed: the 901-body pile 225 against 127) or the schedule is coloured
+    // and the scenes are jointed and small (a barrier per colour costs a cluster
+    // most: passes of 5 and 13 scenes of at most 700 bodies 567 and 545 us
+    // spread, 485 and 498 packed; of 4 and 33 with 2,000 bodies 570 and 599, 627
+    // and 800).  33 scenes: 104 spread over 8 CTAs, 148 over 4, 203 packed; 257:
+    // 244, 193, 209; 1024: 850, 585, 413.  Returns the largest chunk's bodies
+    // (0: some scene exceeds the cap).
     uint32_t pack_solve_chunks() {
         uint32_t largest = 0, total = 0;
         for (const SceneDesc& sd : scenes_host_) {
@@ -734,7 +737,7 @@ class Engine final : public EngineBase {
         if (largest <= solve_cta_cap<P, false>())
             for (uint32_t target : {512u, 768u, 1024u}) {
                 pack_solve(std::min(target, solve_cta_cap<P, false>()), chunks);
-                if (chunks.size() <= (size_t)sms && !solve_chunks_host_.empty()) continue;
+                if (chunks.size() <= (size_t)sms && !(colored && jointed_ && largest <= 768u) && !solve_chunks_host_.empty()) continue;
                 // longest first over the SMs
                 std::vector<double> sm(std::min<size_t>((size_t)sms, chunks.size()), 0.0);
                 auto later = [](double x, double y) { return x > y; };
@@ -1075,6 +1078,7 @@ class Engine final : public EngineBase {
         lbvh_valid_ = false;
         w_.n_joints = 0;  // the world's joints are uploaded below
         sharers_ = 1;
+        jointed_ = 2ull * d->n_constraints >= n;
         DIO_TRY(upload_bodies(d->bodies, n, d->n_hull_vertices));
         if (d->positions_f64 || d->orientations_f64) {
             double* dp = reinterpret_cast<double*>(dstage_);
@@ -2499,6 +2503,7 @@ class Engine final : public EngineBase {
     uint32_t api_bodies_ = 0, api_n_ = 0, api_m_ = 0, api_iters_ = 0, last_np_ = 0;
     uint64_t steps_ = 0;
     bool world_ready_ = false;
+    bool jointed_ = false;  // the uploaded world has a joint for every other body
     uint32_t sharers_ = 1, shape_sharers_ = 1;  // worlds stepped together, now and when the solve was packed
     struct Span {
         cudaEvent_t a, b;
