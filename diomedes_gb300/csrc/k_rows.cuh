@@ -582,13 +582,12 @@ __global__ void k_csr_scatter_dyn(DevWorld<P, R> w, uint32_t* remaining, uint32_
     }
 }
 
-constexpr uint32_t kLongRows = 4096;
 // A thread per end of a row counts the smaller rows of its body's segment: the
 // loads do not wait for one another, and the threads of a pair's rows read the
 // same ones.  (A thread per body with an insertion sort in local memory, longer
 // segments by a CTA each: 15 us cold a step for 8,192 stacked cubes, 13.5 for a
-// 55-cube pyramid of 8-contact pairs; now 6 and 5.)  A segment beyond kLongRows
-// rows is reported and left as it is.
+// 55-cube pyramid of 8-contact pairs; now 6 and 5.)  Counting needs no buffer,
+// so a segment may have any length: every entry that the solve walks is written.
 template <class P, class R>
 __global__ void k_csr_finish_dyn(DevWorld<P, R> w, const uint32_t* loose) {
     pdl_enter();
@@ -599,11 +598,6 @@ __global__ void k_csr_finish_dyn(DevWorld<P, R> w, const uint32_t* loose) {
         const uint32_t i = (t & 1u) ? ab.y : ab.x;
         if (i == kContainer || w.inv[i].w == R(0)) continue;
         const uint32_t j0 = w.row_off[i], j1 = min(w.row_off[i + 1], w.max_incid);
-        if (j0 >= j1) continue;
-        if (j1 - j0 > kLongRows) {
-            atomicOr(&w.ctr->error_flags, kErrIndexOverflow);
-            continue;
-        }
         uint32_t j = j0;
 #pragma unroll 8
         for (uint32_t q = j0; q < j1; ++q) j += loose[q] < r ? 1u : 0u;
