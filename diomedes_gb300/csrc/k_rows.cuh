@@ -375,7 +375,8 @@ __global__ void k_rows(DevWorld<P, R> w, const Slot<R>* slots, uint32_t per, con
     const uint32_t live = ng_dev ? min(*ng_dev, ng) : ng;
     const uint32_t pair_rows = off[ng], cont_rows = off2[n];
     if (blockIdx.x == 0 && threadIdx.x == 0) {
-        w.ctr->pair_rows = pair_rows;
+        // rows that are kept: the next step's warm start searches that many
+        w.ctr->pair_rows = min(pair_rows, w.max_rows);
         w.ctr->container_rows = cont_rows;
         const uint64_t t = (uint64_t)pair_rows + cont_rows;
         w.ctr->rows = t > w.max_rows ? w.max_rows : (uint32_t)t;
