@@ -583,7 +583,9 @@ struct WorldBodies {
         BodyTask<P, R> b;
         b.i = list[t];
         b.j0 = w.row_off[b.i];
-        b.n = w.row_off[b.i + 1] - b.j0;
+        // a caller's offsets may step back: such a body has no rows
+        const uint32_t j1 = w.row_off[b.i + 1];
+        b.n = j1 > b.j0 ? j1 - b.j0 : 0u;
         b.mdt2 = w.mdt2[b.i];
         b.ipos = w.inert_pos[b.i];
         b.irot = w.inert_rot[b.i];
