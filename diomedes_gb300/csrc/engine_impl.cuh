@@ -1077,6 +1077,10 @@ class Engine final : public EngineBase {
         drop_graphs();
         lbvh_valid_ = false;
         w_.n_joints = 0;  // the world's joints are uploaded below
+        // the scene table in force is the former world's: its bodies' scenes say
+        // nothing about these (the list is ordered once the joints are here)
+        solve_chunks_host_.clear();
+        chunked_scenes_ = chunk_world_ = false;
         sharers_ = 1;
         jointed_ = 2ull * d->n_constraints >= n;
         DIO_TRY(upload_bodies(d->bodies, n, d->n_hull_vertices));
@@ -1090,7 +1094,7 @@ class Engine final : public EngineBase {
             k_unpack_pose_f64<P, R><<<grid_for(n, 256), 256, 0, stream_>>>(
                 w_, d->positions_f64 ? dp : nullptr, d->orientations_f64 ? dq : nullptr, n);
         }
-        DIO_TRY(upload_state(d->state, n));
+        DIO_TRY(upload_state(d->state, n, false));
         // scenes
         std::vector<SceneDesc> sc(ns);
         std::vector<A4<P>> org(ns);
