@@ -204,8 +204,12 @@ __device__ __forceinline__ uint32_t container_rows(const DevWorld<P, R>& w, uint
     const V3<R> pos = cast3<R>(sub(xyz(w.pos[0][i]), org));  // as load_nb forms it
     const bool boxy = tag == DIO_SHAPE_CUBE || tag == DIO_SHAPE_BOX;
     R rbound = R(-1);
-    if (tag == DIO_SHAPE_HULL && w.hull_bound) {
-        rbound = w.hull_bound[i];  // over its vertices, kept from the upload
+    const bool hull = tag == DIO_SHAPE_HULL && w.hull_bound;
+    if (hull) {
+        // over its vertices, kept from the upload; an orientation that is not
+        // of unit length scales them by its square
+        const Q4<R> q = narrowq<R>(quat(w.rot[0][i]));
+        rbound = w.hull_bound[i] * fmax_(R(1), q.x * q.x + q.y * q.y + q.z * q.z + q.w * q.w);
     } else if (boxy) {
         rbound = dabs(R(c0.x)) + dabs(R(c0.y)) + dabs(R(c0.z));
     } else if (tag == DIO_SHAPE_SPHERE) {
@@ -223,8 +227,16 @@ __device__ __forceinline__ uint32_t container_rows(const DevWorld<P, R>& w, uint
         for (int k = 0; k < 6; ++k) {
             const A4<R> wall = walls[k];
             const R d = dot(pos, xyz(wall));
-            const R slack = R(1e-4) * (R(1) + dabs(wall.w) + dabs(d));
-            if (!(d + rbound + travel + slack < wall.w)) reach |= 1u << k;
+            R far = rbound + travel, mag = dabs(d);
+            if (hull) {
+                // a vertex may lie on its bound: the wall's normal is taken with
+                // its length (a container's rotation need not be a unit one), and
+                // the rounding of d with its terms
+                far = far * (R(1.0001) * fmax_(R(1), dot(xyz(wall), xyz(wall))));
+                mag = dabs(pos.x * wall.x) + dabs(pos.y * wall.y) + dabs(pos.z * wall.z);
+            }
+            const R slack = R(1e-4) * (R(1) + dabs(wall.w) + mag);
+            if (!(d + far + slack < wall.w)) reach |= 1u << k;
         }
     }
     if (!reach) return 0;
