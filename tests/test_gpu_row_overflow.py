@@ -22,7 +22,7 @@ def test_steps_beyond_the_row_capacity(cap, launch, mode):
         with pytest.raises(abi.DioError) as e:
             w.step(sc.options, 60)
         assert e.value.status == abi.DIO_ERR_CAPACITY
-        assert len(w.contacts()) == cap
+        assert len(w.contacts()) <= cap  # (the last step need not be among those that overflowed)
         if cap < 4:
             return
         ow = O.World(small, solver_mode=mode)
