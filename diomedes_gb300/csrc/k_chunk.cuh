@@ -270,7 +270,9 @@ struct ChunkFetch {
         recover_body_f(w, i, *this, o);
         w.pos[0][i] = c.pos[fin + slot(i)];
         if constexpr (kSplit) {
-            if (o.iterations == 0) w.rot[0][i] = w.init_rot[i];  // the pose before the warm start
+            // without an iteration the two buffers' schedule leaves the pose before
+            // the warm start, the in-place one the warm start itself
+            if (c.step && o.iterations == 0) w.rot[0][i] = w.init_rot[i];
         } else {
             w.rot[0][i] = c.rot[fin + slot(i)];
         }
