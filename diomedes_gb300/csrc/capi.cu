@@ -261,10 +261,16 @@ int dio_world_upload(DioCtx* ctx, const DioWorldDesc* desc) {
     return with_world(ctx, true, [&](dio::EngineBase* e) { return e->world_upload(desc); });
 }
 int dio_step(DioCtx* ctx, const DioAvbdOptions* options, uint32_t steps) {
-    return with_world(ctx, false, [&](dio::EngineBase* e) { return e->step(options, steps); });
+    return with_world(ctx, false, [&](dio::EngineBase* e) {
+        e->share_gpu(1);
+        return e->step(options, steps);
+    });
 }
 int dio_step_async(DioCtx* ctx, const DioAvbdOptions* options, uint32_t steps) {
-    return with_world(ctx, false, [&](dio::EngineBase* e) { return e->step_async(options, steps); });
+    return with_world(ctx, false, [&](dio::EngineBase* e) {
+        e->share_gpu(1);
+        return e->step_async(options, steps);
+    });
 }
 int dio_world_download_async(DioCtx* ctx, DioGpuBody* bodies, DioBodyState* state) {
     return with_world(ctx, false, [&](dio::EngineBase* e) { return e->download_async(bodies, state); });
@@ -275,13 +281,13 @@ int dio_world_set_state(DioCtx* ctx, const DioGpuBody* bodies, const DioBodyStat
 int dio_world_download(DioCtx* ctx, DioGpuBody* bodies, DioBodyState* state) {
     return with_world(ctx, false, [&](dio::EngineBase* e) { return e->download(bodies, state); });
 }
-// worlds that step together lay their launches out for a part of the GPU each
-static void share_gpu(DioCtx* const* ctxs, uint32_t count) {
-    for (uint32_t g = 0; g < count; ++g)
-        with_world(ctxs[g], false, [&](dio::EngineBase* e) {
-            e->share_gpu(count);
-            return DIO_OK;
-        });
+// one step of a world that is stepped with others: worlds that step together
+// lay their launches out for a part of the GPU each
+static int step_together(DioCtx* ctx, uint32_t count, const DioAvbdOptions* options) {
+    return with_world(ctx, false, [&](dio::EngineBase* e) {
+        e->share_gpu(count);
+        return e->step_async(options, 1);
+    });
 }
 int dio_worlds_step_host(DioCtx* const* ctxs, uint32_t count, DioGpuBody* const* bodies,
                          DioBodyState* const* states, const DioAvbdOptions* options, uint32_t steps) {
@@ -289,7 +295,6 @@ int dio_worlds_step_host(DioCtx* const* ctxs, uint32_t count, DioGpuBody* const*
     if (!ctxs || !bodies || !states || !options) return DIO_ERR_INVALID;
     for (uint32_t g = 0; g < count; ++g)
         if (!ctxs[g] || !bodies[g] || !states[g]) return DIO_ERR_INVALID;
-    share_gpu(ctxs, count);
     int rc = DIO_OK;
     // every world's state copy is queued (behind that world's previous
     // read-back) before the host waits on any of them; world g is stepped as
@@ -301,7 +306,7 @@ int dio_worlds_step_host(DioCtx* const* ctxs, uint32_t count, DioGpuBody* const*
                             [&](dio::EngineBase* e) { return e->set_state_begin(bodies[g], states[g]); });
         for (uint32_t g = 0; g < count && !rc; ++g) {
             rc = with_world(ctxs[g], false, [&](dio::EngineBase* e) { return e->set_state_end(); });
-            if (!rc) rc = dio_step_async(ctxs[g], options, 1);
+            if (!rc) rc = step_together(ctxs[g], count, options);
             if (!rc) rc = dio_world_download_async(ctxs[g], bodies[g], states[g]);
         }
     }
@@ -334,7 +339,6 @@ int dio_worlds_step_motion_host(DioCtx* const* ctxs, uint32_t count, DioBodyMoti
     if (!ctxs || !motions || !options) return DIO_ERR_INVALID;
     for (uint32_t g = 0; g < count; ++g)
         if (!ctxs[g] || !motions[g]) return DIO_ERR_INVALID;
-    share_gpu(ctxs, count);
     int rc = DIO_OK;
     // each world's chain (upload, step, read-back) is stream-ordered; the
     // worlds' chains are queued in turn, so one world's copies run beside
@@ -342,7 +346,7 @@ int dio_worlds_step_motion_host(DioCtx* const* ctxs, uint32_t count, DioBodyMoti
     for (uint32_t k = 0; k < steps && !rc; ++k)
         for (uint32_t g = 0; g < count && !rc; ++g) {
             rc = dio_world_set_motion(ctxs[g], motions[g]);
-            if (!rc) rc = dio_step_async(ctxs[g], options, 1);
+            if (!rc) rc = step_together(ctxs[g], count, options);
             if (!rc) rc = dio_world_download_motion_async(ctxs[g], motions[g]);
         }
     for (uint32_t g = 0; g < count; ++g) {
@@ -444,6 +448,7 @@ int dio_autotune(DioCtx* ctx, const DioAvbdOptions* options, uint32_t trial_step
     int rc = world_engine(ctx, false, &e);
     if (rc) return rc;
     if (trial_steps == 0) trial_steps = 5;
+    e->share_gpu(1);  // the trials step it alone
     const std::string key = tune_key(ctx, e);
     DioConfig cfg = ctx->cfg;
     uint32_t v = 0, p = 0, b = 0, t = 0;

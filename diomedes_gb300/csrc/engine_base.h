@@ -67,7 +67,7 @@ struct EngineBase {
     virtual void set_config(const DioConfig& c) = 0;
     // every scene of the uploaded world fits the scene-chunk solve
     virtual bool chunk_solve_possible() const = 0;
-    // how many worlds are stepped together from now on (until the next upload)
+    // how many worlds are stepped together from the next step on
     virtual void share_gpu(uint32_t worlds) = 0;
 
     std::string err;

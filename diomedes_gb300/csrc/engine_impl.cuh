@@ -557,15 +557,12 @@ class Engine final : public EngineBase {
         DIO_TRY(alloc(&joint_off_, (size_t)N + 1));
         DIO_TRY(alloc(&joint_idx_, 2ull * J));
         DIO_TRY(alloc(&jview_, 2ull * J));
-        DIO_TRY(alloc(&dyn_list_, N));
         DIO_TRY(alloc(&dyn_tmp_, N));
         DIO_TRY(alloc(&dyn_keep_, N));
         DIO_TRY(alloc(&list_rows_, N));
-        DIO_TRY(alloc(&list_joints_, N));
-        DIO_TRY(alloc(&list_joint_self_, (size_t)kListJoints * N));
-        DIO_TRY(alloc(&list_joint_other_, (size_t)kListJoints * N));
-        DIO_TRY(alloc(&list_joint_meta_, (size_t)kListJoints * N));
-        w_.solve = SolveList{list_rows_, list_joints_, list_joint_self_, list_joint_other_, list_joint_meta_, N};
+        DIO_TRY(alloc_layout(layouts_[0]));
+        take(layouts_[0]);
+        l_->sharers = 1;
         DIO_TRY(alloc(&color_hist_, kMaxColors + 2));
         const size_t CNT = std::max<size_t>(std::max<size_t>(N, (size_t)PP * per_cap_), 2ull * M) + 2;
         DIO_TRY(alloc(&counts_, CNT));
@@ -575,9 +572,6 @@ class Engine final : public EngineBase {
         DIO_TRY(alloc(&offsets2_, (size_t)N + 2));
         DIO_TRY(alloc(&scenes_, S));
         DIO_TRY(alloc(&chunks_, S));
-        DIO_TRY(alloc(&solve_chunks_, S));
-        DIO_TRY(alloc(&chunk_dyn_, (size_t)S << kMaxClusterShift));
-        DIO_TRY(alloc(&scene_chunk_, S));
         DIO_TRY(alloc(&chunk_tot_, (size_t)S * kTreeParts));
         // pair scratch of the shared-memory trees: scratch_k_ slots per body
         // (at most 16: the write pass stages a chunk's pairs in its boxes' space)
@@ -700,12 +694,10 @@ class Engine final : public EngineBase {
             largest = std::max(largest, sd.body_hi - sd.body_lo);
             total = std::max(total, sd.body_hi);
         }
-        solve_chunks_host_.clear();
-        shape_mode_ = cfg_.solver_mode;
-        shape_block_ = cfg_.block_size;
-        shape_sharers_ = sharers_;
+        Layout& l = *l_;
+        l.chunks.clear();
+        l.estimate = 0.0;
         const int sms = sms_share();
-        solve_estimate_ = 0.0;
         if (scenes_host_.empty() || largest == 0 || largest > kSolveChunkCap) return 0;
         const bool colored = cfg_.solver_mode == DIO_SOLVER_COLORED;
         const double wide = sizeof(P) == sizeof(R) ? (sizeof(P) == 4 ? 1.0 : 3.0) : 1.35;
@@ -714,9 +706,9 @@ class Engine final : public EngineBase {
         auto consider = [&](bool spread, SolveShape sh, double us) {
             if (us >= best) return;
             best = us;
-            spread_ = spread;
-            shape_ = sh;
-            solve_chunks_host_ = chunks;
+            l.spread = spread;
+            l.shape = sh;
+            l.chunks = chunks;
         };
         if (cfg_.block_size == 0 || largest > solve_cta_cap<P, false>()) {
             const uint32_t most = pack_solve(kSolveChunkCap, chunks);
@@ -725,7 +717,7 @@ class Engine final : public EngineBase {
                 while (sh.blk && (most >> sh.blk) < (1u << cl)) --sh.blk;
                 const uint32_t slots = sh.slots(most);
                 if (slots > solve_cta_cap<P, true>() || (cl && most < (4u << cl))) continue;
-                const int held = std::max(1, clusters_held(sh, slots, colored) / (int)sharers_);
+                const int held = std::max(1, clusters_held(sh, slots, colored) / (int)l.sharers);
                 const uint64_t waves = (chunks.size() + held - 1) / held;
                 const double over = double(chunks.size() << cl) / sms - 1.0;  // CTAs beyond one an SM
                 const double share = 1.0 + 0.25 * std::min(1.0, std::max(0.0, over));
@@ -737,7 +729,7 @@ class Engine final : public EngineBase {
         if (largest <= solve_cta_cap<P, false>())
             for (uint32_t target : {512u, 768u, 1024u}) {
                 pack_solve(std::min(target, solve_cta_cap<P, false>()), chunks);
-                if (chunks.size() <= (size_t)sms && !(colored && jointed_ && largest <= 768u) && !solve_chunks_host_.empty()) continue;
+                if (chunks.size() <= (size_t)sms && !(colored && jointed_ && largest <= 768u) && !l.chunks.empty()) continue;
                 // longest first over the SMs
                 std::vector<double> sm(std::min<size_t>((size_t)sms, chunks.size()), 0.0);
                 auto later = [](double x, double y) { return x > y; };
@@ -750,10 +742,10 @@ class Engine final : public EngineBase {
                 const double us = *std::max_element(sm.begin(), sm.end()) * (chunks.size() > (size_t)sms ? 1.35 : 1.0);
                 consider(false, SolveShape{0, 5}, us * wide * (colored ? 1.6 : 1.0));
             }
-        solve_estimate_ = best;
+        l.estimate = best;
         solve_total_ = total;
         uint32_t most = 0;
-        for (const uint2& c : solve_chunks_host_)
+        for (const uint2& c : l.chunks)
             most = std::max(most, scenes_host_[c.y - 1].body_hi - scenes_host_[c.x].body_lo);
         return most;
     }
@@ -761,11 +753,12 @@ class Engine final : public EngineBase {
     // streams take a part each.  Eight 128-scene worlds, frames with motion
     // records: 6.7e8 body-steps/s so, 5.6e8 with the tree count laid out for a
     // whole GPU by each, 4.4e8 with the solve too.
-    int sms_share() const { return std::max(1, sms_ / (int)sharers_); }
+    int sms_share() const { return std::max(1, sms_ / (int)l_->sharers); }
+    // counted in powers of two, so that a group that shrinks or grows by a few
+    // worlds keeps its layout
     void share_gpu(uint32_t worlds) override {
-        if (sharers_ == worlds || !world_ready_) return;
-        sharers_ = worlds;
-        drop_graphs();  // the next step packs its solve again
+        sharers_ = 1;
+        while (sharers_ < worlds && sharers_ < 64u) sharers_ *= 2;
     }
     // clusters of the spread solve that the GPU holds at once
     int clusters_held(const SolveShape& sh, uint32_t slots, bool colored) const {
@@ -799,15 +792,90 @@ class Engine final : public EngineBase {
                          [&](const uint2& a, const uint2& b) { return bodies_of(a) > bodies_of(b); });
         return bodies_of(out.front());
     }
-    // the solve's shape follows the solver mode and the CTA shape asked for;
-    // both may change after the upload
-    int reshape_solve() {
-        if (!chunk_world_ || (shape_mode_ == cfg_.solver_mode && shape_block_ == cfg_.block_size &&
-                              shape_sharers_ == sharers_))
-            return DIO_OK;
-        drop_graphs();
-        DIO_TRY(note_scene_sizes());
-        return order_dyn_list();
+    struct GraphSlot {
+        cudaGraph_t graph = nullptr;
+        cudaGraphExec_t exec = nullptr;
+        DioAvbdOptions opt{};
+        std::vector<std::pair<cudaGraphNode_t, cudaGraphNode_t>> span_nodes;
+        std::vector<int> span_kinds;
+        uint64_t launches = 0;
+    };
+    // How a step is laid out for a number of worlds stepped together, with the
+    // dynamic bodies in that order and the graphs captured with it.
+    struct Layout {
+        uint32_t sharers = 0;          // worlds stepped together (0: not in use)
+        uint32_t mode = 0, block = 0;  // solver_mode, block_size it was chosen for
+        bool ordered = false;          // dyn_list holds the world's dynamic bodies, in order
+        uint64_t used = 0;             // when it was last taken
+        std::vector<uint2> chunks;     // chunks of the scene-chunk solve
+        uint32_t chunk_max = 0;        // bodies of the largest
+        SolveShape shape{0, 5};        // how a chunk is dealt to its cluster's CTAs
+        bool spread = false;           // clusters of small CTAs, or a CTA a chunk
+        double estimate = 0.0;         // of that shape, us
+        uint2* dev_chunks = nullptr;
+        uint2* dyn_runs = nullptr;        // each solve CTA's run of the dynamic-body list
+        uint32_t* scene_chunk = nullptr;  // solve chunk of every scene
+        uint32_t* dyn_list = nullptr;
+        SolveList list{};
+        GraphSlot graphs[4];  // (row-buffer parity, LBVH rebuild or refit)
+    };
+    int alloc_layout(Layout& l) {
+        if (l.dyn_list) return DIO_OK;
+        const size_t N = std::max(1u, cap_.max_bodies), S = std::max(1u, cap_.max_scenes);
+        uint32_t* joints = nullptr;
+        float4 *self = nullptr, *other = nullptr;
+        uint2* meta = nullptr;
+        DIO_TRY(alloc(&l.dev_chunks, S));
+        DIO_TRY(alloc(&l.dyn_runs, S << kMaxClusterShift));
+        DIO_TRY(alloc(&l.scene_chunk, S));
+        DIO_TRY(alloc(&joints, N));
+        DIO_TRY(alloc(&self, kListJoints * N));
+        DIO_TRY(alloc(&other, kListJoints * N));
+        DIO_TRY(alloc(&meta, kListJoints * N));
+        l.list = SolveList{list_rows_, joints, self, other, meta, (uint32_t)N};
+        return alloc(&l.dyn_list, N);
+    }
+    void take(Layout& l) {
+        l_ = &l;
+        l.used = ++layout_clock_;
+        w_.dyn_list = l.dyn_list;
+        w_.solve = l.list;
+    }
+    // The layout for the solver mode, the CTA shape and the number of worlds
+    // stepped together, all of which may change after the upload.  The last
+    // few are kept with their graphs: a caller that steps a world alone and
+    // with others in turn, or in groups of two sizes, packs and captures once
+    // each (worlds of 128 scenes, frames with motion records, us a round: eight
+    // then five 2,500 packed anew and 1,700 so, eight then one step of one alone
+    // 1,310 and 1,260, groups of 8, 7, .. 1 8,000 and 5,100).
+    int choose_layout() {
+        // scenes beyond the shared-memory trees are laid out for the whole GPU
+        const uint32_t sharers = chunk_world_ || !chunks_host_.empty() ? sharers_ : 1u;
+        auto current = [&](const Layout& l) {
+            return l.sharers && l.mode == cfg_.solver_mode && l.block == cfg_.block_size;
+        };
+        Layout* to = nullptr;
+        for (Layout& l : layouts_)
+            if (current(l) && l.sharers == sharers) to = &l;
+        if (to == l_ && to->ordered) return DIO_OK;
+        const bool pack = !to;
+        if (pack) {  // in place of one that no longer holds, else of the one not taken for longest
+            auto age = [&](const Layout& l) { return current(l) ? l.used : 0u; };
+            to = &layouts_[0];
+            for (Layout& l : layouts_)
+                if (age(l) < age(*to)) to = &l;
+            DIO_TRY(alloc_layout(*to));
+            drop_graphs(*to);
+            to->sharers = sharers;
+            to->mode = cfg_.solver_mode;
+            to->block = cfg_.block_size;
+            to->ordered = false;
+        }
+        if (to != l_ && !to->ordered && w_.n_dyn)
+            DIO_CK(cudaMemcpyAsync(to->dyn_list, l_->dyn_list, (size_t)w_.n_dyn * 4, cudaMemcpyDeviceToDevice, stream_));
+        take(*to);
+        if (pack && chunked_scenes_) DIO_TRY(pack_layout());
+        return to->ordered ? DIO_OK : order_dyn_list();
     }
     // largest scene; the chunks of the broad phase's shared-memory trees
     // (scene_tree_cap<R> bodies) and of the scene-chunk solve
@@ -816,22 +884,27 @@ class Engine final : public EngineBase {
         scene_max_ = 0;
         for (const SceneDesc& sd : scenes_host_) scene_max_ = std::max(scene_max_, sd.body_hi - sd.body_lo);
         chunk_max_ = pack_chunks(scene_tree_cap<R>(), chunks_host_);
-        solve_chunk_max_ = pack_solve_chunks();
-        // solve chunk of every scene (when every scene has one)
-        chunked_scenes_ = !solve_chunks_host_.empty() && scene_max_ <= kSolveChunkCap;
-        if (chunked_scenes_) {
-            std::vector<uint32_t> sch(scenes_host_.size(), 0u);
-            for (uint32_t c = 0; c < (uint32_t)solve_chunks_host_.size(); ++c)
-                for (uint32_t sc = solve_chunks_host_[c].x; sc < solve_chunks_host_[c].y; ++sc) sch[sc] = c;
-            DIO_CK(cudaMemcpyAsync(scene_chunk_, sch.data(), sch.size() * 4, cudaMemcpyHostToDevice, stream_));
-            DIO_CK(cudaStreamSynchronize(stream_));  // sch is a host temporary
-        }
         if (!chunks_host_.empty())
             DIO_CK(cudaMemcpyAsync(chunks_, chunks_host_.data(), chunks_host_.size() * sizeof(uint2),
                                    cudaMemcpyHostToDevice, stream_));
-        if (!solve_chunks_host_.empty())
-            DIO_CK(cudaMemcpyAsync(solve_chunks_, solve_chunks_host_.data(),
-                                   solve_chunks_host_.size() * sizeof(uint2), cudaMemcpyHostToDevice, stream_));
+        return pack_layout();
+    }
+    // the layout's solve chunks and the chunk of every scene (when every scene
+    // has one)
+    int pack_layout() {
+        Layout& l = *l_;
+        l.chunk_max = pack_solve_chunks();
+        chunked_scenes_ = !l.chunks.empty() && scene_max_ <= kSolveChunkCap;
+        if (chunked_scenes_) {
+            std::vector<uint32_t> sch(scenes_host_.size(), 0u);
+            for (uint32_t c = 0; c < (uint32_t)l.chunks.size(); ++c)
+                for (uint32_t sc = l.chunks[c].x; sc < l.chunks[c].y; ++sc) sch[sc] = c;
+            DIO_CK(cudaMemcpyAsync(l.scene_chunk, sch.data(), sch.size() * 4, cudaMemcpyHostToDevice, stream_));
+            DIO_CK(cudaStreamSynchronize(stream_));  // sch is a host temporary
+        }
+        if (!l.chunks.empty())
+            DIO_CK(cudaMemcpyAsync(l.dev_chunks, l.chunks.data(), l.chunks.size() * sizeof(uint2),
+                                   cudaMemcpyHostToDevice, stream_));
         return DIO_OK;
     }
 
@@ -1079,9 +1152,13 @@ class Engine final : public EngineBase {
         w_.n_joints = 0;  // the world's joints are uploaded below
         // the scene table in force is the former world's: its bodies' scenes say
         // nothing about these (the list is ordered once the joints are here)
-        solve_chunks_host_.clear();
+        for (Layout& l : layouts_) l.sharers = 0;
+        take(layouts_[0]);
+        l_->sharers = sharers_ = 1;
+        l_->mode = cfg_.solver_mode;
+        l_->block = cfg_.block_size;
+        l_->chunks.clear();
         chunked_scenes_ = chunk_world_ = false;
-        sharers_ = 1;
         jointed_ = 2ull * d->n_constraints >= n;
         DIO_TRY(upload_bodies(d->bodies, n, d->n_hull_vertices));
         if (d->positions_f64 || d->orientations_f64) {
@@ -1157,7 +1234,7 @@ class Engine final : public EngineBase {
     int step_async(const DioAvbdOptions* options, uint32_t steps) override {
         if (!options) return inval("null options");
         if (!world_ready_) return state_err("no world uploaded");
-        DIO_TRY(reshape_solve());
+        DIO_TRY(choose_layout());
         if (cfg_.contact_lag) {
             if (!slots_[1]) DIO_TRY(alloc(&slots_[1], (size_t)cap_.max_pairs * per_cap_));
             if (!lag_primed_) {
@@ -1443,7 +1520,7 @@ class Engine final : public EngineBase {
         k_dyn_flags<P, R><<<grid_for(n, 256), 256, 0, stream_>>>(w_, n, counts2_, dyn_keep_);
         DIO_CK(cudaMemsetAsync(counts2_ + n, 0, 4, stream_));
         DIO_CK(ss_.scan(counts2_, offsets2_, n + 1, false, stream_));
-        k_dyn_fill<<<grid_for(n, 256), 256, 0, stream_>>>(counts2_, offsets2_, n, dyn_list_);
+        k_dyn_fill<<<grid_for(n, 256), 256, 0, stream_>>>(counts2_, offsets2_, n, l_->dyn_list);
         uint32_t nd = 0;
         if (state && n <= kHostCount) {
             for (uint32_t i = 0; i < n; ++i) nd += state[i].inv_mass != 0.0f ? 1u : 0u;
@@ -1453,29 +1530,31 @@ class Engine final : public EngineBase {
         }
         if (w_.n_dyn != nd) drop_graphs();  // launch shapes depend on it
         w_.n_dyn = nd;
-        w_.dyn_list = dyn_list_;
+        for (Layout& l : layouts_) l.ordered = false;
         return order || chunked_scenes_ ? order_dyn_list() : DIO_OK;
     }
     // stable sort of the dynamic-body list by work signature (k_dyn_keys);
     // index order is kept inside a signature
     int order_dyn_list() {
+        Layout& l = *l_;
+        l.ordered = true;
         const uint32_t nd = w_.n_dyn;
-        const uint32_t nc = (uint32_t)solve_chunks_host_.size() << shape_.cl;
-        if (nc) DIO_CK(cudaMemsetAsync(chunk_dyn_, 0, nc * sizeof(uint2), stream_));
+        const uint32_t nc = (uint32_t)l.chunks.size() << l.shape.cl;
+        if (nc) DIO_CK(cudaMemsetAsync(l.dyn_runs, 0, nc * sizeof(uint2), stream_));
         if (!nd) return DIO_OK;
         // in the order of the solve's CTAs when every scene has a solve chunk
         // (a CTA walks its run), else by signature alone
-        const SolveUnits units{chunked_scenes_ ? scene_chunk_ : nullptr, solve_chunks_, scenes_, shape_};
-        k_dyn_keys<P, R><<<grid_for(nd, 256), 256, 0, stream_>>>(w_, dyn_list_, nd, units, counts2_);
+        const SolveUnits units{chunked_scenes_ ? l.scene_chunk : nullptr, l.dev_chunks, scenes_, l.shape};
+        k_dyn_keys<P, R><<<grid_for(nd, 256), 256, 0, stream_>>>(w_, l.dyn_list, nd, units, counts2_);
         const uint32_t end_bit = 7u + (chunked_scenes_ ? bits_for(nc) : 0u);
-        DIO_CK(ss_.sort_pairs(counts2_, offsets2_, dyn_list_, dyn_tmp_, nd, 0u, end_bit, false, stream_));
-        DIO_CK(cudaMemcpyAsync(dyn_list_, dyn_tmp_, (size_t)nd * 4, cudaMemcpyDeviceToDevice, stream_));
+        DIO_CK(ss_.sort_pairs(counts2_, offsets2_, l.dyn_list, dyn_tmp_, nd, 0u, end_bit, false, stream_));
+        DIO_CK(cudaMemcpyAsync(l.dyn_list, dyn_tmp_, (size_t)nd * 4, cudaMemcpyDeviceToDevice, stream_));
         if (chunked_scenes_) {
-            k_chunk_dyn_runs<P, R><<<grid_for(nd, 256), 256, 0, stream_>>>(w_, dyn_list_, nd, units, chunk_dyn_);
+            k_chunk_dyn_runs<P, R><<<grid_for(nd, 256), 256, 0, stream_>>>(w_, l.dyn_list, nd, units, l.dyn_runs);
             if (w_.n_joints)
-                k_list_joints<P, R><<<grid_for(nd, 256), 256, 0, stream_>>>(w_, dyn_list_, nd, list_joints_,
-                                                                            list_joint_self_, list_joint_other_,
-                                                                            list_joint_meta_);
+                k_list_joints<P, R><<<grid_for(nd, 256), 256, 0, stream_>>>(
+                    w_, l.dyn_list, nd, const_cast<uint32_t*>(l.list.joints), const_cast<float4*>(l.list.joint_self),
+                    const_cast<float4*>(l.list.joint_other), const_cast<uint2*>(l.list.joint_meta));
         }
         return DIO_OK;
     }
@@ -1500,7 +1579,7 @@ class Engine final : public EngineBase {
         scene_max_ = n;
         chunk_max_ = pack_chunks(scene_tree_cap<R>(), chunks_host_);
         // these calls solve per phase: no solve chunks, and the list needs no CTA order
-        solve_chunks_host_.clear();
+        l_->chunks.clear();
         chunked_scenes_ = chunk_world_ = false;
         k_single_scene<P, R><<<1, 32, 0, stream_>>>(x, !chunks_host_.empty(), scenes_, chunks_, walls_);
         DIO_CK(cudaGetLastError());
@@ -1526,25 +1605,26 @@ class Engine final : public EngineBase {
     bool use_chunk_solve() const {
         if (!chunk_world_ || cfg_.batched_solver != DIO_SOLVE_AUTO) return false;
         if (sizeof(P) == 4) return true;
-        return solve_estimate_ <= sharers_ * (cfg_.solver_mode == DIO_SOLVER_COLORED ? 500.0 + 2.3e-3 * solve_total_
+        return l_->estimate <= l_->sharers * (cfg_.solver_mode == DIO_SOLVER_COLORED ? 500.0 + 2.3e-3 * solve_total_
                                                                                      : 285.0 + 1.5e-3 * solve_total_);
     }
     bool chunk_solve_possible() const override { return chunk_world_; }
     int solve_chunks(const SolveParams<R>& o) {
-        const uint32_t cap = shape_.slots(solve_chunk_max_);  // shared memory sized to the largest chunk
+        const Layout& l = *l_;
+        const uint32_t cap = l.shape.slots(l.chunk_max);  // shared memory sized to the largest chunk
         cudaEvent_t e0 = span_begin();
-        const int grid = (int)(solve_chunks_host_.size() << shape_.cl);
+        const int grid = (int)(l.chunks.size() << l.shape.cl);
         const bool colored = cfg_.solver_mode == DIO_SOLVER_COLORED;
         auto run = [&](auto* kernel, int threads, size_t smem) {
             // clusters wait for the kernel before: started early they are placed
             // around its last CTAs, two to an SM while others stay free (150
             // coloured scenes 1547 us a pass, 1466 so; 64 CTAs alike; one CTA
             // a chunk is 0.4 % faster started early)
-            return launch_clusters(pdl() && !spread_, spread_ ? 1u << shape_.cl : 0u, kernel, grid, threads, smem, stream_, w_,
-                                   (const uint2*)solve_chunks_, (const uint2*)chunk_dyn_, (const SceneDesc*)scenes_,
-                                   cap, shape_, o);
+            return launch_clusters(pdl() && !l.spread, l.spread ? 1u << l.shape.cl : 0u, kernel, grid, threads, smem, stream_, w_,
+                                   (const uint2*)l.dev_chunks, (const uint2*)l.dyn_runs, (const SceneDesc*)scenes_,
+                                   cap, l.shape, o);
         };
-        if (spread_)
+        if (l.spread)
             DIO_CK(colored ? run(k_solve_chunks_colored<P, R, true, true>, chunk_threads<R, true>(),
                                  chunk_colored_smem_bytes<P, R, true>(cap))
                            : run(k_solve_chunks<P, R, true, true>, chunk_threads<R, true>(), chunk_smem_bytes<P, R, true>(cap)));
@@ -2336,19 +2416,17 @@ class Engine final : public EngineBase {
     }
 
     // ---- CUDA graph of one step, one per row-buffer parity ------------
-    struct GraphSlot {
-        cudaGraph_t graph = nullptr;
-        cudaGraphExec_t exec = nullptr;
-        DioAvbdOptions opt{};
-        std::vector<std::pair<cudaGraphNode_t, cudaGraphNode_t>> span_nodes;
-        std::vector<int> span_kinds;
-    };
-    GraphSlot graphs_[4];  // (row-buffer parity, LBVH rebuild or refit)
+    Layout layouts_[4];
+    Layout* l_ = &layouts_[0];  // the one in force
+    uint64_t layout_clock_ = 0;
     bool rebuild_now_ = true;
     bool lbvh_valid_ = false;
 
     void drop_graphs() {
-        for (auto& g : graphs_) {
+        for (Layout& l : layouts_) drop_graphs(l);
+    }
+    void drop_graphs(Layout& l) {
+        for (auto& g : l.graphs) {
             if (g.exec) cudaGraphExecDestroy(g.exec);
             if (g.graph) cudaGraphDestroy(g.graph);
             g = GraphSlot();
@@ -2364,7 +2442,7 @@ class Engine final : public EngineBase {
         capturing_ = true;
         const uint64_t l0 = launches_;
         int rc = step_body_dev(opt);
-        launches_per_step_ = launches_ - l0;  // counted at replay, not capture
+        const uint64_t launches = launches_ - l0;  // counted at replay, not capture
         launches_ = l0;
         capturing_ = false;
         cudaGraph_t graph = nullptr;
@@ -2401,6 +2479,7 @@ class Engine final : public EngineBase {
         DIO_CK(cudaGraphInstantiate(&g.exec, graph, 0));
         g.graph = graph;  // its node handles address the exec's event nodes
         g.opt = opt;
+        g.launches = launches;
         // the placeholder events now belong to the graph's nodes only
         for (auto& s : cap_spans_) {
             ev_free_.push_back(s.a);
@@ -2412,7 +2491,7 @@ class Engine final : public EngineBase {
 
     int step_graph(const DioAvbdOptions& opt) {
         plan_rebuild();
-        GraphSlot& g = graphs_[cur_ * 2 + (rebuild_now_ ? 1 : 0)];
+        GraphSlot& g = l_->graphs[cur_ * 2 + (rebuild_now_ ? 1 : 0)];
         if (!g.exec || std::memcmp(&g.opt, &opt, sizeof opt) != 0) DIO_TRY(capture(g, opt));
         for (size_t k = 0; k < g.span_nodes.size(); ++k) {
             if (!g.span_nodes[k].first || !g.span_nodes[k].second) continue;
@@ -2422,13 +2501,12 @@ class Engine final : public EngineBase {
             spans_.push_back({e0, e1, g.span_kinds[k]});
         }
         DIO_CK(cudaGraphLaunch(g.exec, stream_));
-        launches_ += launches_per_step_;
+        launches_ += g.launches;
         cur_ = 1 - cur_;
         set_rows(cur_);
         ++steps_;
         return DIO_OK;
     }
-    uint64_t launches_per_step_ = 0;
 
     DioCapacity cap_;
     cudaStream_t stream_;
@@ -2448,7 +2526,6 @@ class Engine final : public EngineBase {
     DioConstraint* joints_ = nullptr;
     uint32_t *joint_off_ = nullptr, *joint_idx_ = nullptr;
     JView* jview_ = nullptr;
-    uint32_t* dyn_list_ = nullptr;
     uint32_t* dyn_tmp_ = nullptr;
     uint32_t* dyn_keep_ = nullptr;  // dynamic flags the list was built from
     uint32_t dyn_list_n_ = 0xFFFFFFFFu;
@@ -2463,21 +2540,9 @@ class Engine final : public EngineBase {
     uint32_t scene_max_ = 0;  // bodies in the largest scene
     uint32_t chunk_max_ = 0;  // bodies in the largest scene chunk
     std::vector<uint2> chunks_host_;
-    std::vector<uint2> solve_chunks_host_;  // chunks of the scene-chunk solve
-    uint2* solve_chunks_ = nullptr;
-    uint2* chunk_dyn_ = nullptr;        // each solve chunk's run of the dynamic-body list
-    uint32_t* scene_chunk_ = nullptr;   // solve chunk of every scene
     bool chunked_scenes_ = false;       // every scene has a solve chunk
-    uint32_t solve_chunk_max_ = 0;      // bodies of the largest solve chunk
-    SolveShape shape_{0, 5};            // how a solve chunk is dealt to its cluster's CTAs
-    bool spread_ = false;               // clusters of small CTAs, or a CTA a chunk
-    uint32_t shape_mode_ = 0, shape_block_ = 0;  // solver_mode, block_size the shape was chosen for
-    double solve_estimate_ = 0.0;       // of the chosen shape, us
     uint32_t solve_total_ = 0;          // bodies of all scenes
-    uint2* list_rows_ = nullptr;        // SolveList arrays
-    uint32_t* list_joints_ = nullptr;
-    float4 *list_joint_self_ = nullptr, *list_joint_other_ = nullptr;
-    uint2* list_joint_meta_ = nullptr;
+    uint2* list_rows_ = nullptr;        // SolveList::rows, written every step
     uint2* chunks_ = nullptr;
     Slot<R>* slots_[2] = {nullptr, nullptr};
     // inside step_body_dev: its scratch zeroing is done by k_roll_counters and
@@ -2508,7 +2573,7 @@ class Engine final : public EngineBase {
     uint64_t steps_ = 0;
     bool world_ready_ = false;
     bool jointed_ = false;  // the uploaded world has a joint for every other body
-    uint32_t sharers_ = 1, shape_sharers_ = 1;  // worlds stepped together, now and when the solve was packed
+    uint32_t sharers_ = 1;  // worlds stepped together from the next step on
     struct Span {
         cudaEvent_t a, b;
         int kind;

@@ -445,7 +445,10 @@ int dio_world_download(DioCtx* ctx, DioGpuBody* bodies, DioBodyState* state);
  * with another world's steps; page-locked host arrays keep the copies
  * asynchronous.  Every context is synchronised before the call returns (device
  * error flags included); the first failure is returned and recorded on the
- * context it came from.  No argument may be NULL; count == 0 is a no-op. */
+ * context it came from.  No argument may be NULL; count == 0 is a no-op.
+ * A world is laid out for its part of the GPU in such a step and for the whole
+ * of it in dio_step / dio_step_async (the same bits either way); the layouts
+ * of the last few world counts are kept with the world. */
 int dio_worlds_step_host(DioCtx* const* ctxs, uint32_t count, DioGpuBody* const* bodies,
                          DioBodyState* const* states, const DioAvbdOptions* options, uint32_t steps);
 /* Extension: replace every body's pose and velocities from `motion` (n
