@@ -805,7 +805,8 @@ class Engine final : public EngineBase {
     struct Layout {
         uint32_t sharers = 0;          // worlds stepped together (0: not in use)
         uint32_t mode = 0, block = 0;  // solver_mode, block_size it was chosen for
-        bool ordered = false;          // dyn_list holds the world's dynamic bodies, in order
+        bool ordered = false;          // dyn_list holds the world's dynamic bodies, in order:
+        bool by_cta = false;           // by the chunk solve's CTAs first, or by signature alone
         uint64_t used = 0;             // when it was last taken
         std::vector<uint2> chunks;     // chunks of the scene-chunk solve
         uint32_t chunk_max = 0;        // bodies of the largest
@@ -857,7 +858,6 @@ class Engine final : public EngineBase {
         Layout* to = nullptr;
         for (Layout& l : layouts_)
             if (current(l) && l.sharers == sharers) to = &l;
-        if (to == l_ && to->ordered) return DIO_OK;
         const bool pack = !to;
         if (pack) {  // in place of one that no longer holds, else of the one not taken for longest
             auto age = [&](const Layout& l) { return current(l) ? l.used : 0u; };
@@ -873,9 +873,9 @@ class Engine final : public EngineBase {
         }
         if (to != l_ && !to->ordered && w_.n_dyn)
             DIO_CK(cudaMemcpyAsync(to->dyn_list, l_->dyn_list, (size_t)w_.n_dyn * 4, cudaMemcpyDeviceToDevice, stream_));
-        take(*to);
+        if (to != l_) take(*to);
         if (pack && chunked_scenes_) DIO_TRY(pack_layout());
-        return to->ordered ? DIO_OK : order_dyn_list();
+        return to->ordered && to->by_cta == use_chunk_solve() ? DIO_OK : order_dyn_list();
     }
     // largest scene; the chunks of the broad phase's shared-memory trees
     // (scene_tree_cap<R> bodies) and of the scene-chunk solve
@@ -1213,11 +1213,11 @@ class Engine final : public EngineBase {
         if (n) k_hull_bounds<P, R><<<grid_for(n, 128), 128, 0, stream_>>>(w_, n, hull_bound_);
         w_.hull_bound = hull_bound_;  // read for hull bodies only
         DIO_CK(cudaMemsetAsync(ctr_, 0, sizeof(Counters), stream_));
-        DIO_TRY(upload_joints(d->constraints, d->n_constraints, n));
         // the scene-chunk solve needs every scene in a chunk and every joint
         // inside one scene (a chunk's shared memory holds its own bodies only)
         chunk_world_ = n && chunked_scenes_ &&
                        joints_within_scenes(d->constraints, d->n_constraints);
+        DIO_TRY(upload_joints(d->constraints, d->n_constraints, n));
         n_prev_rows_ = 0;
         steps_ = 0;
         lag_primed_ = false;
@@ -1531,25 +1531,27 @@ class Engine final : public EngineBase {
         if (w_.n_dyn != nd) drop_graphs();  // launch shapes depend on it
         w_.n_dyn = nd;
         for (Layout& l : layouts_) l.ordered = false;
-        return order || chunked_scenes_ ? order_dyn_list() : DIO_OK;
+        return order ? order_dyn_list() : DIO_OK;
     }
     // stable sort of the dynamic-body list by work signature (k_dyn_keys);
     // index order is kept inside a signature
     int order_dyn_list() {
         Layout& l = *l_;
         l.ordered = true;
+        l.by_cta = use_chunk_solve();
         const uint32_t nd = w_.n_dyn;
-        const uint32_t nc = (uint32_t)l.chunks.size() << l.shape.cl;
+        const uint32_t nc = l.by_cta ? (uint32_t)l.chunks.size() << l.shape.cl : 0u;
         if (nc) DIO_CK(cudaMemsetAsync(l.dyn_runs, 0, nc * sizeof(uint2), stream_));
         if (!nd) return DIO_OK;
-        // in the order of the solve's CTAs when every scene has a solve chunk
-        // (a CTA walks its run), else by signature alone
-        const SolveUnits units{chunked_scenes_ ? l.scene_chunk : nullptr, l.dev_chunks, scenes_, l.shape};
+        // in the order of the chunk solve's CTAs where it runs (a CTA walks its
+        // run), else by signature alone: the per-phase primal of 60 FP64 scenes
+        // takes 1,916 us a step in the CTAs' order and 1,560 so
+        const SolveUnits units{l.by_cta ? l.scene_chunk : nullptr, l.dev_chunks, scenes_, l.shape};
         k_dyn_keys<P, R><<<grid_for(nd, 256), 256, 0, stream_>>>(w_, l.dyn_list, nd, units, counts2_);
-        const uint32_t end_bit = 7u + (chunked_scenes_ ? bits_for(nc) : 0u);
+        const uint32_t end_bit = 7u + (l.by_cta ? bits_for(nc) : 0u);
         DIO_CK(ss_.sort_pairs(counts2_, offsets2_, l.dyn_list, dyn_tmp_, nd, 0u, end_bit, false, stream_));
         DIO_CK(cudaMemcpyAsync(l.dyn_list, dyn_tmp_, (size_t)nd * 4, cudaMemcpyDeviceToDevice, stream_));
-        if (chunked_scenes_) {
+        if (l.by_cta) {
             k_chunk_dyn_runs<P, R><<<grid_for(nd, 256), 256, 0, stream_>>>(w_, l.dyn_list, nd, units, l.dyn_runs);
             if (w_.n_joints)
                 k_list_joints<P, R><<<grid_for(nd, 256), 256, 0, stream_>>>(

@@ -96,3 +96,20 @@ def test_a_world_stepped_alone_is_laid_out_alone():
     assert ran == [(20, 0), (0, 2)] * 2 + [(20, 0)]
     for x in worlds:
         x.close()
+
+
+@pytest.mark.parametrize("precision", [abi.PREC_F32, abi.PREC_SPLIT, abi.PREC_F64])
+@pytest.mark.parametrize("mode", [0, 1])
+def test_solve_launch_switched_after_the_upload(precision, mode):
+    """The chunk solve's list is ordered by its CTAs, the per-phase solve's by
+    signature alone; a bodies' update between them is ordered for the one in
+    force."""
+    sc = scenes.pack([scenes.pyramid(levels=9, gap=-0.01), scenes.constraints_demo(), scenes.box_demo(),
+                      scenes.pyramid(levels=5, gap=-0.01)])
+    ow = O.World(sc, precision=precision, solver_mode=mode)
+    with _world(sc, precision=precision, solver_mode=mode, block_size=640) as w:
+        for launch in (abi.SOLVE_AUTO, abi.SOLVE_PER_PHASE, abi.SOLVE_AUTO, abi.SOLVE_PER_PHASE):
+            w.configure(batched_solver=launch)
+            w.step(sc.options, 2)
+            ow.step(sc.options, 2)
+            _same((*w.download(), w.contacts()), (*ow.download(), ow.contacts()))
