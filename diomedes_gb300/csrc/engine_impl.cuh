@@ -673,21 +673,26 @@ class Engine final : public EngineBase {
     }
     // Chunks of the scene-chunk solve and how each is dealt to CTAs: the
     // cheapest of the spread shapes (clusters of 1 to 8 CTAs) and the packed
-    // ones (a CTA a chunk, chunks of up to `target` bodies), by estimates
-    // fitted to measured solves (us for 10 iterations of the jointed batches
-    // of scenes.batched, 2 to 1024 scenes): a cluster costs 56 plus 47 per
-    // round of 256 bodies of a CTA and a little per body (coloured 139 more;
-    // split precision 1.35 times that, FP64 three times) whatever the number of scenes, until the clusters exceed what the
-    // GPU holds; a packed CTA 18 plus 0.092 a body (coloured 1.6 times), the
-    // SMs taking the next largest chunk as they fall free; packed only when
-    // there are more chunks than SMs (contact-dense scenes are twice as slow
-    // packed: the 901-body pile 225 against 127) or the schedule is coloured
-    // and the scenes are jointed and small (a barrier per colour costs a cluster
-    // most: passes of 5 and 13 scenes of at most 700 bodies 567 and 545 us
-    // spread, 485 and 498 packed; of 4 and 33 with 2,000 bodies 570 and 599, 627
-    // and 800).  33 scenes: 104 spread over 8 CTAs, 148 over 4, 203 packed; 257:
-    // 244, 193, 209; 1024: 850, 585, 413.  Returns the largest chunk's bodies
-    // (0: some scene exceeds the cap).
+    // ones (a CTA a chunk), by estimates fitted to measured solves (us for 10
+    // iterations of the jointed batches of scenes.batched, 2 to 1024 scenes;
+    // FP64: in units of the per-phase estimate of use_chunk_solve).
+    //   Jacobi  a cluster costs 56 plus 47 per round of 256 bodies of a CTA and a
+    // little per body (split precision 1.35 times that, FP64 three times) whatever
+    // the number of scenes, until the clusters exceed what the GPU holds; a
+    // packed CTA 18 plus 0.092 a body, the SMs taking the next largest chunk as
+    // they fall free; packed only when there are more chunks than SMs
+    // (contact-dense scenes are twice as slow packed: the 901-body pile 225
+    // against 127).  33 scenes: 104 spread over 8 CTAs, 148 over 4, 203 packed;
+    // 257: 244, 193, 209; 1024: 850, 585, 413.
+    //   coloured, jointed worlds  a barrier per colour takes most of it: a
+    // cluster 160 plus a little per slot and CTA, a packed CTA 122 plus 0.1 a
+    // body (in FP32 130 against 153 for 100 bodies, 173 and 183 for 408, 197 and 205
+    // for 659; 259 and 198 for 1,609; in split precision 270 and 252, 314 and
+    // 268 for 89 and 367), and chunks as small as the largest scene come first
+    // (five split scenes of 932 bodies in one chunk 316, apart 268).  Other
+    // coloured worlds (contact-dense): as Jacobi, 139 more for a cluster, 1.6 times
+    // packed.
+    // Returns the largest chunk's bodies (0: some scene exceeds the cap).
     uint32_t pack_solve_chunks() {
         uint32_t largest = 0, total = 0;
         for (const SceneDesc& sd : scenes_host_) {
@@ -699,8 +704,18 @@ class Engine final : public EngineBase {
         l.estimate = 0.0;
         const int sms = sms_share();
         if (scenes_host_.empty() || largest == 0 || largest > kSolveChunkCap) return 0;
-        const bool colored = cfg_.solver_mode == DIO_SOLVER_COLORED;
-        const double wide = sizeof(P) == sizeof(R) ? (sizeof(P) == 4 ? 1.0 : 3.0) : 1.35;
+        constexpr bool f32 = sizeof(P) == 4, split = sizeof(P) != sizeof(R);
+        const bool colored = cfg_.solver_mode == DIO_SOLVER_COLORED, sweeps = colored && jointed_;
+        const double wide = f32 ? 1.0 : (split ? 1.35 : 3.0);
+        auto spread_us = [&](uint32_t slots, uint32_t cl) {
+            if (sweeps)
+                return f32 || split ? (160.0 + 0.18 * slots + 5.0 * cl) * (f32 ? 1.0 : 1.5) : 345.0 + 1.7 * slots;
+            return (56.0 + 47.0 * ((slots + 255u) / 256u) + 0.05 * slots + (colored ? 139.0 : 0.0)) * wide;
+        };
+        auto packed_us = [&](uint32_t bodies) {
+            if (sweeps) return f32 || split ? (122.0 + 0.1 * bodies) * (f32 ? 1.0 : 2.1) : 480.0 + 0.55 * bodies;
+            return (18.0 + 0.092 * bodies) * wide * (colored ? 1.6 : 1.0);
+        };
         double best = 1e300;
         std::vector<uint2> chunks;
         auto consider = [&](bool spread, SolveShape sh, double us) {
@@ -710,8 +725,8 @@ class Engine final : public EngineBase {
             l.shape = sh;
             l.chunks = chunks;
         };
-        if (cfg_.block_size == 0 || largest > solve_cta_cap<P, false>()) {
-            const uint32_t most = pack_solve(kSolveChunkCap, chunks);
+        auto spread_to = [&](uint32_t target) {
+            const uint32_t most = pack_solve(target, chunks);
             for (uint32_t cl = 0; cl <= kMaxClusterShift; ++cl) {
                 SolveShape sh{cl, 5};
                 while (sh.blk && (most >> sh.blk) < (1u << cl)) --sh.blk;
@@ -721,27 +736,32 @@ class Engine final : public EngineBase {
                 const uint64_t waves = (chunks.size() + held - 1) / held;
                 const double over = double(chunks.size() << cl) / sms - 1.0;  // CTAs beyond one an SM
                 const double share = 1.0 + 0.25 * std::min(1.0, std::max(0.0, over));
-                const uint32_t rounds = (slots + 255u) / 256u;
-                consider(true, sh,
-                         (56.0 + 47.0 * rounds + 0.05 * slots + (colored ? 139.0 : 0.0)) * wide * share * waves);
+                consider(true, sh, spread_us(slots, cl) * share * waves);
             }
+        };
+        auto packed_to = [&](uint32_t target) {
+            pack_solve(std::min(target, solve_cta_cap<P, false>()), chunks);
+            const double per_sm = double(chunks.size()) / sms;
+            if (per_sm <= 1.0 && !sweeps && !l.chunks.empty()) return;
+            // longest first over the SMs
+            std::vector<double> sm(std::min<size_t>((size_t)sms, chunks.size()), 0.0);
+            auto later = [](double x, double y) { return x > y; };
+            for (const uint2& c : chunks) {
+                std::pop_heap(sm.begin(), sm.end(), later);
+                sm.back() += packed_us(scenes_host_[c.y - 1].body_hi - scenes_host_[c.x].body_lo);
+                std::push_heap(sm.begin(), sm.end(), later);
+            }
+            const double full = per_sm > 1.0 ? 1.35 : (sweeps ? 1.0 + 0.15 * per_sm : 1.0);
+            consider(false, SolveShape{0, 5}, *std::max_element(sm.begin(), sm.end()) * full);
+        };
+        if (cfg_.block_size == 0 || largest > solve_cta_cap<P, false>()) {
+            if (sweeps) spread_to(largest);
+            spread_to(kSolveChunkCap);
         }
-        if (largest <= solve_cta_cap<P, false>())
-            for (uint32_t target : {512u, 768u, 1024u}) {
-                pack_solve(std::min(target, solve_cta_cap<P, false>()), chunks);
-                if (chunks.size() <= (size_t)sms && !(colored && jointed_ && largest <= 768u) && !l.chunks.empty()) continue;
-                // longest first over the SMs
-                std::vector<double> sm(std::min<size_t>((size_t)sms, chunks.size()), 0.0);
-                auto later = [](double x, double y) { return x > y; };
-                for (const uint2& c : chunks) {
-                    const uint32_t bodies = scenes_host_[c.y - 1].body_hi - scenes_host_[c.x].body_lo;
-                    std::pop_heap(sm.begin(), sm.end(), later);
-                    sm.back() += 18.0 + 0.092 * bodies;
-                    std::push_heap(sm.begin(), sm.end(), later);
-                }
-                const double us = *std::max_element(sm.begin(), sm.end()) * (chunks.size() > (size_t)sms ? 1.35 : 1.0);
-                consider(false, SolveShape{0, 5}, us * wide * (colored ? 1.6 : 1.0));
-            }
+        if (largest <= solve_cta_cap<P, false>()) {
+            if (sweeps) packed_to(largest);
+            for (uint32_t target : {512u, 768u, 1024u}) packed_to(target);
+        }
         l.estimate = best;
         solve_total_ = total;
         uint32_t most = 0;

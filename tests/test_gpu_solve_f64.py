@@ -33,8 +33,8 @@ def _same(got, ref):
         assert np.array_equal(np.ascontiguousarray(g).view(np.uint8), np.ascontiguousarray(r).view(np.uint8))
 
 
-@pytest.mark.parametrize("mode", [0, 1])
-@pytest.mark.parametrize("kind,n", [("pyramid", 2), ("pyramid", 9), ("field", 17), ("single", 400), ("batch", 31)])
+@pytest.mark.parametrize("kind,n,mode", [("pyramid", 2, 0), ("pyramid", 9, 0), ("pyramid", 9, 1), ("field", 17, 0),
+                                         ("field", 17, 1), ("single", 400, 0), ("batch", 31, 0)])
 def test_whole_sm_chunks(kind, n, mode):
     sc = _scene(kind, n)
     ow = O.World(sc, precision=abi.PREC_F64, solver_mode=mode, threads=8)
@@ -49,11 +49,13 @@ def test_whole_sm_chunks(kind, n, mode):
 @pytest.mark.parametrize("mode", [0, 1])
 @pytest.mark.parametrize("kind,n", [("pyramid", 3), ("field", 20), ("field", 70), ("single", 1025), ("single", 2047),
                                     ("batch", 31)])
-def test_clusters(kind, n, mode):
+@pytest.mark.parametrize("block", [0, 640])
+def test_worlds_together(kind, n, mode, block):
+    """Clusters, or whole-SM chunks where the scenes fit one (1,024 bodies)."""
     sc = _scene(kind, n)
     ow = O.World(sc, precision=abi.PREC_F64, solver_mode=mode, threads=8)
     ow.step(sc.options, 1)
-    worlds = [_world(sc, solver_mode=mode) for _ in range(3)]
+    worlds = [_world(sc, solver_mode=mode, block_size=block) for _ in range(3)]
     phases = _world(sc, solver_mode=mode, batched_solver=abi.SOLVE_PER_PHASE)
     for k in range(3):
         for group in (worlds, [phases]):
