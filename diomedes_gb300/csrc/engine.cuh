@@ -64,6 +64,7 @@ struct Counters {
     uint32_t dyn_changed;     // a state update turned a body static or dynamic
     uint32_t prev_pairs;      // pairs of the previous step (contact-lag rows)
     uint32_t traverse_pairs;  // pairs appended by the global trees' count pass
+    uint32_t failed_solves;   // warps whose primal held a system outside solve6's one test
 };
 
 // Static part of one contact row (80 B at R = float):

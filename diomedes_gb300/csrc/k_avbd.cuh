@@ -63,7 +63,8 @@ constexpr int kMaskAxisY = (1 << 1) | (1 << 3) | (1 << 5);  // J = (0, s, 0, -s 
 constexpr int kMaskAxisZ = (1 << 2) | (1 << 3) | (1 << 4);  // J = (0, 0, s, s r.y, -s r.x, 0)
 
 // solve6, avbd/src/lib.rs:107-180 (unpivoted LDL^T); solves H x = -g.
-// div(p, a): the quotient of a by pivot p.
+// div(p, v): a column's quotients by pivot p in place; div.each(p, v): one by
+// each pivot.
 template <class R, class Div>
 __device__ __forceinline__ void solve6_with(const Block6<R>& B, R x[6], Div&& div) {
     const R* H = B.h;
@@ -74,76 +75,108 @@ __device__ __forceinline__ void solve6_with(const Block6<R>& B, R x[6], Div&& di
     R a43 = H[tri(3, 2)], a53 = H[tri(4, 2)], a63 = H[tri(5, 2)];
     R a44 = H[tri(3, 3)], a54 = H[tri(4, 3)], a64 = H[tri(5, 3)], a55 = H[tri(4, 4)], a65 = H[tri(5, 4)],
       a66 = H[tri(5, 5)];
-    const auto p1 = div.pivot(a11);
-    R l21 = div(p1, a21), l31 = div(p1, a31), l41 = div(p1, a41), l51 = div(p1, a51), l61 = div(p1, a61);
+    const Pivot<R> p1 = div.pivot(a11);
+    R c1[5] = {a21, a31, a41, a51, a61};
+    div(p1, c1);
+    R l21 = c1[0], l31 = c1[1], l41 = c1[2], l51 = c1[3], l61 = c1[4];
     R d1 = a11;
     R d2 = a22 - l21 * l21 * d1;
-    const auto p2 = div.pivot(d2);
-    R l32 = div(p2, a32 - l21 * l31 * d1);
-    R l42 = div(p2, a42 - l21 * l41 * d1);
-    R l52 = div(p2, a52 - l21 * l51 * d1);
-    R l62 = div(p2, a62 - l21 * l61 * d1);
+    const Pivot<R> p2 = div.pivot(d2);
+    R c2[4] = {a32 - l21 * l31 * d1, a42 - l21 * l41 * d1, a52 - l21 * l51 * d1, a62 - l21 * l61 * d1};
+    div(p2, c2);
+    R l32 = c2[0], l42 = c2[1], l52 = c2[2], l62 = c2[3];
     R d3 = a33 - (l31 * l31 * d1 + l32 * l32 * d2);
-    const auto p3 = div.pivot(d3);
-    R l43 = div(p3, a43 - l31 * l41 * d1 - l32 * l42 * d2);
-    R l53 = div(p3, a53 - l31 * l51 * d1 - l32 * l52 * d2);
-    R l63 = div(p3, a63 - l31 * l61 * d1 - l32 * l62 * d2);
+    const Pivot<R> p3 = div.pivot(d3);
+    R c3[3] = {a43 - l31 * l41 * d1 - l32 * l42 * d2, a53 - l31 * l51 * d1 - l32 * l52 * d2,
+               a63 - l31 * l61 * d1 - l32 * l62 * d2};
+    div(p3, c3);
+    R l43 = c3[0], l53 = c3[1], l63 = c3[2];
     R d4 = a44 - (l41 * l41 * d1 + l42 * l42 * d2 + l43 * l43 * d3);
-    const auto p4 = div.pivot(d4);
-    R l54 = div(p4, a54 - l41 * l51 * d1 - l42 * l52 * d2 - l43 * l53 * d3);
-    R l64 = div(p4, a64 - l41 * l61 * d1 - l42 * l62 * d2 - l43 * l63 * d3);
+    const Pivot<R> p4 = div.pivot(d4);
+    R c4[2] = {a54 - l41 * l51 * d1 - l42 * l52 * d2 - l43 * l53 * d3,
+               a64 - l41 * l61 * d1 - l42 * l62 * d2 - l43 * l63 * d3};
+    div(p4, c4);
+    R l54 = c4[0], l64 = c4[1];
     R d5 = a55 - (l51 * l51 * d1 + l52 * l52 * d2 + l53 * l53 * d3 + l54 * l54 * d4);
-    const auto p5 = div.pivot(d5);
-    R l65 = div(p5, a65 - l51 * l61 * d1 - l52 * l62 * d2 - l53 * l63 * d3 - l54 * l64 * d4);
+    const Pivot<R> p5 = div.pivot(d5);
+    R c5[1] = {a65 - l51 * l61 * d1 - l52 * l62 * d2 - l53 * l63 * d3 - l54 * l64 * d4};
+    div(p5, c5);
+    R l65 = c5[0];
     R d6 = a66 - (l61 * l61 * d1 + l62 * l62 * d2 + l63 * l63 * d3 + l64 * l64 * d4 + l65 * l65 * d5);
-    const auto p6 = div.pivot(d6);
+    const Pivot<R> p[6] = {p1, p2, p3, p4, p5, div.pivot(d6)};
     R b0 = -B.g[0], b1 = -B.g[1], b2 = -B.g[2], b3 = -B.g[3], b4 = -B.g[4], b5 = -B.g[5];
-    R y1 = b0;
-    R y2 = b1 - l21 * y1;
-    R y3 = b2 - l31 * y1 - l32 * y2;
-    R y4 = b3 - l41 * y1 - l42 * y2 - l43 * y3;
-    R y5 = b4 - l51 * y1 - l52 * y2 - l53 * y3 - l54 * y4;
-    R y6 = b5 - l61 * y1 - l62 * y2 - l63 * y3 - l64 * y4 - l65 * y5;
-    R z1 = div(p1, y1), z2 = div(p2, y2), z3 = div(p3, y3), z4 = div(p4, y4), z5 = div(p5, y5), z6 = div(p6, y6);
-    x[5] = z6;
-    x[4] = z5 - l65 * x[5];
-    x[3] = z4 - l54 * x[4] - l64 * x[5];
-    x[2] = z3 - l43 * x[3] - l53 * x[4] - l63 * x[5];
-    x[1] = z2 - l32 * x[2] - l42 * x[3] - l52 * x[4] - l62 * x[5];
-    x[0] = z1 - l21 * x[1] - l31 * x[2] - l41 * x[3] - l51 * x[4] - l61 * x[5];
+    R z[6];
+    z[0] = b0;
+    z[1] = b1 - l21 * z[0];
+    z[2] = b2 - l31 * z[0] - l32 * z[1];
+    z[3] = b3 - l41 * z[0] - l42 * z[1] - l43 * z[2];
+    z[4] = b4 - l51 * z[0] - l52 * z[1] - l53 * z[2] - l54 * z[3];
+    z[5] = b5 - l61 * z[0] - l62 * z[1] - l63 * z[2] - l64 * z[3] - l65 * z[4];
+    div.each(p, z);
+    x[5] = z[5];
+    x[4] = z[4] - l65 * x[5];
+    x[3] = z[3] - l54 * x[4] - l64 * x[5];
+    x[2] = z[2] - l43 * x[3] - l53 * x[4] - l63 * x[5];
+    x[1] = z[1] - l32 * x[2] - l42 * x[3] - l52 * x[4] - l62 * x[5];
+    x[0] = z[0] - l21 * x[1] - l31 * x[2] - l41 * x[3] - l51 * x[4] - l61 * x[5];
 }
-template <class R>
-struct PlainDiv {
-    __device__ __forceinline__ R pivot(R b) const { return b; }
-    __device__ __forceinline__ R operator()(R b, R a) const { return a / b; }
-};
 
 // Each quotient by a pivot is the IEEE quotient: one reciprocal per pivot and
 // a correction step per quotient (div_rn.cuh), with one range test for the
-// whole system; a system outside the range is solved again with IEEE
-// divisions (in line: through a call, the system goes to local memory on
-// every solve, and 1024 scenes take 2816 us a pass instead of 2610; with a
-// test per pivot's column 2658).
+// whole system (OneTest) or one per column, whose quotients are formed again
+// when it fails (ColumnTests).
 template <class R>
-__device__ __forceinline__ void solve6(const Block6<R>& B, R x[6]) {
-    if constexpr (sizeof(R) == 4) {
-        struct Collect {
-            Quotients<R>& q;
-            bool& ok;
-            __device__ __forceinline__ Pivot<R> pivot(R b) const {
-                const Pivot<R> p(b);
-                ok = ok && p.ok();
-                return p;
-            }
-            __device__ __forceinline__ R operator()(const Pivot<R>& p, R a) const { return q.div(p, a); }
-        };
-        Quotients<R> q;
-        bool ok = true;
-        solve6_with(B, x, Collect{q, ok});
-        if (!(ok && q.in_range())) solve6_with(B, x, PlainDiv<R>());
-    } else {
-        solve6_with(B, x, PlainDiv<R>());
+struct OneTest {
+    Quotients<R> q;
+    bool ok = true;
+    __device__ __forceinline__ Pivot<R> pivot(R b) {
+        const Pivot<R> p(b);
+        ok = ok && p.ok();
+        return p;
     }
+    template <int N>
+    __device__ __forceinline__ void operator()(const Pivot<R>& p, R (&v)[N]) {
+#pragma unroll
+        for (int k = 0; k < N; ++k) v[k] = q.div(p, v[k]);
+    }
+    __device__ __forceinline__ void each(const Pivot<R> (&p)[6], R (&v)[6]) {
+#pragma unroll
+        for (int k = 0; k < 6; ++k) v[k] = q.div(p[k], v[k]);
+    }
+};
+template <class R>
+struct ColumnTests {
+    __device__ __forceinline__ Pivot<R> pivot(R b) const { return Pivot<R>(b); }
+    template <int N>
+    __device__ __forceinline__ void operator()(const Pivot<R>& p, R (&v)[N]) const {
+        divide_all(p, v);
+    }
+    __device__ __forceinline__ void each(const Pivot<R> (&p)[6], R (&v)[6]) const { divide_each(p, v); }
+};
+// hint: where a caller remembers that its systems have failed the one test.
+// Such systems come again in every iteration, and a warp that solves one twice
+// holds up its colour or phase (us a step or launch, all quotients divided
+// again, then as it is: 13 coloured scenes without such a body 178, with one 236
+// and 199; 33 scenes 113 and 98; the 400 x 500 split wall, where four systems in
+// five fail, 106 and 101).  The second solve is in line: through a call, the
+// system goes to local memory on every solve, and 1024 scenes take 2816 us a
+// pass instead of 2610; with a test per column alone 2658.
+struct NoHint {
+    __device__ __forceinline__ bool careful() const { return false; }
+    __device__ __forceinline__ void be_careful() const {}
+};
+template <class R, class Hint = NoHint>
+__device__ __forceinline__ void solve6(const Block6<R>& B, R x[6], const Hint& hint = Hint()) {
+    bool done = false;
+    if constexpr (sizeof(R) == 4) {
+        if (!hint.careful()) {
+            OneTest<R> div;
+            solve6_with(B, x, div);
+            done = div.ok && div.q.in_range();
+            if (!done) hint.be_careful();
+        }
+    }
+    if (!done) solve6_with(B, x, ColumnTests<R>());
 }
 
 // avbd_init, avbd/src/lib.rs:202-254, for one body: the inertial target and
@@ -264,7 +297,7 @@ __global__ void __launch_bounds__(256) k_init(DevWorld<P, R> w, uint32_t lo, uin
 
 // Where the primal and the dual find poses.  pos: a position; rot: a body's
 // own rotation; rot_r: a rotation rounded to R; moved: what rows take; store:
-// a body's new pose.
+// a body's new pose; careful, be_careful: solve6's hint.
 // PoseFetch: pose buffer rd in global memory, displacements formed here.
 template <class P, class R>
 struct PoseFetch {
@@ -285,6 +318,11 @@ template <class P, class R>
 struct GlobalFetch {
     const DevWorld<P, R>& w;
     int rd, wr;
+    // warps that held a failing system this step, once they are an eighth of all
+    __device__ __forceinline__ bool careful() const { return w.ctr->failed_solves > w.n_dyn / 256u; }
+    __device__ __forceinline__ void be_careful() const {
+        if ((threadIdx.x & 31u) == (uint32_t)__ffs(__activemask()) - 1u) atomicAdd(&w.ctr->failed_solves, 1u);
+    }
     __device__ __forceinline__ A4<P> pos(uint32_t j) const { return w.pos[rd][j]; }
     __device__ __forceinline__ A4<P> rot(uint32_t j) const { return w.rot[rd][j]; }
     __device__ __forceinline__ Q4<R> rot_r(uint32_t j) const { return quat(w.rot_r[rd][j]); }
@@ -308,6 +346,8 @@ struct TileFetch {
     const A4<P>* sq;
     const A4<P>* si;
     const A4<P>* sr;
+    __device__ __forceinline__ bool careful() const { return g.careful(); }
+    __device__ __forceinline__ void be_careful() const { g.be_careful(); }
     __device__ __forceinline__ bool in(uint32_t j) const { return j - lo < (uint32_t)T; }
     __device__ __forceinline__ A4<P> pos(uint32_t j) const { return in(j) ? sp[j - lo] : g.pos(j); }
     __device__ __forceinline__ A4<P> rot(uint32_t j) const { return in(j) ? sq[j - lo] : g.rot(j); }
@@ -656,7 +696,7 @@ __device__ __forceinline__ void primal_finish(const S& bodies, uint32_t t, uint3
         primal_jview_f<P, R>(jv, fetch, sp, sqr, B);
     }
     R dx[6];
-    solve6(B, dx);
+    solve6(B, dx, fetch);
     const A4<P> np = pack(add(sp, widen3<P>(V3<R>{dx[0], dx[1], dx[2]})));
     if constexpr (std::is_same<P, R>::value)
         fetch.store(i, np, packq(quat_step(sq, V3<P>{dx[3], dx[4], dx[5]})));

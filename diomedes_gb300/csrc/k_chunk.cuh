@@ -193,6 +193,9 @@ struct ChunkFetch {
     uint32_t rd, wr;  // snapshot and output buffer, as offsets
     uint32_t lo, rank;
     SolveShape shape;
+    volatile uint32_t* failed = nullptr;  // set: a system of this CTA failed solve6's one test
+    __device__ __forceinline__ bool careful() const { return *failed; }
+    __device__ __forceinline__ void be_careful() const { *failed = 1u; }
     template <class T>
     __device__ __forceinline__ T get(const T* a, uint32_t j) const {
         const uint32_t d = j - lo;
@@ -464,7 +467,7 @@ __global__ void __launch_bounds__(chunk_threads<R, kSpread>(), sizeof(R) == 4 &&
                    SolveShape shape, SolveParams<R> o) {
     extern __shared__ __align__(16) unsigned char chunk_smem[];
     __shared__ uint32_t s_rows[4];
-    __shared__ uint32_t s_cursor[2];
+    __shared__ uint32_t s_cursor[2], s_failed;
     __shared__ uint32_t s_warp[chunk_threads<R, kSpread>() / 32];
     pdl_enter();
     // layout: poses, staging, the groups' first bodies
@@ -476,6 +479,7 @@ __global__ void __launch_bounds__(chunk_threads<R, kSpread>(), sizeof(R) == 4 &&
     ChunkCta c = chunk_cta(chunks, dyn_runs, scenes, shape);
     chunk_row_bounds(w.ab, w.ctr, c, s_rows);
     if (tid < 2) s_cursor[tid] = 0u;
+    if (tid == 2) s_failed = 0u;
     using Fetch = ChunkFetch<P, R, kCluster>;
     chunk_init(w, c, shape, o, Fetch{w, poses, 0u, cap, c.lo, c.rank, shape});
     chunk_sync<kCluster>();
@@ -490,8 +494,8 @@ __global__ void __launch_bounds__(chunk_threads<R, kSpread>(), sizeof(R) == 4 &&
     for (uint32_t k = 0; k < o.iterations; ++k) {
         const uint32_t rd = (k & 1u) * cap, wr = cap - rd;
         if (tid == 0) s_cursor[(k + 1u) & 1u] = 0u;  // last used before the previous barrier
-        chunk_primal<kSpread>(w, ListBodies<P, R>{w}, groups, range, o, Fetch{w, poses, rd, wr, c.lo, c.rank, shape},
-                              stage, &s_cursor[k & 1u]);
+        chunk_primal<kSpread>(w, ListBodies<P, R>{w}, groups, range, o,
+                              Fetch{w, poses, rd, wr, c.lo, c.rank, shape, &s_failed}, stage, &s_cursor[k & 1u]);
         chunk_sync<kCluster>();
         if (!c.rows) continue;  // the same for all CTAs of the chunk
         const Fetch fd{w, poses, wr, wr, c.lo, c.rank, shape};
@@ -542,7 +546,7 @@ __global__ void __launch_bounds__(chunk_threads<R, kSpread>(), sizeof(R) == 4 &&
                            uint32_t cap, SolveShape shape, SolveParams<R> o) {
     extern __shared__ __align__(16) unsigned char chunk_smem[];
     __shared__ uint32_t s_rows[4];
-    __shared__ uint32_t s_cursor[2];
+    __shared__ uint32_t s_cursor[2], s_failed;
     __shared__ uint32_t s_colored, s_ncolors, s_ndyn;
     pdl_enter();
     const uint32_t tid = threadIdx.x, nt = blockDim.x;
@@ -562,6 +566,7 @@ __global__ void __launch_bounds__(chunk_threads<R, kSpread>(), sizeof(R) == 4 &&
         s_colored = 0;
         s_ncolors = 0;
         s_ndyn = ndyn;
+        s_failed = 0;
     }
     if (tid < 2) s_cursor[tid] = 0u;
     for (uint32_t q = tid; q <= kMaxColors; q += nt) {
@@ -569,7 +574,7 @@ __global__ void __launch_bounds__(chunk_threads<R, kSpread>(), sizeof(R) == 4 &&
         s_next[q] = 0;
     }
     // init (the in-place schedule reads and writes one buffer) and colours reset
-    const ChunkFetch<P, R, kCluster> f{w, poses, 0u, 0u, lo, c.rank, shape};
+    const ChunkFetch<P, R, kCluster> f{w, poses, 0u, 0u, lo, c.rank, shape, &s_failed};
     chunk_init(w, c, shape, o, f);
     for (uint32_t s = tid; s < shape.slots(c.nb); s += nt) s_color[s] = kNoColor;
     chunk_sync<kCluster>();

@@ -569,6 +569,7 @@ static __global__ void k_roll_counters(Counters* c, uint32_t* zero0, uint32_t* z
     c->epa_next = 0;
     c->colors = 0;
     c->traverse_pairs = 0;
+    c->failed_solves = 0;
 }
 
 // CSR of the dynamic bodies only (the primal never visits a static body):
