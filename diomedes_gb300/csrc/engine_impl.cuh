@@ -1621,16 +1621,17 @@ class Engine final : public EngineBase {
         }
         return true;
     }
-    // the whole solve of a world step as one launch (k_solve_chunks)
-    // unless, with FP64 poses, the per-phase launches are the faster: 285 us
+    // the whole solve of a world step as one launch (k_solve_chunks) unless,
+    // with FP64 poses, the per-phase launches are estimated the faster: 285 us
     // plus 1.5 per 1,000 bodies (coloured 500 plus 2.3), measured as above
-    bool use_chunk_solve() const {
-        if (!chunk_world_ || cfg_.batched_solver != DIO_SOLVE_AUTO) return false;
+    bool use_chunk_solve() const { return cfg_.batched_solver == DIO_SOLVE_AUTO && auto_chunk_solve(); }
+    bool auto_chunk_solve() const {
+        if (!chunk_world_) return false;
         if (sizeof(P) == 4) return true;
         return l_->estimate <= l_->sharers * (cfg_.solver_mode == DIO_SOLVER_COLORED ? 500.0 + 2.3e-3 * solve_total_
                                                                                      : 285.0 + 1.5e-3 * solve_total_);
     }
-    bool chunk_solve_possible() const override { return chunk_world_; }
+    bool chunk_solve_taken() override { return choose_layout() == DIO_OK && auto_chunk_solve(); }
     int solve_chunks(const SolveParams<R>& o) {
         const Layout& l = *l_;
         const uint32_t cap = l.shape.slots(l.chunk_max);  // shared memory sized to the largest chunk

@@ -113,3 +113,16 @@ def test_solve_launch_switched_after_the_upload(precision, mode):
             w.step(sc.options, 2)
             ow.step(sc.options, 2)
             _same((*w.download(), w.contacts()), (*ow.download(), ow.contacts()))
+
+
+def test_tuner_times_the_primal_shapes_where_no_chunk_solve_runs():
+    """An FP64 batch whose scenes fit the chunk solve but go per phase either
+    way: the tuner goes on to the primal shapes."""
+    sc = scenes.batched(n_scenes=12, lo=600, hi=1600, seed=5)
+    with _world(sc, precision=abi.PREC_F64, profile=1) as w:
+        w.step(sc.options, 1)
+        assert w.stats()["chunk_launches"] == 0
+        w.configure(profile=0)
+        before = w.download_f64()
+        assert w.autotune(sc.options, trial_steps=1)["batched_solver"] == abi.SOLVE_PER_PHASE
+        _same(w.download_f64(), before)
