@@ -143,6 +143,21 @@ __global__ void k_unpack_contacts(RowStatics<R> rs, RowDuals<P, R> rd, uint2* ab
     }
 }
 
+// rows [r0, r0 + n) of a buffer as records, or from them
+template <class P, class R>
+__global__ void k_row_records(RowStatics<R> rs, RowDuals<P, R> rd, uint32_t r0, uint32_t n, RowStatic<R>* s,
+                              RowDual<P, R>* d, bool take) {
+    for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < n; k += gridDim.x * blockDim.x) {
+        if (take) {
+            rs.put(r0 + k, s[k]);
+            rd.put(r0 + k, d[k]);
+        } else {
+            s[k] = rs[r0 + k];
+            d[k] = rd[r0 + k];
+        }
+    }
+}
+
 template <class P, class R>
 __global__ void k_pack_contacts(RowStatics<R> rs, RowDuals<P, R> rd, const uint2* ab, DioContact* out,
                                 const uint32_t* m_dev) {
@@ -2077,21 +2092,32 @@ class Engine final : public EngineBase {
         }
         return o;
     }
-    // the image keeps rows as records (RowStatic, RowDual), the device field
-    // by field: strided copies between the two
+    // the image keeps rows as records (RowStatic, RowDual), the device field by
+    // field: records are formed or taken apart in the staging buffer, as many at
+    // a time as it holds, and copied in one piece (strided copies of a field each:
+    // a resume of 126,000 rows 1.5 ms, so 0.9)
     int copy_rows(char* statics, char* duals, int buf, uint32_t rows, bool to_device) {
-        auto field = [&](char* host, size_t pitch, void* dev, size_t bytes) {
-            return to_device ? cudaMemcpy2DAsync(dev, bytes, host, pitch, bytes, rows, cudaMemcpyHostToDevice, stream_)
-                             : cudaMemcpy2DAsync(host, pitch, dev, bytes, bytes, rows, cudaMemcpyDeviceToHost, stream_);
-        };
-        for (size_t f = 0; f < 5; ++f)
-            DIO_CK(field(statics + f * sizeof(A4<R>), sizeof(RowStatic<R>), rs_[buf].v + f * rs_[buf].stride,
-                         sizeof(A4<R>)));
-        DIO_CK(field(duals + offsetof(DualRecord, penalty), sizeof(DualRecord), rd_[buf].penalty, sizeof(A4<R>)));
-        DIO_CK(field(duals + offsetof(DualRecord, lambda), sizeof(DualRecord), rd_[buf].lambda, sizeof(A4<P>)));
+        const uint32_t most = (uint32_t)std::min<size_t>(
+            rows, (stage_bytes_ - 256) / (sizeof(RowStatic<R>) + sizeof(RowDual<P, R>)));
+        auto* ds = reinterpret_cast<RowStatic<R>*>(dstage_);
+        auto* dd = reinterpret_cast<RowDual<P, R>*>(static_cast<char*>(dstage_) +
+                                                    align256((size_t)most * sizeof(RowStatic<R>)));
+        for (uint32_t r = 0; r < rows; r += most) {
+            const uint32_t k = std::min(most, rows - r);
+            char *hs = statics + (size_t)r * sizeof(RowStatic<R>), *hd = duals + (size_t)r * sizeof(RowDual<P, R>);
+            const size_t bs = (size_t)k * sizeof(RowStatic<R>), bd = (size_t)k * sizeof(RowDual<P, R>);
+            if (to_device) {
+                DIO_CK(cudaMemcpyAsync(ds, hs, bs, cudaMemcpyHostToDevice, stream_));
+                DIO_CK(cudaMemcpyAsync(dd, hd, bd, cudaMemcpyHostToDevice, stream_));
+            }
+            k_row_records<P, R><<<grid_for(k, 256), 256, 0, stream_>>>(rs_[buf], rd_[buf], r, k, ds, dd, to_device);
+            if (!to_device) {
+                DIO_CK(cudaMemcpyAsync(hs, ds, bs, cudaMemcpyDeviceToHost, stream_));
+                DIO_CK(cudaMemcpyAsync(hd, dd, bd, cudaMemcpyDeviceToHost, stream_));
+            }
+        }
         return DIO_OK;
     }
-    using DualRecord = RowDual<P, R>;
     static constexpr char kCkptMagic[8] = {'D', 'I', 'O', 'C', 'K', 'P', 'T', '1'};
 
    public:
