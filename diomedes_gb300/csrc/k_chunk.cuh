@@ -193,9 +193,11 @@ struct ChunkFetch {
     uint32_t rd, wr;  // snapshot and output buffer, as offsets
     uint32_t lo, rank;
     SolveShape shape;
-    volatile uint32_t* failed = nullptr;  // set: a system of this CTA failed solve6's one test
-    __device__ __forceinline__ bool careful() const { return *failed; }
-    __device__ __forceinline__ void be_careful() const { *failed = 1u; }
+    // a bit per group of bodies: one of its systems has failed solve6's one test
+    uint32_t* failed = nullptr;
+    uint32_t group = 0;
+    __device__ __forceinline__ bool careful() const { return (failed[group >> 5] >> (group & 31u)) & 1u; }
+    __device__ __forceinline__ void be_careful() const { atomicOr(&failed[group >> 5], 1u << (group & 31u)); }
     template <class T>
     __device__ __forceinline__ T get(const T* a, uint32_t j) const {
         const uint32_t d = j - lo;
@@ -418,10 +420,11 @@ __device__ __forceinline__ uint32_t chunk_groups(const DevWorld<P, R>& w, const 
 // The primal of `groups` groups by the CTA's warps, taken from the end
 // through a shared cursor: the end of a CTA's run holds the bodies without
 // joints, whose contact rows make them the longest.  range(k, t, n): group
-// k's first position and bodies.
+// k's first position, from t0 on, and bodies.
 template <bool kSpread, class P, class R, class F, class S, class Range>
-__device__ __forceinline__ void chunk_primal(const DevWorld<P, R>& w, const S& bodies, uint32_t groups, Range&& range,
-                                             const SolveParams<R>& o, const F& fetch, R* stage, uint32_t* cursor) {
+__device__ __forceinline__ void chunk_primal(const DevWorld<P, R>& w, const S& bodies, uint32_t groups, uint32_t t0,
+                                             Range&& range, const SolveParams<R>& o, F fetch, R* stage,
+                                             uint32_t* cursor) {
     const uint32_t lane = threadIdx.x & 31u;
     for (;;) {
         uint32_t k = 0;
@@ -430,6 +433,7 @@ __device__ __forceinline__ void chunk_primal(const DevWorld<P, R>& w, const S& b
         if (k >= groups) break;
         uint32_t t, n;
         range(groups - 1u - k, t, n);
+        fetch.group = t - t0;
         primal_group<kSpread>(w, bodies, t, n, o, fetch, stage, lane);
     }
 }
@@ -467,7 +471,7 @@ __global__ void __launch_bounds__(chunk_threads<R, kSpread>(), sizeof(R) == 4 &&
                    SolveShape shape, SolveParams<R> o) {
     extern __shared__ __align__(16) unsigned char chunk_smem[];
     __shared__ uint32_t s_rows[4];
-    __shared__ uint32_t s_cursor[2], s_failed;
+    __shared__ uint32_t s_cursor[2], s_failed[kSolveChunkCap / 32];
     __shared__ uint32_t s_warp[chunk_threads<R, kSpread>() / 32];
     pdl_enter();
     // layout: poses, staging, the groups' first bodies
@@ -479,7 +483,7 @@ __global__ void __launch_bounds__(chunk_threads<R, kSpread>(), sizeof(R) == 4 &&
     ChunkCta c = chunk_cta(chunks, dyn_runs, scenes, shape);
     chunk_row_bounds(w.ab, w.ctr, c, s_rows);
     if (tid < 2) s_cursor[tid] = 0u;
-    if (tid == 2) s_failed = 0u;
+    if (tid < kSolveChunkCap / 32) s_failed[tid] = 0u;
     using Fetch = ChunkFetch<P, R, kCluster>;
     chunk_init(w, c, shape, o, Fetch{w, poses, 0u, cap, c.lo, c.rank, shape});
     chunk_sync<kCluster>();
@@ -494,8 +498,8 @@ __global__ void __launch_bounds__(chunk_threads<R, kSpread>(), sizeof(R) == 4 &&
     for (uint32_t k = 0; k < o.iterations; ++k) {
         const uint32_t rd = (k & 1u) * cap, wr = cap - rd;
         if (tid == 0) s_cursor[(k + 1u) & 1u] = 0u;  // last used before the previous barrier
-        chunk_primal<kSpread>(w, ListBodies<P, R>{w}, groups, range, o,
-                              Fetch{w, poses, rd, wr, c.lo, c.rank, shape, &s_failed}, stage, &s_cursor[k & 1u]);
+        chunk_primal<kSpread>(w, ListBodies<P, R>{w}, groups, c.dyn.x, range, o,
+                              Fetch{w, poses, rd, wr, c.lo, c.rank, shape, s_failed}, stage, &s_cursor[k & 1u]);
         chunk_sync<kCluster>();
         if (!c.rows) continue;  // the same for all CTAs of the chunk
         const Fetch fd{w, poses, wr, wr, c.lo, c.rank, shape};
@@ -546,7 +550,7 @@ __global__ void __launch_bounds__(chunk_threads<R, kSpread>(), sizeof(R) == 4 &&
                            uint32_t cap, SolveShape shape, SolveParams<R> o) {
     extern __shared__ __align__(16) unsigned char chunk_smem[];
     __shared__ uint32_t s_rows[4];
-    __shared__ uint32_t s_cursor[2], s_failed;
+    __shared__ uint32_t s_cursor[2], s_failed[kSolveChunkCap / 32];
     __shared__ uint32_t s_colored, s_ncolors, s_ndyn;
     pdl_enter();
     const uint32_t tid = threadIdx.x, nt = blockDim.x;
@@ -566,15 +570,15 @@ __global__ void __launch_bounds__(chunk_threads<R, kSpread>(), sizeof(R) == 4 &&
         s_colored = 0;
         s_ncolors = 0;
         s_ndyn = ndyn;
-        s_failed = 0;
     }
+    if (tid < kSolveChunkCap / 32) s_failed[tid] = 0u;
     if (tid < 2) s_cursor[tid] = 0u;
     for (uint32_t q = tid; q <= kMaxColors; q += nt) {
         s_cstart[q] = 0;
         s_next[q] = 0;
     }
     // init (the in-place schedule reads and writes one buffer) and colours reset
-    const ChunkFetch<P, R, kCluster> f{w, poses, 0u, 0u, lo, c.rank, shape, &s_failed};
+    const ChunkFetch<P, R, kCluster> f{w, poses, 0u, 0u, lo, c.rank, shape, s_failed};
     chunk_init(w, c, shape, o, f);
     for (uint32_t s = tid; s < shape.slots(c.nb); s += nt) s_color[s] = kNoColor;
     chunk_sync<kCluster>();
@@ -665,7 +669,7 @@ __global__ void __launch_bounds__(chunk_threads<R, kSpread>(), sizeof(R) == 4 &&
                 t = q0 + e * g;
                 n = min(g, qn - e * g);
             };
-            chunk_primal<kSpread>(w, OrderedBodies<P, R>{{w}, s_order}, (qn + g - 1) / g, range, o, f, stage,
+            chunk_primal<kSpread>(w, OrderedBodies<P, R>{{w}, s_order}, (qn + g - 1) / g, 0u, range, o, f, stage,
                                   &s_cursor[turn]);
             chunk_sync<kCluster>();
         }
