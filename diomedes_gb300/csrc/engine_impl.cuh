@@ -138,8 +138,9 @@ __global__ void k_unpack_contacts(RowStatics<R> rs, RowDuals<P, R> rd, uint2* ab
         d.penalty = A4<R>{R(x.penalty[0]), R(x.penalty[1]), R(x.penalty[2]), R(0)};
         d.lambda = A4<P>{P(x.lambda[0]), P(x.lambda[1]), P(x.lambda[2]), P(0)};
         rd.put(r, d);
-        ab[r] = make_uint2(x.a, x.b);
-        if (x.a >= n || (x.b != kContainer && x.b >= n)) atomicOr(err, kErrBadIndex);
+        const bool bad_a = x.a >= n, bad_b = x.b != kContainer && x.b >= n;
+        if (bad_a || bad_b) atomicOr(err, kErrBadIndex);
+        ab[r] = make_uint2(bad_a ? 0u : x.a, bad_b ? kContainer : x.b);  // nothing reads beyond the bodies
     }
 }
 
@@ -195,13 +196,22 @@ __global__ void k_pack_contacts(RowStatics<R> rs, RowDuals<P, R> rd, const uint2
 }
 
 // Given the reference CSR (offsets, indices), derive the other-body array.
-static __global__ void k_csr_other(const uint32_t* off, const uint32_t* idx, const uint2* ab, uint32_t* oth, uint32_t n,
-                            uint32_t m, uint32_t* err) {
+// The other body of each of a caller's incidences.  What lies out of range -- a
+// list beyond the ninc incidences, a row beyond the m -- is reported and brought
+// into range, so that the solve, whose result is refused, reads no further than
+// the buffers go.  row_off: off so.
+static __global__ void k_csr_other(const uint32_t* off, uint32_t* row_off, uint32_t* idx, const uint2* ab, uint32_t* oth,
+                            uint32_t n, uint32_t m, uint32_t ninc, uint32_t* err) {
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        for (uint32_t j = off[i]; j < off[i + 1]; ++j) {
+        const uint32_t j0 = off[i], j1 = off[i + 1];
+        if (j0 < j1 && j1 > ninc) atomicOr(err, kErrBadIndex);
+        row_off[i] = min(j0, ninc);
+        if (i + 1u == n) row_off[n] = min(j1, ninc);
+        for (uint32_t j = j0; j < min(j1, ninc); ++j) {
             uint32_t r = idx[j];
             if (r >= m) {
                 atomicOr(err, kErrBadIndex);
+                idx[j] = 0u;
                 oth[j] = kContainer;
                 continue;
             }
@@ -1129,10 +1139,10 @@ class Engine final : public EngineBase {
             k_unpack_contacts<P, R><<<grid_for(m, 256), 256, 0, stream_>>>(w_.rs, w_.rd, w_.ab, dc, m, n,
                                                                            &ctr_->error_flags);
         }
-        DIO_CK(cudaMemcpyAsync(w_.row_off, offsets, ((size_t)n + 1) * 4, cudaMemcpyHostToDevice, stream_));
+        DIO_CK(cudaMemcpyAsync(offsets2_, offsets, ((size_t)n + 1) * 4, cudaMemcpyHostToDevice, stream_));
         if (ninc) DIO_CK(cudaMemcpyAsync(w_.row_idx, indices, (size_t)ninc * 4, cudaMemcpyHostToDevice, stream_));
-        k_csr_other<<<grid_for(n, 128), 128, 0, stream_>>>(w_.row_off, w_.row_idx, w_.ab, w_.row_oth, n, m,
-                                                          &ctr_->error_flags);
+        k_csr_other<<<grid_for(n, 128), 128, 0, stream_>>>(offsets2_, w_.row_off, w_.row_idx, w_.ab, w_.row_oth, n, m,
+                                                          ninc, &ctr_->error_flags);
         DIO_TRY(upload_joints(constraints, nj, n));
         k_set_u32<<<1, 1, 0, stream_>>>(&ctr_->rows, m);
         SolveParams<R> o = solve_params(options->dt, options->gravity, options->alpha, options->beta_lin,
@@ -2095,7 +2105,7 @@ class Engine final : public EngineBase {
     // the image keeps rows as records (RowStatic, RowDual), the device field by
     // field: records are formed or taken apart in the staging buffer, as many at
     // a time as it holds, and copied in one piece (strided copies of a field each:
-    // a resume of 126,000 rows 1.5 ms, so 0.9)
+    // a resume of 160,000 rows 1.55 ms, so 0.99)
     int copy_rows(char* statics, char* duals, int buf, uint32_t rows, bool to_device) {
         const uint32_t most = (uint32_t)std::min<size_t>(
             rows, (stage_bytes_ - 256) / (sizeof(RowStatic<R>) + sizeof(RowDual<P, R>)));
