@@ -795,9 +795,9 @@ class Engine final : public EngineBase {
         return most;
     }
     // The SMs that this world counts on: worlds stepped together on their
-    // streams take a part each.  Eight 128-scene worlds, frames with motion
-    // records: 6.7e8 body-steps/s so, 5.6e8 with the tree count laid out for a
-    // whole GPU by each, 4.4e8 with the solve too.
+    // streams take a part each.  The benchmark's eight 128-scene worlds, frames with
+    // motion records after its 310 steps: 6.7e8 body-steps/s so, 5.6e8 with the tree
+    // count laid out for a whole GPU by each, 4.4e8 with the solve too.
     int sms_share() const { return std::max(1, sms_ / (int)l_->sharers); }
     // counted in powers of two, so that a group that shrinks or grows by a few
     // worlds keeps its layout

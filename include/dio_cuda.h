@@ -244,7 +244,9 @@ typedef struct DioConfig {
                                    whole scenes with the poses in shared
                                    memory, when every scene fits a chunk
                                    (2048 bodies) and no joint crosses
-                                   scenes; DIO_SOLVE_PER_PHASE (1) always
+                                   scenes -- with FP64 poses (split, FP64)
+                                   where that is estimated the faster;
+                                   DIO_SOLVE_PER_PHASE (1) always
                                    launches init / primal / dual / recover
                                    kernels.  Both give identical results. */
     uint32_t profile;           /* time primal / dual launches with events */
