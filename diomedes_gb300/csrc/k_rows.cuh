@@ -602,6 +602,8 @@ __global__ void k_csr_scatter_dyn(DevWorld<P, R> w, uint32_t* remaining, uint32_
 // segments by a CTA each: 15 us cold a step for 8,192 stacked cubes, 13.5 for a
 // 55-cube pyramid of 8-contact pairs; now 6 and 5.)  Counting needs no buffer,
 // so a segment may have any length: every entry that the solve walks is written.
+// (A plate of 3,455 and of 9,705 rows: the whole rows phase 106 and 290 us a
+// step, beside a solve of 2,200 and 6,600 for that body's sums.)
 template <class P, class R>
 __global__ void k_csr_finish_dyn(DevWorld<P, R> w, const uint32_t* loose) {
     pdl_enter();
